@@ -131,7 +131,7 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
 
   if (warp == 0) {
     // ================================================================ TMA producer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       // launched with programmatic serialization behind the split pass: everything up to here
       // ran while that pass was still draining; the panels are complete after this
       ptx::griddep_wait();
@@ -162,7 +162,7 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
     }
   } else if (warp == 1) {
     // ================================================================ MMA issuer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       const uint32_t d0 = tmem_base;
       const uint32_t d1 = tmem_base + D1_COL;
       bool ok = true;

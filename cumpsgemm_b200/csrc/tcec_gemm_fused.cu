@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) tcec_gemm_fused_kernel(const F
   if (warp >= MMA_WARP) {
     // ================================================================ MMA issuer
     ptx::setmaxnreg_dec<REGS_MMA>();
-    if (warp == MMA_WARP && lane == 0) {
+    if (warp == MMA_WARP && ptx::elect_one()) {
       bool ok = true;
       const uint32_t chunk = p.drain_chunk;
       const uint32_t first = p.first_chunk;
@@ -639,10 +639,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) tcec_gemm_fused_kernel(const F
           ptx::tc_fence_after();
           const uint64_t a_hi = desc0 + s * kStageDesc;
           const uint64_t a_lo = a_hi + kALo, b_hi = a_hi + kBHi;
-          // Issuing one tcgen05.mma costs the issuing thread about 120 cycles whatever its
-          // size, which is more than a 128 x 128 x 16 product takes to execute.  The B_hi and
-          // B_lo tiles of a stage are adjacent in shared memory, so A_hi x [B_hi; B_lo] is ONE
-          // instruction of twice the width that yields hi*hi (columns 0..BN) and hi*lo
+          // Every tcgen05.mma reads its A tile from shared memory anew, and a 128 x 128 x 16
+          // product is as long as that read.  The B_hi and B_lo tiles of a stage are adjacent in
+          // shared memory, so A_hi x [B_hi; B_lo] is ONE instruction of twice the width that yields hi*hi (columns 0..BN) and hi*lo
           // (columns BN..2BN); lo*hi is added onto the second half.  Eight instructions per
           // stage instead of twelve, and all three products of a chunk leave TMEM together.
 #pragma unroll

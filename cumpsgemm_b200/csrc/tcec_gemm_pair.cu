@@ -194,7 +194,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
 
   if (warp == 0) {
     // ================================================================ TMA producer (both CTAs)
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       uint32_t it = 0; // stage uses since kernel start, across tiles
       bool ok = true;
       bool pace = leader && p.wave_counter != nullptr && work_items > num_clusters;
@@ -248,7 +248,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
     }
   } else if (warp == 1) {
     // ================================================================ MMA issuer (leader only)
-    if (leader && lane == 0) {
+    if (leader && ptx::elect_one()) {
       const uint32_t d0 = tmem_base;
       const uint32_t d1 = tmem_base + D1_COL;
       constexpr uint16_t BOTH = 0x3;
