@@ -19,6 +19,7 @@
 // While the tensor core runs the two correction products of a stage the
 // epilogue warps drain D0 of the same stage, so D0 needs no double buffering
 // and the two accumulators fill the 512 TMEM columns at BN = 256.
+#include "epilogue.cuh"
 #include "gemm_common.cuh"
 #include "ptx.cuh"
 
@@ -246,17 +247,11 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
       ok = ptx::mbar_wait(ptx::smem_u32(d1_full), 0u, abort_flag, p.status, ptx::kErrWaitD1Full);
       if (ok) {
         ptx::tc_fence_after();
-        const float lsi = p.lo_scale_inv;
-#pragma unroll
-        for (int pc = 0; pc < CPT / 32; ++pc) {
-          uint32_t v[32];
-          ptx::tmem_ld_32x32b_x32(tmem_base + D1_COL + lane_addr + col_base + pc * 32, v);
-          ptx::tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            acc[pc * 32 + i] = fmaf(__uint_as_float(v[i]), lsi, acc[pc * 32 + i]);
-        }
+        add_corrections_in_tmem<CPT>(tmem_base + D1_COL + lane_addr + col_base, acc,
+                                     p.lo_scale_inv);
       }
+    } else if (ok) {
+      sums_to_tmem<CPT>(tmem_base + D1_COL + lane_addr + col_base, acc);
     }
 
     if (ok) {
@@ -266,47 +261,14 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
       const float unscale = (p.dyn != nullptr && p.k_slices == 1) ? p.dyn->unscale_c : 1.f;
       const float ar = p.alpha_r * unscale, ai = p.alpha_i * unscale;
       const float br = p.beta_r, bi = p.beta_i;
-      const bool read_c = (br != 0.f) || (bi != 0.f);
       const uint32_t row = static_cast<uint32_t>(m0) + quarter * 32u + static_cast<uint32_t>(lane);
-      const bool row_ok = row < p.m;
       float *cbase = ((p.c_array != nullptr) ? p.c_array[batch_id]
                                               : p.c + static_cast<uint64_t>(batch_id) * p.stride_c +
                                                     static_cast<uint64_t>(slice) * p.slice_stride) +
                      row;
-      const float sgn = (lane & 1) ? 1.f : -1.f; // odd rows hold imaginary parts
-      // Columns go in groups: all loads of a group are issued before its first store (the
-      // compiler must assume a store may alias the next load, which would put one memory
-      // latency per column on the tile's critical path when beta != 0).
-      constexpr int EPI_BATCH = (CPT >= 8) ? 8 : CPT;
-#pragma unroll
-      for (int i0 = 0; i0 < CPT; i0 += EPI_BATCH) {
-        float old[EPI_BATCH];
-#pragma unroll
-        for (int j = 0; j < EPI_BATCH; ++j) {
-          const uint32_t col = static_cast<uint32_t>(n0) + col_base + static_cast<uint32_t>(i0 + j);
-          old[j] = (read_c && row_ok && col < p.n)
-                       ? __ldcs(cbase + static_cast<uint64_t>(col) * p.ldc)
-                       : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < EPI_BATCH; ++j) {
-          const int i = i0 + j;
-          const uint32_t col = static_cast<uint32_t>(n0) + col_base + static_cast<uint32_t>(i);
-          if (col < p.n) { // uniform over the warp
-            float out;
-            if (p.is_complex) {
-              const float acc_o = __shfl_xor_sync(0xffffffffu, acc[i], 1);
-              const float old_o = __shfl_xor_sync(0xffffffffu, old[j], 1);
-              out = ar * acc[i] + sgn * ai * acc_o;
-              if (read_c) out += br * old[j] + sgn * bi * old_o;
-            } else {
-              out = ar * acc[i];
-              if (read_c) out = fmaf(br, old[j], out);
-            }
-            if (row_ok) cbase[static_cast<uint64_t>(col) * p.ldc] = out;
-          }
-        }
-      }
+      store_tile<CPT>(tmem_base + D1_COL + lane_addr + col_base, cbase, p.ldc,
+                      static_cast<uint32_t>(n0) + col_base, p.n, row < p.m, ar, ai, br, bi,
+                      p.is_complex != 0);
     }
   }
 

@@ -29,6 +29,7 @@
 //   d1_full   in both CTAs: commit multicast after the last stage of a tile
 //   d1_empty  leader's only: 16 arrivals, after the epilogue warps have read D1
 // Every wait is bounded; no TMA multicast is used.
+#include "epilogue.cuh"
 #include "gemm_common.cuh"
 #include "ptx.cuh"
 
@@ -315,67 +316,50 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
     }
   } else if (warp >= 4) {
     // ================================================================ drain + epilogue (both CTAs)
-    const uint32_t quarter = static_cast<uint32_t>(warp & 3);
-    const uint32_t half = static_cast<uint32_t>((warp - 4) >> 2);
-    const uint32_t lane_addr = (quarter * 32u) << 16;
-    const uint32_t col_base = half * CPT;
+    const uint32_t t_base = tmem_base + ((static_cast<uint32_t>(warp & 3) * 32u) << 16) +
+                            static_cast<uint32_t>((warp - 4) >> 2) * CPT;
     const uint32_t d0_empty_leader = ptx::map_to_cta(ptx::smem_u32(d0_empty), 0);
-    const uint32_t d1_empty_leader = ptx::map_to_cta(ptx::smem_u32(d1_empty), 0);
-    const float unscale = (p.dyn != nullptr) ? p.dyn->unscale_c : 1.f;
-    const float ar = p.alpha_r * unscale, ai = p.alpha_i * unscale;
-    const float br = p.beta_r, bi = p.beta_i;
-    const bool read_c = (br != 0.f) || (bi != 0.f);
-    const float sgn = (lane & 1) ? 1.f : -1.f; // odd rows hold imaginary parts
-    const float lsi = p.lo_scale_inv;
 
     uint32_t chunk_idx = 0, tile_iter = 0, tail_phase = 0;
     bool ok = true;
     for (uint32_t w = cluster_id; w < work_items && ok; w += num_clusters, ++tile_iter) {
-      const WorkItem wi = work_item(w, tail, k_blocks);
-      const bool split = w >= tail.split_begin; // this item is one K slice of a tile
-      const uint32_t n_chunks =
-          1u + ((wi.kbn > p.first_chunk)
-                    ? (wi.kbn - p.first_chunk + p.drain_chunk - 1) / p.drain_chunk
-                    : 0u);
-      const TileCoord tc = tile_coord(wi.tile, p, rank);
+      uint32_t n_chunks, prefetch_at;
+      {
+        const uint32_t kbn = work_item(w, tail, k_blocks).kbn;
+        n_chunks = 1u + ((kbn > p.first_chunk)
+                             ? (kbn - p.first_chunk + p.drain_chunk - 1) / p.drain_chunk
+                             : 0u);
+        const bool read_c = (p.beta_r != 0.f) || (p.beta_i != 0.f);
+        prefetch_at = (!read_c || w >= tail.split_begin) ? n_chunks
+                      : (n_chunks > C_PREFETCH_LEAD)     ? n_chunks - C_PREFETCH_LEAD
+                                                         : 0u;
+      }
       float acc[CPT];
 #pragma unroll
       for (int i = 0; i < CPT; ++i) acc[i] = 0.f;
 
-      // C(row, col): lanes hold consecutive rows of the column-major C, so each warp access
-      // covers 128 contiguous bytes of one column.
-      const uint32_t row =
-          static_cast<uint32_t>(tc.m0) + quarter * 32u + static_cast<uint32_t>(lane);
-      const bool row_ok = row < p.m;
-      float *cbase = ((p.c_array != nullptr) ? p.c_array[tc.batch]
-                                              : p.c + static_cast<uint64_t>(tc.batch) * p.stride_c) +
-                     row;
-      const uint32_t prefetch_at = (n_chunks > C_PREFETCH_LEAD) ? n_chunks - C_PREFETCH_LEAD : 0u;
-
+#pragma unroll 1
       for (uint32_t c = 0; c < n_chunks; ++c, ++chunk_idx) {
-        if (read_c && !split && c == prefetch_at) {
+        if (c == prefetch_at) {
           // beta != 0: pull this warp's part of the C tile into L2 a few chunks before the
           // epilogue reads it (lane l fetches the line of columns l, l+32, ...)
-#pragma unroll
+          const TileCoord tc = tile_coord(work_item(opaque(w), tail, k_blocks).tile, p, rank);
+          const uint32_t row = static_cast<uint32_t>(tc.m0) + static_cast<uint32_t>(warp & 3) * 32u;
+          const float *cp =
+              ((p.c_array != nullptr) ? p.c_array[tc.batch]
+                                      : p.c + static_cast<uint64_t>(tc.batch) * p.stride_c) + row;
+#pragma unroll 1
           for (int q = 0; q < CPT / 32; ++q) {
-            const uint32_t col = static_cast<uint32_t>(tc.n0) + col_base +
-                                 static_cast<uint32_t>(q * 32 + lane);
-            if (col < p.n && row - lane < p.m)
-              ptx::prefetch_l2(cbase - lane + static_cast<uint64_t>(col) * p.ldc);
+            const uint32_t col = static_cast<uint32_t>(tc.n0) +
+                                 static_cast<uint32_t>(((warp - 4) >> 2) * CPT + q * 32 + lane);
+            if (col < p.n && row < p.m) ptx::prefetch_l2(cp + static_cast<uint64_t>(col) * p.ldc);
           }
         }
-        ok = ptx::mbar_wait_timed(ptx::smem_u32(d0_full), chunk_idx & 1u, abort_flag, p.status,
-                                  ptx::kErrWaitD0Full, dbg, &dbg_wait);
+        ok = ptx::mbar_wait(ptx::smem_u32(d0_full), chunk_idx & 1u, abort_flag, p.status,
+                            ptx::kErrWaitD0Full);
         if (!ok) break;
         ptx::tc_fence_after();
-#pragma unroll
-        for (int pc = 0; pc < CPT / 32; ++pc) {
-          uint32_t v[32];
-          ptx::tmem_ld_32x32b_x32(tmem_base + lane_addr + col_base + pc * 32, v);
-          ptx::tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) acc[pc * 32 + i] += __uint_as_float(v[i]);
-        }
+        drain_sums<CPT>(t_base, acc);
         ptx::tc_fence_before();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive_cluster(d0_empty_leader);
@@ -386,19 +370,22 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
                           ptx::kErrWaitD1Full);
       if (!ok) break;
       ptx::tc_fence_after();
-#pragma unroll
-      for (int pc = 0; pc < CPT / 32; ++pc) {
-        uint32_t v[32];
-        ptx::tmem_ld_32x32b_x32(tmem_base + D1_COL + lane_addr + col_base + pc * 32, v);
-        ptx::tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          acc[pc * 32 + i] = fmaf(__uint_as_float(v[i]), lsi, acc[pc * 32 + i]);
-      }
-      // D1 is in registers: the issuer may start the next tile's correction products
-      ptx::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive_cluster(d1_empty_leader);
+      // the finished sums stay in the D1 columns; from here on they are read from there, and what
+      // the epilogue needs to know of the tile is worked out only now (epilogue.cuh)
+      const uint32_t t_sums = t_base + D1_COL;
+      add_corrections_in_tmem<CPT>(t_sums, acc, p.lo_scale_inv);
+      const WorkItem wi = work_item(opaque(w), tail, k_blocks);
+      const bool split = w >= tail.split_begin; // this item is one K slice of a tile
+      const TileCoord tc = tile_coord(wi.tile, p, rank);
+      const uint32_t quarter = static_cast<uint32_t>(warp & 3);
+      const uint32_t col_base = static_cast<uint32_t>((warp - 4) >> 2) * CPT;
+      const uint32_t d1_empty_leader = ptx::map_to_cta(ptx::smem_u32(d1_empty), 0);
+      // D1 is no longer needed: the issuer may start the next tile's correction products
+      auto release_d1 = [&]() {
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster(d1_empty_leader);
+      };
 
       if (split) {
         // one K slice of a tile: park the partial sums, take a ticket, and go on to the
@@ -406,10 +393,17 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
         const uint32_t ti = wi.tile - tail.split_begin;
         constexpr uint32_t HALF = BN_PAIR * BM_CTA; // floats of one CTA's 128 x 256 half
         float *tbase = tail.partial + (static_cast<uint64_t>(ti) * tail.slices * 2u + rank) * HALF +
-                       quarter * 32u + static_cast<uint32_t>(lane);
+                       col_base * BM_CTA + quarter * 32u + static_cast<uint32_t>(lane);
         float *mine = tbase + static_cast<uint64_t>(wi.slice) * 2u * HALF;
+#pragma unroll 1
+        for (int c = 0; c < CPT; c += kEpiGroup) {
+          uint32_t v[kEpiGroup];
+          ptx::tmem_ld_32x32b_x16(t_sums + c, v);
+          ptx::tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < CPT; ++i) __stcg(mine + (col_base + i) * BM_CTA, acc[i]);
+          for (int i = 0; i < kEpiGroup; ++i)
+            __stcg(mine + (c + i) * BM_CTA, __uint_as_float(v[i]));
+        }
         __threadfence();
         // the eight epilogue warps meet twice (all partial sums stored; ticket published) on
         // an mbarrier of their own, with the bounded wait every other wait here uses
@@ -426,54 +420,42 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
         if (warp == 4 && lane == 0) *ticket_smem = atomicAdd(tail.counters + ti * 2u + rank, 1u);
         ok = meet();
         if (!ok) break;
-        if (*ticket_smem != tail.slices - 1u) continue;
-        __threadfence();
-#pragma unroll
-        for (int i = 0; i < CPT; ++i) acc[i] = __ldcg(tbase + (col_base + i) * BM_CTA);
-        for (uint32_t sl = 1; sl < tail.slices; ++sl) {
-          const float *other = tbase + static_cast<uint64_t>(sl) * 2u * HALF;
-#pragma unroll
-          for (int i = 0; i < CPT; ++i) acc[i] += __ldcg(other + (col_base + i) * BM_CTA);
+        if (*ticket_smem != tail.slices - 1u) {
+          release_d1();
+          continue;
         }
+        __threadfence();
+#pragma unroll 1
+        for (int c = 0; c < CPT; c += kEpiGroup) {
+          float sum[kEpiGroup];
+#pragma unroll
+          for (int i = 0; i < kEpiGroup; ++i) sum[i] = __ldcg(tbase + (c + i) * BM_CTA);
+          for (uint32_t sl = 1; sl < tail.slices; ++sl) {
+            const float *other = tbase + static_cast<uint64_t>(sl) * 2u * HALF;
+#pragma unroll
+            for (int i = 0; i < kEpiGroup; ++i) sum[i] += __ldcg(other + (c + i) * BM_CTA);
+          }
+          uint32_t v[kEpiGroup];
+#pragma unroll
+          for (int i = 0; i < kEpiGroup; ++i) v[i] = __float_as_uint(sum[i]);
+          ptx::tmem_st_32x32b_x16(t_sums + c, v);
+        }
+        ptx::tmem_st_wait();
       }
 
-      // C(row, col) = alpha * acc + beta * C(row, col)
-      // Columns go in groups of EPI_BATCH: all loads of a group are issued before its first
-      // store, otherwise every load would wait for the store before it (the compiler must
-      // assume they alias) and a tile would spend 128 memory latencies here.
-      constexpr int EPI_BATCH = 8;
-#pragma unroll
-      for (int i0 = 0; i0 < CPT; i0 += EPI_BATCH) {
-        float old[EPI_BATCH];
-#pragma unroll
-        for (int j = 0; j < EPI_BATCH; ++j) {
-          const uint32_t col =
-              static_cast<uint32_t>(tc.n0) + col_base + static_cast<uint32_t>(i0 + j);
-          old[j] = (read_c && row_ok && col < p.n)
-                       ? __ldcs(cbase + static_cast<uint64_t>(col) * p.ldc)
-                       : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < EPI_BATCH; ++j) {
-          const int i = i0 + j;
-          const uint32_t col = static_cast<uint32_t>(tc.n0) + col_base + static_cast<uint32_t>(i);
-          if (col < p.n) { // uniform over the warp
-            float out;
-            if (p.is_complex) {
-              const float acc_o = __shfl_xor_sync(0xffffffffu, acc[i], 1);
-              const float old_o = __shfl_xor_sync(0xffffffffu, old[j], 1);
-              out = ar * acc[i] + sgn * ai * acc_o;
-              if (read_c) out += br * old[j] + sgn * bi * old_o;
-            } else {
-              out = ar * acc[i];
-              if (read_c) out = fmaf(br, old[j], out);
-            }
-            if (row_ok) cbase[static_cast<uint64_t>(col) * p.ldc] = out;
-          }
-        }
-      }
+      // C(row, col): lanes hold consecutive rows of the column-major C, so each warp access
+      // covers 128 contiguous bytes of one column.
+      const uint32_t row =
+          static_cast<uint32_t>(tc.m0) + quarter * 32u + static_cast<uint32_t>(lane);
+      float *cbase = ((p.c_array != nullptr) ? p.c_array[tc.batch]
+                                              : p.c + static_cast<uint64_t>(tc.batch) * p.stride_c) +
+                     row;
+      const float unscale = (p.dyn != nullptr) ? p.dyn->unscale_c : 1.f;
+      store_tile<CPT>(t_sums, cbase, p.ldc, static_cast<uint32_t>(tc.n0) + col_base, p.n, row < p.m,
+                      p.alpha_r * unscale, p.alpha_i * unscale, p.beta_r, p.beta_i,
+                      p.is_complex != 0);
+      release_d1();
     }
-    if (dbg && warp == 4 && lane == 0) atomicAdd(p.debug + 3, dbg_wait);
   }
 
   // ---------------------------------------------------------------- teardown
