@@ -220,7 +220,7 @@ class Handle:
         self._lib.cuMpSGEMM_set_workspace_limit(self._h, nbytes)
 
     def reload_tuning_env(self) -> None:
-        """Read the CUMPSGEMM_TILE_N / PAIR / DRAIN_CHUNK / FIRST_CHUNK / PACE / FUSED variables
+        """Read the CUMPSGEMM_TILE_N / PAIR / DRAIN_CHUNK / FIRST_CHUNK / PACE / FUSED / STREAM variables
         again (a handle reads them once, at creation)."""
         self._lib.cuMpSGEMM_reload_tuning_env(self._h)
 

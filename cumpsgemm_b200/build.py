@@ -34,6 +34,7 @@ CUDA_SOURCES = [
     "tcec_gemm.cu",
     "tcec_gemm_pair.cu",
     "tcec_gemm_fused.cu",
+    "tcec_gemm_stream.cu",
     "gemm_api.cu",
     "ext_api.cu",
     "static_scratch_gemm.cu",

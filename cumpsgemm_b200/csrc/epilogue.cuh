@@ -76,6 +76,31 @@ __device__ __forceinline__ void add_corrections_in_tmem(uint32_t taddr, const fl
   ptx::tmem_st_wait();
 }
 
+// C(row, col) = alpha * acc for columns [col0, col0 + CPT), straight from the registers
+template <int CPT>
+__device__ __forceinline__ void store_registers(const float (&acc)[CPT], float *cbase, uint64_t ldc,
+                                                uint32_t col0, uint32_t n, bool row_ok, float ar,
+                                                float ai) {
+  if (col0 >= n) return; // uniform over the warp
+  const uint32_t cols = n - col0;
+  float *cp = cbase + static_cast<uint64_t>(col0) * ldc;
+  if (ai == 0.f) {
+#pragma unroll
+    for (int i = 0; i < CPT; ++i) {
+      if (row_ok && static_cast<uint32_t>(i) < cols) __stcs(cp, ar * acc[i]);
+      cp += ldc;
+    }
+  } else {
+    const float sai = (threadIdx.x & 1) ? ai : -ai; // odd rows hold imaginary parts
+#pragma unroll
+    for (int i = 0; i < CPT; ++i) {
+      const float out = ar * acc[i] + sai * __shfl_xor_sync(0xffffffffu, acc[i], 1);
+      if (row_ok && static_cast<uint32_t>(i) < cols) __stcs(cp, out);
+      cp += ldc;
+    }
+  }
+}
+
 template <int CPT, bool READ_C, bool COMPLEX>
 __device__ __forceinline__ void store_loop(uint32_t taddr, float *cp, uint64_t ldc, uint32_t cols,
                                            bool row_ok, float ar, float ai, float br, float bi) {
@@ -88,10 +113,14 @@ __device__ __forceinline__ void store_loop(uint32_t taddr, float *cp, uint64_t l
 #pragma unroll
     for (uint32_t j = 0; j < G; ++j, lp += ldc) old[j] = (row_ok && j < cols) ? __ldcs(lp) : 0.f;
   }
+  uint32_t v[G];
+  ptx::tmem_ld_32x32b_x16(taddr, v);
+  ptx::tmem_ld_wait();
 #pragma unroll 1
   for (uint32_t c = 0; c < cols; c += G) {
-    uint32_t v[G];
-    ptx::tmem_ld_32x32b_x16(taddr + c, v);
+    // the next group (the last iteration fetches its own again) is on its way during the stores
+    uint32_t nv[G];
+    ptx::tmem_ld_32x32b_x16(taddr + min(c + G, static_cast<uint32_t>(CPT) - G), nv);
     float next[G];
     if constexpr (READ_C) {
       const float *lp = cp + static_cast<uint64_t>(G) * ldc;
@@ -99,7 +128,6 @@ __device__ __forceinline__ void store_loop(uint32_t taddr, float *cp, uint64_t l
       for (uint32_t j = 0; j < G; ++j, lp += ldc)
         next[j] = (row_ok && c + G + j < cols) ? __ldcs(lp) : 0.f;
     }
-    ptx::tmem_ld_wait();
 #pragma unroll
     for (uint32_t j = 0; j < G; ++j) {
       const float x = __uint_as_float(v[j]);
@@ -113,6 +141,9 @@ __device__ __forceinline__ void store_loop(uint32_t taddr, float *cp, uint64_t l
       if (row_ok && c + j < cols) *cp = out;
       cp += ldc;
     }
+    ptx::tmem_ld_wait();
+#pragma unroll
+    for (uint32_t j = 0; j < G; ++j) v[j] = nv[j];
   }
 }
 

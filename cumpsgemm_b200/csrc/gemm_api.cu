@@ -168,6 +168,85 @@ bool fused_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperati
   return true;
 }
 
+// Where the streaming kernel (tcec_gemm_stream.cu) is the faster path.  It saves the split pass,
+// its workspace traffic and a launch, and pays with about 2,450 cycles per 64 k values of a
+// 256 x 256 pair tile where the pre-split pair kernel takes 1,600, and with a longer start-up.
+// Measured (B200, us per call, paths that applied before / this kernel with the width chosen here):
+//   strided batches of small matrices, FP16TCEC          TF32TCEC
+//     64 x 256^3          23.9 / 18.1                      512 x 256^3           262 / 104
+//     512 x 256^3          123 / 80                        2048 x 128^3          460 / 154
+//     64 x 512^3           114 / 68                        16 x 1024^3           219 / 161
+//     16 x 1024^3          126 / 112                       128 x complex 256^3   191 / 94
+//     512 x complex 128^3   83 / 50 (128 wide)
+//     512 x 512 x 64 x 512 130 / 78 (128 wide)
+//     32 x 1024 x 1024 x 64 43 / 43, and a lone 4096 x 4096 x 512 55 / 64: where every operand element
+//     is used by many tiles the pre-split panels win, hence the limit on m and n.
+//   few tiles, long K (slices)
+//     256 x 256 x 65536     67 / 45      512 x 512 x 16384  48 / 37      4096 x 128 x 4096  42 / 33
+//     256 x 1024 x 8192     31 / 27      384 x 384 x 8192 25 / 25        512 x 512 x 4096   19 / 20
+//     256 x 256 x 4096      15 / 17
+bool stream_pays(const StreamPlan &plan, std::uint64_t m_exp, std::uint64_t n, std::uint64_t batch,
+                 int clusters) {
+  const std::uint64_t tiles = plan.total_tiles;
+  if (plan.slices > 1) return plan.units >= 256 || tiles * plan.units >= 512;
+  return batch >= 8 && m_exp <= 1024 && n <= 1024 &&
+         2 * tiles >= static_cast<std::uint64_t>(clusters);
+}
+
+// Operands of a call for the streaming pair kernel (tcec_gemm_stream.cu).  TMA reads them in
+// place, so bases, leading dimensions and batch strides have to be multiples of 16 bytes; every
+// op and both kinds are handled.  Returns false when the call has to take another path.
+template <class T>
+bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperation_t op_B,
+                 std::uint64_t m, std::uint64_t n, std::uint64_t k, const T *a, std::uint64_t lda,
+                 std::uint64_t stridea, const T *b, std::uint64_t ldb, std::uint64_t strideb,
+                 std::uint64_t batch, StreamKind kind, StreamGemmArgs *out) {
+  constexpr bool is_complex = std::is_same<T, cuComplex>::value;
+  constexpr std::uint64_t fpe = is_complex ? 2 : 1;
+  const Tuning &t = h->tuning;
+  if (t.stream == 0 || (t.stream == -1 && t.others_forced())) return false;
+  const std::uint64_t sa = batch > 1 ? stridea * fpe : 0, sb = batch > 1 ? strideb * fpe : 0;
+  const bool aligned = (reinterpret_cast<std::uintptr_t>(a) % 16 == 0) &&
+                       (reinterpret_cast<std::uintptr_t>(b) % 16 == 0) && (lda * fpe) % 4 == 0 &&
+                       (ldb * fpe) % 4 == 0 && sa % 4 == 0 && sb % 4 == 0;
+  constexpr std::uint64_t kMaxStride = (1ull << 38) - 1; // floats: TMA strides are below 2^40 bytes
+  if (!aligned || lda * fpe > kMaxStride || ldb * fpe > kMaxStride || sa > kMaxStride ||
+      sb > kMaxStride)
+    return false;
+  const std::uint64_t m_exp = m * fpe, k_exp = k * fpe;
+  if (batch > 0x3fffffffull) return false;
+  const int tile_n = (t.stream == 128 || t.stream == 256) ? t.stream : (n <= 128 ? 128 : 256);
+  int clusters = 0;
+  if (stream_max_clusters(tile_n, &clusters) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const StreamPlan plan = plan_stream(t, tile_n, m_exp, n, k_exp, batch,
+                                      static_cast<std::uint32_t>(clusters));
+  if (plan.total_tiles == 0) return false;
+  if (t.stream == -1 && !stream_pays(plan, m_exp, n, batch, clusters)) return false;
+  *out = StreamGemmArgs{};
+  out->kind = kind;
+  out->a = StreamOperand{reinterpret_cast<const float *>(a), lda * fpe, sa};
+  out->b = StreamOperand{reinterpret_cast<const float *>(b), ldb * fpe, sb};
+  if (is_complex) {
+    out->layout_a = (op_A == CUBLAS_OP_N) ? 2 : 3;
+    out->layout_b = (op_B == CUBLAS_OP_N) ? 0 : 4;
+    out->conj_a = (op_A == CUBLAS_OP_C);
+    out->conj_b = (op_B == CUBLAS_OP_C);
+  } else {
+    out->layout_a = (op_A == CUBLAS_OP_N) ? 1 : 0;
+    out->layout_b = (op_B == CUBLAS_OP_N) ? 0 : 1;
+  }
+  out->is_complex = is_complex;
+  out->m = static_cast<std::uint32_t>(m_exp);
+  out->n = static_cast<std::uint32_t>(n);
+  out->k = static_cast<std::uint32_t>(k_exp);
+  out->batch = static_cast<std::uint32_t>(batch);
+  out->plan = plan;
+  return true;
+}
+
 } // namespace
 
 template <class T>
@@ -232,10 +311,90 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
   const std::uint64_t m_exp = m * fpe; // rows of the expanded real problem
   const std::uint64_t k_exp = k * fpe;
 
-  // ---- one launch, no workspace: operands split inside the GEMM kernel
+  // ---- one launch on CTA pairs, operands split between TMA and the tensor core
+  StreamGemmArgs ga;
+  const StreamKind stream_kind = (want_fp16 && want_tf32) ? StreamKind::device
+                                 : want_fp16              ? StreamKind::fp16
+                                                          : StreamKind::tf32;
+  // (batches of matrices with at most 128 rows would leave one CTA of every pair idle: the kernel
+  // below serves those it can, 2048 x 128^3 82 us against 95-110 here)
   FusedGemmArgs fa;
-  if (mode == CUMPSGEMM_FP16TCEC && !ptr_arrays &&
-      fused_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, &fa)) {
+  const bool fused = mode == CUMPSGEMM_FP16TCEC && !ptr_arrays &&
+                     fused_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch,
+                                   &fa);
+  if (ec && !ptr_arrays && !(fused && batch >= 8 && m_exp <= 128 && h->tuning.stream == -1) &&
+      stream_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, stream_kind,
+                     &ga)) {
+    bool room = true;
+    if (ga.plan.piece_clusters > 0) {
+      const std::size_t bytes = stream_scratch_bytes(ga.plan, ga.m, ga.n, ga.batch);
+      const std::size_t limit =
+          h->workspace_limit_bytes ? h->workspace_limit_bytes : kDefaultWorkspaceLimit;
+      room = bytes <= limit && ensure_workspace(h, bytes);
+    }
+    if (room) {
+      ga.c = reinterpret_cast<float *>(c);
+      ga.ldc = ldc * fpe;
+      ga.stride_c = stridec * fpe;
+      ga.alpha_r = Scalar<T>::re(alpha);
+      ga.alpha_i = Scalar<T>::im(alpha);
+      ga.beta_r = Scalar<T>::re(beta);
+      ga.beta_i = Scalar<T>::im(beta);
+      ga.dyn = dyn;
+      ga.dev_status = h->dev_status;
+      ga.debug = h->debug_buffer;
+      ga.partial = reinterpret_cast<float *>(h->workspace);
+      ga.counters = reinterpret_cast<unsigned int *>(h->dev_status + 2 + kPairTailCounters);
+      if (used_kernel_module_id != nullptr) {
+        const int tn = pick_tile(h->tuning, h->num_sms, m_exp, n, batch, true).tile_n;
+        *used_kernel_module_id = (ga.plan.slices > 1) ? 100u : (tn == 256) ? 0u : (tn == 128) ? 1u : 2u;
+      }
+      const bool prof = h->exp_stats.profiling_enabled;
+      if (prof) h->exp_stats.profiler.start("gemm_kernel", h->cuda_stream);
+      cuMpSGEMM_handle::TimingTriple tt{};
+      if (h->kernel_timing) {
+        for (auto &e : tt.e) cudaEventCreate(&e);
+        cudaEventRecord(tt.e[0], h->cuda_stream);
+        cudaEventRecord(tt.e[1], h->cuda_stream);
+      }
+      cudaError_t gerr = launch_tcec_gemm_stream(ga, h->cuda_stream);
+      const bool addressable = gerr != cudaErrorNotSupported;
+      if (gerr == cudaSuccess && ga.plan.slices > 1) {
+        TcecGemmArgs r = {};
+        r.m = ga.m;
+        r.n = ga.n;
+        r.batch = ga.batch;
+        r.c = ga.c;
+        r.ldc = ga.ldc;
+        r.stride_c = ga.stride_c;
+        r.alpha_r = ga.alpha_r;
+        r.alpha_i = ga.alpha_i;
+        r.beta_r = ga.beta_r;
+        r.beta_i = ga.beta_i;
+        r.is_complex = ga.is_complex;
+        r.dyn = ga.dyn;
+        r.k_slices = ga.plan.slices;
+        r.partial = ga.partial;
+        gerr = launch_splitk_reduce(r, h->cuda_stream);
+      }
+      if (h->kernel_timing) {
+        cudaEventRecord(tt.e[2], h->cuda_stream);
+        h->timing_events.push_back(tt);
+      }
+      if (prof) h->exp_stats.profiler.stop("gemm_kernel", h->cuda_stream);
+      if (addressable) {
+        mark_stream_work(h);
+        if (gerr != cudaSuccess) {
+          log_error(std::string("kernel launch failed: ") + cudaGetErrorString(gerr));
+          return CUBLAS_STATUS_EXECUTION_FAILED;
+        }
+        return CUBLAS_STATUS_SUCCESS;
+      }
+    }
+  }
+
+  // ---- one launch, no workspace: operands split inside the GEMM kernel
+  if (fused) {
     fa.c = reinterpret_cast<float *>(c);
     fa.ldc = ldc * fpe;
     fa.stride_c = stridec * fpe;

@@ -55,6 +55,11 @@ static_assert(sizeof(GemmKernelParams) <= 128, "see the comment at the top of th
 bool make_panel_map(CUtensorMap *map, SplitKind kind, const void *panel, uint32_t k_pad,
                     uint32_t rows_pad, uint32_t planes, uint32_t box_rows);
 
+// Tensor map over FP32 data in global memory: dims[0] contiguous, strides (bytes) of dims 1 and 2,
+// optional 128-byte swizzle (box[0] = 32 then).  Returns false if the driver rejects it.
+bool make_float_map(CUtensorMap *map, const float *base, const uint64_t (&dims)[3],
+                    const uint64_t (&strides)[2], const uint32_t (&box)[3], bool swizzle);
+
 // CTA-pair kernel (tcec_gemm_pair.cu): 256 x 256 tile per cluster of two CTAs.
 cudaError_t launch_tcec_gemm_pair(const TcecGemmArgs &a, cudaStream_t stream);
 cudaError_t launch_tcec_gemm_pair_auto(const TcecGemmArgs &a, cudaStream_t stream);

@@ -83,6 +83,13 @@ struct Tuning {
   int fused = -1;      // -1 = by rule
   int split_k = -1;    // CUMPSGEMM_SPLIT_K: 0 = never, -1 = by rule, n > 1 = that many slices
   int tail_split = -1; // CUMPSGEMM_TAIL_SPLIT: 0 = never, -1 = by rule, n > 1 = at most n slices
+  int stream = -1;     // CUMPSGEMM_STREAM: 0 / 1 the pair kernel that splits its operands off / on
+                       // wherever it is applicable, 256 / 128 on with that tile width, -1 by rule
+  // a switch of one of the other kernels or of their schedules is set
+  bool others_forced() const {
+    return tile_n != 0 || pair != -1 || drain_chunk != 0 || first_chunk != 0 || pace != 1 ||
+           fused != -1 || split_k > 0 || tail_split > 0;
+  }
 };
 Tuning read_tuning_env();
 
@@ -139,7 +146,9 @@ struct cuMpSGEMM_handle {
   cumpsgemm_b200::Tuning tuning;
 
   // Device status word the GEMM kernel writes when a bounded wait gives up.
-  int *dev_status = nullptr; // [0] kernel status word, [1] wave counter of the pair kernel
+  // [0] kernel status word, [1] wave counter of the pair kernel, [2 ...] its tail-split counters,
+  // then the counters of the streaming kernel
+  int *dev_status = nullptr;
 
   // Optional per-launch timing: events recorded on the launching stream before the split
   // pass, between split pass and GEMM kernel, and after the GEMM kernel.
@@ -333,6 +342,47 @@ struct FusedGemmArgs {
   float *partial = nullptr;
 };
 cudaError_t launch_tcec_gemm_fused(const FusedGemmArgs &a, cudaStream_t stream);
+// GEMM on CTA pairs that splits its operands between TMA and the tensor core
+// (tcec_gemm_stream.cu): no workspace for panels, error-corrected kinds only, strided batches.
+// Sizes are those of the real (expanded) problem, leading dimensions and strides in floats.
+enum class StreamKind : int { fp16 = 0, tf32 = 1, device = 2 }; // device: dyn->gemm_mode decides
+struct StreamOperand {
+  const float *src;
+  std::uint64_t ld, stride; // multiples of 4 (TMA: 16 bytes); stride 0: one matrix for all batches
+};
+// How the tiles of a launch are dealt to the CTA pairs; see tcec_gemm_stream.cu.
+struct StreamPlan {
+  int tile_n;                    // 256 or 128 columns per pair tile (256 rows)
+  std::uint32_t total_tiles;
+  std::uint32_t units;           // K loop in units of 64 k values
+  std::uint32_t whole_tiles;     // dealt whole, in waves
+  std::uint32_t piece_clusters;  // clusters sharing the k range of the other tiles (0: none)
+  std::uint32_t slices;          // > 1: every tile in that many slices plus a reduction kernel
+};
+StreamPlan plan_stream(const Tuning &tuning, int tile_n, std::uint64_t m, std::uint64_t n,
+                       std::uint64_t k, std::uint64_t batch, std::uint32_t clusters);
+struct StreamGemmArgs {
+  StreamKind kind;
+  StreamOperand a, b;
+  int layout_a, layout_b; // RawLayout of tcec_gemm_stream.cu
+  bool conj_a, conj_b, is_complex;
+  std::uint32_t m, n, k, batch;
+  float *c;
+  std::uint64_t ldc, stride_c;
+  float alpha_r, alpha_i, beta_r, beta_i;
+  const DynParams *dyn; // nullable: scale factors and the un-scaling of C
+  int *dev_status;
+  unsigned long long *debug;
+  StreamPlan plan;
+  float *partial;         // stream_scratch_bytes() bytes when the plan cuts tiles along K
+  unsigned int *counters; // kStreamCounters words, zero (the kernel leaves them at zero)
+};
+constexpr int kStreamCounters = 512; // two per tile that is cut in pieces
+constexpr int kStatusWords = 2 + kPairTailCounters + kStreamCounters; // of handle::dev_status
+std::size_t stream_scratch_bytes(const StreamPlan &plan, std::uint32_t m, std::uint32_t n,
+                                 std::uint32_t batch);
+cudaError_t stream_max_clusters(int tile_n, int *clusters); // of the current device
+cudaError_t launch_tcec_gemm_stream(const StreamGemmArgs &a, cudaStream_t stream);
 // Self-test of the bounded mbarrier wait (see cuMpSGEMM_selftest_bounded_wait).
 cudaError_t launch_bounded_wait_selftest(int *dev_status, unsigned long long limit_ns,
                                          unsigned long long *dev_waited_ns, cudaStream_t stream);

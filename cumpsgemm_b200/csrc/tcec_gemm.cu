@@ -355,6 +355,22 @@ bool make_panel_map(CUtensorMap *map, SplitKind kind, const void *panel, uint32_
   return r == CUDA_SUCCESS;
 }
 
+bool make_float_map(CUtensorMap *map, const float *base, const uint64_t (&dims)[3],
+                    const uint64_t (&strides)[2], const uint32_t (&box)[3], bool swizzle) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (fn == nullptr) return false;
+  const cuuint64_t d[3] = {dims[0], dims[1], dims[2]};
+  const cuuint64_t st[2] = {strides[0], strides[1]};
+  const cuuint32_t bx[3] = {box[0], box[1], box[2]};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r =
+      fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(base), d, st, bx, estr,
+         CU_TENSOR_MAP_INTERLEAVE_NONE,
+         swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+
 namespace {
 
 // Tensor maps, kernel parameters and grid size of one kind.

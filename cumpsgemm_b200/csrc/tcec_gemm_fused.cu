@@ -64,8 +64,8 @@
 // All need 16-byte aligned bases, leading dimensions and batch strides.
 #include "gemm_common.cuh"
 #include "ptx.cuh"
+#include "split_math.cuh"
 
-#include <cuda_fp16.h>
 #include <mutex>
 
 namespace cumpsgemm_b200 {
@@ -121,35 +121,6 @@ template <int BN> struct FusedCfg {
   static constexpr uint32_t TMEM_COLS = 4u * BN;
 };
 
-// Byte offset of (row r, 16-byte chunk c) inside a K-major tile with 128-byte rows and the
-// 128-byte swizzle: 8-row groups of 1 KiB, chunk index XORed with the row index modulo 8.
-__device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t c) {
-  return (r >> 3) * 1024u + (r & 7u) * 128u + ((c ^ (r & 7u)) << 4);
-}
-
-// hi = RN_fp16(v), lo = RN_fp16((v - hi) * 2^11) for two values, packed (v0 in the low half)
-__device__ __forceinline__ void split2(float v0, float v1, uint32_t &hi, uint32_t &lo) {
-  const __half2 h = __floats2half2_rn(v0, v1);
-  const float2 hf = __half22float2(h);
-  const __half2 l = __floats2half2_rn((v0 - hf.x) * 2048.f, (v1 - hf.y) * 2048.f);
-  hi = *reinterpret_cast<const uint32_t *>(&h);
-  lo = *reinterpret_cast<const uint32_t *>(&l);
-}
-
-__device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t x, uint32_t y, uint32_t z,
-                                             uint32_t w) {
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x), "r"(y), "r"(z),
-               "r"(w)
-               : "memory");
-}
-// generic-proxy writes to shared memory become visible to the async proxy (the tensor core)
-__device__ __forceinline__ void fence_proxy_async_shared() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 // 4 floats at p, zero filled outside [.., limit) / when !ok
 __device__ __forceinline__ float4 ld4(const float *p, uint64_t first, uint64_t limit, bool ok) {
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -167,10 +138,6 @@ __device__ __forceinline__ float4 ld4(const float *p, uint64_t first, uint64_t l
 // (cw = 0..7).  Every body issues all of a thread's loads (up to eight float4) before the
 // first conversion, reads whole 128-byte lines per warp instruction, and stores without
 // shared-memory bank conflicts.
-
-__device__ __forceinline__ void st_shared_v2(uint32_t addr, uint32_t x, uint32_t y) {
-  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(x), "r"(y) : "memory");
-}
 
 // K-contiguous source.  One warp instruction covers 2 rows x 64 k: lanes 0-15 read the 256
 // contiguous bytes of one row, lanes 16-31 those of the next.  A lane's four values are half

@@ -1,0 +1,1063 @@
+// Error-corrected tensor-core GEMM on CTA pairs that splits its FP32 operands on the way from
+// TMA to the tensor core: no split pass, no operand workspace, one launch.
+//
+// The reference splits every FP32 value at fragment load, inside the GEMM kernel
+// (src/device_tcec_wrapper.hpp:72-80 called from src/cumpsgemm_kernel.cuh:58-100).  Here a
+// cluster of two CTAs owns a 256 x BN tile of C (BN = 256 or 128); each CTA
+//   * fetches its own 128 rows of op(A) and its own BN / 2 rows of op(B) as plain FP32 through TMA
+//     into a ring of raw slots (32 k values each; edges are zero filled by TMA, so no thread
+//     tests bounds),
+//   * has eight converter warps split the raw values into hi / lo (same bits as split_kernels.cu)
+//     and write them as 128-byte-swizzled K-major tiles into a ring of operand stages,
+//   * and holds its 128 rows of the two TMEM accumulators (D0 = hi*hi, drained every stage into
+//     FP32 registers; D1 = lo*hi + hi*lo, drained once per tile), which its eight epilogue warps
+//     drain.
+// The even CTA's single issuing thread drives the tensor cores of both SMs (cta_group::2).
+//
+// Why pairs, and why raw slots in shared memory.  Per SM and 64 k values a 256 x 256 pair tile
+// converts 128 + 128 rows for a 128 x 256 share of C, half of what a 128 x 128 tile of
+// tcec_gemm_fused.cu converts per product.  Letting TMA run three slots ahead takes the
+// global-memory latency off the converter warps, which was a third of their time when they loaded
+// for themselves.
+//
+// What bounds it: shared-memory traffic.  Per stage of 64 k values an SM's shared memory takes 64 KiB
+// from TMA, gives 64 KiB to the converters, takes 64 KiB of hi / lo tiles back and feeds 96 KiB
+// to the tensor core: 2304 cycles at 128 bytes per cycle, against 1536 of tensor-core work.
+// Measured 2450 cycles per stage (m = n = k = 2048), and with short tiles about 4,500 per tile for
+// the hand-over of D1 on top.  Measured per call, paths that applied before / here (us): 512 x
+// complex 256^3 FP16TCEC_SCALING (one third of it the scan) 558 / 374, 512 x 256^3 123 / 80,
+// TF32TCEC 512 x 256^3 262 / 104, 256 x 256 x 65536 68.7 / 48.7.  Errors against 64-bit products
+// are equal or smaller (those two: 2.1e-7 -> 1.5e-7 and 4.1e-7 -> 2.1e-7), because D0 is drained
+// every 64 FP16 / 32 TF32 values.
+//
+// Work distribution.  Tiles are dealt to the clusters in whole waves; what is left over
+// (total mod clusters, or everything when there are fewer tiles than clusters) can be cut along K:
+//   ticket mode   the left-over tiles' k range is laid out end to end and cut into equal pieces,
+//                 one per cluster, so a piece may end one tile and begin the next.  A piece that
+//                 is not a whole tile parks its FP32 partial sums in scratch memory and takes a
+//                 ticket of the tile's counter; the CTA that draws the last ticket adds the pieces
+//                 in ascending k (whoever it is, the result is the same) and runs the alpha / beta
+//                 epilogue, then puts the counter back to zero.  Nobody waits for anybody.
+//   reduce mode   few tiles: every tile is cut into the same number of slices, which write plain
+//                 partial sums that splitk_reduce_kernel adds in ascending order.
+// Both are the deterministic successors of the reference's atomic split-K kernel
+// (src/cumpsgemm.cu:272-304, src/dmem_accessor.hpp:352-395).
+//
+// Threads: 640 = warp 0 TMA producer, warp 1 TMEM allocation + MMA issue (even CTA), warps 2-3
+// idle, warps 4-11 drain / epilogue, warps 12-19 converters.  Launched with 96 registers per
+// thread = 61440; setmaxnreg gives the epilogue warps 160 (they hold 128 running sums each), the
+// converters 56 and the rest 48: 256*160 + 256*56 + 128*48 = 61440, so the increase can always be
+// served.
+//
+// Barriers (per CTA, same shared-memory offsets; "leader" = even CTA):
+//   raw_full[r]    1 arrival (producer, expect_tx) + TMA bytes      own CTA
+//   raw_empty[r]   8 arrivals, one per converter warp               own CTA
+//   full[s]        leader's only: 16 arrivals, 8 converter warps of each CTA
+//   empty[s]       tcgen05.commit multicast from the leader         both CTAs
+//   d0_full, d0_empty, d1_full, d1_empty, tail: as in tcec_gemm_pair.cu
+// Every wait is bounded; no TMA multicast is used.
+#include "epilogue.cuh"
+#include "gemm_common.cuh"
+#include "ptx.cuh"
+#include "split_math.cuh"
+
+#include <mutex>
+
+namespace cumpsgemm_b200 {
+namespace {
+
+constexpr int BM_CTA = 128;
+constexpr int ROW_BYTES = kGemmRowBytes;
+constexpr int SLOT_K = 32; // k values of a raw slot (128 bytes of FP32)
+constexpr int NUM_THREADS = 640;
+constexpr int FIRST_EPI_WARP = 4, NUM_EPI_WARPS = 8;
+constexpr int FIRST_CVT_WARP = 12, NUM_CVT_WARPS = 8;
+constexpr int LAUNCH_REGS = 96;
+constexpr int REGS_EPI = 160, REGS_CVT = 56, REGS_REST = 48;
+static_assert(256 * REGS_EPI + 256 * REGS_CVT + 128 * REGS_REST <= NUM_THREADS * LAUNCH_REGS,
+              "register re-allocation must fit what the CTA was launched with");
+constexpr uint32_t C_PREFETCH_LEAD = 8; // stages between the L2 prefetch of C and its use
+
+// Raw layouts a converter can read (values of StreamGemmArgs::layout_a / layout_b).
+enum RawLayout : int {
+  kRawK = 0,    // element (r, k) at [r * ld + k]: K contiguous, 128-byte rows, 128-byte swizzle
+  kRawR = 1,    // element (r, k) at [k * ld + r]: rows contiguous
+  kRawCplxAR = 2, // complex A, op N: rows contiguous
+  kRawCplxAK = 3, // complex A, op T / C: K contiguous, swizzled
+  kRawCplxBR = 4  // complex B, op T / C: rows contiguous   (complex B, op N is kRawK)
+};
+
+struct StreamParams {
+  float *c;
+  const DynParams *dyn;
+  int *status;
+  float *partial;         // ticket mode: [cluster][2][CTA rank][BN columns][128 rows]
+  unsigned int *counters; // ticket mode: [left-over tile][CTA rank], zero between launches
+  unsigned long long *debug;
+  uint64_t ldc, stride_c, slice_stride;
+  uint32_t m, n;
+  uint32_t units; // K loop in units of 64 k values
+  uint32_t tiles_m, tiles_n;
+  uint32_t total_tiles;
+  uint32_t whole_tiles; // tiles [0, whole_tiles) are dealt whole
+  float alpha_r, alpha_i, beta_r, beta_i;
+  uint16_t piece_clusters; // clusters that share the left-over tiles' k range (0: none left over)
+  uint16_t slices;         // reduce mode: slices per tile; 0 or 1: ticket mode
+  uint8_t layout_a, layout_b;
+  uint8_t flags; // k* below
+};
+static_assert(sizeof(StreamParams) <= 128, "kernel parameter structs stay within 128 bytes");
+constexpr uint32_t kIsComplex = 1, kConjA = 2, kConjB = 4, kBatchA = 8, kBatchB = 16,
+                   kDirectStores = 32;
+
+template <int BN> struct StreamCfg {
+  static constexpr int B_ROWS = BN / 2; // rows of op(B) per CTA
+  static constexpr int A_TILE = BM_CTA * ROW_BYTES;
+  static constexpr int B_TILE = B_ROWS * ROW_BYTES;
+  static constexpr int STAGE_BYTES = 2 * (A_TILE + B_TILE);
+  static constexpr int STAGES = (BN == 256) ? 2 : 3;
+  static constexpr int RAW_A = BM_CTA * SLOT_K * 4;
+  static constexpr int RAW_BYTES = RAW_A + B_ROWS * SLOT_K * 4;
+  static constexpr int RAW_SLOTS = 3;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + RAW_SLOTS * RAW_BYTES + 1024 + 256;
+  static constexpr uint32_t TMEM_COLS = 2 * BN;
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
+};
+
+struct TileCoord {
+  uint32_t batch;
+  int m0; // first row of this CTA's 128 rows
+  int n0; // first column of the pair's BN columns
+};
+
+template <int BN>
+__device__ __forceinline__ TileCoord tile_coord(uint32_t tile, const StreamParams &p,
+                                                uint32_t rank) {
+  constexpr uint32_t GROUP_M = 8;
+  const uint32_t tiles_per_batch = p.tiles_m * p.tiles_n;
+  TileCoord c;
+  c.batch = tile / tiles_per_batch;
+  const uint32_t t = tile - c.batch * tiles_per_batch;
+  const uint32_t tiles_in_group = GROUP_M * p.tiles_n;
+  const uint32_t group_id = t / tiles_in_group;
+  const uint32_t first_m = group_id * GROUP_M;
+  const uint32_t group_rows = min(p.tiles_m - first_m, GROUP_M);
+  const uint32_t in_group = t - group_id * tiles_in_group;
+  c.m0 = static_cast<int>((first_m + in_group % group_rows) * 2 * BM_CTA + rank * BM_CTA);
+  c.n0 = static_cast<int>((in_group / group_rows) * BN);
+  return c;
+}
+
+// First unit (of the left-over tiles' concatenated k range) of cluster c's piece.
+__device__ __forceinline__ uint32_t piece_start(uint32_t c, uint32_t total_units,
+                                                uint32_t clusters) {
+  return static_cast<uint32_t>(static_cast<uint64_t>(c) * total_units / clusters);
+}
+
+// One work item: units [u0, u0 + un) of a tile's K loop.
+struct WorkItem {
+  uint32_t tile, u0, un;
+  uint32_t slot; // ticket mode: which of the cluster's two scratch tiles a partial item uses
+};
+// The items of one cluster, in the order every role walks them.
+struct WorkList {
+  uint32_t w, step; // whole tiles
+  uint32_t u, u_end, first;
+  __device__ __forceinline__ WorkList(const StreamParams &p, uint32_t cluster, uint32_t clusters)
+      : w(cluster), step(clusters), u(0), u_end(0), first(1) {
+    if (cluster < p.piece_clusters) {
+      const uint32_t total = (p.total_tiles - p.whole_tiles) * p.units;
+      u = piece_start(cluster, total, p.piece_clusters);
+      u_end = piece_start(cluster + 1, total, p.piece_clusters);
+    }
+  }
+  __device__ __forceinline__ bool next(const StreamParams &p, WorkItem &x) {
+    if (w < p.whole_tiles) {
+      x.tile = w;
+      x.u0 = 0;
+      x.un = p.units;
+      x.slot = 0;
+      w += step;
+      return true;
+    }
+    if (u < u_end) {
+      const uint32_t ti = u / p.units;
+      x.tile = p.whole_tiles + ti;
+      x.u0 = u - ti * p.units;
+      x.un = min(p.units - x.u0, u_end - u);
+      x.slot = first ? 0u : 1u;
+      first = 0;
+      u += x.un;
+      return true;
+    }
+    return false;
+  }
+};
+
+template <int KIND>
+__device__ __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                         uint32_t acc) {
+  if constexpr (KIND == 0) {
+    ptx::mma_f16_ss_pair(d, a, b, idesc, acc);
+  } else {
+    ptx::mma_tf32_ss_pair(d, a, b, idesc, acc);
+  }
+}
+
+// ---------------------------------------------------------------- converters
+// One warp converts 32 rows (lane = row) of one operand: of every raw slot JOBS groups of eight
+// consecutive k values, of which a slot has four.  Each layout has a loop of its own: a warp runs
+// one of them, so the code it cycles through stays small (a first version chose the layout per
+// group inside one unrolled loop: 5,000 cycles per stage, most of them instruction fetches and
+// spills).  Shared-memory accesses are free of bank conflicts: K-contiguous tiles are swizzled by
+// TMA (eight lanes of a 16-byte access hit eight different 16-byte positions), row-contiguous
+// ones are read 4 or 8 bytes per lane along the row.  Row r's 16-byte chunk q of a swizzled
+// tile is at r * 128 + ((q ^ (r & 7)) << 4), i.e. at (r * 128 + ((r & 7) << 4)) ^ (q << 4).
+struct ConverterState {
+  uint64_t *raw_full, *raw_empty, *empty;
+  uint32_t full_leader; // shared::cluster address of full[0] in the leader
+  uint32_t raw, dst;    // shared addresses of slot 0's raw tile and stage 0's hi tile of the operand
+  uint32_t lo_delta;
+  uint32_t row;         // this lane's row of the tile
+  uint32_t group0;      // first of the warp's 8-k groups in a slot
+  float scale;
+  uint32_t conj_mask;   // sign bit if the operand is conjugated, else 0
+  volatile int *abort_flag;
+  int *status;
+  bool timed;
+  unsigned long long wait_raw, wait_empty;
+};
+
+__device__ __forceinline__ float flip_sign(float x, uint32_t mask) {
+  return __uint_as_float(__float_as_uint(x) ^ mask);
+}
+
+// Eight consecutive expanded k values (group g of the slot) of the lane's row; `raw` is the slot's
+// tile, lane_addr the lane's precomputed address inside it.
+// Complex A expands to rows (2i, 2i+1) x columns (2l, 2l+1) = [[re, -im], [im, re]].
+template <int LAYOUT, int ROWS>
+__device__ __forceinline__ void load_raw8(uint32_t lane_addr, uint32_t g, const ConverterState &st,
+                                          float (&v)[8]) {
+  if constexpr (LAYOUT == kRawK) {
+    const float4 x = ld_shared_f4(lane_addr ^ ((2u * g) << 4));
+    const float4 y = ld_shared_f4(lane_addr ^ ((2u * g + 1u) << 4));
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+    v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+  } else if constexpr (LAYOUT == kRawR) {
+#pragma unroll
+    for (uint32_t e = 0; e < 8; ++e) v[e] = ld_shared_f1(lane_addr + (8u * g + e) * ROWS * 4u);
+  } else if constexpr (LAYOUT == kRawCplxBR) {
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) {
+      const float2 x = ld_shared_f2(lane_addr + (4u * g + e) * ROWS * 8u);
+      v[2 * e] = x.x;
+      v[2 * e + 1] = flip_sign(x.y, st.conj_mask);
+    }
+  } else {
+    float2 x[4];
+    if constexpr (LAYOUT == kRawCplxAR) {
+#pragma unroll
+      for (uint32_t e = 0; e < 4; ++e) x[e] = ld_shared_f2(lane_addr + (4u * g + e) * ROWS * 4u);
+    } else {
+#pragma unroll
+      for (uint32_t h = 0; h < 2; ++h) {
+        const float4 y = ld_shared_f4(lane_addr ^ ((2u * g + h) << 4));
+        x[2 * h] = make_float2(y.x, flip_sign(y.y, st.conj_mask));
+        x[2 * h + 1] = make_float2(y.z, flip_sign(y.w, st.conj_mask));
+      }
+    }
+    const bool im_row = (st.row & 1u) != 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      v[2 * e] = im_row ? x[e].y : x[e].x;
+      v[2 * e + 1] = im_row ? x[e].x : -x[e].y;
+    }
+  }
+}
+
+// Splits eight consecutive k values and stores them at 8-k group kc of the stage.
+template <int KIND>
+__device__ __forceinline__ void split_store8(const float (&v)[8], uint32_t lane_dst,
+                                             uint32_t lo_delta, uint32_t kc) {
+  if constexpr (KIND == 0) {
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) split2(v[2 * t], v[2 * t + 1], h[t], l[t]);
+    const uint32_t addr = lane_dst ^ (kc << 4);
+    st_shared_v4(addr, h[0], h[1], h[2], h[3]);
+    st_shared_v4(addr + lo_delta, l[0], l[1], l[2], l[3]);
+  } else {
+#pragma unroll
+    for (uint32_t g = 0; g < 2; ++g) {
+      uint32_t h[4], l[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) split_tf32(v[4 * g + t], h[t], l[t]);
+      const uint32_t addr = lane_dst ^ ((2u * kc + g) << 4);
+      st_shared_v4(addr, h[0], h[1], h[2], h[3]);
+      st_shared_v4(addr + lo_delta, l[0], l[1], l[2], l[3]);
+    }
+  }
+}
+
+template <int KIND, int BN, int LAYOUT, int ROWS, int JOBS>
+__device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterState &st) {
+  using Cfg = StreamCfg<BN>;
+  constexpr uint32_t SLOTS_PER_STAGE = (KIND == 0) ? 2 : 1;
+  const uint32_t r = st.row;
+  const int lane = static_cast<int>(threadIdx.x & 31);
+  uint32_t lane_raw;
+  if constexpr (LAYOUT == kRawK) lane_raw = st.raw + r * 128u + ((r & 7u) << 4);
+  else if constexpr (LAYOUT == kRawR) lane_raw = st.raw + r * 4u;
+  else if constexpr (LAYOUT == kRawCplxBR) lane_raw = st.raw + r * 8u;
+  else if constexpr (LAYOUT == kRawCplxAR) lane_raw = st.raw + (r >> 1) * 8u;
+  else lane_raw = st.raw + (r >> 1) * 128u + (((r >> 1) & 7u) << 4);
+  const uint32_t lane_dst = st.dst + r * 128u + ((r & 7u) << 4);
+  const bool scaled = st.scale != 1.f;
+  uint32_t rs = 0, rph = 0, s = 0, ph = 0;
+#pragma unroll 1
+  for (uint32_t i = 0; i < total_stages; ++i) {
+#pragma unroll 1
+    for (uint32_t half = 0; half < SLOTS_PER_STAGE; ++half) {
+      if (!ptx::mbar_wait_timed(ptx::smem_u32(&st.raw_full[rs]), rph, st.abort_flag, st.status,
+                                ptx::kErrWaitFull, st.timed, &st.wait_raw))
+        return;
+      if (half == 0) {
+        if (!ptx::mbar_wait_timed(ptx::smem_u32(&st.empty[s]), ph ^ 1u, st.abort_flag, st.status,
+                                  ptx::kErrWaitEmpty, st.timed, &st.wait_empty))
+          return;
+      }
+      // two groups at a time: enough independent arithmetic, and no spills at this register count
+      const uint32_t raw_addr = lane_raw + rs * Cfg::RAW_BYTES;
+      const uint32_t dst_addr = lane_dst + s * Cfg::STAGE_BYTES;
+#pragma unroll
+      for (int j = 0; j < JOBS; j += 2) {
+        float v[2][8];
+        load_raw8<LAYOUT, ROWS>(raw_addr, st.group0 + j, st, v[0]);
+        load_raw8<LAYOUT, ROWS>(raw_addr, st.group0 + j + 1, st, v[1]);
+        if (scaled) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            v[0][e] *= st.scale;
+            v[1][e] *= st.scale;
+          }
+        }
+        split_store8<KIND>(v[0], dst_addr, st.lo_delta, 4u * half + st.group0 + j);
+        split_store8<KIND>(v[1], dst_addr, st.lo_delta, 4u * half + st.group0 + j + 1);
+      }
+      // every value of the slot has been read: it may be refilled
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&st.raw_empty[rs]));
+      if (++rs == Cfg::RAW_SLOTS) {
+        rs = 0;
+        rph ^= 1u;
+      }
+    }
+    fence_proxy_async_shared();
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive_cluster(st.full_leader + 8u * s);
+    if (++s == Cfg::STAGES) {
+      s = 0;
+      ph ^= 1u;
+    }
+  }
+}
+
+template <int KIND, int BN>
+__device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUtensorMap &map_b,
+                                            const StreamParams &p) {
+  using Cfg = StreamCfg<BN>;
+  constexpr int STAGES = Cfg::STAGES, RAW_SLOTS = Cfg::RAW_SLOTS;
+  constexpr int K_STEPS = ROW_BYTES / 32;
+  constexpr uint32_t SLOTS_PER_STAGE = (KIND == 0) ? 2 : 1;
+  constexpr uint32_t STAGES_PER_UNIT = (KIND == 0) ? 1 : 2;
+  constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, 2 * BM_CTA, BN);
+  constexpr float LO_SCALE_INV = (KIND == 0) ? (1.f / 2048.f) : 1.f;
+  constexpr uint32_t D1_COL = BN;
+  constexpr int CPT = BN / 2; // accumulator columns per epilogue thread
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t *raw_smem = smem + STAGES * Cfg::STAGE_BYTES;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(raw_smem + RAW_SLOTS * Cfg::RAW_BYTES);
+  uint64_t *raw_full = bars;
+  uint64_t *raw_empty = raw_full + RAW_SLOTS;
+  uint64_t *full_bar = raw_empty + RAW_SLOTS;
+  uint64_t *empty_bar = full_bar + STAGES;
+  uint64_t *d0_full = empty_bar + STAGES;
+  uint64_t *d0_empty = d0_full + 1;
+  uint64_t *d1_full = d0_full + 2;
+  uint64_t *d1_empty = d0_full + 3;
+  uint64_t *tail_bar = d0_full + 4; // the eight epilogue warps of this CTA (ticket mode)
+  uint32_t *tmem_base_ptr = reinterpret_cast<uint32_t *>(d0_full + 5);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_base_ptr + 1);
+  volatile uint32_t *ticket_smem = reinterpret_cast<volatile uint32_t *>(tmem_base_ptr + 2);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = ptx::cluster_ctarank();
+  const bool leader = (rank == 0);
+  const uint32_t cluster_id = blockIdx.x >> 1;
+  const uint32_t num_clusters = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < RAW_SLOTS; ++s) {
+      ptx::mbar_init(ptx::smem_u32(&raw_full[s]), 1);
+      ptx::mbar_init(ptx::smem_u32(&raw_empty[s]), NUM_CVT_WARPS);
+    }
+    for (int s = 0; s < STAGES; ++s) {
+      ptx::mbar_init(ptx::smem_u32(&full_bar[s]), 2 * NUM_CVT_WARPS);
+      ptx::mbar_init(ptx::smem_u32(&empty_bar[s]), 1);
+    }
+    ptx::mbar_init(ptx::smem_u32(d0_full), 1);
+    ptx::mbar_init(ptx::smem_u32(d0_empty), 2 * NUM_EPI_WARPS);
+    ptx::mbar_init(ptx::smem_u32(d1_full), 1);
+    ptx::mbar_init(ptx::smem_u32(d1_empty), 2 * NUM_EPI_WARPS);
+    ptx::mbar_init(ptx::smem_u32(tail_bar), NUM_EPI_WARPS);
+    *abort_flag = 0;
+    ptx::mbar_init_fence();
+    ptx::prefetch_tensormap(&map_a);
+    ptx::prefetch_tensormap(&map_b);
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc_pair(ptx::smem_u32(tmem_base_ptr), Cfg::TMEM_COLS);
+    ptx::tmem_relinquish_pair();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  // both CTAs' barriers must exist before any remote arrive
+  ptx::cluster_arrive();
+  ptx::cluster_wait();
+  ptx::tc_fence_after();
+  const uint32_t tmem_base = *tmem_base_ptr;
+  // launched behind the previous kernel of the stream (programmatic serialization): from here
+  // on global memory is read and written
+  ptx::griddep_wait();
+  const bool dbg = (p.debug != nullptr);
+  unsigned long long dbg_wait = 0, dbg_wait2 = 0;
+
+  if (warp < FIRST_EPI_WARP) {
+    ptx::setmaxnreg_dec<REGS_REST>();
+    if (warp == 0) {
+      if (ptx::elect_one()) {
+        // ============================================================== TMA producer (both CTAs)
+        const bool a_k = p.layout_a == kRawK || p.layout_a == kRawCplxAK;
+        const bool a_cplx = p.layout_a == kRawCplxAR || p.layout_a == kRawCplxAK;
+        const bool b_k = p.layout_b == kRawK;
+        const bool b_cplx = p.layout_b == kRawCplxBR;
+        // coordinate steps per slot: x for K-contiguous operands, y for row-contiguous ones
+        const int a_dy = a_cplx ? SLOT_K / 2 : SLOT_K;
+        const int b_dy = b_cplx ? SLOT_K / 2 : SLOT_K;
+        const uint32_t bytes = (a_cplx ? Cfg::RAW_A / 2 : Cfg::RAW_A) +
+                               static_cast<uint32_t>(Cfg::B_ROWS * SLOT_K * 4);
+        uint32_t s = 0, ph = 0;
+        bool ok = true;
+        WorkList list(p, cluster_id, num_clusters);
+        WorkItem x;
+        while (ok && list.next(p, x)) {
+          const TileCoord tc = tile_coord<BN>(x.tile, p, rank);
+          const int b_row = tc.n0 + static_cast<int>(rank) * Cfg::B_ROWS;
+          const int t0 = static_cast<int>(2u * x.u0);
+          int ax = a_k ? t0 * SLOT_K : tc.m0;
+          int ay = a_k ? (a_cplx ? tc.m0 >> 1 : tc.m0) : t0 * a_dy;
+          int bx = b_k ? t0 * SLOT_K : (b_cplx ? 2 * b_row : b_row);
+          int by = b_k ? b_row : t0 * b_dy;
+          const int az = (p.flags & kBatchA) ? static_cast<int>(tc.batch) : 0;
+          const int bz = (p.flags & kBatchB) ? static_cast<int>(tc.batch) : 0;
+          for (uint32_t t = 0; t < 2u * x.un; ++t) {
+            ok = ptx::mbar_wait(ptx::smem_u32(&raw_empty[s]), ph ^ 1u, abort_flag, p.status,
+                                ptx::kErrWaitEmpty);
+            if (!ok) break;
+            const uint32_t fb = ptx::smem_u32(&raw_full[s]);
+            ptx::mbar_arrive_expect_tx(fb, bytes);
+            const uint32_t dst = ptx::smem_u32(raw_smem + s * Cfg::RAW_BYTES);
+            ptx::tma_load_3d(dst, &map_a, fb, ax, ay, az);
+            ptx::tma_load_3d(dst + Cfg::RAW_A, &map_b, fb, bx, by, bz);
+            if (a_k) ax += SLOT_K;
+            else ay += a_dy;
+            if (b_k) bx += SLOT_K;
+            else by += b_dy;
+            if (++s == RAW_SLOTS) {
+              s = 0;
+              ph ^= 1u;
+            }
+          }
+        }
+      }
+    } else if (warp == 1 && leader) {
+      if (ptx::elect_one()) {
+        // ============================================================== MMA issuer (leader only)
+        const uint32_t d0 = tmem_base, d1 = tmem_base + D1_COL;
+        constexpr uint16_t BOTH = 0x3;
+        const uint64_t desc0 = ptx::make_kmajor_desc<ROW_BYTES>(ptx::smem_u32(smem));
+        constexpr uint64_t kStage = Cfg::STAGE_BYTES >> 4;
+        constexpr uint64_t kALo = Cfg::A_TILE >> 4, kBHi = (2 * Cfg::A_TILE) >> 4,
+                           kBLo = (2 * Cfg::A_TILE + Cfg::B_TILE) >> 4;
+        uint32_t s = 0, ph = 0, d0_ph = 1, d1_ph = 1;
+        bool ok = true;
+        const long long dbg_t0 = clock64();
+        WorkList list(p, cluster_id, num_clusters);
+        WorkItem x;
+        while (ok && list.next(p, x)) {
+          const uint32_t kbn = x.un * STAGES_PER_UNIT;
+          for (uint32_t kb = 0; kb < kbn; ++kb) {
+            ok = ptx::mbar_wait_timed(ptx::smem_u32(&full_bar[s]), ph, abort_flag, p.status,
+                                      ptx::kErrWaitFull, dbg, &dbg_wait);
+            if (!ok) break;
+            ptx::tc_fence_after();
+            const uint64_t a_hi = desc0 + s * kStage;
+            const uint64_t a_lo = a_hi + kALo, b_hi = a_hi + kBHi, b_lo = a_hi + kBLo;
+            auto corrections = [&](uint32_t acc_first) {
+#pragma unroll
+              for (int ks = 0; ks < K_STEPS; ++ks)
+                mma_pair<KIND>(d1, a_lo + 2 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : acc_first);
+#pragma unroll
+              for (int ks = 0; ks < K_STEPS; ++ks)
+                mma_pair<KIND>(d1, a_hi + 2 * ks, b_lo + 2 * ks, IDESC, 1u);
+            };
+            // D0 is drained every stage.  The corrections come before the hi*hi products, so that
+            // the drain of the previous stage's D0 hides behind them; in the first stage of an
+            // item they come after, because they have to wait until the epilogue has given D1 back.
+            if (kb > 0) corrections(1u);
+            ok = ptx::mbar_wait_timed(ptx::smem_u32(d0_empty), d0_ph, abort_flag, p.status,
+                                      ptx::kErrWaitD0Empty, dbg, &dbg_wait2);
+            if (!ok) break;
+            d0_ph ^= 1u;
+            ptx::tc_fence_after();
+#pragma unroll
+            for (int ks = 0; ks < K_STEPS; ++ks)
+              mma_pair<KIND>(d0, a_hi + 2 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : 0u);
+            ptx::tc_commit_pair(ptx::smem_u32(d0_full), BOTH);
+            if (kb == 0) {
+              ok = ptx::mbar_wait_timed(ptx::smem_u32(d1_empty), d1_ph, abort_flag, p.status,
+                                        ptx::kErrWaitD1Empty, dbg, &dbg_wait2);
+              if (!ok) break;
+              d1_ph ^= 1u;
+              ptx::tc_fence_after();
+              corrections(0u);
+            }
+            ptx::tc_commit_pair(ptx::smem_u32(&empty_bar[s]), BOTH);
+            if (++s == STAGES) {
+              s = 0;
+              ph ^= 1u;
+            }
+          }
+          if (ok) ptx::tc_commit_pair(ptx::smem_u32(d1_full), BOTH);
+        }
+        if (dbg) {
+          atomicAdd(p.debug + 0, dbg_wait);
+          atomicAdd(p.debug + 1, dbg_wait2);
+          atomicAdd(p.debug + 4, static_cast<unsigned long long>(clock64() - dbg_t0));
+          atomicAdd(p.debug + 5, 1ull);
+        }
+      }
+    }
+  } else if (warp >= FIRST_CVT_WARP) {
+    // ================================================================ converters (both CTAs)
+    ptx::setmaxnreg_dec<REGS_CVT>();
+    // warps 0-3: the four 32-row blocks of A; warps 4-7: those of B (BN = 128: two warps to each
+    // of its two blocks, half of a slot's groups each)
+    constexpr int B_JOBS = (BN == 256) ? 4 : 2;
+    const uint32_t cw = static_cast<uint32_t>(warp - FIRST_CVT_WARP);
+    const bool for_a = cw < 4;
+    // the converters see a plain stream of stages; only its length depends on the work items
+    uint32_t total_stages = 0;
+    {
+      WorkList list(p, cluster_id, num_clusters);
+      WorkItem x;
+      while (list.next(p, x)) total_stages += x.un * STAGES_PER_UNIT;
+    }
+    ConverterState st;
+    st.raw_full = raw_full;
+    st.raw_empty = raw_empty;
+    st.empty = empty_bar;
+    st.full_leader = ptx::map_to_cta(ptx::smem_u32(full_bar), 0);
+    st.raw = ptx::smem_u32(raw_smem) + (for_a ? 0u : Cfg::RAW_A);
+    st.dst = ptx::smem_u32(smem) + (for_a ? 0u : 2u * Cfg::A_TILE);
+    st.lo_delta = for_a ? Cfg::A_TILE : Cfg::B_TILE;
+    st.row = (for_a ? cw : (BN == 256 ? cw - 4u : (cw - 4u) >> 1)) * 32u + lane;
+    st.group0 = (for_a || BN == 256) ? 0u : 2u * (cw & 1u);
+    st.scale = 1.f;
+    if (p.dyn != nullptr) st.scale = for_a ? p.dyn->scale_a : p.dyn->scale_b;
+    st.conj_mask = (p.flags & (for_a ? kConjA : kConjB)) ? 0x80000000u : 0u;
+    st.abort_flag = abort_flag;
+    st.status = p.status;
+    st.timed = dbg;
+    st.wait_raw = st.wait_empty = 0;
+    if (for_a) {
+      switch (p.layout_a) {
+      case kRawK:
+        convert_loop<KIND, BN, kRawK, BM_CTA, 4>(total_stages, st);
+        break;
+      case kRawR:
+        convert_loop<KIND, BN, kRawR, BM_CTA, 4>(total_stages, st);
+        break;
+      case kRawCplxAR:
+        convert_loop<KIND, BN, kRawCplxAR, BM_CTA, 4>(total_stages, st);
+        break;
+      default:
+        convert_loop<KIND, BN, kRawCplxAK, BM_CTA, 4>(total_stages, st);
+        break;
+      }
+    } else {
+      switch (p.layout_b) {
+      case kRawK:
+        convert_loop<KIND, BN, kRawK, Cfg::B_ROWS, B_JOBS>(total_stages, st);
+        break;
+      case kRawR:
+        convert_loop<KIND, BN, kRawR, Cfg::B_ROWS, B_JOBS>(total_stages, st);
+        break;
+      default:
+        convert_loop<KIND, BN, kRawCplxBR, Cfg::B_ROWS, B_JOBS>(total_stages, st);
+        break;
+      }
+    }
+    if (dbg && cw == 0 && lane == 0) {
+      atomicAdd(p.debug + 2, st.wait_raw);
+      atomicAdd(p.debug + 3, st.wait_empty);
+    }
+  } else {
+    // ================================================================ drain + epilogue (both CTAs)
+    ptx::setmaxnreg_inc<REGS_EPI>();
+    const uint32_t t_base = tmem_base + ((static_cast<uint32_t>(warp & 3) * 32u) << 16) +
+                            static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2) * CPT;
+    const uint32_t d0_empty_leader = ptx::map_to_cta(ptx::smem_u32(d0_empty), 0);
+
+    uint32_t d0_ph = 0, d1_ph = 0, tail_phase = 0;
+    bool ok = true;
+    WorkList list(p, cluster_id, num_clusters);
+    WorkItem x;
+    while (ok && list.next(p, x)) {
+      const uint32_t drains = x.un * STAGES_PER_UNIT;
+      const uint32_t prefetch_at = (p.beta_r == 0.f && p.beta_i == 0.f) ? drains
+                                   : (drains > C_PREFETCH_LEAD)         ? drains - C_PREFETCH_LEAD
+                                                                        : 0u;
+      float acc[CPT];
+#pragma unroll
+      for (int i = 0; i < CPT; ++i) acc[i] = 0.f;
+
+#pragma unroll 1
+      for (uint32_t c = 0; c < drains; ++c) {
+        if (c == prefetch_at) {
+          // beta != 0: pull this warp's part of the C tile into L2 before the epilogue reads it
+          const TileCoord tc = tile_coord<BN>(opaque(x.tile), p, rank);
+          const uint32_t row = static_cast<uint32_t>(tc.m0) + static_cast<uint32_t>(warp & 3) * 32u;
+          const float *cp = p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row;
+#pragma unroll 1
+          for (int q = 0; q < CPT / 32; ++q) {
+            const uint32_t col =
+                static_cast<uint32_t>(tc.n0) +
+                static_cast<uint32_t>(((warp - FIRST_EPI_WARP) >> 2) * CPT + q * 32 + lane);
+            if (col < p.n && row < p.m) ptx::prefetch_l2(cp + static_cast<uint64_t>(col) * p.ldc);
+          }
+        }
+        ok = ptx::mbar_wait(ptx::smem_u32(d0_full), d0_ph, abort_flag, p.status, ptx::kErrWaitD0Full);
+        if (!ok) break;
+        d0_ph ^= 1u;
+        ptx::tc_fence_after();
+        drain_sums<CPT>(t_base, acc);
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster(d0_empty_leader);
+      }
+      if (!ok) break;
+
+      ok = ptx::mbar_wait(ptx::smem_u32(d1_full), d1_ph, abort_flag, p.status, ptx::kErrWaitD1Full);
+      if (!ok) break;
+      d1_ph ^= 1u;
+      ptx::tc_fence_after();
+      const uint32_t t_sums = t_base + D1_COL;
+      if (BN == 128 && (p.flags & kDirectStores)) {
+        // Many short tiles per cluster, C not read: stores straight from the registers.  That is
+        // long code, but it stays in the instruction cache from tile to tile, and D1 goes back to
+        // the issuer before the stores instead of after them.
+#pragma unroll
+        for (int c = 0; c < CPT; c += 16) {
+          uint32_t v[16];
+          ptx::tmem_ld_32x32b_x16(t_sums + c, v);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            acc[c + i] = fmaf(__uint_as_float(v[i]), LO_SCALE_INV, acc[c + i]);
+        }
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0)
+          ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(d1_empty), 0));
+        const TileCoord tc = tile_coord<BN>(opaque(x.tile), p, rank);
+        const uint32_t row = static_cast<uint32_t>(tc.m0) + static_cast<uint32_t>(warp & 3) * 32u +
+                             static_cast<uint32_t>(lane);
+        const uint32_t col0 = static_cast<uint32_t>(tc.n0) +
+                              static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2) * CPT;
+        const float unscale = (p.dyn != nullptr) ? p.dyn->unscale_c : 1.f;
+        store_registers<CPT>(acc, p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row, p.ldc,
+                             col0, p.n, row < p.m, p.alpha_r * unscale, p.alpha_i * unscale);
+        continue;
+      }
+      // the finished sums stay in the D1 columns; from here on they are read from there, and what
+      // the epilogue needs to know of the tile is worked out only now (epilogue.cuh)
+      add_corrections_in_tmem<CPT>(t_sums, acc, LO_SCALE_INV);
+      const bool part = x.un != p.units; // this item is a piece of a tile
+      const TileCoord tc = tile_coord<BN>(opaque(x.tile), p, rank);
+      const uint32_t quarter = static_cast<uint32_t>(warp & 3);
+      const uint32_t col_base = static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2) * CPT;
+      const uint32_t row =
+          static_cast<uint32_t>(tc.m0) + quarter * 32u + static_cast<uint32_t>(lane);
+      float *cbase = p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row;
+      if (p.slices > 1) // reduce mode: slice index = position of the cluster within its tile
+        cbase += static_cast<uint64_t>(cluster_id % p.slices) * p.slice_stride;
+      const uint32_t d1_empty_leader = ptx::map_to_cta(ptx::smem_u32(d1_empty), 0);
+      auto release_d1 = [&]() {
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster(d1_empty_leader);
+      };
+
+      if (part && p.slices <= 1) {
+        // ticket mode: park the partial sums, take a ticket, and go on to the epilogue only with
+        // the last ticket of this CTA's half of the tile
+        constexpr uint32_t HALF = BN * BM_CTA; // floats of one CTA's half of a tile
+        const uint32_t lane_off = col_base * BM_CTA + quarter * 32u + static_cast<uint32_t>(lane);
+        float *mine = p.partial + static_cast<uint64_t>((cluster_id * 2u + x.slot) * 2u + rank) * HALF +
+                      lane_off;
+#pragma unroll 1
+        for (int c = 0; c < CPT; c += kEpiGroup) {
+          uint32_t v[kEpiGroup];
+          ptx::tmem_ld_32x32b_x16(t_sums + c, v);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < kEpiGroup; ++i)
+            __stcg(mine + (c + i) * BM_CTA, __uint_as_float(v[i]));
+        }
+        __threadfence();
+        // the eight epilogue warps meet twice: all partial sums stored; ticket published
+        auto meet = [&]() -> bool {
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(tail_bar));
+          const bool met = ptx::mbar_wait(ptx::smem_u32(tail_bar), tail_phase, abort_flag,
+                                          p.status, ptx::kErrWaitTail);
+          tail_phase ^= 1u;
+          return met;
+        };
+        ok = meet();
+        if (!ok) break;
+        // the clusters whose pieces make up this tile: those owning its first and last unit
+        const uint32_t ti = x.tile - p.whole_tiles;
+        const uint32_t total = (p.total_tiles - p.whole_tiles) * p.units;
+        const uint32_t pcs = p.piece_clusters;
+        const uint32_t ua = ti * p.units, ub = ua + p.units - 1u;
+        uint32_t c0 = static_cast<uint32_t>(static_cast<uint64_t>(ua) * pcs / total);
+        while (piece_start(c0 + 1u, total, pcs) <= ua) ++c0;
+        while (piece_start(c0, total, pcs) > ua) --c0;
+        uint32_t c1 = static_cast<uint32_t>(static_cast<uint64_t>(ub) * pcs / total);
+        while (piece_start(c1 + 1u, total, pcs) <= ub) ++c1;
+        while (piece_start(c1, total, pcs) > ub) --c1;
+        unsigned int *counter = p.counters + ti * 2u + rank;
+        if (warp == FIRST_EPI_WARP && lane == 0) {
+          const uint32_t t = atomicAdd(counter, 1u);
+          if (t == c1 - c0) *counter = 0; // all pieces are in: ready for the next launch
+          *ticket_smem = t;
+        }
+        ok = meet();
+        if (!ok) break;
+        if (*ticket_smem != c1 - c0) {
+          release_d1();
+          continue;
+        }
+        __threadfence();
+        // pieces in ascending k: the first is its cluster's second item unless that cluster's
+        // range begins with this tile; all others are their clusters' first items
+        const uint32_t slot0 = (piece_start(c0, total, pcs) < ua) ? 1u : 0u;
+        const float *src0 = p.partial + static_cast<uint64_t>((c0 * 2u + slot0) * 2u + rank) * HALF +
+                            lane_off;
+        const float *src1 = p.partial + static_cast<uint64_t>((c0 + 1u) * 4u + rank) * HALF + lane_off;
+#pragma unroll 1
+        for (int c = 0; c < CPT; c += kEpiGroup) {
+          float sum[kEpiGroup];
+#pragma unroll
+          for (int i = 0; i < kEpiGroup; ++i) sum[i] = __ldcg(src0 + (c + i) * BM_CTA);
+          const float *src = src1;
+          for (uint32_t cc = c0 + 1u; cc <= c1; ++cc, src += 4u * HALF) {
+#pragma unroll
+            for (int i = 0; i < kEpiGroup; ++i) sum[i] += __ldcg(src + (c + i) * BM_CTA);
+          }
+          uint32_t v[kEpiGroup];
+#pragma unroll
+          for (int i = 0; i < kEpiGroup; ++i) v[i] = __float_as_uint(sum[i]);
+          ptx::tmem_st_32x32b_x16(t_sums + c, v);
+        }
+        ptx::tmem_st_wait();
+      }
+
+      const float unscale = (p.dyn != nullptr && p.slices <= 1) ? p.dyn->unscale_c : 1.f;
+      store_tile<CPT>(t_sums, cbase, p.ldc, static_cast<uint32_t>(tc.n0) + col_base, p.n, row < p.m,
+                      p.alpha_r * unscale, p.alpha_i * unscale, p.beta_r, p.beta_i,
+                      (p.flags & kIsComplex) != 0);
+      release_d1();
+    }
+  }
+
+  // ---------------------------------------------------------------- teardown
+  // neither CTA leaves while the other still uses its shared memory or TMEM
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::cluster_arrive();
+  ptx::cluster_wait();
+  if (*abort_flag) {
+    // a wait gave up: let copies and tensor-core work still in flight land
+    const uint64_t t0 = ptx::globaltimer_ns();
+    while (ptx::globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
+  }
+}
+
+// KIND: 0 = FP16, 1 = TF32, 2 = decided on the device (AUTO)
+template <int KIND, int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
+    tcec_gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a,
+                            const __grid_constant__ CUtensorMap map_b, const StreamParams p) {
+  if constexpr (KIND == 2) {
+    ptx::griddep_wait(); // the decision is written by an earlier kernel of the call
+    if (p.dyn->gemm_mode == CUMPSGEMM_TF32TCEC)
+      stream_body<1, BN>(map_a, map_b, p);
+    else
+      stream_body<0, BN>(map_a, map_b, p);
+  } else {
+    stream_body<KIND, BN>(map_a, map_b, p);
+  }
+}
+
+// Per device and kernel, once: shared-memory attribute, register count, resident clusters.
+template <int KIND, int BN> cudaError_t stream_setup(int *clusters_out) {
+  static std::once_flag once[64];
+  static cudaError_t setup_error[64];
+  static int max_clusters[64];
+  auto kernel = tcec_gemm_stream_kernel<KIND, BN>;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  std::call_once(once[dev], [&]() {
+    constexpr int smem = StreamCfg<BN>::SMEM_BYTES;
+    setup_error[dev] =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // the register re-allocation inside the kernel draws on what the CTA was launched with: an
+    // increase that cannot be served would wait for ever, so refuse to launch with fewer
+    cudaFuncAttributes attr;
+    if (setup_error[dev] == cudaSuccess) {
+      setup_error[dev] = cudaFuncGetAttributes(&attr, kernel);
+      if (setup_error[dev] == cudaSuccess && attr.numRegs < LAUNCH_REGS)
+        setup_error[dev] = cudaErrorLaunchOutOfResources;
+    }
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int clusters = sms / 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(2 * clusters));
+    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    int active = 0;
+    if (setup_error[dev] == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&active, kernel, &cfg) == cudaSuccess) {
+      if (active > 0 && active < clusters) clusters = active;
+    } else {
+      cudaGetLastError();
+    }
+    max_clusters[dev] = clusters > 0 ? clusters : 1;
+  });
+  *clusters_out = max_clusters[dev];
+  return setup_error[dev];
+}
+
+// Tensor maps of the raw operands (see RawLayout).  Box: one slot of one CTA's rows.
+bool raw_map(CUtensorMap *map, const StreamOperand &o, int layout, uint64_t rows, uint64_t k,
+             uint32_t batch, uint32_t box_rows) {
+  // rows, k: extents of the expanded real operand
+  uint64_t d0, d1;
+  uint32_t b0, b1;
+  bool swizzle = false;
+  switch (layout) {
+  case kRawK:
+    d0 = k, d1 = rows, b0 = SLOT_K, b1 = box_rows, swizzle = true;
+    break;
+  case kRawR:
+    d0 = rows, d1 = k, b0 = box_rows, b1 = SLOT_K;
+    break;
+  case kRawCplxAR: // floats of a column = expanded rows
+    d0 = rows, d1 = k / 2, b0 = box_rows, b1 = SLOT_K / 2;
+    break;
+  case kRawCplxAK: // floats of a row = expanded k
+    d0 = k, d1 = rows / 2, b0 = SLOT_K, b1 = box_rows / 2, swizzle = true;
+    break;
+  default: // kRawCplxBR: two floats per row of B'
+    d0 = 2 * rows, d1 = k / 2, b0 = 2 * box_rows, b1 = SLOT_K / 2;
+    break;
+  }
+  const uint64_t nb = (o.stride != 0 && batch > 1) ? batch : 1;
+  const uint64_t ld_bytes = o.ld * sizeof(float);
+  const uint64_t stride_bytes = (nb > 1) ? o.stride * sizeof(float) : ld_bytes;
+  const uint64_t dims[3] = {d0, d1, nb};
+  const uint64_t strides[2] = {ld_bytes, stride_bytes};
+  const uint32_t box[3] = {b0, b1, 1};
+  return make_float_map(map, o.src, dims, strides, box, swizzle);
+}
+
+template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, cudaStream_t stream) {
+  int max_clusters = 1;
+  const cudaError_t se = stream_setup<KIND, BN>(&max_clusters);
+  if (se != cudaSuccess) return se;
+  CUtensorMap map_a, map_b;
+  if (!raw_map(&map_a, a.a, a.layout_a, a.m, a.k, a.batch, BM_CTA) ||
+      !raw_map(&map_b, a.b, a.layout_b, a.n, a.k, a.batch, BN / 2))
+    return cudaErrorNotSupported; // an extent TMA cannot address: the caller takes another path
+  StreamParams p;
+  p.c = a.c;
+  p.dyn = a.dyn;
+  p.status = a.dev_status;
+  p.partial = a.partial;
+  p.counters = a.counters;
+  p.debug = a.debug;
+  p.ldc = a.ldc;
+  p.stride_c = a.stride_c;
+  p.slice_stride = 0;
+  p.m = a.m;
+  p.n = a.n;
+  p.units = (a.k + 63) / 64;
+  p.tiles_m = (a.m + 2 * BM_CTA - 1) / (2 * BM_CTA);
+  p.tiles_n = (a.n + BN - 1) / BN;
+  p.total_tiles = p.tiles_m * p.tiles_n * a.batch;
+  p.alpha_r = a.alpha_r;
+  p.alpha_i = a.alpha_i;
+  p.beta_r = a.beta_r;
+  p.beta_i = a.beta_i;
+  p.layout_a = static_cast<uint8_t>(a.layout_a);
+  p.layout_b = static_cast<uint8_t>(a.layout_b);
+  p.flags = static_cast<uint8_t>((a.is_complex ? kIsComplex : 0) | (a.conj_a ? kConjA : 0) |
+                                 (a.conj_b ? kConjB : 0) |
+                                 (a.batch > 1 && a.a.stride != 0 ? kBatchA : 0) |
+                                 (a.batch > 1 && a.b.stride != 0 ? kBatchB : 0));
+  const StreamPlan &plan = a.plan;
+  if (plan.tile_n != BN || plan.total_tiles != p.total_tiles || plan.units != p.units)
+    return cudaErrorInvalidValue;
+  p.whole_tiles = plan.whole_tiles;
+  p.piece_clusters = static_cast<uint16_t>(plan.piece_clusters);
+  p.slices = static_cast<uint16_t>(plan.slices);
+  if (plan.slices > 1) {
+    p.c = a.partial;
+    p.ldc = a.m;
+    p.stride_c = static_cast<uint64_t>(a.m) * a.n;
+    p.slice_stride = p.stride_c * a.batch;
+    p.alpha_r = 1.f;
+    p.alpha_i = 0.f;
+    p.beta_r = 0.f;
+    p.beta_i = 0.f;
+    p.flags = static_cast<uint8_t>(p.flags & ~kIsComplex);
+  }
+  // direct stores: at least three waves of whole tiles of a short K loop, beta = 0 (with 256 columns
+  // the sums leave too few registers for it)
+  if (BN == 128 && plan.piece_clusters == 0 && plan.whole_tiles >= 3u * static_cast<uint32_t>(max_clusters) &&
+      p.units <= 16 && a.beta_r == 0.f && a.beta_i == 0.f)
+    p.flags |= kDirectStores;
+  uint32_t clusters = plan.whole_tiles > plan.piece_clusters ? plan.whole_tiles : plan.piece_clusters;
+  if (clusters > static_cast<uint32_t>(max_clusters)) clusters = static_cast<uint32_t>(max_clusters);
+  if (clusters == 0 || plan.piece_clusters > clusters) return cudaErrorInvalidValue;
+  return launch_chained(tcec_gemm_stream_kernel<KIND, BN>, 2 * clusters, NUM_THREADS,
+                        StreamCfg<BN>::SMEM_BYTES, stream, map_a, map_b, p);
+}
+
+template <int BN> cudaError_t launch_by_kind(const StreamGemmArgs &a, cudaStream_t stream) {
+  switch (a.kind) {
+  case StreamKind::fp16:
+    return launch_variant<0, BN>(a, stream);
+  case StreamKind::tf32:
+    return launch_variant<1, BN>(a, stream);
+  default:
+    return a.dyn != nullptr ? launch_variant<2, BN>(a, stream) : cudaErrorInvalidValue;
+  }
+}
+
+} // namespace
+
+// Left-over tiles (total mod clusters, or all of them when there are fewer tiles than clusters)
+// are cut along K where that saves more than it costs.
+StreamPlan plan_stream(const Tuning &tuning, int tile_n, uint64_t m, uint64_t n, uint64_t k,
+                       uint64_t batch, uint32_t clusters) {
+  StreamPlan pl = {};
+  pl.tile_n = tile_n;
+  const uint64_t total =
+      ((m + 2 * BM_CTA - 1) / (2 * BM_CTA)) * ((n + tile_n - 1) / tile_n) * batch;
+  const uint64_t units = (k + 63) / 64;
+  if (total == 0 || total > 0x3fffffffull || units == 0 || units > 0x3fffffull || clusters == 0)
+    return StreamPlan{};
+  pl.total_tiles = static_cast<uint32_t>(total);
+  pl.units = static_cast<uint32_t>(units);
+  pl.whole_tiles = pl.total_tiles;
+  const uint32_t rem = pl.total_tiles % clusters;
+  if (rem == 0 || 2 * rem > static_cast<uint32_t>(kStreamCounters)) return pl;
+  constexpr uint32_t kMinSliceUnits = 3;  // shortest slice / piece, in units of 64 k values
+  constexpr uint32_t kMinSavedUnits = 6;  // a cut has to save that much of a tile's K loop
+  if (3 * pl.total_tiles <= clusters && tuning.split_k != 0) {
+    // few tiles: slices and a reduction kernel
+    uint32_t s = clusters / pl.total_tiles;
+    if (s > pl.units / kMinSliceUnits) s = pl.units / kMinSliceUnits;
+    if (s >= 2 && pl.units - pl.units / s >= kMinSavedUnits) {
+      pl.whole_tiles = 0;
+      pl.slices = s;
+      pl.piece_clusters = s * pl.total_tiles;
+    }
+    return pl;
+  }
+  if (tuning.split_k == 0 || tuning.tail_split == 0) return pl;
+  const uint64_t left = static_cast<uint64_t>(rem) * pl.units;
+  uint32_t pc = clusters;
+  if (left / kMinSliceUnits < pc) pc = static_cast<uint32_t>(left / kMinSliceUnits);
+  // pieces of equal length that end where the tiles end need one ticket less per tile
+  if (pc > rem && pc < 2 * rem + rem / 4 && pc >= 2 * rem) pc = 2 * rem;
+  if (pc <= rem) return pl;
+  const uint32_t per = static_cast<uint32_t>((left + pc - 1) / pc);
+  if (per + kMinSavedUnits > pl.units) return pl;
+  pl.whole_tiles = pl.total_tiles - rem;
+  pl.piece_clusters = pc;
+  return pl;
+}
+
+std::size_t stream_scratch_bytes(const StreamPlan &plan, uint32_t m, uint32_t n, uint32_t batch) {
+  if (plan.slices > 1)
+    return static_cast<std::size_t>(plan.slices) * m * n * batch * sizeof(float);
+  return static_cast<std::size_t>(plan.piece_clusters) * 2u * 2u * BM_CTA *
+         static_cast<std::size_t>(plan.tile_n) * sizeof(float);
+}
+
+cudaError_t launch_tcec_gemm_stream(const StreamGemmArgs &a, cudaStream_t stream) {
+  if (a.plan.tile_n == 256) return launch_by_kind<256>(a, stream);
+  if (a.plan.tile_n == 128) return launch_by_kind<128>(a, stream);
+  return cudaErrorInvalidValue;
+}
+
+cudaError_t stream_max_clusters(int tile_n, int *clusters) {
+  return tile_n == 256 ? stream_setup<0, 256>(clusters) : stream_setup<0, 128>(clusters);
+}
+
+} // namespace cumpsgemm_b200
+
+extern "C" int cuMpSGEMM_plan_stream(uint64_t m, uint64_t n, uint64_t k, uint64_t batch, int tile_n,
+                                     unsigned clusters, unsigned *total_tiles, unsigned *units,
+                                     unsigned *whole_tiles, unsigned *piece_clusters,
+                                     unsigned *slices) {
+  using namespace cumpsgemm_b200;
+  if (m == 0 || n == 0 || k == 0 || batch == 0 || (tile_n != 256 && tile_n != 128) ||
+      clusters == 0 || total_tiles == nullptr || units == nullptr || whole_tiles == nullptr ||
+      piece_clusters == nullptr || slices == nullptr)
+    return 1;
+  const StreamPlan pl = plan_stream(Tuning{}, tile_n, m, n, k, batch, clusters);
+  if (pl.total_tiles == 0) return 1;
+  *total_tiles = pl.total_tiles;
+  *units = pl.units;
+  *whole_tiles = pl.whole_tiles;
+  *piece_clusters = pl.piece_clusters;
+  *slices = pl.slices;
+  return 0;
+}

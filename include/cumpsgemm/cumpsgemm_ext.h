@@ -148,7 +148,7 @@ void cuMpSGEMM_set_workspace_limit(cuMpSGEMM_handle_t handle, size_t bytes);
 void cuMpSGEMM_set_count_tail_padding(cuMpSGEMM_handle_t handle, int enable);
 /* A handle reads the tuning variables (CUMPSGEMM_TILE_N, CUMPSGEMM_PAIR, CUMPSGEMM_DRAIN_CHUNK,
  * CUMPSGEMM_FIRST_CHUNK, CUMPSGEMM_PACE, CUMPSGEMM_FUSED, CUMPSGEMM_SPLIT_K,
- * CUMPSGEMM_TAIL_SPLIT) once, when it is created, so that a GEMM call does not query the
+ * CUMPSGEMM_TAIL_SPLIT, CUMPSGEMM_STREAM) once, when it is created, so that a GEMM call does not query the
  * environment; this reads them again. */
 void cuMpSGEMM_reload_tuning_env(cuMpSGEMM_handle_t handle);
 /* Host-only query (no GPU needed): how the CTA-pair kernel would schedule `total_tiles` tiles
@@ -161,6 +161,16 @@ void cuMpSGEMM_reload_tuning_env(cuMpSGEMM_handle_t handle);
 int cuMpSGEMM_plan_pair_tail(unsigned total_tiles, unsigned clusters, unsigned k_pad, int tf32,
                              unsigned *split_begin, unsigned *slices, unsigned *slice_k,
                              unsigned *work_items);
+/* Host-only query (no GPU needed): how the kernel that splits its operands between TMA and the
+ * tensor core would deal an m x n x k x batch problem (sizes of the real, expanded problem) in
+ * 256 x tile_n pair tiles (tile_n 256 or 128) to `clusters` CTA pairs.  *units is the K loop in
+ * units of 64 values; tiles [0, *whole_tiles) of *total_tiles run whole; the k range of the
+ * others, laid end to end, is shared by *piece_clusters pairs, pair c taking units
+ * [c * u / p, (c + 1) * u / p) of the u units; *slices > 1: every tile is cut into that many and
+ * a second kernel adds them.  Returns 0, or 1 for invalid arguments. */
+int cuMpSGEMM_plan_stream(uint64_t m, uint64_t n, uint64_t k, uint64_t batch, int tile_n,
+                          unsigned clusters, unsigned *total_tiles, unsigned *units,
+                          unsigned *whole_tiles, unsigned *piece_clusters, unsigned *slices);
 /* Per-launch device timing with CUDA events on the handle's stream (off by default).  While
  * enabled every split + GEMM launch group records three events; get_kernel_timing
  * synchronises the stream, returns the number of launch groups since the last query and the
