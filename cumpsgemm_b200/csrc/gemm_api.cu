@@ -10,8 +10,10 @@
 // src/instance_sm80.cu) collapses to three tile widths because op N/T/C,
 // leading dimensions and edges are absorbed by the split pass.
 #include "gemm_common.cuh"
+#include "work_list.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 namespace cumpsgemm_b200 {
@@ -53,35 +55,98 @@ template <> struct Scalar<cuComplex> {
   static float im(const cuComplex *p) { return p->y; }
 };
 
-// Tile for a problem: width 256 / 128 / 64 of the single-CTA kernel (128 rows), or the CTA-pair
-// kernel's 256 x 256 tile (error-corrected modes only).  CUMPSGEMM_TILE_N forces the width,
-// CUMPSGEMM_PAIR=0/1 the kernel.  Measured on B200 (GEMM kernel only, us, FP16TCEC, beta=0.5,
-// 30 calls back to back):
-//   m=n=k   128x64   128x128   128x256   pairs 256x256
-//   1024     22.0     24.4      32.4       37.0      (16 pair tiles)
-//   1536     50.4     31.3      40.8       46.7      (36)
-//   2048    121       76.3      56.7       65.9      (64 pair tiles on 74 pair slots)
-//   3072      -      198       155        154        (144)
-//   4096      -      449       384        362        (256)
-// The pair kernel wins once there is more than one wave of pair tiles; below that the widest
-// single-CTA tile that still gives about two thirds of the SMs a tile is fastest: narrower
-// tiles move the same operand bytes for fewer MMAs.
+// ---------------------------------------------------------------- which kernel
+//
+// Estimated time of a call on each path, in microseconds.  A call is one or more waves of tiles,
+// each as long as its K loop; what the paths trade is idle SMs against operand traffic, the split
+// pass against converting every operand element once per tile that uses it, and cutting tiles
+// along K against adding the pieces.  The constants are least-squares fits to 104 problems of
+// 1-80 pair tiles and k = 128-8192 with every path forced in turn (B200, mean error 5-9 %);
+// taking the path with the smallest estimate was 0.5 % slower on average than the best path of
+// each problem, the fixed rule it replaces 7 %.  Examples, us per call (K slices of 128 x 256
+// tiles / 128 x 128 tiles / pairs in K pieces / streaming):
+//   2048 x 1024 x 2048     43 / 30 / 37 / 40        464 x 3256 x 7240      113 / 102 / 98 / 80
+//   1536 x 1536 x 4096     69 / 58 / 63 / 62        512 x 4096 x 4096       77 / 64 / 67 / 62
+//   complex 1280 x 960 x 1500  - / 75 / 65 / 70     TF32TCEC 4096 x 1024 x 2048  - / 104 / 95 / 82
+// A unit of 64 k values is one stage in FP16TCEC and two in TF32TCEC, for all paths alike.
+struct PathModel {
+  double units, stages, sms, pairs;
+  double split; // megabytes the split pass reads and writes
+  std::uint64_t m, n, batch;
+
+  static double waves(std::uint64_t tiles, double slots) { return std::ceil(tiles / slots); }
+  PathModel(unsigned num_sms, std::uint64_t m_, std::uint64_t n_, std::uint64_t k,
+            std::uint64_t batch_, bool tf32)
+      : units(static_cast<double>((k + 63) / 64)), stages(tf32 ? 2 * units : units), sms(num_sms),
+        pairs(num_sms / 2), m(m_), n(n_), batch(batch_) {
+    split = 1e-6 * static_cast<double>(m + n) * k * batch * (tf32 ? 12 : 8);
+  }
+  std::uint64_t tiles(std::uint64_t bm, std::uint64_t bn) const {
+    return ((m + bm - 1) / bm) * ((n + bn - 1) / bn) * batch;
+  }
+  // One CTA per 128 x bn tile.  A stage takes longer the more SMs compete for L2 (and power).
+  double single(int bn) const {
+    const std::uint64_t t = tiles(128, bn);
+    const double busy = std::min(1.0, t / sms);
+    const double w = waves(t, sms) * stages;
+    if (bn == 64) return 5.7 + 0.073 * split + w * (0.45 + 0.11 * busy);
+    if (bn == 128) return 6.1 + 0.100 * split + w * (0.53 + 0.15 * busy);
+    return 6.8 + 0.108 * split + w * (0.97 + 0.26 * busy);
+  }
+  double pair(const WorkPlan &w) const { // 256 x 256 tiles, left-over ones perhaps in K pieces
+    double length = waves(w.whole_tiles, pairs) * units, t = 8.8 + 0.169 * split;
+    if (w.piece_clusters > 0) {
+      const double left = w.total_tiles - w.whole_tiles;
+      length += w.slice_units != 0 ? w.slice_units : std::ceil(left * units / w.piece_clusters);
+      t += 4.0 + 0.06 * left;
+    }
+    return t + length * stages / units * (0.86 + 0.29 * std::min(1.0, w.total_tiles / pairs));
+  }
+  double split_k(std::uint32_t slices) const { // K slices of the widest tiles, then a reduction
+    return 2.0 + 0.15 * split + 1.32 * std::ceil(stages / slices) +
+           0.69e-6 * 4 * static_cast<double>(m) * n * batch * slices;
+  }
+  double stream(const StreamPlan &pl) const { // tcec_gemm_stream.cu
+    const bool tf32 = stages > units, wide = pl.tile_n == 256;
+    double length = waves(pl.whole_tiles, pairs) * units, t = tf32 ? 8.5 : 7.8;
+    if (pl.piece_clusters > 0) {
+      const double left = pl.total_tiles - pl.whole_tiles;
+      length += std::ceil(left * units / pl.piece_clusters);
+      t += (tf32 ? 4.9 : 2.9) + 0.19 * left;
+    }
+    return t + length * (tf32 ? (wide ? 2.33 : 1.85) : (wide ? 1.56 : 1.35));
+  }
+};
+
+// Tile of the pre-split path: width 256 / 128 / 64 of the single-CTA kernel (128 rows), or the
+// CTA-pair kernel's 256 x 256 tile (error-corrected modes only).  CUMPSGEMM_TILE_N forces the
+// width, CUMPSGEMM_PAIR=0/1 the kernel.
 } // namespace
 
 TileChoice pick_tile(const Tuning &tuning, unsigned num_sms, std::uint64_t m_exp, std::uint64_t n,
-                     std::uint64_t batch, bool ec) {
+                     std::uint64_t k_exp, std::uint64_t batch, bool ec, bool tf32, bool can_cut) {
   const bool pair_off = tuning.pair == 0;
-  const bool pair_on = tuning.pair == 1;
-  if (tuning.tile_n == 256) return {256, ec && !pair_off};
-  if (tuning.tile_n == 128 || tuning.tile_n == 64) return {tuning.tile_n, false};
-  const std::uint64_t sms = static_cast<std::uint64_t>(num_sms);
-  const std::uint64_t pair_tiles = ((m_exp + 255) / 256) * ((n + 255) / 256) * batch;
-  const std::uint64_t tiles_256 = ((m_exp + 127) / 128) * ((n + 255) / 256) * batch;
-  const std::uint64_t tiles_128 = ((m_exp + 127) / 128) * ((n + 127) / 128) * batch;
-  if (ec && !pair_off && (pair_on || pair_tiles > sms / 2)) return {256, true};
-  if (3 * tiles_256 >= 2 * sms) return {256, false};
-  if (3 * tiles_128 >= 2 * sms) return {128, false};
-  return {64, false};
+  if (tuning.tile_n == 256) return {256, ec && !pair_off, 0.0};
+  if (tuning.tile_n == 128 || tuning.tile_n == 64) return {tuning.tile_n, false, 0.0};
+  const PathModel model(num_sms, m_exp, n, k_exp, batch, tf32);
+  if (!ec) { // a third of the products: the widest tile that gives two thirds of the SMs one
+    const std::uint64_t sms = num_sms;
+    if (3 * model.tiles(128, 256) >= 2 * sms) return {256, false, 0.0};
+    return {3 * model.tiles(128, 128) >= 2 * sms ? 128 : 64, false, 0.0};
+  }
+  TileChoice best = {64, false, model.single(64)};
+  for (int bn : {128, 256})
+    if (const double t = model.single(bn); t < best.us) best = {bn, false, t};
+  const std::uint64_t pair_tiles = model.tiles(256, 256);
+  if (!pair_off && num_sms >= 2 && pair_tiles <= 0x7fffffffull) {
+    // (more than one wave of pair tiles: always pairs, 4096^3 277 us against 338 for 128 x 256
+    // tiles, GEMM kernel; the model is fitted to less)
+    const WorkPlan w = plan_pair(tuning, tf32, can_cut, static_cast<std::uint32_t>(pair_tiles),
+                                 static_cast<std::uint32_t>(model.units), num_sms / 2);
+    const double t = model.pair(w);
+    if (tuning.pair == 1 || pair_tiles > num_sms / 2 || t < best.us) best = {256, true, t};
+  }
+  return best;
 }
 
 namespace {
@@ -168,29 +233,18 @@ bool fused_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperati
   return true;
 }
 
-// Where the streaming kernel (tcec_gemm_stream.cu) is the faster path.  It saves the split pass,
-// its workspace traffic and a launch, and pays with about 2,450 cycles per 64 k values of a
-// 256 x 256 pair tile where the pre-split pair kernel takes 1,600, and with a longer start-up.
-// Measured (B200, us per call, paths that applied before / this kernel with the width chosen here):
-//   strided batches of small matrices, FP16TCEC          TF32TCEC
-//     64 x 256^3          23.9 / 18.1                      512 x 256^3           262 / 104
-//     512 x 256^3          123 / 80                        2048 x 128^3          460 / 154
-//     64 x 512^3           114 / 68                        16 x 1024^3           219 / 161
-//     16 x 1024^3          126 / 112                       128 x complex 256^3   191 / 94
-//     512 x complex 128^3   83 / 50 (128 wide)
-//     512 x 512 x 64 x 512 130 / 78 (128 wide)
-//     32 x 1024 x 1024 x 64 43 / 43, and a lone 4096 x 4096 x 512 55 / 64: where every operand element
-//     is used by many tiles the pre-split panels win, hence the limit on m and n.
-//   few tiles, long K (slices)
-//     256 x 256 x 65536     67 / 45      512 x 512 x 16384  48 / 37      4096 x 128 x 4096  42 / 33
-//     256 x 1024 x 8192     31 / 27      384 x 384 x 8192 25 / 25        512 x 512 x 4096   19 / 20
-//     256 x 256 x 4096      15 / 17
-bool stream_pays(const StreamPlan &plan, std::uint64_t m_exp, std::uint64_t n, std::uint64_t batch,
-                 int clusters) {
-  const std::uint64_t tiles = plan.total_tiles;
-  if (plan.slices > 1) return plan.units >= 256 || tiles * plan.units >= 512;
+// Batches of small matrices take the streaming kernel (tcec_gemm_stream.cu): the split pass and its
+// workspace traffic weigh as much as the products there.  Measured (B200, us per call, paths that
+// applied before / this kernel with the width chosen here):
+//   FP16TCEC   64 x 256^3 23.9 / 18.1      512 x 256^3 123 / 80        64 x 512^3 114 / 68
+//              16 x 1024^3 126 / 112       512 x complex 128^3 83 / 50 (128 wide)
+//              32 x 1024 x 1024 x 64 43 / 43
+//   TF32TCEC   512 x 256^3 262 / 104       2048 x 128^3 460 / 154      16 x 1024^3 219 / 161
+//              128 x complex 256^3 191 / 94
+bool small_matrix_batch(const StreamPlan &plan, std::uint64_t m_exp, std::uint64_t n,
+                        std::uint64_t batch, int clusters) {
   return batch >= 8 && m_exp <= 1024 && n <= 1024 &&
-         2 * tiles >= static_cast<std::uint64_t>(clusters);
+         2ull * plan.total_tiles >= static_cast<std::uint64_t>(clusters);
 }
 
 // Operands of a call for the streaming pair kernel (tcec_gemm_stream.cu).  TMA reads them in
@@ -200,7 +254,7 @@ template <class T>
 bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperation_t op_B,
                  std::uint64_t m, std::uint64_t n, std::uint64_t k, const T *a, std::uint64_t lda,
                  std::uint64_t stridea, const T *b, std::uint64_t ldb, std::uint64_t strideb,
-                 std::uint64_t batch, StreamKind kind, StreamGemmArgs *out) {
+                 std::uint64_t batch, StreamKind kind, double presplit_us, StreamGemmArgs *out) {
   constexpr bool is_complex = std::is_same<T, cuComplex>::value;
   constexpr std::uint64_t fpe = is_complex ? 2 : 1;
   const Tuning &t = h->tuning;
@@ -224,7 +278,19 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
   const StreamPlan plan = plan_stream(t, tile_n, m_exp, n, k_exp, batch,
                                       static_cast<std::uint32_t>(clusters));
   if (plan.total_tiles == 0) return false;
-  if (t.stream == -1 && !stream_pays(plan, m_exp, n, batch, clusters)) return false;
+  if (t.stream == -1 && !small_matrix_batch(plan, m_exp, n, batch, clusters)) {
+    // beyond one and a half waves the operands are reused by too many tiles to convert them again
+    // for each (4096^3 TF32TCEC: 600 us against 560), and the model is not fitted to it
+    if (2ull * plan.total_tiles > 3ull * static_cast<std::uint64_t>(clusters)) return false;
+    // (the kind of an AUTO call is not known here: the mean of both)
+    double us = 0.0;
+    if (kind != StreamKind::tf32)
+      us += PathModel(h->num_sms, m_exp, n, k_exp, batch, false).stream(plan);
+    if (kind != StreamKind::fp16)
+      us += PathModel(h->num_sms, m_exp, n, k_exp, batch, true).stream(plan);
+    if (kind == StreamKind::device) us *= 0.5;
+    if (us >= presplit_us) return false;
+  }
   *out = StreamGemmArgs{};
   out->kind = kind;
   out->a = StreamOperand{reinterpret_cast<const float *>(a), lda * fpe, sa};
@@ -246,6 +312,50 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
   out->plan = plan;
   return true;
 }
+
+// Tile or K slices of the pre-split path.
+struct PresplitChoice {
+  TileChoice tile;
+  std::uint32_t k_slices; // > 1: K slices of single-CTA tiles, added by a second kernel
+  double us;
+};
+PresplitChoice choose_presplit(const cuMpSGEMM_handle *h, std::uint64_t m_exp, std::uint64_t n,
+                               std::uint64_t k_exp, std::uint64_t batch, bool ec, bool tf32,
+                               bool can_slice) {
+  const Tuning &t = h->tuning;
+  PresplitChoice c;
+  c.tile = pick_tile(t, h->num_sms, m_exp, n, k_exp, batch, ec, tf32, true);
+  c.k_slices = 1;
+  c.us = c.tile.us;
+  // Few tiles and a long K loop (the shapes the reference hands to its atomic split-K kernel,
+  // src/cumpsgemm.cu:272-304): cut K into slices, one CTA each, so that the tiles fill the
+  // GPU; the slices' partial sums are added in a fixed order by a second kernel.  The widest
+  // tile the problem fills is taken (fewest operand bytes per product), and each slice keeps
+  // at least 256 k values.
+  const std::uint32_t k_pad64 = static_cast<std::uint32_t>(round_up(k_exp, 64));
+  const int wide = t.tile_n != 0 ? t.tile_n : (n > 128) ? 256 : (n > 64 ? 128 : 64);
+  const std::uint64_t tiles = ((m_exp + 127) / 128) * ((n + wide - 1) / wide) * batch;
+  const bool forced = t.split_k > 1;
+  if (can_slice && t.split_k != 0 && t.pair != 1 &&
+      (forced || (k_pad64 >= 2048 && 2 * tiles <= h->num_sms))) {
+    std::uint32_t wanted = static_cast<std::uint32_t>(h->num_sms / tiles);
+    wanted = std::min<std::uint32_t>(wanted, k_pad64 / 256);
+    if (forced) wanted = static_cast<std::uint32_t>(t.split_k);
+    const std::uint32_t slices = split_k_slices(k_pad64, wanted);
+    const double us = slices > 1 ? PathModel(h->num_sms, m_exp, n, k_exp, batch, tf32)
+                                       .split_k(slices)
+                                 : 0.0;
+    if (slices > 1 && (forced || !ec || t.tile_n != 0 || us < c.us)) {
+      c.k_slices = slices;
+      c.tile = TileChoice{wide, false, us};
+      c.us = us;
+    }
+  }
+  return c;
+}
+
+// The reference's module ids name tile classes.
+inline unsigned tile_class(int tile_n) { return (tile_n == 256) ? 0u : (tile_n == 128) ? 1u : 2u; }
 
 } // namespace
 
@@ -311,11 +421,16 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
   const std::uint64_t m_exp = m * fpe; // rows of the expanded real problem
   const std::uint64_t k_exp = k * fpe;
 
+  // ---- the pre-split path's tile or K slices, and what it would take
+  const bool auto_kind = want_fp16 && want_tf32;
+  const StreamKind stream_kind = auto_kind ? StreamKind::device
+                                 : want_fp16 ? StreamKind::fp16 : StreamKind::tf32;
+  PresplitChoice pre = choose_presplit(h, m_exp, n, k_exp, batch, ec, want_tf32, !ptr_arrays);
+  if (auto_kind)
+    pre.us = 0.5 * (pre.us + choose_presplit(h, m_exp, n, k_exp, batch, ec, false, !ptr_arrays).us);
+
   // ---- one launch on CTA pairs, operands split between TMA and the tensor core
   StreamGemmArgs ga;
-  const StreamKind stream_kind = (want_fp16 && want_tf32) ? StreamKind::device
-                                 : want_fp16              ? StreamKind::fp16
-                                                          : StreamKind::tf32;
   // (batches of matrices with at most 128 rows would leave one CTA of every pair idle: the kernel
   // below serves those it can, 2048 x 128^3 82 us against 95-110 here)
   FusedGemmArgs fa;
@@ -324,10 +439,10 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
                                    &fa);
   if (ec && !ptr_arrays && !(fused && batch >= 8 && m_exp <= 128 && h->tuning.stream == -1) &&
       stream_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, stream_kind,
-                     &ga)) {
+                     pre.us, &ga)) {
     bool room = true;
     if (ga.plan.piece_clusters > 0) {
-      const std::size_t bytes = stream_scratch_bytes(ga.plan, ga.m, ga.n, ga.batch);
+      const std::size_t bytes = stream_scratch_bytes(ga.plan);
       const std::size_t limit =
           h->workspace_limit_bytes ? h->workspace_limit_bytes : kDefaultWorkspaceLimit;
       room = bytes <= limit && ensure_workspace(h, bytes);
@@ -344,10 +459,8 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
       ga.dev_status = h->dev_status;
       ga.debug = h->debug_buffer;
       ga.partial = reinterpret_cast<float *>(h->workspace);
-      ga.counters = reinterpret_cast<unsigned int *>(h->dev_status + 2 + kPairTailCounters);
       if (used_kernel_module_id != nullptr) {
-        const int tn = pick_tile(h->tuning, h->num_sms, m_exp, n, batch, true).tile_n;
-        *used_kernel_module_id = (ga.plan.slices > 1) ? 100u : (tn == 256) ? 0u : (tn == 128) ? 1u : 2u;
+        *used_kernel_module_id = (ga.plan.slices > 1) ? 100u : tile_class(pre.tile.tile_n);
       }
       const bool prof = h->exp_stats.profiling_enabled;
       if (prof) h->exp_stats.profiler.start("gemm_kernel", h->cuda_stream);
@@ -359,24 +472,6 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
       }
       cudaError_t gerr = launch_tcec_gemm_stream(ga, h->cuda_stream);
       const bool addressable = gerr != cudaErrorNotSupported;
-      if (gerr == cudaSuccess && ga.plan.slices > 1) {
-        TcecGemmArgs r = {};
-        r.m = ga.m;
-        r.n = ga.n;
-        r.batch = ga.batch;
-        r.c = ga.c;
-        r.ldc = ga.ldc;
-        r.stride_c = ga.stride_c;
-        r.alpha_r = ga.alpha_r;
-        r.alpha_i = ga.alpha_i;
-        r.beta_r = ga.beta_r;
-        r.beta_i = ga.beta_i;
-        r.is_complex = ga.is_complex;
-        r.dyn = ga.dyn;
-        r.k_slices = ga.plan.slices;
-        r.partial = ga.partial;
-        gerr = launch_splitk_reduce(r, h->cuda_stream);
-      }
       if (h->kernel_timing) {
         cudaEventRecord(tt.e[2], h->cuda_stream);
         h->timing_events.push_back(tt);
@@ -454,34 +549,12 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
     return CUBLAS_STATUS_SUCCESS;
   }
 
-  TileChoice choice = pick_tile(h->tuning, h->num_sms, m_exp, n, batch, ec);
-  // Few tiles and a long K loop (the shapes the reference hands to its atomic split-K kernel,
-  // src/cumpsgemm.cu:272-304): cut K into slices, one CTA each, so that the tiles fill the
-  // GPU; the slices' partial sums are added in a fixed order by a second kernel.  The widest
-  // tile the problem fills is taken (fewest operand bytes per product), and each slice keeps
-  // at least 256 k values.
-  std::uint32_t k_slices = 1;
-  {
-    const std::uint32_t k_pad64 = static_cast<std::uint32_t>(round_up(k_exp, 64));
-    int wide = (n > 128) ? 256 : (n > 64 ? 128 : 64);
-    if (h->tuning.tile_n != 0) wide = h->tuning.tile_n;
-    const std::uint64_t tiles = ((m_exp + 127) / 128) * ((n + wide - 1) / wide) * batch;
-    const bool forced = h->tuning.split_k > 1;
-    if (!ptr_arrays && h->tuning.split_k != 0 && h->tuning.pair != 1 &&
-        (forced || (k_pad64 >= 2048 && 2 * tiles <= h->num_sms))) {
-      std::uint32_t wanted = static_cast<std::uint32_t>(h->num_sms / tiles);
-      wanted = std::min<std::uint32_t>(wanted, k_pad64 / 256);
-      if (forced) wanted = static_cast<std::uint32_t>(h->tuning.split_k);
-      k_slices = split_k_slices(k_pad64, wanted);
-      if (k_slices > 1) choice = TileChoice{wide, false};
-    }
-  }
-  const int tile_n = choice.tile_n;
-  const bool use_pair = choice.pair;
+  const std::uint32_t k_slices = pre.k_slices;
+  const int tile_n = pre.tile.tile_n;
+  const bool use_pair = pre.tile.pair;
   // tile class, or 100 for the split-K path as in the reference (src/cumpsgemm.cu:283-285)
   if (used_kernel_module_id != nullptr)
-    *used_kernel_module_id =
-        (k_slices > 1) ? 100u : (tile_n == 256) ? 0u : (tile_n == 128 ? 1u : 2u);
+    *used_kernel_module_id = (k_slices > 1) ? 100u : tile_class(tile_n);
 
   const std::uint32_t rows_pad_a =
       static_cast<std::uint32_t>(round_up(m_exp, use_pair ? 256 : 128));
@@ -517,7 +590,6 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
     const std::uint32_t nb = static_cast<std::uint32_t>(std::min<std::uint64_t>(chunk, batch - b0));
     // AUTO: one split launch and one GEMM launch whose kernels read the device-side decision
     // and run the FP16 or the TF32 pipeline; every other mode: the one kind it names.
-    const bool auto_kind = want_fp16 && want_tf32;
     const SplitKind kind = want_fp16 ? SplitKind::fp16 : SplitKind::tf32;
     SplitArgs sa;
     sa.kind = kind;
@@ -537,6 +609,7 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
     sa.k_pad = k_pad;
     sa.with_lo = ec;
     sa.dyn = dyn;
+    if (use_pair) sa.zero_word = reinterpret_cast<unsigned int *>(h->dev_status + 1);
     cuMpSGEMM_handle::TimingTriple tt{};
     if (h->kernel_timing) {
       for (auto &e : tt.e) cudaEventCreate(&e);

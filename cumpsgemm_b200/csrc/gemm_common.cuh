@@ -60,6 +60,25 @@ bool make_panel_map(CUtensorMap *map, SplitKind kind, const void *panel, uint32_
 bool make_float_map(CUtensorMap *map, const float *base, const uint64_t (&dims)[3],
                     const uint64_t (&strides)[2], const uint32_t (&box)[3], bool swizzle);
 
+// How the pair kernel deals `total_tiles` tiles with `units` x 64 k values to at most
+// `max_clusters` CTA pairs (tcec_gemm_pair.cu).
+struct WorkPlan;
+WorkPlan plan_pair(const Tuning &tuning, bool tf32, bool can_cut, uint32_t total_tiles,
+                   uint32_t units, uint32_t max_clusters);
+
+// Sum and epilogue of the tiles a launch cut along K (piece_fixup.cu).
+struct PieceFixupArgs {
+  const float *partial;
+  float *c;
+  float *const *c_array;
+  const DynParams *dyn;
+  uint64_t ldc, stride_c;
+  uint32_t m, n, tiles_m, tiles_n, tile_n;
+  float alpha_r, alpha_i, beta_r, beta_i;
+  bool is_complex;
+};
+cudaError_t launch_piece_fixup(const PieceFixupArgs &a, const WorkPlan &w, cudaStream_t stream);
+
 // CTA-pair kernel (tcec_gemm_pair.cu): 256 x 256 tile per cluster of two CTAs.
 cudaError_t launch_tcec_gemm_pair(const TcecGemmArgs &a, cudaStream_t stream);
 cudaError_t launch_tcec_gemm_pair_auto(const TcecGemmArgs &a, cudaStream_t stream);

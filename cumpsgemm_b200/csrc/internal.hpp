@@ -146,9 +146,7 @@ struct cuMpSGEMM_handle {
   cumpsgemm_b200::Tuning tuning;
 
   // Device status word the GEMM kernel writes when a bounded wait gives up.
-  // [0] kernel status word, [1] wave counter of the pair kernel, [2 ...] its tail-split counters,
-  // then the counters of the streaming kernel
-  int *dev_status = nullptr;
+  int *dev_status = nullptr; // [0] kernel status word, [1] wave counter of the pair kernel
 
   // Optional per-launch timing: events recorded on the launching stream before the split
   // pass, between split pass and GEMM kernel, and after the GEMM kernel.
@@ -229,6 +227,8 @@ struct SplitArgs {
   std::uint32_t k_pad;     // padded expanded K (multiple of 64)
   bool with_lo;            // also write the lo panel
   const DynParams *dyn;    // nullable: scale factor and gating
+  // device word the pass sets to zero for the kernel behind it (taken from the first operand)
+  unsigned int *zero_word = nullptr;
 };
 // Splits op(A) and op(B) of one GEMM in a single launch.
 cudaError_t launch_split_pair(const SplitArgs &a, const SplitArgs &b, cudaStream_t stream);
@@ -286,8 +286,8 @@ struct TcecGemmArgs {
   int tile_n;           // 256, 128 or 64
   int *dev_status;
   unsigned long long *debug = nullptr; // optional stall breakdown buffer (8 x u64)
-  // Optional device word the persistent pair kernel uses to keep its clusters in step
-  // (zeroed by the launcher before every launch); null switches the pacing off.
+  // Optional device word the persistent pair kernel uses to keep its clusters in step (zero at
+  // launch: the split pass zeroes it); null switches the pacing off.
   unsigned int *wave_counter = nullptr;
   Tuning tuning;
   // Split-K (single-CTA kernel only): k_slices > 1 cuts the K loop into that many CTAs per tile,
@@ -296,16 +296,13 @@ struct TcecGemmArgs {
   // slice the same whole number of 64-k-value units (0 or 1: no split).
   std::uint32_t k_slices = 1;
   float *partial = nullptr;
-  // Pair kernel only: scratch for the K-split of the last, partly filled wave of tiles
-  // (pair_tail_scratch_bytes() bytes) and kPairTailCounters zeroed device words behind
-  // `wave_counter`; null switches the tail split off.
+  // Pair kernel only: scratch for the K pieces of the last, partly filled wave of tiles
+  // (pair_tail_scratch_bytes() bytes); null switches the cutting off.
   float *tail_partial = nullptr;
 };
-// Device words the pair kernel's tail split needs behind the wave counter (two per tail tile).
-constexpr int kPairTailCounters = 256;
-// Bytes of `tail_partial` on a device with num_sms SMs: one 256 x 256 FP32 tile per CTA pair.
+// Bytes of `tail_partial` on a device with num_sms SMs: two 256 x 256 FP32 tiles per CTA pair.
 inline std::size_t pair_tail_scratch_bytes(int num_sms) {
-  return static_cast<std::size_t>(num_sms / 2) * 256u * 256u * sizeof(float);
+  return static_cast<std::size_t>(num_sms / 2) * 2u * 256u * 256u * sizeof(float);
 }
 // Slices actually used when `wanted` are asked for a K loop of k_pad values.
 std::uint32_t split_k_slices(std::uint32_t k_pad, std::uint32_t wanted);
@@ -357,7 +354,7 @@ struct StreamPlan {
   std::uint32_t units;           // K loop in units of 64 k values
   std::uint32_t whole_tiles;     // dealt whole, in waves
   std::uint32_t piece_clusters;  // clusters sharing the k range of the other tiles (0: none)
-  std::uint32_t slices;          // > 1: every tile in that many slices plus a reduction kernel
+  std::uint32_t slices;          // > 1: every tile in that many pieces of its own
 };
 StreamPlan plan_stream(const Tuning &tuning, int tile_n, std::uint64_t m, std::uint64_t n,
                        std::uint64_t k, std::uint64_t batch, std::uint32_t clusters);
@@ -374,13 +371,9 @@ struct StreamGemmArgs {
   int *dev_status;
   unsigned long long *debug;
   StreamPlan plan;
-  float *partial;         // stream_scratch_bytes() bytes when the plan cuts tiles along K
-  unsigned int *counters; // kStreamCounters words, zero (the kernel leaves them at zero)
+  float *partial; // stream_scratch_bytes() bytes when the plan cuts tiles along K
 };
-constexpr int kStreamCounters = 512; // two per tile that is cut in pieces
-constexpr int kStatusWords = 2 + kPairTailCounters + kStreamCounters; // of handle::dev_status
-std::size_t stream_scratch_bytes(const StreamPlan &plan, std::uint32_t m, std::uint32_t n,
-                                 std::uint32_t batch);
+std::size_t stream_scratch_bytes(const StreamPlan &plan);
 cudaError_t stream_max_clusters(int tile_n, int *clusters); // of the current device
 cudaError_t launch_tcec_gemm_stream(const StreamGemmArgs &a, cudaStream_t stream);
 // Self-test of the bounded mbarrier wait (see cuMpSGEMM_selftest_bounded_wait).
@@ -437,15 +430,18 @@ cublasStatus_t tiny_gemm(cuMpSGEMM_handle *h, bool long_is_m, cublasOperation_t 
                          std::uint64_t stride_c, std::uint64_t batch);
 
 // ---------------------------------------------------------------- GEMM dispatch
-// Tile for a problem: width 256 / 128 / 64 of the single-CTA kernel (128 rows), or the CTA-pair
-// kernel's 256 x 256 tile (error-corrected modes only).  m_exp = rows of the real problem
-// (twice m for complex).  The one rule every entry point uses.
+// Tile of the pre-split path: width 256 / 128 / 64 of the single-CTA kernel (128 rows), or the
+// CTA-pair kernel's 256 x 256 tile (error-corrected modes only), and its estimated time.  Sizes
+// are those of the real problem (complex operands expanded).  The one rule every entry point
+// uses.  can_cut: the caller has scratch memory for K pieces of pair tiles.
 struct TileChoice {
   int tile_n;
   bool pair;
+  double us;
 };
 TileChoice pick_tile(const Tuning &tuning, unsigned num_sms, std::uint64_t m_exp, std::uint64_t n,
-                     std::uint64_t batch, bool error_correction);
+                     std::uint64_t k_exp, std::uint64_t batch, bool error_correction, bool tf32,
+                     bool can_cut);
 
 // Shared implementation behind gemm<T> / gemm_stridedBatch<T>.
 // `dyn` != nullptr selects the fused scaling path (scale in the split pass,

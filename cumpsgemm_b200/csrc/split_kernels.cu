@@ -356,13 +356,21 @@ struct SplitJob {
   uint32_t gx, gy, gz;
 };
 
+// The wave counter of the pair kernel behind the split pass starts from zero: written here it
+// costs nothing, where a memset between the two kernels would cost a launch and keep them from
+// being chained (4 us a call).
+__device__ __forceinline__ void zero_word(unsigned int *z) {
+  if (z != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *z = 0u;
+}
+
 template <int KIND, bool VEC>
-__global__ void __launch_bounds__(THREADS, VEC ? 5 : 6) split_dual_kernel(const SplitJob a, const SplitJob b) {
+__global__ void __launch_bounds__(THREADS, VEC ? 5 : 6) split_dual_kernel(const SplitJob a, const SplitJob b, unsigned int *z) {
   __shared__ float tile[TILE][TILE + 1]; // transposing staging tile shared by all paths
   // Chained behind the kernel that writes the scaling constants (AUTO / FP16TCEC_SCALING), and
   // the GEMM kernel that follows may be scheduled while this one drains: its prologue does not
   // depend on the panels, and its first panel load waits for this grid to complete.
   CUMPSGEMM_CHAINED_KERNEL_ENTRY();
+  zero_word(z);
   const uint32_t blocks_a = a.gx * a.gy * a.gz;
   uint32_t id = blockIdx.x;
   const SplitJob &j = (id < blocks_a) ? a : b;
@@ -377,9 +385,10 @@ __global__ void __launch_bounds__(THREADS, VEC ? 5 : 6) split_dual_kernel(const 
 // deselected one exit, src/cumpsgemm_kernel.cuh:478-489).
 template <bool VEC>
 __global__ void __launch_bounds__(THREADS, VEC ? 5 : 6)
-    split_dual_auto_kernel(const SplitJob a, const SplitJob b) {
+    split_dual_auto_kernel(const SplitJob a, const SplitJob b, unsigned int *z) {
   __shared__ float tile[TILE][TILE + 1];
   CUMPSGEMM_CHAINED_KERNEL_ENTRY(); // see split_dual_kernel
+  zero_word(z);
   const uint32_t blocks_a = a.gx * a.gy * a.gz;
   uint32_t id = blockIdx.x;
   const SplitJob &j = (id < blocks_a) ? a : b;
@@ -433,19 +442,21 @@ bool make_job(const SplitArgs &a, SplitJob *job) {
 cudaError_t launch_split_pair_auto(const SplitArgs &a, const SplitArgs &b, cudaStream_t stream) {
   if (a.dyn == nullptr || b.dyn != a.dyn) return cudaErrorInvalidValue;
   SplitJob ja, jb;
+  unsigned int *z = a.zero_word;
   if (!make_job(a, &ja) || !make_job(b, &jb)) return cudaErrorInvalidValue;
   const uint64_t blocks = static_cast<uint64_t>(ja.gx) * ja.gy * ja.gz +
                           static_cast<uint64_t>(jb.gx) * jb.gy * jb.gz;
   if (blocks == 0 || blocks > 0x7fffffffull) return cudaErrorInvalidValue;
   const bool vec = (ja.path >= kPathKContig) || (jb.path >= kPathKContig);
   const unsigned grid = static_cast<unsigned>(blocks);
-  if (vec) return launch_chained(split_dual_auto_kernel<true>, grid, THREADS, 0, stream, ja, jb);
-  return launch_chained(split_dual_auto_kernel<false>, grid, THREADS, 0, stream, ja, jb);
+  if (vec) return launch_chained(split_dual_auto_kernel<true>, grid, THREADS, 0, stream, ja, jb, z);
+  return launch_chained(split_dual_auto_kernel<false>, grid, THREADS, 0, stream, ja, jb, z);
 }
 
 cudaError_t launch_split_pair(const SplitArgs &a, const SplitArgs &b, cudaStream_t stream) {
   if (a.kind != b.kind) return cudaErrorInvalidValue;
   SplitJob ja, jb;
+  unsigned int *z = a.zero_word;
   if (!make_job(a, &ja) || !make_job(b, &jb)) return cudaErrorInvalidValue;
   const uint64_t blocks = static_cast<uint64_t>(ja.gx) * ja.gy * ja.gz +
                           static_cast<uint64_t>(jb.gx) * jb.gy * jb.gz;
@@ -453,11 +464,11 @@ cudaError_t launch_split_pair(const SplitArgs &a, const SplitArgs &b, cudaStream
   const bool vec = (ja.path >= kPathKContig) || (jb.path >= kPathKContig);
   const unsigned grid = static_cast<unsigned>(blocks);
   if (a.kind == SplitKind::fp16) {
-    if (vec) return launch_chained(split_dual_kernel<0, true>, grid, THREADS, 0, stream, ja, jb);
-    return launch_chained(split_dual_kernel<0, false>, grid, THREADS, 0, stream, ja, jb);
+    if (vec) return launch_chained(split_dual_kernel<0, true>, grid, THREADS, 0, stream, ja, jb, z);
+    return launch_chained(split_dual_kernel<0, false>, grid, THREADS, 0, stream, ja, jb, z);
   }
-  if (vec) return launch_chained(split_dual_kernel<1, true>, grid, THREADS, 0, stream, ja, jb);
-  return launch_chained(split_dual_kernel<1, false>, grid, THREADS, 0, stream, ja, jb);
+  if (vec) return launch_chained(split_dual_kernel<1, true>, grid, THREADS, 0, stream, ja, jb, z);
+  return launch_chained(split_dual_kernel<1, false>, grid, THREADS, 0, stream, ja, jb, z);
 }
 
 } // namespace cumpsgemm_b200

@@ -105,7 +105,8 @@ extern "C" cublasStatus_t cuMpSGEMM_sgemm_static_scratch(
   const std::size_t es = (kind == SplitKind::fp16) ? 2 : 4;
   // the tile rule of the regular entry points, so that both run the same kernels
   const Tuning tuning = read_tuning_env(); // no handle to cache them in
-  const TileChoice choice = pick_tile(tuning, static_cast<unsigned>(pd->num_sms), m, n, 1, true);
+  const TileChoice choice = pick_tile(tuning, static_cast<unsigned>(pd->num_sms), m, n, k, 1, true,
+                                      kind == SplitKind::tf32, false);
   const int tile_n = choice.tile_n;
   const bool use_pair = choice.pair;
   const std::uint64_t rows_pad_a = round_up(m, use_pair ? 256 : 128);

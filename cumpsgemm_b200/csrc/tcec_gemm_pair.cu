@@ -32,6 +32,7 @@
 #include "epilogue.cuh"
 #include "gemm_common.cuh"
 #include "ptx.cuh"
+#include "work_list.cuh"
 
 #include <mutex>
 
@@ -68,72 +69,30 @@ struct TileCoord {
   int n0; // first column of the pair's 256 columns
 };
 
-// Grouped raster over pair tiles: tiles that run at the same time share A and B panels in L2.
 __device__ __forceinline__ TileCoord tile_coord(uint32_t tile, const GemmKernelParams &p,
                                                 uint32_t rank) {
-  constexpr uint32_t GROUP_M = 8;
-  const uint32_t tiles_per_batch = p.tiles_m * p.tiles_n;
+  const TilePos t = tile_raster(tile, p.tiles_m, p.tiles_n);
   TileCoord c;
-  c.batch = tile / tiles_per_batch;
-  const uint32_t t = tile - c.batch * tiles_per_batch;
-  const uint32_t tiles_in_group = GROUP_M * p.tiles_n;
-  const uint32_t group_id = t / tiles_in_group;
-  const uint32_t first_m = group_id * GROUP_M;
-  const uint32_t group_rows = min(p.tiles_m - first_m, GROUP_M);
-  const uint32_t in_group = t - group_id * tiles_in_group;
-  const uint32_t tile_m = first_m + in_group % group_rows;
-  const uint32_t tile_n = in_group / group_rows;
-  c.m0 = static_cast<int>(tile_m * 2 * BM_CTA + rank * BM_CTA);
-  c.n0 = static_cast<int>(tile_n * BN_PAIR);
+  c.batch = t.batch;
+  c.m0 = static_cast<int>(t.tm * 2 * BM_CTA + rank * BM_CTA);
+  c.n0 = static_cast<int>(t.tn * BN_PAIR);
   return c;
 }
 
-// K-split of the last, partly filled wave.  With T tiles on C clusters the last wave has
-// T mod C tiles; when that is at most half of C, each of those tiles is cut into `slices` K
-// ranges that run on different clusters at the same time, so the wave takes 1/slices of a
-// tile's time instead of a whole one (m=n=k=4096: 256 tiles on 74 clusters = 3.46 waves, the
-// last 34 tiles are cut in two and the launch takes 3.5 tile times instead of 4).  Every slice
-// writes its plain FP32 partial sums to scratch memory and takes a ticket from the tile's
-// counter; the CTA that draws the last ticket adds the slices in ascending order (so the
-// result does not depend on which one that is) and runs the alpha / beta epilogue.  Nobody
-// waits for anybody, hence no assumption about which clusters are resident together.
-// Work item w of a launch: w < split_begin is tile w with its whole K loop; beyond that,
-// item split_begin + u is slice u % slices of tile split_begin + u / slices.
-struct PairTail {
-  float *partial;          // [tail tile][slice][CTA rank][256 columns][128 rows]
-  unsigned int *counters;  // [tail tile][CTA rank], zero at launch
-  uint32_t split_begin;    // first tile that is split (= total tiles when nothing is split)
-  uint32_t slices;         // K slices per split tile (1: nothing is split)
-  uint32_t slice_blocks;   // stages per slice (the last one may be shorter)
-  uint32_t work_items;     // split_begin + (total tiles - split_begin) * slices
+// Tiles left over from the whole waves are cut along K (work_list.cuh) when that shortens the
+// launch: m=n=k=4096 has 256 tiles on 74 clusters = 3.46 waves, the last 34 tiles are cut in two
+// and the launch takes 3.5 tile times instead of 4.  Every piece parks its plain FP32 partial
+// sums in scratch memory; piece_fixup.cu adds them.
+struct PairPlan {
+  float *partial; // [cluster][2][CTA rank][256 columns][128 rows]
+  WorkPlan w;
 };
-
-struct WorkItem {
-  uint32_t tile, kb0, kbn, slice;
-};
-
-__device__ __forceinline__ WorkItem work_item(uint32_t w, const PairTail &t, uint32_t k_blocks) {
-  WorkItem x;
-  if (w < t.split_begin) {
-    x.tile = w;
-    x.kb0 = 0;
-    x.kbn = k_blocks;
-    x.slice = 0;
-  } else {
-    const uint32_t u = w - t.split_begin;
-    const uint32_t ti = u / t.slices;
-    x.tile = t.split_begin + ti;
-    x.slice = u - ti * t.slices;
-    x.kb0 = x.slice * t.slice_blocks;
-    x.kbn = min(t.slice_blocks, k_blocks - x.kb0);
-  }
-  return x;
-}
 
 template <int KIND>
 __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtensorMap &map_b,
-                                          const GemmKernelParams &p, const PairTail &tail) {
+                                          const GemmKernelParams &p, const PairPlan &plan) {
   constexpr int K_STEPS = ROW_BYTES / 32;
+  constexpr uint32_t STAGES_PER_UNIT = (KIND == 0) ? 1 : 2; // a unit is 64 k values
   constexpr int MY_MODE = (KIND == 0) ? CUMPSGEMM_FP16TCEC : CUMPSGEMM_TF32TCEC;
   constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, 2 * BM_CTA, BN_PAIR);
   constexpr int CPT = BN_PAIR / 2;
@@ -150,10 +109,8 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
   uint64_t *d0_empty = bars + 2 * STAGES + 1;
   uint64_t *d1_full = bars + 2 * STAGES + 2;
   uint64_t *d1_empty = bars + 2 * STAGES + 3;
-  uint64_t *tail_bar = bars + 2 * STAGES + 4; // the eight epilogue warps of this CTA (tail split)
-  uint32_t *tmem_base_ptr = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 5);
+  uint32_t *tmem_base_ptr = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_base_ptr + 1);
-  volatile uint32_t *ticket_smem = reinterpret_cast<volatile uint32_t *>(tmem_base_ptr + 2);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -161,7 +118,6 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
   const bool leader = (rank == 0);
   const uint32_t cluster_id = blockIdx.x >> 1;
   const uint32_t num_clusters = gridDim.x >> 1;
-  const uint32_t work_items = tail.work_items;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -172,7 +128,6 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
     ptx::mbar_init(ptx::smem_u32(d0_empty), 2 * NUM_EPI_WARPS);
     ptx::mbar_init(ptx::smem_u32(d1_full), 1);
     ptx::mbar_init(ptx::smem_u32(d1_empty), 2 * NUM_EPI_WARPS);
-    ptx::mbar_init(ptx::smem_u32(tail_bar), NUM_EPI_WARPS);
     *abort_flag = 0;
     ptx::mbar_init_fence();
     ptx::prefetch_tensormap(&map_a);
@@ -196,16 +151,20 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
   if (warp == 0) {
     // ================================================================ TMA producer (both CTAs)
     if (ptx::elect_one()) {
+      // launched with programmatic serialization behind the split pass, which also zeroes the
+      // wave counter: both are complete after this
+      ptx::griddep_wait();
       uint32_t it = 0; // stage uses since kernel start, across tiles
       bool ok = true;
-      bool pace = leader && p.wave_counter != nullptr && work_items > num_clusters;
+      bool pace = leader && p.wave_counter != nullptr && plan.w.whole_tiles > num_clusters;
       uint32_t wave = 0;
-      for (uint32_t w = cluster_id; w < work_items && ok; w += num_clusters, ++wave) {
-        const WorkItem wi = work_item(w, tail, k_blocks);
-        const TileCoord tc = tile_coord(wi.tile, p, rank);
+      WorkList list(plan.w, cluster_id, num_clusters);
+      WorkItem x;
+      while (ok && list.next(plan.w, x)) {
+        const TileCoord tc = tile_coord(x.tile, p, rank);
         const int za = static_cast<int>(tc.batch * 2u);
         const int nb0 = tc.n0 + static_cast<int>(rank) * 128; // this CTA's rows of the B tile
-        if (pace) {
+        if (pace && x.tile < plan.w.whole_tiles) {
           // Keep the clusters in step.  Clusters that run at the same time share panel rows
           // through L2 only while they are at about the same k; left alone they drift apart
           // by about 2 % per tile and, once the drift exceeds what L2 retains, most loads go
@@ -215,7 +174,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
           // then this cluster stops pacing for the rest of the launch, so clusters that are
           // not resident at the same time cost one time-out and never a wrong result.
           atomicAdd(p.wave_counter, 1u);
-          const uint32_t target = min(work_items, (wave + 1) * num_clusters);
+          const uint32_t target = min(plan.w.whole_tiles, (++wave) * num_clusters);
           const uint64_t t0 = ptx::globaltimer_ns();
           while (*reinterpret_cast<volatile unsigned int *>(p.wave_counter) < target) {
             if (ptx::globaltimer_ns() - t0 > 100000ull) {
@@ -225,7 +184,8 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
             __nanosleep(64);
           }
         }
-        for (uint32_t kb = 0; kb < wi.kbn; ++kb, ++it) {
+        const uint32_t kb0 = x.u0 * STAGES_PER_UNIT, kbn = x.un * STAGES_PER_UNIT;
+        for (uint32_t kb = 0; kb < kbn; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1u;
           ok = ptx::mbar_wait_timed(ptx::smem_u32(&empty_bar[s]), ph ^ 1u, abort_flag, p.status,
@@ -237,7 +197,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
           const uint32_t st = ptx::smem_u32(smem + s * STAGE_BYTES);
           // coordinates: (element in the K block, row, plane * k_blocks + K block); each box
           // is one contiguous 16 KiB run of the K-blocked panel
-          const int zh = static_cast<int>(static_cast<uint32_t>(za) * k_blocks + wi.kb0 + kb);
+          const int zh = static_cast<int>(static_cast<uint32_t>(za) * k_blocks + kb0 + kb);
           const int zl = zh + static_cast<int>(k_blocks);
           ptx::tma_load_3d_pair(st, &map_a, fb, 0, tc.m0, zh);
           ptx::tma_load_3d_pair(st + TILE_BYTES, &map_a, fb, 0, tc.m0, zl);
@@ -256,54 +216,65 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
       bool ok = true;
       const long long dbg_t0 = clock64();
       const uint32_t chunk = p.drain_chunk;
-      const uint32_t first = p.first_chunk; // stages in the first chunk of every tile
-      // Chunks of a tile: [0, first), then pieces of `chunk` stages.
-      auto chunk_start = [&](uint32_t kb) {
-        return kb == 0 || (kb >= first && (kb - first) % chunk == 0);
-      };
-      uint32_t it = 0, chunk_idx = 0, tile_iter = 0;
-      for (uint32_t w = cluster_id; w < work_items && ok; w += num_clusters, ++tile_iter) {
-        const uint32_t kbn = work_item(w, tail, k_blocks).kbn;
-        for (uint32_t kb = 0; kb < kbn && ok; ++kb, ++it) {
-          const bool first_in_chunk = chunk_start(kb);
-          const uint32_t s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1u;
+      const uint64_t desc0 = ptx::make_kmajor_desc<ROW_BYTES>(ptx::smem_u32(smem));
+      constexpr uint64_t kStage = STAGE_BYTES >> 4, kTile = TILE_BYTES >> 4;
+      uint32_t s = 0, ph = 0, d0_ph = 1, d1_ph = 1;
+      WorkList list(plan.w, cluster_id, num_clusters);
+      WorkItem x;
+      while (ok && list.next(plan.w, x)) {
+        const uint32_t kbn = x.un * STAGES_PER_UNIT;
+        uint32_t chunk_end = 0; // first stage after the current chunk
+        for (uint32_t kb = 0; kb < kbn; ++kb) {
+          const bool first_in_chunk = (kb == chunk_end);
+          if (first_in_chunk) chunk_end = min(kb + chunk, kbn);
           ok = ptx::mbar_wait_timed(ptx::smem_u32(&full_bar[s]), ph, abort_flag, p.status,
                                     ptx::kErrWaitFull, dbg, &dbg_wait);
           if (!ok) break;
+          ptx::tc_fence_after();
+          const uint64_t a_hi = desc0 + s * kStage;
+          const uint64_t a_lo = a_hi + kTile, b_hi = a_hi + 2 * kTile, b_lo = a_hi + 3 * kTile;
+          auto corrections = [&](uint32_t acc_first) {
+#pragma unroll
+            for (int ks = 0; ks < K_STEPS; ++ks)
+              mma_pair<KIND>(d1, a_lo + 2 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : acc_first);
+#pragma unroll
+            for (int ks = 0; ks < K_STEPS; ++ks)
+              mma_pair<KIND>(d1, a_hi + 2 * ks, b_lo + 2 * ks, IDESC, 1u);
+          };
+          // The corrections of a chunk's first stage come before its hi*hi products, those of
+          // its last stage after them: the drain of D0 in between has two stages' corrections
+          // to hide behind (one with single-stage chunks).  In the first stage of an item they
+          // come after, because they have to wait until the epilogue has given D1 back.
+          const bool corrections_first = first_in_chunk && kb > 0;
+          if (corrections_first) corrections(1u);
           if (first_in_chunk) {
             // D0 of the previous chunk must have been drained before it is overwritten.
-            ok = ptx::mbar_wait_timed(ptx::smem_u32(d0_empty), (chunk_idx & 1u) ^ 1u, abort_flag,
-                                      p.status, ptx::kErrWaitD0Empty, dbg, &dbg_wait2);
+            ok = ptx::mbar_wait_timed(ptx::smem_u32(d0_empty), d0_ph, abort_flag, p.status,
+                                      ptx::kErrWaitD0Empty, dbg, &dbg_wait2);
             if (!ok) break;
-          }
-          ptx::tc_fence_after();
-          const uint32_t st = ptx::smem_u32(smem + s * STAGE_BYTES);
-          const uint64_t a_hi = ptx::make_kmajor_desc<ROW_BYTES>(st);
-          const uint64_t a_lo = ptx::make_kmajor_desc<ROW_BYTES>(st + TILE_BYTES);
-          const uint64_t b_hi = ptx::make_kmajor_desc<ROW_BYTES>(st + 2 * TILE_BYTES);
-          const uint64_t b_lo = ptx::make_kmajor_desc<ROW_BYTES>(st + 3 * TILE_BYTES);
-#pragma unroll
-          for (int ks = 0; ks < K_STEPS; ++ks)
-            mma_pair<KIND>(d0, a_hi + 2 * ks, b_hi + 2 * ks, IDESC,
-                           (!first_in_chunk || ks > 0) ? 1u : 0u);
-          const bool last_in_chunk = (kb + 1 == kbn) || chunk_start(kb + 1);
-          if (last_in_chunk) ptx::tc_commit_pair(ptx::smem_u32(d0_full), BOTH);
-          if (kb == 0) {
-            // D1 still holds the previous tile's corrections until its epilogue has read them.
-            ok = ptx::mbar_wait_timed(ptx::smem_u32(d1_empty), (tile_iter & 1u) ^ 1u, abort_flag,
-                                      p.status, ptx::kErrWaitD1Empty, dbg, &dbg_wait2);
-            if (!ok) break;
+            d0_ph ^= 1u;
             ptx::tc_fence_after();
           }
 #pragma unroll
           for (int ks = 0; ks < K_STEPS; ++ks)
-            mma_pair<KIND>(d1, a_lo + 2 * ks, b_hi + 2 * ks, IDESC, (kb > 0 || ks > 0) ? 1u : 0u);
-#pragma unroll
-          for (int ks = 0; ks < K_STEPS; ++ks)
-            mma_pair<KIND>(d1, a_hi + 2 * ks, b_lo + 2 * ks, IDESC, 1u);
+            mma_pair<KIND>(d0, a_hi + 2 * ks, b_hi + 2 * ks, IDESC,
+                           (!first_in_chunk || ks > 0) ? 1u : 0u);
+          if (kb + 1 == chunk_end) ptx::tc_commit_pair(ptx::smem_u32(d0_full), BOTH);
+          if (!corrections_first) {
+            if (kb == 0) {
+              ok = ptx::mbar_wait_timed(ptx::smem_u32(d1_empty), d1_ph, abort_flag, p.status,
+                                        ptx::kErrWaitD1Empty, dbg, &dbg_wait2);
+              if (!ok) break;
+              d1_ph ^= 1u;
+              ptx::tc_fence_after();
+            }
+            corrections(kb > 0 ? 1u : 0u);
+          }
           ptx::tc_commit_pair(ptx::smem_u32(&empty_bar[s]), BOTH);
-          if (last_in_chunk) ++chunk_idx;
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
         if (ok) ptx::tc_commit_pair(ptx::smem_u32(d1_full), BOTH);
       }
@@ -320,30 +291,29 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
                             static_cast<uint32_t>((warp - 4) >> 2) * CPT;
     const uint32_t d0_empty_leader = ptx::map_to_cta(ptx::smem_u32(d0_empty), 0);
 
-    uint32_t chunk_idx = 0, tile_iter = 0, tail_phase = 0;
+    // the split pass has read its sources and zeroed nothing these warps touch before the first
+    // finished chunk, but the wait keeps every global access of this kernel behind it
+    ptx::griddep_wait();
+    uint32_t d0_ph = 0, d1_ph = 0;
     bool ok = true;
-    for (uint32_t w = cluster_id; w < work_items && ok; w += num_clusters, ++tile_iter) {
-      uint32_t n_chunks, prefetch_at;
-      {
-        const uint32_t kbn = work_item(w, tail, k_blocks).kbn;
-        n_chunks = 1u + ((kbn > p.first_chunk)
-                             ? (kbn - p.first_chunk + p.drain_chunk - 1) / p.drain_chunk
-                             : 0u);
-        const bool read_c = (p.beta_r != 0.f) || (p.beta_i != 0.f);
-        prefetch_at = (!read_c || w >= tail.split_begin) ? n_chunks
-                      : (n_chunks > C_PREFETCH_LEAD)     ? n_chunks - C_PREFETCH_LEAD
-                                                         : 0u;
-      }
+    WorkList list(plan.w, cluster_id, num_clusters);
+    WorkItem x;
+    while (ok && list.next(plan.w, x)) {
+      const uint32_t n_chunks = (x.un * STAGES_PER_UNIT + p.drain_chunk - 1u) / p.drain_chunk;
+      const uint32_t prefetch_at =
+          ((p.beta_r == 0.f && p.beta_i == 0.f) || x.un != plan.w.units) ? n_chunks
+          : (n_chunks > C_PREFETCH_LEAD) ? n_chunks - C_PREFETCH_LEAD
+                                         : 0u;
       float acc[CPT];
 #pragma unroll
       for (int i = 0; i < CPT; ++i) acc[i] = 0.f;
 
 #pragma unroll 1
-      for (uint32_t c = 0; c < n_chunks; ++c, ++chunk_idx) {
+      for (uint32_t c = 0; c < n_chunks; ++c) {
         if (c == prefetch_at) {
           // beta != 0: pull this warp's part of the C tile into L2 a few chunks before the
           // epilogue reads it (lane l fetches the line of columns l, l+32, ...)
-          const TileCoord tc = tile_coord(work_item(opaque(w), tail, k_blocks).tile, p, rank);
+          const TileCoord tc = tile_coord(opaque(x.tile), p, rank);
           const uint32_t row = static_cast<uint32_t>(tc.m0) + static_cast<uint32_t>(warp & 3) * 32u;
           const float *cp =
               ((p.c_array != nullptr) ? p.c_array[tc.batch]
@@ -355,9 +325,9 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
             if (col < p.n && row < p.m) ptx::prefetch_l2(cp + static_cast<uint64_t>(col) * p.ldc);
           }
         }
-        ok = ptx::mbar_wait(ptx::smem_u32(d0_full), chunk_idx & 1u, abort_flag, p.status,
-                            ptx::kErrWaitD0Full);
+        ok = ptx::mbar_wait(ptx::smem_u32(d0_full), d0_ph, abort_flag, p.status, ptx::kErrWaitD0Full);
         if (!ok) break;
+        d0_ph ^= 1u;
         ptx::tc_fence_after();
         drain_sums<CPT>(t_base, acc);
         ptx::tc_fence_before();
@@ -366,17 +336,16 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
       }
       if (!ok) break;
 
-      ok = ptx::mbar_wait(ptx::smem_u32(d1_full), tile_iter & 1u, abort_flag, p.status,
-                          ptx::kErrWaitD1Full);
+      ok = ptx::mbar_wait(ptx::smem_u32(d1_full), d1_ph, abort_flag, p.status, ptx::kErrWaitD1Full);
       if (!ok) break;
+      d1_ph ^= 1u;
       ptx::tc_fence_after();
       // the finished sums stay in the D1 columns; from here on they are read from there, and what
       // the epilogue needs to know of the tile is worked out only now (epilogue.cuh)
       const uint32_t t_sums = t_base + D1_COL;
       add_corrections_in_tmem<CPT>(t_sums, acc, p.lo_scale_inv);
-      const WorkItem wi = work_item(opaque(w), tail, k_blocks);
-      const bool split = w >= tail.split_begin; // this item is one K slice of a tile
-      const TileCoord tc = tile_coord(wi.tile, p, rank);
+      const bool part = x.un != plan.w.units; // this item is a piece of a tile
+      const TileCoord tc = tile_coord(opaque(x.tile), p, rank);
       const uint32_t quarter = static_cast<uint32_t>(warp & 3);
       const uint32_t col_base = static_cast<uint32_t>((warp - 4) >> 2) * CPT;
       const uint32_t d1_empty_leader = ptx::map_to_cta(ptx::smem_u32(d1_empty), 0);
@@ -387,14 +356,12 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
         if (lane == 0) ptx::mbar_arrive_cluster(d1_empty_leader);
       };
 
-      if (split) {
-        // one K slice of a tile: park the partial sums, take a ticket, and go on to the
-        // epilogue only with the last ticket of this CTA's half of the tile
-        const uint32_t ti = wi.tile - tail.split_begin;
+      if (part) {
+        // a piece of a tile: park the partial sums for the kernel that adds the pieces
         constexpr uint32_t HALF = BN_PAIR * BM_CTA; // floats of one CTA's 128 x 256 half
-        float *tbase = tail.partial + (static_cast<uint64_t>(ti) * tail.slices * 2u + rank) * HALF +
-                       col_base * BM_CTA + quarter * 32u + static_cast<uint32_t>(lane);
-        float *mine = tbase + static_cast<uint64_t>(wi.slice) * 2u * HALF;
+        const uint32_t lane_off = col_base * BM_CTA + quarter * 32u + static_cast<uint32_t>(lane);
+        float *mine = plan.partial +
+                      static_cast<uint64_t>((cluster_id * 2u + x.slot) * 2u + rank) * HALF + lane_off;
 #pragma unroll 1
         for (int c = 0; c < CPT; c += kEpiGroup) {
           uint32_t v[kEpiGroup];
@@ -404,43 +371,8 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
           for (int i = 0; i < kEpiGroup; ++i)
             __stcg(mine + (c + i) * BM_CTA, __uint_as_float(v[i]));
         }
-        __threadfence();
-        // the eight epilogue warps meet twice (all partial sums stored; ticket published) on
-        // an mbarrier of their own, with the bounded wait every other wait here uses
-        auto meet = [&]() -> bool {
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(tail_bar));
-          const bool met = ptx::mbar_wait(ptx::smem_u32(tail_bar), tail_phase, abort_flag,
-                                          p.status, ptx::kErrWaitTail);
-          tail_phase ^= 1u;
-          return met;
-        };
-        ok = meet();
-        if (!ok) break;
-        if (warp == 4 && lane == 0) *ticket_smem = atomicAdd(tail.counters + ti * 2u + rank, 1u);
-        ok = meet();
-        if (!ok) break;
-        if (*ticket_smem != tail.slices - 1u) {
-          release_d1();
-          continue;
-        }
-        __threadfence();
-#pragma unroll 1
-        for (int c = 0; c < CPT; c += kEpiGroup) {
-          float sum[kEpiGroup];
-#pragma unroll
-          for (int i = 0; i < kEpiGroup; ++i) sum[i] = __ldcg(tbase + (c + i) * BM_CTA);
-          for (uint32_t sl = 1; sl < tail.slices; ++sl) {
-            const float *other = tbase + static_cast<uint64_t>(sl) * 2u * HALF;
-#pragma unroll
-            for (int i = 0; i < kEpiGroup; ++i) sum[i] += __ldcg(other + (c + i) * BM_CTA);
-          }
-          uint32_t v[kEpiGroup];
-#pragma unroll
-          for (int i = 0; i < kEpiGroup; ++i) v[i] = __float_as_uint(sum[i]);
-          ptx::tmem_st_32x32b_x16(t_sums + c, v);
-        }
-        ptx::tmem_st_wait();
+        release_d1();
+        continue;
       }
 
       // C(row, col): lanes hold consecutive rows of the column-major C, so each warp access
@@ -481,8 +413,8 @@ template <int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     tcec_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
                           const __grid_constant__ CUtensorMap map_b, const GemmKernelParams p,
-                          const PairTail tail) {
-  pair_body<KIND>(map_a, map_b, p, tail);
+                          const PairPlan plan) {
+  pair_body<KIND>(map_a, map_b, p, plan);
 }
 
 // AUTO: both kinds' tensor maps and parameters travel with the launch; the device-side
@@ -494,12 +426,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
                                const GemmKernelParams p16,
                                const __grid_constant__ CUtensorMap map_a32,
                                const __grid_constant__ CUtensorMap map_b32,
-                               const GemmKernelParams p32, const PairTail tail16,
-                               const PairTail tail32) {
+                               const GemmKernelParams p32, const PairPlan plan) {
   if (p16.dyn->gemm_mode == CUMPSGEMM_TF32TCEC) {
-    pair_body<1>(map_a32, map_b32, p32, tail32);
+    pair_body<1>(map_a32, map_b32, p32, plan);
   } else {
-    pair_body<0>(map_a16, map_b16, p16, tail16);
+    pair_body<0>(map_a16, map_b16, p16, plan);
   }
 }
 
@@ -538,8 +469,8 @@ template <int TAG, class Kernel> cudaError_t pair_setup(Kernel kernel, int *clus
 }
 
 // Tensor maps and kernel parameters of one kind.  Returns false on invalid sizes.
-bool pair_prepare(const TcecGemmArgs &a, SplitKind kind, CUtensorMap *map_a, CUtensorMap *map_b,
-                  GemmKernelParams *pp) {
+bool pair_prepare(const TcecGemmArgs &a, SplitKind kind, int max_clusters, CUtensorMap *map_a,
+                  CUtensorMap *map_b, GemmKernelParams *pp) {
   const uint32_t planes = a.batch * 2u;
   if (!make_panel_map(map_a, kind, a.panel_a, a.k_pad, a.rows_pad_a, planes, 128) ||
       !make_panel_map(map_b, kind, a.panel_b, a.k_pad, a.rows_pad_b, planes, 128)) {
@@ -567,29 +498,15 @@ bool pair_prepare(const TcecGemmArgs &a, SplitKind kind, CUtensorMap *map_a, CUt
   p.debug = a.debug;
   {
     const int v = a.tuning.drain_chunk;
-    // Default: two stages (128 FP16 / 64 TF32 k values) per drain.  Measured at m=n=k=16384,
-    // uniform(-1,1): residual 3.1e-7 / 2.8e-7 / 3.7e-7 / 6.5e-7 / 2.5e-6 / 1.9e-5 for 1 / 2 / 4 /
-    // 8 / 32 / 256 stages per drain (FP32 cuBLAS SGEMM on the same inputs: 2.3e-6).
-    p.drain_chunk = static_cast<uint16_t>((v >= 1) ? (v > 0xffff ? 0xffff : v) : 2);
-    // The first chunk of every tile is longer: while it accumulates, the epilogue warps are
-    // still storing the previous tile, and the issuer would otherwise wait about 17,000 cycles
-    // per tile for them to drain a short first chunk (measured: 5 % of a tile at k=16384, 18 %
-    // at k=4096).  Its length is bounded by accuracy: the tensor core's own accumulation loses
-    // about 1.2e-9 relative accuracy per accumulated k value, and the first chunk's share of
-    // the result is sqrt(first / k), so the result stays as close to the FP64 product as with
-    // short chunks only if first^1.5 <= ~80 sqrt(k).  Measured residuals (FP16TCEC, m=n=4096,
-    // FP32 cuBLAS in brackets): k=512 with 128 / 256 / 512 values in the first chunk 2.0e-7 /
-    // 2.8e-7 / 6.5e-7 (4.1e-7); k=4096 with 256 / 512: 2.3e-7 / 3.1e-7 (1.2e-6); k=16384 with
-    // 128 / 512 / 1024: 2.8e-7 / 3.0e-7 / 4.2e-7 (2.3e-6).  TF32 products carry more bits into
-    // the accumulator and lose twice as much, so that kind gets half the length.
-    const uint32_t k_per_stage = ROW_BYTES / es;
-    const uint32_t k_total = p.k_blocks * k_per_stage;
-    uint32_t first_k = (k_total >= 8192u) ? 512u : (k_total >= 2048u ? 256u : 128u);
-    if (kind != SplitKind::fp16) first_k /= 2u;
-    const int fv = a.tuning.first_chunk;
-    const uint32_t first = (fv >= 1) ? static_cast<uint32_t>(fv) : first_k / k_per_stage;
-    p.first_chunk = static_cast<uint16_t>(first > 0xffffu ? 0xffffu : first);
-    if (p.first_chunk < p.drain_chunk) p.first_chunk = p.drain_chunk;
+    // Two stages (128 FP16 / 64 TF32 k values) per drain.  Measured at m=n=k=16384, uniform(-1,1):
+    // residual 3.1e-7 / 2.8e-7 / 3.7e-7 / 6.5e-7 / 2.5e-6 / 1.9e-5 for 1 / 2 / 4 / 8 / 32 / 256
+    // stages per drain (FP32 cuBLAS SGEMM on the same inputs: 2.3e-6).  One stage where there is at
+    // most one wave of tiles, as in the single-CTA kernel that shares those sizes (m=n=k=2048:
+    // 1.7e-7 instead of 2.3e-7 for 3 % of the time).
+    const uint32_t pairs = static_cast<uint32_t>(max_clusters);
+    const uint32_t dflt = (static_cast<uint64_t>(p.tiles_m) * p.tiles_n * a.batch > pairs) ? 2 : 1;
+    p.drain_chunk = static_cast<uint16_t>((v >= 1) ? (v > 0xffff ? 0xffff : v) : dflt);
+    p.first_chunk = p.drain_chunk; // (the fused kernel's field)
   }
   const uint64_t total = static_cast<uint64_t>(p.tiles_m) * p.tiles_n * a.batch;
   if (total == 0 || total > 0x7fffffffull) return false;
@@ -599,75 +516,99 @@ bool pair_prepare(const TcecGemmArgs &a, SplitKind kind, CUtensorMap *map_a, CUt
   return true;
 }
 
-// Plan of the tail split (see PairTail) for a launch on at most `max_clusters` clusters.  A
-// slice keeps at least 1024 k values, so that a slice's prologue and drain stay amortised.
-PairTail plan_tail(const TcecGemmArgs &a, SplitKind kind, const GemmKernelParams &p,
-                   uint32_t max_clusters) {
-  PairTail t;
-  t.partial = nullptr;
-  t.counters = nullptr;
-  t.split_begin = p.total_tiles;
-  t.slices = 1;
-  t.slice_blocks = p.k_blocks;
-  t.work_items = p.total_tiles;
-  if (a.tail_partial == nullptr || a.wave_counter == nullptr || a.tuning.tail_split == 0) return t;
-  const uint32_t rem = p.total_tiles % max_clusters;
-  if (rem == 0 || 2 * rem > max_clusters || 2 * rem > static_cast<uint32_t>(kPairTailCounters))
+} // namespace
+
+// Plan of a launch on at most `max_clusters` clusters: how the tiles left over from the whole
+// waves are cut along K.
+//   At most half a wave of them: every tile in equal slices, one cluster each.  A slice keeps at
+//   least 1024 k values, so that its prologue and drain stay amortised.
+//   More than half a wave: their k range laid end to end and shared by all clusters.
+// Either way only if the launch gets shorter by more than the pieces cost: parking and adding
+// them takes about 0.35 us per left-over tile, a unit of 64 k values 0.9 us (FP16) or 1.8 (TF32).
+WorkPlan plan_pair(const Tuning &tuning, bool tf32, bool can_cut, uint32_t total_tiles,
+                   uint32_t units, uint32_t max_clusters) {
+  WorkPlan t;
+  t.total_tiles = total_tiles;
+  t.whole_tiles = total_tiles;
+  t.units = units;
+  t.slice_units = 0;
+  t.piece_clusters = 0;
+  t.slices = 0;
+  const uint32_t rem = max_clusters > 0 ? total_tiles % max_clusters : 0;
+  if (!can_cut || tuning.tail_split == 0 || rem == 0 || max_clusters > 0xffffu) return t;
+  const uint32_t min_saved = 2 + (tf32 ? rem / 5 : 2 * rem / 5);
+  if (2 * rem <= max_clusters) {
+    uint32_t slices = max_clusters / rem;
+    if (slices > units / 16u) slices = units / 16u;
+    if (slices > 8u) slices = 8u;
+    if (tuning.tail_split > 1 && slices > static_cast<uint32_t>(tuning.tail_split))
+      slices = static_cast<uint32_t>(tuning.tail_split);
+    if (slices < 2u) return t;
+    const uint32_t per = (units + slices - 1) / slices;
+    slices = (units + per - 1) / per; // no empty slice
+    if (slices < 2u || per + min_saved > units) return t;
+    t.whole_tiles = total_tiles - rem;
+    t.slices = static_cast<uint16_t>(slices);
+    t.slice_units = per;
+    t.piece_clusters = static_cast<uint16_t>(rem * slices);
     return t;
-  const uint32_t k_per_stage = ROW_BYTES / ((kind == SplitKind::fp16) ? 2u : 4u);
-  const uint32_t min_stages = 1024u / k_per_stage;
-  uint32_t slices = max_clusters / rem;
-  if (slices > p.k_blocks / min_stages) slices = p.k_blocks / min_stages;
-  if (slices > 8u) slices = 8u;
-  if (a.tuning.tail_split > 1 && slices > static_cast<uint32_t>(a.tuning.tail_split))
-    slices = static_cast<uint32_t>(a.tuning.tail_split);
-  if (slices < 2u) return t;
-  const uint32_t per = (p.k_blocks + slices - 1) / slices;
-  slices = (p.k_blocks + per - 1) / per; // no empty slice
-  if (slices < 2u) return t;
-  t.partial = a.tail_partial;
-  t.counters = a.wave_counter + 1;
-  t.split_begin = p.total_tiles - rem;
-  t.slices = slices;
-  t.slice_blocks = per;
-  t.work_items = t.split_begin + rem * slices;
+  }
+  const uint64_t left = static_cast<uint64_t>(rem) * units;
+  const uint32_t per = static_cast<uint32_t>((left + max_clusters - 1) / max_clusters);
+  if (tuning.tail_split > 1 || per + min_saved > units || left > 0x7fffffffull) return t;
+  t.whole_tiles = total_tiles - rem;
+  t.piece_clusters = static_cast<uint16_t>(max_clusters);
   return t;
 }
+
+namespace {
 
 // Pacing pays when tiles are long (the drift it removes is 2 % of a tile) and clusters share
 // panel rows; for short tiles a barrier per tile costs more than it saves.
 bool wants_pacing(const TcecGemmArgs &a, uint32_t clusters, const GemmKernelParams &p,
-                  const PairTail &t) {
-  return a.wave_counter != nullptr && t.work_items > clusters && p.k_blocks >= kPaceMinStages &&
+                  const WorkPlan &w) {
+  return a.wave_counter != nullptr && w.whole_tiles > clusters && p.k_blocks >= kPaceMinStages &&
          a.tuning.pace != 0;
 }
 
-// The wave counter and the tail-split counters behind it start every launch at zero.
-cudaError_t reset_counters(const TcecGemmArgs &a, bool tail, cudaStream_t stream) {
-  return cudaMemsetAsync(a.wave_counter, 0,
-                         sizeof(unsigned int) * (tail ? 1 + kPairTailCounters : 1), stream);
+// Grid and plan of a launch, in units of 64 k values.
+PairPlan make_plan(const TcecGemmArgs &a, bool tf32, uint32_t total_tiles, int max_clusters,
+                   uint32_t *clusters) {
+  PairPlan plan;
+  plan.partial = a.tail_partial;
+  plan.w = plan_pair(a.tuning, tf32, a.tail_partial != nullptr, total_tiles,
+                     a.k_pad / 64, static_cast<uint32_t>(max_clusters));
+  *clusters = plan.w.whole_tiles > plan.w.piece_clusters ? plan.w.whole_tiles
+                                                          : plan.w.piece_clusters;
+  if (*clusters > static_cast<uint32_t>(max_clusters)) *clusters = static_cast<uint32_t>(max_clusters);
+  return plan;
+}
+
+// The kernel that adds the pieces, if the plan cut any tile.
+cudaError_t fix_up(const TcecGemmArgs &a, const GemmKernelParams &p, const PairPlan &plan,
+                   cudaStream_t stream) {
+  if (plan.w.piece_clusters == 0) return cudaSuccess;
+  const PieceFixupArgs f = {plan.partial, a.c,       a.c_array, a.dyn,     a.ldc,
+                            a.stride_c,   a.m,       a.n,       p.tiles_m, p.tiles_n,
+                            BN_PAIR,      a.alpha_r, a.alpha_i, a.beta_r,  a.beta_i,
+                            a.is_complex};
+  return launch_piece_fixup(f, plan.w, stream);
 }
 
 template <int KIND> cudaError_t launch_pair(const TcecGemmArgs &a, cudaStream_t stream) {
-  auto kernel = tcec_gemm_pair_kernel<KIND>;
   int max_clusters = 1;
-  const cudaError_t se = pair_setup<KIND>(kernel, &max_clusters);
+  const cudaError_t se = pair_setup<KIND>(tcec_gemm_pair_kernel<KIND>, &max_clusters);
   if (se != cudaSuccess) return se;
   constexpr SplitKind kind = KIND == 0 ? SplitKind::fp16 : SplitKind::tf32;
   CUtensorMap map_a, map_b;
   GemmKernelParams p;
-  if (!pair_prepare(a, kind, &map_a, &map_b, &p)) return cudaErrorInvalidValue;
-  const PairTail tail = plan_tail(a, kind, p, static_cast<uint32_t>(max_clusters));
-  const uint32_t clusters =
-      tail.work_items < static_cast<uint32_t>(max_clusters) ? tail.work_items : max_clusters;
-  const bool pace = wants_pacing(a, clusters, p, tail);
-  if (pace) p.wave_counter = a.wave_counter;
-  if (pace || tail.slices > 1) {
-    const cudaError_t me = reset_counters(a, tail.slices > 1, stream);
-    if (me != cudaSuccess) return me;
-  }
-  kernel<<<2 * clusters, NUM_THREADS, SMEM_BYTES, stream>>>(map_a, map_b, p, tail);
-  return cudaGetLastError();
+  if (!pair_prepare(a, kind, max_clusters, &map_a, &map_b, &p)) return cudaErrorInvalidValue;
+  uint32_t clusters = 0;
+  const PairPlan plan = make_plan(a, KIND == 1, p.total_tiles, max_clusters, &clusters);
+  if (wants_pacing(a, clusters, p, plan.w)) p.wave_counter = a.wave_counter;
+  const cudaError_t e = launch_chained(tcec_gemm_pair_kernel<KIND>, 2 * clusters, NUM_THREADS,
+                                       SMEM_BYTES, stream, map_a, map_b, p, plan);
+  return e != cudaSuccess ? e : fix_up(a, p, plan, stream);
 }
 
 } // namespace
@@ -679,31 +620,23 @@ cudaError_t launch_tcec_gemm_pair(const TcecGemmArgs &a, cudaStream_t stream) {
 
 cudaError_t launch_tcec_gemm_pair_auto(const TcecGemmArgs &a, cudaStream_t stream) {
   if (!a.error_correction || a.dyn == nullptr) return cudaErrorInvalidValue;
-  auto kernel = tcec_gemm_pair_auto_kernel;
   int max_clusters = 1;
-  const cudaError_t se = pair_setup<2>(kernel, &max_clusters);
+  const cudaError_t se = pair_setup<2>(tcec_gemm_pair_auto_kernel, &max_clusters);
   if (se != cudaSuccess) return se;
   CUtensorMap a16, b16, a32, b32;
   GemmKernelParams p16, p32;
-  if (!pair_prepare(a, SplitKind::fp16, &a16, &b16, &p16) ||
-      !pair_prepare(a, SplitKind::tf32, &a32, &b32, &p32))
+  if (!pair_prepare(a, SplitKind::fp16, max_clusters, &a16, &b16, &p16) ||
+      !pair_prepare(a, SplitKind::tf32, max_clusters, &a32, &b32, &p32))
     return cudaErrorInvalidValue;
-  const PairTail t16 = plan_tail(a, SplitKind::fp16, p16, static_cast<uint32_t>(max_clusters));
-  const PairTail t32 = plan_tail(a, SplitKind::tf32, p32, static_cast<uint32_t>(max_clusters));
-  // one grid for whichever kind runs: the larger of the two work lists, capped at what fits
-  uint32_t clusters = t16.work_items > t32.work_items ? t16.work_items : t32.work_items;
-  if (clusters > static_cast<uint32_t>(max_clusters)) clusters = max_clusters;
+  uint32_t clusters = 0;
+  // (one plan for whichever kind runs)
+  const PairPlan plan = make_plan(a, false, p16.total_tiles, max_clusters, &clusters);
   // pacing depends on the K loop length, which differs by kind: one counter serves whichever runs
-  const bool pace16 = wants_pacing(a, clusters, p16, t16), pace32 = wants_pacing(a, clusters, p32, t32);
-  if (pace16) p16.wave_counter = a.wave_counter;
-  if (pace32) p32.wave_counter = a.wave_counter;
-  const bool tail = t16.slices > 1 || t32.slices > 1;
-  if (pace16 || pace32 || tail) {
-    const cudaError_t me = reset_counters(a, tail, stream);
-    if (me != cudaSuccess) return me;
-  }
-  kernel<<<2 * clusters, NUM_THREADS, SMEM_BYTES, stream>>>(a16, b16, p16, a32, b32, p32, t16, t32);
-  return cudaGetLastError();
+  if (wants_pacing(a, clusters, p16, plan.w)) p16.wave_counter = a.wave_counter;
+  if (wants_pacing(a, clusters, p32, plan.w)) p32.wave_counter = a.wave_counter;
+  const cudaError_t e = launch_chained(tcec_gemm_pair_auto_kernel, 2 * clusters, NUM_THREADS,
+                                       SMEM_BYTES, stream, a16, b16, p16, a32, b32, p32, plan);
+  return e != cudaSuccess ? e : fix_up(a, p16, plan, stream);
 }
 
 } // namespace cumpsgemm_b200
@@ -715,22 +648,11 @@ extern "C" int cuMpSGEMM_plan_pair_tail(unsigned total_tiles, unsigned clusters,
   if (total_tiles == 0 || clusters == 0 || k_pad == 0 || k_pad % 64 != 0 ||
       split_begin == nullptr || slices == nullptr || slice_k == nullptr || work_items == nullptr)
     return 1;
-  const SplitKind kind = tf32 ? SplitKind::tf32 : SplitKind::fp16;
-  const unsigned k_per_stage = ROW_BYTES / (tf32 ? 4u : 2u);
-  // the plan only looks at whether scratch and counters exist, never at their contents
-  static float scratch_marker;
-  static unsigned int counter_marker[2];
-  TcecGemmArgs a = {};
-  a.tail_partial = &scratch_marker;
-  a.wave_counter = counter_marker;
-  a.tuning = Tuning{};
-  GemmKernelParams p = {};
-  p.total_tiles = total_tiles;
-  p.k_blocks = k_pad / k_per_stage;
-  const PairTail t = plan_tail(a, kind, p, clusters);
-  *split_begin = t.split_begin;
-  *slices = t.slices;
-  *slice_k = t.slice_blocks * k_per_stage;
-  *work_items = t.work_items;
+  const WorkPlan t = plan_pair(Tuning{}, tf32 != 0, true, total_tiles, k_pad / 64, clusters);
+  const bool sliced = t.slice_units != 0;
+  *split_begin = sliced ? t.whole_tiles : total_tiles;
+  *slices = sliced ? t.slices : 1;
+  *slice_k = sliced ? t.slice_units * 64 : k_pad;
+  *work_items = sliced ? t.whole_tiles + t.piece_clusters : total_tiles;
   return 0;
 }

@@ -30,18 +30,9 @@
 // are equal or smaller (those two: 2.1e-7 -> 1.5e-7 and 4.1e-7 -> 2.1e-7), because D0 is drained
 // every 64 FP16 / 32 TF32 values.
 //
-// Work distribution.  Tiles are dealt to the clusters in whole waves; what is left over
-// (total mod clusters, or everything when there are fewer tiles than clusters) can be cut along K:
-//   ticket mode   the left-over tiles' k range is laid out end to end and cut into equal pieces,
-//                 one per cluster, so a piece may end one tile and begin the next.  A piece that
-//                 is not a whole tile parks its FP32 partial sums in scratch memory and takes a
-//                 ticket of the tile's counter; the CTA that draws the last ticket adds the pieces
-//                 in ascending k (whoever it is, the result is the same) and runs the alpha / beta
-//                 epilogue, then puts the counter back to zero.  Nobody waits for anybody.
-//   reduce mode   few tiles: every tile is cut into the same number of slices, which write plain
-//                 partial sums that splitk_reduce_kernel adds in ascending order.
-// Both are the deterministic successors of the reference's atomic split-K kernel
-// (src/cumpsgemm.cu:272-304, src/dmem_accessor.hpp:352-395).
+// Work distribution: work_list.cuh.  What is left over from whole waves (total mod clusters, or
+// everything when there are fewer tiles than clusters) can be cut along K; piece_fixup.cu then
+// adds the pieces and runs their epilogue.
 //
 // Threads: 640 = warp 0 TMA producer, warp 1 TMEM allocation + MMA issue (even CTA), warps 2-3
 // idle, warps 4-11 drain / epilogue, warps 12-19 converters.  Launched with 96 registers per
@@ -54,12 +45,13 @@
 //   raw_empty[r]   8 arrivals, one per converter warp               own CTA
 //   full[s]        leader's only: 16 arrivals, 8 converter warps of each CTA
 //   empty[s]       tcgen05.commit multicast from the leader         both CTAs
-//   d0_full, d0_empty, d1_full, d1_empty, tail: as in tcec_gemm_pair.cu
+//   d0_full, d0_empty, d1_full, d1_empty: as in tcec_gemm_pair.cu
 // Every wait is bounded; no TMA multicast is used.
 #include "epilogue.cuh"
 #include "gemm_common.cuh"
 #include "ptx.cuh"
 #include "split_math.cuh"
+#include "work_list.cuh"
 
 #include <mutex>
 
@@ -91,18 +83,13 @@ struct StreamParams {
   float *c;
   const DynParams *dyn;
   int *status;
-  float *partial;         // ticket mode: [cluster][2][CTA rank][BN columns][128 rows]
-  unsigned int *counters; // ticket mode: [left-over tile][CTA rank], zero between launches
+  float *partial; // [cluster][2][CTA rank][BN columns][128 rows]
   unsigned long long *debug;
-  uint64_t ldc, stride_c, slice_stride;
+  uint64_t ldc, stride_c;
   uint32_t m, n;
-  uint32_t units; // K loop in units of 64 k values
   uint32_t tiles_m, tiles_n;
-  uint32_t total_tiles;
-  uint32_t whole_tiles; // tiles [0, whole_tiles) are dealt whole
   float alpha_r, alpha_i, beta_r, beta_i;
-  uint16_t piece_clusters; // clusters that share the left-over tiles' k range (0: none left over)
-  uint16_t slices;         // reduce mode: slices per tile; 0 or 1: ticket mode
+  WorkPlan w;
   uint8_t layout_a, layout_b;
   uint8_t flags; // k* below
 };
@@ -133,66 +120,13 @@ struct TileCoord {
 template <int BN>
 __device__ __forceinline__ TileCoord tile_coord(uint32_t tile, const StreamParams &p,
                                                 uint32_t rank) {
-  constexpr uint32_t GROUP_M = 8;
-  const uint32_t tiles_per_batch = p.tiles_m * p.tiles_n;
+  const TilePos t = tile_raster(tile, p.tiles_m, p.tiles_n);
   TileCoord c;
-  c.batch = tile / tiles_per_batch;
-  const uint32_t t = tile - c.batch * tiles_per_batch;
-  const uint32_t tiles_in_group = GROUP_M * p.tiles_n;
-  const uint32_t group_id = t / tiles_in_group;
-  const uint32_t first_m = group_id * GROUP_M;
-  const uint32_t group_rows = min(p.tiles_m - first_m, GROUP_M);
-  const uint32_t in_group = t - group_id * tiles_in_group;
-  c.m0 = static_cast<int>((first_m + in_group % group_rows) * 2 * BM_CTA + rank * BM_CTA);
-  c.n0 = static_cast<int>((in_group / group_rows) * BN);
+  c.batch = t.batch;
+  c.m0 = static_cast<int>(t.tm * 2 * BM_CTA + rank * BM_CTA);
+  c.n0 = static_cast<int>(t.tn * BN);
   return c;
 }
-
-// First unit (of the left-over tiles' concatenated k range) of cluster c's piece.
-__device__ __forceinline__ uint32_t piece_start(uint32_t c, uint32_t total_units,
-                                                uint32_t clusters) {
-  return static_cast<uint32_t>(static_cast<uint64_t>(c) * total_units / clusters);
-}
-
-// One work item: units [u0, u0 + un) of a tile's K loop.
-struct WorkItem {
-  uint32_t tile, u0, un;
-  uint32_t slot; // ticket mode: which of the cluster's two scratch tiles a partial item uses
-};
-// The items of one cluster, in the order every role walks them.
-struct WorkList {
-  uint32_t w, step; // whole tiles
-  uint32_t u, u_end, first;
-  __device__ __forceinline__ WorkList(const StreamParams &p, uint32_t cluster, uint32_t clusters)
-      : w(cluster), step(clusters), u(0), u_end(0), first(1) {
-    if (cluster < p.piece_clusters) {
-      const uint32_t total = (p.total_tiles - p.whole_tiles) * p.units;
-      u = piece_start(cluster, total, p.piece_clusters);
-      u_end = piece_start(cluster + 1, total, p.piece_clusters);
-    }
-  }
-  __device__ __forceinline__ bool next(const StreamParams &p, WorkItem &x) {
-    if (w < p.whole_tiles) {
-      x.tile = w;
-      x.u0 = 0;
-      x.un = p.units;
-      x.slot = 0;
-      w += step;
-      return true;
-    }
-    if (u < u_end) {
-      const uint32_t ti = u / p.units;
-      x.tile = p.whole_tiles + ti;
-      x.u0 = u - ti * p.units;
-      x.un = min(p.units - x.u0, u_end - u);
-      x.slot = first ? 0u : 1u;
-      first = 0;
-      u += x.un;
-      return true;
-    }
-    return false;
-  }
-};
 
 template <int KIND>
 __device__ __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
@@ -388,10 +322,8 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   uint64_t *d0_empty = d0_full + 1;
   uint64_t *d1_full = d0_full + 2;
   uint64_t *d1_empty = d0_full + 3;
-  uint64_t *tail_bar = d0_full + 4; // the eight epilogue warps of this CTA (ticket mode)
-  uint32_t *tmem_base_ptr = reinterpret_cast<uint32_t *>(d0_full + 5);
+  uint32_t *tmem_base_ptr = reinterpret_cast<uint32_t *>(d0_full + 4);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_base_ptr + 1);
-  volatile uint32_t *ticket_smem = reinterpret_cast<volatile uint32_t *>(tmem_base_ptr + 2);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -413,7 +345,6 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     ptx::mbar_init(ptx::smem_u32(d0_empty), 2 * NUM_EPI_WARPS);
     ptx::mbar_init(ptx::smem_u32(d1_full), 1);
     ptx::mbar_init(ptx::smem_u32(d1_empty), 2 * NUM_EPI_WARPS);
-    ptx::mbar_init(ptx::smem_u32(tail_bar), NUM_EPI_WARPS);
     *abort_flag = 0;
     ptx::mbar_init_fence();
     ptx::prefetch_tensormap(&map_a);
@@ -452,9 +383,9 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
                                static_cast<uint32_t>(Cfg::B_ROWS * SLOT_K * 4);
         uint32_t s = 0, ph = 0;
         bool ok = true;
-        WorkList list(p, cluster_id, num_clusters);
+        WorkList list(p.w, cluster_id, num_clusters);
         WorkItem x;
-        while (ok && list.next(p, x)) {
+        while (ok && list.next(p.w, x)) {
           const TileCoord tc = tile_coord<BN>(x.tile, p, rank);
           const int b_row = tc.n0 + static_cast<int>(rank) * Cfg::B_ROWS;
           const int t0 = static_cast<int>(2u * x.u0);
@@ -496,9 +427,9 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
         uint32_t s = 0, ph = 0, d0_ph = 1, d1_ph = 1;
         bool ok = true;
         const long long dbg_t0 = clock64();
-        WorkList list(p, cluster_id, num_clusters);
+        WorkList list(p.w, cluster_id, num_clusters);
         WorkItem x;
-        while (ok && list.next(p, x)) {
+        while (ok && list.next(p.w, x)) {
           const uint32_t kbn = x.un * STAGES_PER_UNIT;
           for (uint32_t kb = 0; kb < kbn; ++kb) {
             ok = ptx::mbar_wait_timed(ptx::smem_u32(&full_bar[s]), ph, abort_flag, p.status,
@@ -563,9 +494,9 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     // the converters see a plain stream of stages; only its length depends on the work items
     uint32_t total_stages = 0;
     {
-      WorkList list(p, cluster_id, num_clusters);
+      WorkList list(p.w, cluster_id, num_clusters);
       WorkItem x;
-      while (list.next(p, x)) total_stages += x.un * STAGES_PER_UNIT;
+      while (list.next(p.w, x)) total_stages += x.un * STAGES_PER_UNIT;
     }
     ConverterState st;
     st.raw_full = raw_full;
@@ -623,11 +554,11 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
                             static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2) * CPT;
     const uint32_t d0_empty_leader = ptx::map_to_cta(ptx::smem_u32(d0_empty), 0);
 
-    uint32_t d0_ph = 0, d1_ph = 0, tail_phase = 0;
+    uint32_t d0_ph = 0, d1_ph = 0;
     bool ok = true;
-    WorkList list(p, cluster_id, num_clusters);
+    WorkList list(p.w, cluster_id, num_clusters);
     WorkItem x;
-    while (ok && list.next(p, x)) {
+    while (ok && list.next(p.w, x)) {
       const uint32_t drains = x.un * STAGES_PER_UNIT;
       const uint32_t prefetch_at = (p.beta_r == 0.f && p.beta_i == 0.f) ? drains
                                    : (drains > C_PREFETCH_LEAD)         ? drains - C_PREFETCH_LEAD
@@ -697,15 +628,13 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
       // the finished sums stay in the D1 columns; from here on they are read from there, and what
       // the epilogue needs to know of the tile is worked out only now (epilogue.cuh)
       add_corrections_in_tmem<CPT>(t_sums, acc, LO_SCALE_INV);
-      const bool part = x.un != p.units; // this item is a piece of a tile
+      const bool part = x.un != p.w.units; // this item is a piece of a tile
       const TileCoord tc = tile_coord<BN>(opaque(x.tile), p, rank);
       const uint32_t quarter = static_cast<uint32_t>(warp & 3);
       const uint32_t col_base = static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2) * CPT;
       const uint32_t row =
           static_cast<uint32_t>(tc.m0) + quarter * 32u + static_cast<uint32_t>(lane);
       float *cbase = p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row;
-      if (p.slices > 1) // reduce mode: slice index = position of the cluster within its tile
-        cbase += static_cast<uint64_t>(cluster_id % p.slices) * p.slice_stride;
       const uint32_t d1_empty_leader = ptx::map_to_cta(ptx::smem_u32(d1_empty), 0);
       auto release_d1 = [&]() {
         ptx::tc_fence_before();
@@ -713,9 +642,8 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
         if (lane == 0) ptx::mbar_arrive_cluster(d1_empty_leader);
       };
 
-      if (part && p.slices <= 1) {
-        // ticket mode: park the partial sums, take a ticket, and go on to the epilogue only with
-        // the last ticket of this CTA's half of the tile
+      if (part) {
+        // park the partial sums for the kernel that adds the pieces
         constexpr uint32_t HALF = BN * BM_CTA; // floats of one CTA's half of a tile
         const uint32_t lane_off = col_base * BM_CTA + quarter * 32u + static_cast<uint32_t>(lane);
         float *mine = p.partial + static_cast<uint64_t>((cluster_id * 2u + x.slot) * 2u + rank) * HALF +
@@ -729,67 +657,11 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
           for (int i = 0; i < kEpiGroup; ++i)
             __stcg(mine + (c + i) * BM_CTA, __uint_as_float(v[i]));
         }
-        __threadfence();
-        // the eight epilogue warps meet twice: all partial sums stored; ticket published
-        auto meet = [&]() -> bool {
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(tail_bar));
-          const bool met = ptx::mbar_wait(ptx::smem_u32(tail_bar), tail_phase, abort_flag,
-                                          p.status, ptx::kErrWaitTail);
-          tail_phase ^= 1u;
-          return met;
-        };
-        ok = meet();
-        if (!ok) break;
-        // the clusters whose pieces make up this tile: those owning its first and last unit
-        const uint32_t ti = x.tile - p.whole_tiles;
-        const uint32_t total = (p.total_tiles - p.whole_tiles) * p.units;
-        const uint32_t pcs = p.piece_clusters;
-        const uint32_t ua = ti * p.units, ub = ua + p.units - 1u;
-        uint32_t c0 = static_cast<uint32_t>(static_cast<uint64_t>(ua) * pcs / total);
-        while (piece_start(c0 + 1u, total, pcs) <= ua) ++c0;
-        while (piece_start(c0, total, pcs) > ua) --c0;
-        uint32_t c1 = static_cast<uint32_t>(static_cast<uint64_t>(ub) * pcs / total);
-        while (piece_start(c1 + 1u, total, pcs) <= ub) ++c1;
-        while (piece_start(c1, total, pcs) > ub) --c1;
-        unsigned int *counter = p.counters + ti * 2u + rank;
-        if (warp == FIRST_EPI_WARP && lane == 0) {
-          const uint32_t t = atomicAdd(counter, 1u);
-          if (t == c1 - c0) *counter = 0; // all pieces are in: ready for the next launch
-          *ticket_smem = t;
-        }
-        ok = meet();
-        if (!ok) break;
-        if (*ticket_smem != c1 - c0) {
-          release_d1();
-          continue;
-        }
-        __threadfence();
-        // pieces in ascending k: the first is its cluster's second item unless that cluster's
-        // range begins with this tile; all others are their clusters' first items
-        const uint32_t slot0 = (piece_start(c0, total, pcs) < ua) ? 1u : 0u;
-        const float *src0 = p.partial + static_cast<uint64_t>((c0 * 2u + slot0) * 2u + rank) * HALF +
-                            lane_off;
-        const float *src1 = p.partial + static_cast<uint64_t>((c0 + 1u) * 4u + rank) * HALF + lane_off;
-#pragma unroll 1
-        for (int c = 0; c < CPT; c += kEpiGroup) {
-          float sum[kEpiGroup];
-#pragma unroll
-          for (int i = 0; i < kEpiGroup; ++i) sum[i] = __ldcg(src0 + (c + i) * BM_CTA);
-          const float *src = src1;
-          for (uint32_t cc = c0 + 1u; cc <= c1; ++cc, src += 4u * HALF) {
-#pragma unroll
-            for (int i = 0; i < kEpiGroup; ++i) sum[i] += __ldcg(src + (c + i) * BM_CTA);
-          }
-          uint32_t v[kEpiGroup];
-#pragma unroll
-          for (int i = 0; i < kEpiGroup; ++i) v[i] = __float_as_uint(sum[i]);
-          ptx::tmem_st_32x32b_x16(t_sums + c, v);
-        }
-        ptx::tmem_st_wait();
+        release_d1();
+        continue;
       }
 
-      const float unscale = (p.dyn != nullptr && p.slices <= 1) ? p.dyn->unscale_c : 1.f;
+      const float unscale = (p.dyn != nullptr) ? p.dyn->unscale_c : 1.f;
       store_tile<CPT>(t_sums, cbase, p.ldc, static_cast<uint32_t>(tc.n0) + col_base, p.n, row < p.m,
                       p.alpha_r * unscale, p.alpha_i * unscale, p.beta_r, p.beta_i,
                       (p.flags & kIsComplex) != 0);
@@ -918,17 +790,13 @@ template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, 
   p.dyn = a.dyn;
   p.status = a.dev_status;
   p.partial = a.partial;
-  p.counters = a.counters;
   p.debug = a.debug;
   p.ldc = a.ldc;
   p.stride_c = a.stride_c;
-  p.slice_stride = 0;
   p.m = a.m;
   p.n = a.n;
-  p.units = (a.k + 63) / 64;
   p.tiles_m = (a.m + 2 * BM_CTA - 1) / (2 * BM_CTA);
   p.tiles_n = (a.n + BN - 1) / BN;
-  p.total_tiles = p.tiles_m * p.tiles_n * a.batch;
   p.alpha_r = a.alpha_r;
   p.alpha_i = a.alpha_i;
   p.beta_r = a.beta_r;
@@ -940,32 +808,31 @@ template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, 
                                  (a.batch > 1 && a.a.stride != 0 ? kBatchA : 0) |
                                  (a.batch > 1 && a.b.stride != 0 ? kBatchB : 0));
   const StreamPlan &plan = a.plan;
-  if (plan.tile_n != BN || plan.total_tiles != p.total_tiles || plan.units != p.units)
+  if (plan.tile_n != BN || plan.total_tiles != p.tiles_m * p.tiles_n * a.batch ||
+      plan.units != (a.k + 63) / 64)
     return cudaErrorInvalidValue;
-  p.whole_tiles = plan.whole_tiles;
-  p.piece_clusters = static_cast<uint16_t>(plan.piece_clusters);
-  p.slices = static_cast<uint16_t>(plan.slices);
-  if (plan.slices > 1) {
-    p.c = a.partial;
-    p.ldc = a.m;
-    p.stride_c = static_cast<uint64_t>(a.m) * a.n;
-    p.slice_stride = p.stride_c * a.batch;
-    p.alpha_r = 1.f;
-    p.alpha_i = 0.f;
-    p.beta_r = 0.f;
-    p.beta_i = 0.f;
-    p.flags = static_cast<uint8_t>(p.flags & ~kIsComplex);
-  }
+  p.w.total_tiles = plan.total_tiles;
+  p.w.whole_tiles = plan.whole_tiles;
+  p.w.units = plan.units;
+  p.w.slice_units = 0;
+  p.w.piece_clusters = static_cast<uint16_t>(plan.piece_clusters);
+  p.w.slices = static_cast<uint16_t>(plan.slices);
   // direct stores: at least three waves of whole tiles of a short K loop, beta = 0 (with 256 columns
   // the sums leave too few registers for it)
   if (BN == 128 && plan.piece_clusters == 0 && plan.whole_tiles >= 3u * static_cast<uint32_t>(max_clusters) &&
-      p.units <= 16 && a.beta_r == 0.f && a.beta_i == 0.f)
+      plan.units <= 16 && a.beta_r == 0.f && a.beta_i == 0.f)
     p.flags |= kDirectStores;
   uint32_t clusters = plan.whole_tiles > plan.piece_clusters ? plan.whole_tiles : plan.piece_clusters;
   if (clusters > static_cast<uint32_t>(max_clusters)) clusters = static_cast<uint32_t>(max_clusters);
   if (clusters == 0 || plan.piece_clusters > clusters) return cudaErrorInvalidValue;
-  return launch_chained(tcec_gemm_stream_kernel<KIND, BN>, 2 * clusters, NUM_THREADS,
-                        StreamCfg<BN>::SMEM_BYTES, stream, map_a, map_b, p);
+  const cudaError_t e = launch_chained(tcec_gemm_stream_kernel<KIND, BN>, 2 * clusters, NUM_THREADS,
+                                       StreamCfg<BN>::SMEM_BYTES, stream, map_a, map_b, p);
+  if (e != cudaSuccess || plan.piece_clusters == 0) return e;
+  const PieceFixupArgs f = {a.partial,  a.c,       nullptr,   a.dyn,     a.ldc,
+                            a.stride_c, a.m,       a.n,       p.tiles_m, p.tiles_n,
+                            BN,         a.alpha_r, a.alpha_i, a.beta_r,  a.beta_i,
+                            a.is_complex};
+  return launch_piece_fixup(f, p.w, stream);
 }
 
 template <int BN> cudaError_t launch_by_kind(const StreamGemmArgs &a, cudaStream_t stream) {
@@ -996,14 +863,16 @@ StreamPlan plan_stream(const Tuning &tuning, int tile_n, uint64_t m, uint64_t n,
   pl.units = static_cast<uint32_t>(units);
   pl.whole_tiles = pl.total_tiles;
   const uint32_t rem = pl.total_tiles % clusters;
-  if (rem == 0 || 2 * rem > static_cast<uint32_t>(kStreamCounters)) return pl;
-  constexpr uint32_t kMinSliceUnits = 3;  // shortest slice / piece, in units of 64 k values
-  constexpr uint32_t kMinSavedUnits = 6;  // a cut has to save that much of a tile's K loop
+  if (rem == 0 || clusters > 0xffffu) return pl;
+  constexpr uint32_t kMinSliceUnits = 3; // shortest slice / piece, in units of 64 k values
+  // a cut has to save more than parking and adding the pieces costs: about 0.3 us per left-over
+  // tile, at 1.45 us per unit
+  const uint32_t min_saved = 2 + rem / 5;
   if (3 * pl.total_tiles <= clusters && tuning.split_k != 0) {
-    // few tiles: slices and a reduction kernel
+    // few tiles: each in the same number of slices
     uint32_t s = clusters / pl.total_tiles;
     if (s > pl.units / kMinSliceUnits) s = pl.units / kMinSliceUnits;
-    if (s >= 2 && pl.units - pl.units / s >= kMinSavedUnits) {
+    if (s >= 2 && pl.units - pl.units / s >= min_saved + 2) {
       pl.whole_tiles = 0;
       pl.slices = s;
       pl.piece_clusters = s * pl.total_tiles;
@@ -1014,19 +883,15 @@ StreamPlan plan_stream(const Tuning &tuning, int tile_n, uint64_t m, uint64_t n,
   const uint64_t left = static_cast<uint64_t>(rem) * pl.units;
   uint32_t pc = clusters;
   if (left / kMinSliceUnits < pc) pc = static_cast<uint32_t>(left / kMinSliceUnits);
-  // pieces of equal length that end where the tiles end need one ticket less per tile
-  if (pc > rem && pc < 2 * rem + rem / 4 && pc >= 2 * rem) pc = 2 * rem;
   if (pc <= rem) return pl;
   const uint32_t per = static_cast<uint32_t>((left + pc - 1) / pc);
-  if (per + kMinSavedUnits > pl.units) return pl;
+  if (per + min_saved > pl.units) return pl;
   pl.whole_tiles = pl.total_tiles - rem;
   pl.piece_clusters = pc;
   return pl;
 }
 
-std::size_t stream_scratch_bytes(const StreamPlan &plan, uint32_t m, uint32_t n, uint32_t batch) {
-  if (plan.slices > 1)
-    return static_cast<std::size_t>(plan.slices) * m * n * batch * sizeof(float);
+std::size_t stream_scratch_bytes(const StreamPlan &plan) {
   return static_cast<std::size_t>(plan.piece_clusters) * 2u * 2u * BM_CTA *
          static_cast<std::size_t>(plan.tile_n) * sizeof(float);
 }

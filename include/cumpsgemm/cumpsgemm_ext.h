@@ -155,7 +155,8 @@ void cuMpSGEMM_reload_tuning_env(cuMpSGEMM_handle_t handle);
  * of 256 x 256 with a K loop of k_pad values (a multiple of 64; tf32 != 0 for the TF32 kinds) on
  * `clusters` CTA pairs.  Tiles [0, *split_begin) run whole; each later tile (the last, partly
  * filled wave) is cut into *slices K slices of *slice_k values, *work_items work items in
- * all.  *slices == 1: nothing is cut.  Returns 0, or 1 for invalid arguments.  No counterpart
+ * all.  *slices == 1: nothing is cut into slices (a last wave that is more than half full may
+ * instead be shared by all pairs in K pieces of equal length).  Returns 0, or 1 for invalid arguments.  No counterpart
  * in the reference (its atomic split-K kernel, src/cumpsgemm.cu:272-304, is the nearest
  * relative). */
 int cuMpSGEMM_plan_pair_tail(unsigned total_tiles, unsigned clusters, unsigned k_pad, int tf32,
