@@ -47,6 +47,52 @@ __device__ __forceinline__ uint64_t panel_offset(uint64_t r, uint64_t kk, uint32
   return ((kk / KBE) * rows_pad + r) * KBE + (kk % KBE);
 }
 
+// Eight lanes (g = 0..7) share the 64 k values of a row.  Which of them lane g converts is chosen so
+// that every 16-byte store of the eight lanes together fills whole 128-byte lines of the panel: 8g
+// ... 8g + 7 for FP16 (one store per plane), 4g ... 4g + 3 and 32 + 4g ... for TF32 (two).
+template <int KIND> __device__ __forceinline__ int k_of(int g, int j) {
+  if constexpr (KIND == 0) return 8 * g + j;
+  return (j < 4) ? 4 * g + j : 32 + 4 * g + (j - 4);
+}
+
+// Splits lane g's eight values of row r, k values k0 + k_of(g, j), and stores them to the panel
+// (`batch_off`: first element of this batch entry's hi plane).
+template <int KIND>
+__device__ __forceinline__ void convert_store8(const float (&v)[8], void *panel, uint64_t batch_off,
+                                               uint64_t r, uint64_t k0, int g, uint32_t rows_pad,
+                                               uint64_t plane_elems, uint32_t planes) {
+  if constexpr (KIND == 0) {
+    __align__(16) __half hi[8];
+    __align__(16) __half lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      hi[j] = __float2half_rn(v[j]);
+      lo[j] = __float2half_rn((v[j] - __half2float(hi[j])) * 2048.f);
+    }
+    __half *ph = reinterpret_cast<__half *>(panel) + batch_off +
+                 panel_offset<KIND>(r, k0 + 8 * g, rows_pad);
+    *reinterpret_cast<uint4 *>(ph) = *reinterpret_cast<const uint4 *>(hi);
+    if (planes == 2)
+      *reinterpret_cast<uint4 *>(ph + plane_elems) = *reinterpret_cast<const uint4 *>(lo);
+  } else {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      __align__(16) float hi[4];
+      __align__(16) float lo[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        hi[j] = to_tf32(v[4 * half + j]);
+        lo[j] = to_tf32(v[4 * half + j] - hi[j]);
+      }
+      float *ph = reinterpret_cast<float *>(panel) + batch_off +
+                  panel_offset<KIND>(r, k0 + 32 * half + 4 * g, rows_pad);
+      *reinterpret_cast<uint4 *>(ph) = *reinterpret_cast<const uint4 *>(hi);
+      if (planes == 2)
+        *reinterpret_cast<uint4 *>(ph + plane_elems) = *reinterpret_cast<const uint4 *>(lo);
+    }
+  }
+}
+
 struct SplitParams {
   const float *src; // complex sources are addressed as pairs of floats
   const float *const *src_array; // pointer-array batches: matrix b starts at src_array[b]
@@ -111,36 +157,42 @@ __device__ __forceinline__ void split_generic_body(const SplitParams &p, const u
       tile[r][2 * kk + 1] = (p.conj ? -v[q].y : v[q].y) * scale;
     }
   } else {
-    for (int idx = threadIdx.x; idx < SR * SK; idx += THREADS) {
-      int r, kk;
-      if (p.src_k_contig) {
-        kk = idx % SK;
-        r = idx / SK;
-      } else {
-        r = idx % SR;
-        kk = idx / SR;
-      }
-      const uint64_t gr = r0 + r, gk = k0 + kk;
-      float re = 0.f;
-      if (gr < p.rows && gk < p.k)
-        re = src[p.src_k_contig ? (gk + gr * p.ld) : (gr + gk * p.ld)] * scale;
-      tile[r][kk] = re;
+    // Real: sources whose rows do not start on 16-byte boundaries, read 4 bytes per lane along the
+    // contiguous dimension, all sixteen loads of a thread issued before the first store.  (One load
+    // per store and a division per element, as first written: 47 us for the 56 MB of operands of
+    // 1999 x 3001 x 2777, now 22; the panels are another 58 MB.)
+    constexpr int PER = SR * SK / THREADS;
+    const int fast = threadIdx.x % TILE, slow = threadIdx.x / TILE; // SR == SK == TILE
+    constexpr int STEP = THREADS / TILE;
+    float v[PER];
+    const bool kc = p.src_k_contig != 0;
+    const uint64_t f0 = (kc ? k0 : r0) + fast, s0 = (kc ? r0 : k0) + slow;
+    const uint64_t f_end = kc ? p.k : p.rows, s_end = kc ? p.rows : p.k;
+    const float *q = src + f0 + s0 * p.ld;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      v[i] = (f0 < f_end && s0 + i * STEP < s_end) ? *q : 0.f;
+      q += STEP * p.ld;
     }
+    // lanes run along k or along the rows; a row of the tile is 65 floats, so neither conflicts
+    float *t = kc ? &tile[slow][fast] : &tile[fast][slow];
+    const int step = kc ? STEP * (TILE + 1) : STEP;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) t[i * step] = v[i] * scale;
   }
   __syncthreads();
 
-  // ---- phase 2: each thread converts 8 consecutive expanded-K values of one expanded row
+  // ---- phase 2: each thread converts 8 expanded-K values of one expanded row
   const uint64_t er0 = static_cast<uint64_t>(bid.y) * TILE; // expanded row origin
   const uint64_t ek0 = static_cast<uint64_t>(bid.x) * TILE; // expanded K origin
   const uint64_t plane_elems = static_cast<uint64_t>(p.rows_pad) * p.k_pad;
 #pragma unroll
   for (int it = 0; it < TILE * TILE / (THREADS * 8); ++it) {
     const int er = (threadIdx.x >> 3) + it * (THREADS >> 3);
-    const int ek = (threadIdx.x & 7) * 8;
     float v[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int c = ek + j;
+      const int c = k_of<KIND>(threadIdx.x & 7, j);
       if constexpr (MODE == 0 || MODE == 2) {
         v[j] = tile[er][c];
       } else {
@@ -152,76 +204,14 @@ __device__ __forceinline__ void split_generic_body(const SplitParams &p, const u
         v[j] = (!im_row && odd) ? -x : x;
       }
     }
-    const uint64_t out_off = panel_offset<KIND>(er0 + er, ek0 + ek, p.rows_pad);
-    if constexpr (KIND == 0) {
-      __align__(16) __half hi[8];
-      __align__(16) __half lo[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        hi[j] = __float2half_rn(v[j]);
-        lo[j] = __float2half_rn((v[j] - __half2float(hi[j])) * 2048.f);
-      }
-      __half *ph = reinterpret_cast<__half *>(p.panel) +
-                   static_cast<uint64_t>(b) * p.planes * plane_elems + out_off;
-      *reinterpret_cast<uint4 *>(ph) = *reinterpret_cast<const uint4 *>(hi);
-      if (p.planes == 2)
-        *reinterpret_cast<uint4 *>(ph + plane_elems) = *reinterpret_cast<const uint4 *>(lo);
-    } else {
-      __align__(16) float hi[8];
-      __align__(16) float lo[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        hi[j] = to_tf32(v[j]);
-        lo[j] = to_tf32(v[j] - hi[j]);
-      }
-      float *ph = reinterpret_cast<float *>(p.panel) +
-                  static_cast<uint64_t>(b) * p.planes * plane_elems + out_off;
-      reinterpret_cast<uint4 *>(ph)[0] = reinterpret_cast<const uint4 *>(hi)[0];
-      reinterpret_cast<uint4 *>(ph)[1] = reinterpret_cast<const uint4 *>(hi)[1];
-      if (p.planes == 2) {
-        reinterpret_cast<uint4 *>(ph + plane_elems)[0] = reinterpret_cast<const uint4 *>(lo)[0];
-        reinterpret_cast<uint4 *>(ph + plane_elems)[1] = reinterpret_cast<const uint4 *>(lo)[1];
-      }
-    }
+    convert_store8<KIND>(v, p.panel, static_cast<uint64_t>(b) * p.planes * plane_elems, er0 + er, ek0,
+                         threadIdx.x & 7, p.rows_pad, plane_elems, p.planes);
   }
 }
 
 // ---------------------------------------------------------------- vectorised real paths
 // Used when the source base address, leading dimension and batch stride are multiples of
 // 16 bytes; anything else (and every complex operand) takes split_kernel above.
-
-template <int KIND>
-__device__ __forceinline__ void convert_store8(const float (&v)[8], void *panel, uint64_t off,
-                                               uint64_t plane_elems, uint32_t planes) {
-  if constexpr (KIND == 0) {
-    __align__(16) __half hi[8];
-    __align__(16) __half lo[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      hi[j] = __float2half_rn(v[j]);
-      lo[j] = __float2half_rn((v[j] - __half2float(hi[j])) * 2048.f);
-    }
-    __half *ph = reinterpret_cast<__half *>(panel) + off;
-    *reinterpret_cast<uint4 *>(ph) = *reinterpret_cast<const uint4 *>(hi);
-    if (planes == 2)
-      *reinterpret_cast<uint4 *>(ph + plane_elems) = *reinterpret_cast<const uint4 *>(lo);
-  } else {
-    __align__(16) float hi[8];
-    __align__(16) float lo[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      hi[j] = to_tf32(v[j]);
-      lo[j] = to_tf32(v[j] - hi[j]);
-    }
-    float *ph = reinterpret_cast<float *>(panel) + off;
-    reinterpret_cast<uint4 *>(ph)[0] = reinterpret_cast<const uint4 *>(hi)[0];
-    reinterpret_cast<uint4 *>(ph)[1] = reinterpret_cast<const uint4 *>(hi)[1];
-    if (planes == 2) {
-      reinterpret_cast<uint4 *>(ph + plane_elems)[0] = reinterpret_cast<const uint4 *>(lo)[0];
-      reinterpret_cast<uint4 *>(ph + plane_elems)[1] = reinterpret_cast<const uint4 *>(lo)[1];
-    }
-  }
-}
 
 // float4 at p if the whole vector is inside [.., limit), element-wise with zero fill otherwise
 __device__ __forceinline__ float4 load4_guarded(const float *p, uint64_t first, uint64_t limit,
@@ -247,7 +237,9 @@ __device__ __forceinline__ void split_kcontig_body(const SplitParams &p, const u
   }
   const uint32_t b = bid.z;
   const float *src = p.src + static_cast<uint64_t>(b) * p.stride;
-  const uint64_t k0 = static_cast<uint64_t>(bid.x) * 64 + (threadIdx.x & 7) * 8;
+  const int g = threadIdx.x & 7;
+  const uint64_t k0 = static_cast<uint64_t>(bid.x) * 64;
+  const uint64_t ka = k0 + k_of<KIND>(g, 0), kb = k0 + k_of<KIND>(g, 4); // its two groups of four
   const uint64_t r_base = static_cast<uint64_t>(bid.y) * 128 + (threadIdx.x >> 3);
   const uint64_t plane_elems = static_cast<uint64_t>(p.rows_pad) * p.k_pad;
   float4 x[4][2];
@@ -255,9 +247,9 @@ __device__ __forceinline__ void split_kcontig_body(const SplitParams &p, const u
   for (int i = 0; i < 4; ++i) {
     const uint64_t r = r_base + i * 32;
     const bool row_ok = r < p.rows;
-    const float *q = src + r * p.ld + k0;
-    x[i][0] = load4_guarded(q, k0, p.k, row_ok);
-    x[i][1] = load4_guarded(q + 4, k0 + 4, p.k, row_ok);
+    const float *q = src + r * p.ld;
+    x[i][0] = load4_guarded(q + ka, ka, p.k, row_ok);
+    x[i][1] = load4_guarded(q + kb, kb, p.k, row_ok);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -265,10 +257,8 @@ __device__ __forceinline__ void split_kcontig_body(const SplitParams &p, const u
     if (r >= p.rows_pad) continue;
     const float v[8] = {x[i][0].x * scale, x[i][0].y * scale, x[i][0].z * scale, x[i][0].w * scale,
                         x[i][1].x * scale, x[i][1].y * scale, x[i][1].z * scale, x[i][1].w * scale};
-    convert_store8<KIND>(v, p.panel,
-                         static_cast<uint64_t>(b) * p.planes * plane_elems +
-                             panel_offset<KIND>(r, k0, p.rows_pad),
-                         plane_elems, p.planes);
+    convert_store8<KIND>(v, p.panel, static_cast<uint64_t>(b) * p.planes * plane_elems, r, k0, g,
+                         p.rows_pad, plane_elems, p.planes);
   }
 }
 
@@ -308,43 +298,43 @@ __device__ __forceinline__ void split_rcontig_body(const SplitParams &p, const u
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
     const int er = (threadIdx.x >> 3) + it * 32;
-    const int ek = (threadIdx.x & 7) * 8;
     float v[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = tile[er][ek + j];
-    convert_store8<KIND>(v, p.panel,
-                         static_cast<uint64_t>(b) * p.planes * plane_elems +
-                             panel_offset<KIND>(r0 + er, k0 + ek, p.rows_pad),
-                         plane_elems, p.planes);
+    for (int j = 0; j < 8; ++j) v[j] = tile[er][k_of<KIND>(threadIdx.x & 7, j)];
+    convert_store8<KIND>(v, p.panel, static_cast<uint64_t>(b) * p.planes * plane_elems, r0 + er, k0,
+                         threadIdx.x & 7, p.rows_pad, plane_elems, p.planes);
   }
 }
 
 // Which body handles an operand.
 enum SplitPath : int { kPathReal = 0, kPathComplexA = 1, kPathComplexB = 2, kPathKContig = 3, kPathRContig = 4 };
 
-// VEC = false leaves the vectorised bodies out, which keeps the register count of the
-// latency-bound generic bodies low (30 instead of 64: twice the resident blocks).
-template <int KIND, bool VEC>
+// Which bodies a kernel contains.  Both operands of a call are real or both complex; keeping the
+// sets apart keeps the register counts of the latency-bound generic bodies low, which is what
+// decides how many of their blocks are resident.
+enum SplitSet : int { kSetComplex = 0, kSetReal = 1, kSetRealVec = 2 };
+template <int SET> constexpr int min_blocks() { return SET == kSetRealVec ? 5 : 6; }
+
+template <int KIND, int SET>
 __device__ __forceinline__ void split_dispatch(const SplitParams &p, int path, const uint3 bid,
                                                float (*tile)[TILE + 1]) {
-  if constexpr (!VEC) {
-    if (path == kPathReal) split_generic_body<KIND, 0>(p, bid, tile);
-    else if (path == kPathComplexA) split_generic_body<KIND, 1>(p, bid, tile);
+  if constexpr (SET == kSetComplex) {
+    if (path == kPathComplexA) split_generic_body<KIND, 1>(p, bid, tile);
     else split_generic_body<KIND, 2>(p, bid, tile);
-    return;
-  }
-  // Both operands of a call are real or both complex, and complex ones never take a
-  // vectorised body, so this instantiation leaves the complex bodies (and their registers) out.
-  switch (path) {
-  case kPathReal:
+  } else if constexpr (SET == kSetReal) {
     split_generic_body<KIND, 0>(p, bid, tile);
-    break;
-  case kPathKContig:
-    split_kcontig_body<KIND>(p, bid);
-    break;
-  default:
-    split_rcontig_body<KIND>(p, bid, tile);
-    break;
+  } else {
+    switch (path) {
+    case kPathReal:
+      split_generic_body<KIND, 0>(p, bid, tile);
+      break;
+    case kPathKContig:
+      split_kcontig_body<KIND>(p, bid);
+      break;
+    default:
+      split_rcontig_body<KIND>(p, bid, tile);
+      break;
+    }
   }
 }
 
@@ -363,8 +353,9 @@ __device__ __forceinline__ void zero_word(unsigned int *z) {
   if (z != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *z = 0u;
 }
 
-template <int KIND, bool VEC>
-__global__ void __launch_bounds__(THREADS, VEC ? 5 : 6) split_dual_kernel(const SplitJob a, const SplitJob b, unsigned int *z) {
+template <int KIND, int SET>
+__global__ void __launch_bounds__(THREADS, min_blocks<SET>())
+    split_dual_kernel(const SplitJob a, const SplitJob b, unsigned int *z) {
   __shared__ float tile[TILE][TILE + 1]; // transposing staging tile shared by all paths
   // Chained behind the kernel that writes the scaling constants (AUTO / FP16TCEC_SCALING), and
   // the GEMM kernel that follows may be scheduled while this one drains: its prologue does not
@@ -376,15 +367,15 @@ __global__ void __launch_bounds__(THREADS, VEC ? 5 : 6) split_dual_kernel(const 
   const SplitJob &j = (id < blocks_a) ? a : b;
   if (id >= blocks_a) id -= blocks_a;
   const uint3 bid = make_uint3(id % j.gx, (id / j.gx) % j.gy, id / (j.gx * j.gy));
-  split_dispatch<KIND, VEC>(j.p, j.path, bid, tile);
+  split_dispatch<KIND, SET>(j.p, j.path, bid, tile);
 }
 
 // AUTO: the kind (FP16 or TF32 panels) is decided on the device.  Job geometry, source
 // addressing and the workspace are the same for both kinds, so one launch reads the decision
 // and runs the matching bodies (the reference launches the kernels of both kinds and lets the
 // deselected one exit, src/cumpsgemm_kernel.cuh:478-489).
-template <bool VEC>
-__global__ void __launch_bounds__(THREADS, VEC ? 5 : 6)
+template <int SET>
+__global__ void __launch_bounds__(THREADS, min_blocks<SET>())
     split_dual_auto_kernel(const SplitJob a, const SplitJob b, unsigned int *z) {
   __shared__ float tile[TILE][TILE + 1];
   CUMPSGEMM_CHAINED_KERNEL_ENTRY(); // see split_dual_kernel
@@ -395,9 +386,9 @@ __global__ void __launch_bounds__(THREADS, VEC ? 5 : 6)
   if (id >= blocks_a) id -= blocks_a;
   const uint3 bid = make_uint3(id % j.gx, (id / j.gx) % j.gy, id / (j.gx * j.gy));
   if (j.p.dyn->gemm_mode == CUMPSGEMM_TF32TCEC)
-    split_dispatch<1, VEC>(j.p, j.path, bid, tile);
+    split_dispatch<1, SET>(j.p, j.path, bid, tile);
   else
-    split_dispatch<0, VEC>(j.p, j.path, bid, tile);
+    split_dispatch<0, SET>(j.p, j.path, bid, tile);
 }
 
 bool make_job(const SplitArgs &a, SplitJob *job) {
@@ -437,6 +428,11 @@ bool make_job(const SplitArgs &a, SplitJob *job) {
   return static_cast<uint64_t>(job->gx) * job->gy * job->gz <= 0x3fffffffull;
 }
 
+SplitSet split_set(const SplitArgs &a, const SplitJob &ja, const SplitJob &jb) {
+  if (a.is_complex) return kSetComplex;
+  return (ja.path >= kPathKContig || jb.path >= kPathKContig) ? kSetRealVec : kSetReal;
+}
+
 } // namespace
 
 cudaError_t launch_split_pair_auto(const SplitArgs &a, const SplitArgs &b, cudaStream_t stream) {
@@ -447,11 +443,31 @@ cudaError_t launch_split_pair_auto(const SplitArgs &a, const SplitArgs &b, cudaS
   const uint64_t blocks = static_cast<uint64_t>(ja.gx) * ja.gy * ja.gz +
                           static_cast<uint64_t>(jb.gx) * jb.gy * jb.gz;
   if (blocks == 0 || blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-  const bool vec = (ja.path >= kPathKContig) || (jb.path >= kPathKContig);
   const unsigned grid = static_cast<unsigned>(blocks);
-  if (vec) return launch_chained(split_dual_auto_kernel<true>, grid, THREADS, 0, stream, ja, jb, z);
-  return launch_chained(split_dual_auto_kernel<false>, grid, THREADS, 0, stream, ja, jb, z);
+  switch (split_set(a, ja, jb)) {
+  case kSetComplex:
+    return launch_chained(split_dual_auto_kernel<kSetComplex>, grid, THREADS, 0, stream, ja, jb, z);
+  case kSetReal:
+    return launch_chained(split_dual_auto_kernel<kSetReal>, grid, THREADS, 0, stream, ja, jb, z);
+  default:
+    return launch_chained(split_dual_auto_kernel<kSetRealVec>, grid, THREADS, 0, stream, ja, jb, z);
+  }
 }
+
+namespace {
+template <int KIND>
+cudaError_t launch_set(SplitSet set, unsigned grid, cudaStream_t stream, const SplitJob &ja,
+                       const SplitJob &jb, unsigned int *z) {
+  switch (set) {
+  case kSetComplex:
+    return launch_chained(split_dual_kernel<KIND, kSetComplex>, grid, THREADS, 0, stream, ja, jb, z);
+  case kSetReal:
+    return launch_chained(split_dual_kernel<KIND, kSetReal>, grid, THREADS, 0, stream, ja, jb, z);
+  default:
+    return launch_chained(split_dual_kernel<KIND, kSetRealVec>, grid, THREADS, 0, stream, ja, jb, z);
+  }
+}
+} // namespace
 
 cudaError_t launch_split_pair(const SplitArgs &a, const SplitArgs &b, cudaStream_t stream) {
   if (a.kind != b.kind) return cudaErrorInvalidValue;
@@ -461,14 +477,10 @@ cudaError_t launch_split_pair(const SplitArgs &a, const SplitArgs &b, cudaStream
   const uint64_t blocks = static_cast<uint64_t>(ja.gx) * ja.gy * ja.gz +
                           static_cast<uint64_t>(jb.gx) * jb.gy * jb.gz;
   if (blocks == 0 || blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-  const bool vec = (ja.path >= kPathKContig) || (jb.path >= kPathKContig);
   const unsigned grid = static_cast<unsigned>(blocks);
-  if (a.kind == SplitKind::fp16) {
-    if (vec) return launch_chained(split_dual_kernel<0, true>, grid, THREADS, 0, stream, ja, jb, z);
-    return launch_chained(split_dual_kernel<0, false>, grid, THREADS, 0, stream, ja, jb, z);
-  }
-  if (vec) return launch_chained(split_dual_kernel<1, true>, grid, THREADS, 0, stream, ja, jb, z);
-  return launch_chained(split_dual_kernel<1, false>, grid, THREADS, 0, stream, ja, jb, z);
+  const SplitSet set = split_set(a, ja, jb);
+  return a.kind == SplitKind::fp16 ? launch_set<0>(set, grid, stream, ja, jb, z)
+                                   : launch_set<1>(set, grid, stream, ja, jb, z);
 }
 
 } // namespace cumpsgemm_b200
