@@ -78,10 +78,15 @@ __device__ __forceinline__ void scale_items(const ScaleParams &s, float coef) {
   }
 }
 
+// All kernels here and the scans are chained (launch_chained): a caller that drives statistics,
+// scaling, GEMM and un-scaling itself issues thirteen launches, nine of them 2 us long, and the
+// gaps between them were as long again (4096 x 1024 x 2048: 152 -> 129 us for the whole sequence).
+
 // which: 0 = operand A, 1 = operand B.  inverse = false: X *= 2^14 / max; true: X *= max / 2^14.
 __global__ void __launch_bounds__(THREADS)
     scale_ab_kernel(const ScaleParams s, const int *flag, const float *max_slot, int which,
                     int inverse) {
+  CUMPSGEMM_CHAINED_KERNEL_ENTRY();
   if (flag != nullptr) {
     const int f = *flag;
     if (which == 0 && !flag_scale_a(f)) return;
@@ -95,6 +100,7 @@ __global__ void __launch_bounds__(THREADS)
 
 __global__ void __launch_bounds__(THREADS)
     scale_c_kernel(const ScaleParams s, const int *flag, const float *max_a, const float *max_b) {
+  CUMPSGEMM_CHAINED_KERNEL_ENTRY();
   const float ma = *max_a, mb = *max_b;
   if (ma == 0.f || mb == 0.f) return;
   float coef = 1.f;
@@ -110,6 +116,7 @@ __global__ void __launch_bounds__(THREADS)
 }
 
 __global__ void flag_from_stats_kernel(int *flag, const int *mode_a, const int *mode_b) {
+  CUMPSGEMM_CHAINED_KERNEL_ENTRY();
   const int pa = *mode_a, pb = *mode_b;
   if (pa == CUMPSGEMM_TF32TCEC || pb == CUMPSGEMM_TF32TCEC) {
     *flag = CUMPSGEMM_TF32TCEC;
@@ -200,19 +207,22 @@ void launch_scaling(cuMpSGEMM_handle *h, ScaleOp op, unsigned m, unsigned n, T *
   case ScaleOp::scale_a:
   case ScaleOp::scale_b:
     if (prof) h->exp_stats.profiler.start("scaling_AB", h->cuda_stream);
-    scale_ab_kernel<<<grid, THREADS, 0, h->cuda_stream>>>(
-        s, flag, h->exp_stats.dev_max + stats_id_a, op == ScaleOp::scale_a ? 0 : 1, 0);
+    launch_chained(scale_ab_kernel, grid, THREADS, 0, h->cuda_stream, s, flag,
+                   static_cast<const float *>(h->exp_stats.dev_max + stats_id_a),
+                   op == ScaleOp::scale_a ? 0 : 1, 0);
     if (prof) h->exp_stats.profiler.stop("scaling_AB", h->cuda_stream);
     break;
   case ScaleOp::reset_a:
   case ScaleOp::reset_b:
-    scale_ab_kernel<<<grid, THREADS, 0, h->cuda_stream>>>(
-        s, flag, h->exp_stats.dev_max + stats_id_a, op == ScaleOp::reset_a ? 0 : 1, 1);
+    launch_chained(scale_ab_kernel, grid, THREADS, 0, h->cuda_stream, s, flag,
+                   static_cast<const float *>(h->exp_stats.dev_max + stats_id_a),
+                   op == ScaleOp::reset_a ? 0 : 1, 1);
     break;
   case ScaleOp::scale_c:
     if (prof) h->exp_stats.profiler.start("scaling_C", h->cuda_stream);
-    scale_c_kernel<<<grid, THREADS, 0, h->cuda_stream>>>(s, flag, h->exp_stats.dev_max + stats_id_a,
-                                                         h->exp_stats.dev_max + stats_id_b);
+    launch_chained(scale_c_kernel, grid, THREADS, 0, h->cuda_stream, s, flag,
+                   static_cast<const float *>(h->exp_stats.dev_max + stats_id_a),
+                   static_cast<const float *>(h->exp_stats.dev_max + stats_id_b));
     if (prof) h->exp_stats.profiler.stop("scaling_C", h->cuda_stream);
     break;
   }
@@ -344,9 +354,9 @@ void set_dynamic_launch_buffer_by_exp_stats(cuMpSGEMM_handle *handle,
                                             const unsigned A_exp_stats_buffer_id,
                                             const unsigned B_exp_stats_buffer_id) {
   DeviceGuard guard(handle->device);
-  flag_from_stats_kernel<<<1, 1, 0, handle->cuda_stream>>>(
-      handle->dyn_launch.flag_buffer + dynamic_launch_buffer_id,
-      handle->exp_stats.dev_mode + A_exp_stats_buffer_id,
-      handle->exp_stats.dev_mode + B_exp_stats_buffer_id);
+  launch_chained(flag_from_stats_kernel, 1, 1, 0, handle->cuda_stream,
+                 handle->dyn_launch.flag_buffer + dynamic_launch_buffer_id,
+                 static_cast<const int *>(handle->exp_stats.dev_mode + A_exp_stats_buffer_id),
+                 static_cast<const int *>(handle->exp_stats.dev_mode + B_exp_stats_buffer_id));
 }
 } // namespace cumpsgemm

@@ -25,7 +25,10 @@ namespace cumpsgemm_b200 {
 namespace {
 
 constexpr int THREADS = 256;
-constexpr int CHUNK = 16384; // floats of one column handled per work item
+// Floats of one column handled per work item: CHUNK_STEP (four 16-byte loads per thread, all in
+// flight) times 1 to 4, the fewest that leaves no more items than resident CTAs.  With four always,
+// a 1024 x 2048 matrix kept 128 CTAs busy for 10 us per scan.
+constexpr uint32_t CHUNK_STEP = 4096;
 
 struct ScanParams {
   const float *ptr;   // complex input viewed as floats
@@ -36,6 +39,7 @@ struct ScanParams {
   uint32_t batch;
   uint64_t chunks_per_col;
   uint64_t items;     // batch * n * chunks_per_col
+  uint32_t chunk;     // floats per item
   int vec_ok;         // pointer, ld and stride allow aligned float4 access
   // Zero values the reference's stage kernels append to the tail of every matrix when m*n is
   // not a multiple of 4 and then count like data (0 unless the compatibility switch is on).
@@ -43,8 +47,9 @@ struct ScanParams {
 };
 
 // Collapse contiguous storage into one long column so that small matrices still vectorise.
-ScanParams make_scan(const void *ptr, uint64_t m, uint64_t n, uint64_t ld, uint32_t batch,
-                     uint64_t stride, int floats_per_elem, bool count_tail_padding = false) {
+ScanParams make_scan(const cuMpSGEMM_handle *h, const void *ptr, uint64_t m, uint64_t n, uint64_t ld,
+                     uint32_t batch, uint64_t stride, int floats_per_elem,
+                     bool count_tail_padding = false) {
   ScanParams s;
   s.pad_values = 0;
   if (count_tail_padding) {
@@ -67,7 +72,11 @@ ScanParams make_scan(const void *ptr, uint64_t m, uint64_t n, uint64_t ld, uint3
       s.batch = 1;
     }
   }
-  s.chunks_per_col = (s.m + CHUNK - 1) / CHUNK;
+  const uint64_t steps = static_cast<uint64_t>(s.batch) * s.n * ((s.m + CHUNK_STEP - 1) / CHUNK_STEP);
+  const uint64_t ctas = static_cast<uint64_t>(h->num_sms) * 8;
+  s.chunk = CHUNK_STEP *
+            (steps <= ctas ? 1u : steps <= 2 * ctas ? 2u : steps <= 3 * ctas ? 3u : 4u);
+  s.chunks_per_col = (s.m + s.chunk - 1) / s.chunk;
   s.items = static_cast<uint64_t>(s.batch) * s.n * s.chunks_per_col;
   s.vec_ok = ((reinterpret_cast<uintptr_t>(ptr) & 15u) == 0) && (s.ld % 4 == 0) &&
              (s.stride % 4 == 0);
@@ -100,13 +109,23 @@ __device__ __forceinline__ void scan_items(const ScanParams &s, Acc &a, float ig
                                            float uf_thr, unsigned int bid = blockIdx.x,
                                            unsigned int nblocks = gridDim.x) {
   for (uint64_t item = bid; item < s.items; item += nblocks) {
-    const uint64_t chunk = item % s.chunks_per_col;
-    const uint64_t col_id = item / s.chunks_per_col;
-    const uint64_t col = col_id % s.n;
-    const uint64_t b = col_id / s.n;
+    uint64_t chunk, col, b;
+    if (s.items <= 0xffffffffull) { // (then every factor fits too: short 32-bit divisions)
+      const uint32_t i32 = static_cast<uint32_t>(item);
+      const uint32_t cpc = static_cast<uint32_t>(s.chunks_per_col), n32 = static_cast<uint32_t>(s.n);
+      const uint32_t col_id = i32 / cpc;
+      chunk = i32 - col_id * cpc;
+      b = col_id / n32;
+      col = col_id - static_cast<uint32_t>(b) * n32;
+    } else {
+      chunk = item % s.chunks_per_col;
+      const uint64_t col_id = item / s.chunks_per_col;
+      col = col_id % s.n;
+      b = col_id / s.n;
+    }
     const float *p = s.ptr + b * s.stride + col * s.ld;
-    const uint64_t begin = chunk * CHUNK;
-    const uint64_t end = min(s.m, begin + CHUNK);
+    const uint64_t begin = chunk * s.chunk;
+    const uint64_t end = min(s.m, begin + s.chunk);
     if (s.vec_ok) {
       // begin is a multiple of 4 and the column start is 16-byte aligned
       const uint64_t vec_end = begin + ((end - begin) & ~3ull);
@@ -407,6 +426,7 @@ __device__ __forceinline__ void fused_max_body(const ScanParams &s, float *max_s
 __global__ void __launch_bounds__(THREADS, 8)
     fused_stage1_kernel(const ScanParams s, const StatSlots o, float ignore_thr, float uf_thr,
                         float tolerance, ScanPartial *partials, unsigned int *ticket) {
+  CUMPSGEMM_CHAINED_KERNEL_ENTRY();
   fused_stage1_body(s, o, ignore_thr, uf_thr, tolerance, partials, ticket, blockIdx.x, gridDim.x);
 }
 
@@ -414,6 +434,7 @@ __global__ void __launch_bounds__(THREADS, 8)
     fused_stage2_kernel(const ScanParams s, const StatSlots o, float half_ignore_thr,
                         float half_uf_thr, float tolerance, ScanPartial *partials,
                         unsigned int *ticket) {
+  CUMPSGEMM_CHAINED_KERNEL_ENTRY();
   fused_stage2_body(s, o, half_ignore_thr, half_uf_thr, tolerance, partials, ticket, blockIdx.x,
                     gridDim.x);
 }
@@ -421,6 +442,7 @@ __global__ void __launch_bounds__(THREADS, 8)
 __global__ void __launch_bounds__(THREADS, 8)
     fused_max_only_kernel(const ScanParams s, float *max_slot, ScanPartial *partials,
                           unsigned int *ticket) {
+  CUMPSGEMM_CHAINED_KERNEL_ENTRY();
   fused_max_body(s, max_slot, partials, ticket, blockIdx.x, gridDim.x);
 }
 
@@ -544,7 +566,7 @@ void exp_stats_init_slot(cuMpSGEMM_handle *h, unsigned id) {
 template <class T>
 void exp_stats_stage1(cuMpSGEMM_handle *h, unsigned id, unsigned m, unsigned n, const T *ptr,
                       unsigned ld, unsigned batch, unsigned stride) {
-  const ScanParams s = make_scan(ptr, m, n, ld, batch, stride, floats_per_elem<T>(),
+  const ScanParams s = make_scan(h, ptr, m, n, ld, batch, stride, floats_per_elem<T>(),
                                  h->exp_stats.count_tail_padding);
   stage1_kernel<<<scan_grid(h, s), THREADS, 0, h->cuda_stream>>>(
       s, h->exp_stats.dev_max + id, h->exp_stats.dev_total + id, h->exp_stats.dev_underflow + id,
@@ -560,7 +582,7 @@ void exp_stats_decide1(cuMpSGEMM_handle *h, unsigned id) {
 template <class T>
 void exp_stats_stage2(cuMpSGEMM_handle *h, unsigned id, unsigned m, unsigned n, const T *ptr,
                       unsigned ld, unsigned batch, unsigned stride) {
-  const ScanParams s = make_scan(ptr, m, n, ld, batch, stride, floats_per_elem<T>(),
+  const ScanParams s = make_scan(h, ptr, m, n, ld, batch, stride, floats_per_elem<T>(),
                                  h->exp_stats.count_tail_padding);
   stage2_kernel<<<scan_grid(h, s), THREADS, 0, h->cuda_stream>>>(
       s, h->exp_stats.dev_mode + id, h->exp_stats.dev_max + id, h->exp_stats.dev_total + id,
@@ -583,7 +605,7 @@ void exp_max_only(cuMpSGEMM_handle *h, unsigned id, unsigned m, unsigned n, cons
     init_slot_kernel<<<1, 1, 0, h->cuda_stream>>>(h->exp_stats.dev_max + id, nullptr, nullptr);
   }
   ScopedTimer t(h, "exp_max");
-  const ScanParams s = make_scan(ptr, m, n, ld, batch, stride, floats_per_elem<T>());
+  const ScanParams s = make_scan(h, ptr, m, n, ld, batch, stride, floats_per_elem<T>());
   max_only_kernel<<<scan_grid(h, s), THREADS, 0, h->cuda_stream>>>(s, h->exp_stats.dev_max + id);
 }
 
@@ -604,23 +626,23 @@ inline StatSlots stat_slots(cuMpSGEMM_handle *h, unsigned id) {
 template <class T>
 void exp_stats_fused(cuMpSGEMM_handle *h, unsigned id, unsigned m, unsigned n, const T *ptr,
                      unsigned ld, unsigned batch, unsigned stride) {
-  const ScanParams s = make_scan(ptr, m, n, ld, batch, stride, floats_per_elem<T>(),
+  const ScanParams s = make_scan(h, ptr, m, n, ld, batch, stride, floats_per_elem<T>(),
                                  h->exp_stats.count_tail_padding);
   auto &es = h->exp_stats;
-  fused_stage1_kernel<<<scan_grid(h, s), THREADS, 0, h->cuda_stream>>>(
-      s, stat_slots(h, id), es.ignore_threshold, es.underflow_threshold,
-      es.underflow_tolerance_rate, scan_partials(h), scan_tickets(h));
-  fused_stage2_kernel<<<scan_grid(h, s), THREADS, 0, h->cuda_stream>>>(
-      s, stat_slots(h, id), es.ignore_threshold / 2, es.underflow_threshold / 2,
-      es.underflow_tolerance_rate, scan_partials(h), scan_tickets(h));
+  launch_chained(fused_stage1_kernel, scan_grid(h, s), THREADS, 0, h->cuda_stream, s,
+                 stat_slots(h, id), es.ignore_threshold, es.underflow_threshold,
+                 es.underflow_tolerance_rate, scan_partials(h), scan_tickets(h));
+  launch_chained(fused_stage2_kernel, scan_grid(h, s), THREADS, 0, h->cuda_stream, s,
+                 stat_slots(h, id), es.ignore_threshold / 2, es.underflow_threshold / 2,
+                 es.underflow_tolerance_rate, scan_partials(h), scan_tickets(h));
 }
 
 template <class T>
 void exp_max_fused(cuMpSGEMM_handle *h, unsigned id, unsigned m, unsigned n, const T *ptr,
                    unsigned ld, unsigned batch, unsigned stride) {
-  const ScanParams s = make_scan(ptr, m, n, ld, batch, stride, floats_per_elem<T>());
-  fused_max_only_kernel<<<scan_grid(h, s), THREADS, 0, h->cuda_stream>>>(
-      s, h->exp_stats.dev_max + id, scan_partials(h), scan_tickets(h));
+  const ScanParams s = make_scan(h, ptr, m, n, ld, batch, stride, floats_per_elem<T>());
+  launch_chained(fused_max_only_kernel, scan_grid(h, s), THREADS, 0, h->cuda_stream, s,
+                 h->exp_stats.dev_max + id, scan_partials(h), scan_tickets(h));
 }
 
 // Statistics (full = true) or maximum exponent only of the two operands of a GEMM, two slots,
@@ -631,8 +653,8 @@ void exp_stats_pair(cuMpSGEMM_handle *h, bool full, unsigned id_a, unsigned am, 
                     unsigned bn, const T *b, unsigned ldb, unsigned stride_b, unsigned batch) {
   DualScan d;
   const bool pad = full && h->exp_stats.count_tail_padding;
-  d.s[0] = make_scan(a, am, an, lda, batch, stride_a, floats_per_elem<T>(), pad);
-  d.s[1] = make_scan(b, bm, bn, ldb, batch, stride_b, floats_per_elem<T>(), pad);
+  d.s[0] = make_scan(h, a, am, an, lda, batch, stride_a, floats_per_elem<T>(), pad);
+  d.s[1] = make_scan(h, b, bm, bn, ldb, batch, stride_b, floats_per_elem<T>(), pad);
   d.o[0] = stat_slots(h, id_a);
   d.o[1] = stat_slots(h, id_b);
   d.grid_a = scan_grid(h, d.s[0]);

@@ -37,7 +37,19 @@ bool ensure_workspace(cuMpSGEMM_handle *h, std::size_t bytes) {
   return true;
 }
 
+// Whether the workspace can be grown now: not while the stream is being captured into a graph,
+// where an allocation would end the capture.
+bool may_allocate(const cuMpSGEMM_handle *h) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->cuda_stream, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return cap == cudaStreamCaptureStatusNone;
+}
+
 __global__ void dyn_params_from_flag_kernel(DynParams *out, const int *flag) {
+  CUMPSGEMM_CHAINED_KERNEL_ENTRY();
   out->scale_a = 1.f;
   out->scale_b = 1.f;
   out->unscale_c = 1.f;
@@ -268,7 +280,7 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
       sb > kMaxStride)
     return false;
   const std::uint64_t m_exp = m * fpe, k_exp = k * fpe;
-  if (batch > 0x3fffffffull) return false;
+  if (batch > 0x3fffffffull || n > 0x3fffffffull) return false; // (TMA coordinates are 32-bit)
   const int tile_n = (t.stream == 128 || t.stream == 256) ? t.stream : (n <= 128 ? 128 : 256);
   int clusters = 0;
   if (stream_max_clusters(tile_n, &clusters) != cudaSuccess) {
@@ -413,7 +425,8 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
     DynParams *slot = h->dev_dyn_params + h->dyn_params_next;
     h->dyn_params_next = (h->dyn_params_next + 1) % h->dyn_params_length;
     const unsigned id = h->dyn_launch.enabled ? h->dyn_launch.enabled_id : 0u;
-    dyn_params_from_flag_kernel<<<1, 1, 0, h->cuda_stream>>>(slot, h->dyn_launch.flag_buffer + id);
+    launch_chained(dyn_params_from_flag_kernel, 1, 1, 0, h->cuda_stream, slot,
+                   static_cast<const int *>(h->dyn_launch.flag_buffer + id));
     dyn = slot;
   }
 
@@ -445,7 +458,14 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
       const std::size_t bytes = stream_scratch_bytes(ga.plan);
       const std::size_t limit =
           h->workspace_limit_bytes ? h->workspace_limit_bytes : kDefaultWorkspaceLimit;
-      room = bytes <= limit && ensure_workspace(h, bytes);
+      if (h->workspace_bytes < bytes && (bytes > limit || !may_allocate(h))) {
+        // no room for the pieces' sums: whole tiles only, which need no memory
+        ga.plan.whole_tiles = ga.plan.total_tiles;
+        ga.plan.piece_clusters = 0;
+        ga.plan.slices = 0;
+      } else {
+        room = ensure_workspace(h, bytes);
+      }
     }
     if (room) {
       ga.c = reinterpret_cast<float *>(c);
@@ -472,9 +492,11 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
       }
       cudaError_t gerr = launch_tcec_gemm_stream(ga, h->cuda_stream);
       const bool addressable = gerr != cudaErrorNotSupported;
-      if (h->kernel_timing) {
+      if (h->kernel_timing && addressable) {
         cudaEventRecord(tt.e[2], h->cuda_stream);
         h->timing_events.push_back(tt);
+      } else if (h->kernel_timing) {
+        for (auto &e : tt.e) cudaEventDestroy(e);
       }
       if (prof) h->exp_stats.profiler.stop("gemm_kernel", h->cuda_stream);
       if (addressable) {
@@ -569,12 +591,16 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
   // split-K partial sums: k_slices blocks of m x n floats per batch entry, behind the panels
   const std::size_t bytes_p_1 =
       (k_slices > 1) ? static_cast<std::size_t>(k_slices) * m_exp * n * sizeof(float) : 0;
-  // scratch of the pair kernel's tail split (once per call, behind everything else)
-  const std::size_t bytes_tail = use_pair ? pair_tail_scratch_bytes(h->num_sms) : 0;
+  // scratch for the K pieces of pair tiles (once per call, behind everything else)
+  std::size_t bytes_tail = use_pair ? pair_tail_scratch_bytes(h->num_sms) : 0;
   std::uint64_t chunk = std::max<std::uint64_t>(1, limit / (bytes_a_1 + bytes_b_1 + bytes_p_1));
   chunk = std::min<std::uint64_t>(chunk, batch);
   chunk = std::min<std::uint64_t>(chunk, 32768); // planes of a tensor map, tiles of a launch
-  if (!ensure_workspace(h, chunk * (bytes_a_1 + bytes_b_1 + bytes_p_1) + bytes_tail)) {
+  const std::size_t bytes_panels = chunk * (bytes_a_1 + bytes_b_1 + bytes_p_1);
+  if (bytes_tail > 0 && h->workspace_bytes < bytes_panels + bytes_tail &&
+      h->workspace_bytes >= bytes_panels && !may_allocate(h))
+    bytes_tail = 0; // captured with a workspace that only holds the panels: no pieces
+  if (!ensure_workspace(h, bytes_panels + bytes_tail)) {
     log_error("failed to allocate the operand workspace");
     return CUBLAS_STATUS_ALLOC_FAILED;
   }
@@ -659,7 +685,7 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
     g.tuning = h->tuning;
     g.k_slices = k_slices;
     g.partial = (k_slices > 1) ? ws_p : nullptr;
-    g.tail_partial = use_pair ? ws_t : nullptr;
+    g.tail_partial = bytes_tail > 0 ? ws_t : nullptr;
     if (auto_kind)
       err = use_pair ? launch_tcec_gemm_pair_auto(g, h->cuda_stream)
                      : launch_tcec_gemm_auto(g, h->cuda_stream);

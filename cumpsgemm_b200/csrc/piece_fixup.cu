@@ -49,6 +49,15 @@ __global__ void __launch_bounds__(256 * GROUPS) piece_fixup_kernel(const FixupPa
   const uint32_t pieces = tp.c1 - tp.c0 + 1u;
   const uint32_t group = threadIdx.x >> 8;
   const uint32_t first = pieces * group / GROUPS, last = pieces * (group + 1u) / GROUPS;
+  const bool read_c = (p.beta_r != 0.f) || (p.beta_i != 0.f);
+  const bool row_ok = row < p.m;
+  float *cp = ((p.c_array != nullptr) ? p.c_array[pos.batch]
+                                      : p.c + static_cast<uint64_t>(pos.batch) * p.stride_c) +
+              static_cast<uint64_t>(col0) * p.ldc + row;
+  float old[COLS]; // on their way while the pieces are added
+#pragma unroll
+  for (uint32_t j = 0; j < COLS; ++j)
+    old[j] = (read_c && group == 0 && row_ok && col0 + j < p.n) ? __ldcs(cp + j * p.ldc) : 0.f;
   float sum[COLS];
 #pragma unroll
   for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
@@ -74,15 +83,6 @@ __global__ void __launch_bounds__(256 * GROUPS) piece_fixup_kernel(const FixupPa
   const float unscale = (p.dyn != nullptr) ? p.dyn->unscale_c : 1.f;
   const float ar = p.alpha_r * unscale, ai = p.alpha_i * unscale;
   const float sgn = (r & 1u) ? 1.f : -1.f; // odd rows hold imaginary parts
-  const bool read_c = (p.beta_r != 0.f) || (p.beta_i != 0.f);
-  const bool row_ok = row < p.m;
-  float *cp = ((p.c_array != nullptr) ? p.c_array[pos.batch]
-                                      : p.c + static_cast<uint64_t>(pos.batch) * p.stride_c) +
-              static_cast<uint64_t>(col0) * p.ldc + row;
-  float old[COLS];
-#pragma unroll
-  for (uint32_t j = 0; j < COLS; ++j)
-    old[j] = (read_c && row_ok && col0 + j < p.n) ? __ldcs(cp + j * p.ldc) : 0.f;
 #pragma unroll
   for (uint32_t j = 0; j < COLS; ++j) {
     float out = ar * sum[j];
