@@ -57,6 +57,11 @@ DevPtr = Union[int, "torch.Tensor"]  # noqa: F821
 
 
 def _ptr(x: DevPtr) -> int:
+    try:  # a CUDA tensor, the usual case: three operands per call come through here
+        if x.is_cuda:
+            return x.data_ptr()
+    except AttributeError:
+        pass
     if isinstance(x, int):
         return x
     if hasattr(x, "data_ptr"):
@@ -69,18 +74,22 @@ def _ptr(x: DevPtr) -> int:
 def _is_complex(x: DevPtr, hint: Optional[bool]) -> bool:
     if hint is not None:
         return hint
-    if hasattr(x, "is_complex"):
-        return bool(x.is_complex())
+    try:
+        return x.is_complex()
+    except AttributeError:
+        pass
     raise ValueError("pass complex=True/False when operands are raw addresses")
 
 
+_ComplexScalar = C.c_float * 2
+
+
 def _scalar(value, is_complex: bool):
+    """alpha / beta as a pointer argument (the argument keeps its storage alive)."""
     if is_complex:
         z = complex(value)
-        arr = (C.c_float * 2)(z.real, z.imag)
-    else:
-        arr = (C.c_float * 1)(float(value))
-    return arr
+        return C.byref(_ComplexScalar(z.real, z.imag))
+    return C.byref(C.c_float(float(value)))
 
 
 def compute_mode_string(mode: int) -> str:
@@ -141,8 +150,8 @@ class Handle:
         cplx = _is_complex(A, complex)
         fn = self._lib.cuMpSGEMM_cgemm if cplx else self._lib.cuMpSGEMM_sgemm
         a, b = _scalar(alpha, cplx), _scalar(beta, cplx)
-        st = fn(self._h, op_A, op_B, m, n, k, C.cast(a, C.c_void_p), _ptr(A), lda, _ptr(B), ldb,
-                C.cast(b, C.c_void_p), _ptr(Cmat), ldc, int(mode))
+        st = fn(self._h, op_A, op_B, m, n, k, a, _ptr(A), lda, _ptr(B), ldb,
+                b, _ptr(Cmat), ldc, int(mode))
         if check and st != CUBLAS_STATUS_SUCCESS:
             raise CuMpSGEMMError(st, "cuMpSGEMM_cgemm" if cplx else "cuMpSGEMM_sgemm")
         return st
@@ -156,8 +165,8 @@ class Handle:
         fn = (self._lib.cuMpSGEMM_cgemm_strided_batch if cplx
               else self._lib.cuMpSGEMM_sgemm_strided_batch)
         a, b = _scalar(alpha, cplx), _scalar(beta, cplx)
-        st = fn(self._h, op_A, op_B, m, n, k, C.cast(a, C.c_void_p), _ptr(A), lda, stridea,
-                _ptr(B), ldb, strideb, C.cast(b, C.c_void_p), _ptr(Cmat), ldc, stridec,
+        st = fn(self._h, op_A, op_B, m, n, k, a, _ptr(A), lda, stridea,
+                _ptr(B), ldb, strideb, b, _ptr(Cmat), ldc, stridec,
                 batch_count, int(mode))
         if check and st != CUBLAS_STATUS_SUCCESS:
             raise CuMpSGEMMError(st, "cuMpSGEMM_*gemm_strided_batch")
@@ -172,8 +181,8 @@ class Handle:
         fn = (self._lib.cuMpSGEMM_cgemm_strided_batch_with_stats if cplx
               else self._lib.cuMpSGEMM_sgemm_strided_batch_with_stats)
         a, b = _scalar(alpha, cplx), _scalar(beta, cplx)
-        st = fn(self._h, op_A, op_B, m, n, k, C.cast(a, C.c_void_p), _ptr(A), lda, stridea,
-                _ptr(B), ldb, strideb, C.cast(b, C.c_void_p), _ptr(Cmat), ldc, stridec,
+        st = fn(self._h, op_A, op_B, m, n, k, a, _ptr(A), lda, stridea,
+                _ptr(B), ldb, strideb, b, _ptr(Cmat), ldc, stridec,
                 batch_count, int(mode), stats_id_a, stats_id_b)
         if st != CUBLAS_STATUS_SUCCESS:
             raise CuMpSGEMMError(st, "cuMpSGEMM_*gemm_strided_batch_with_stats")
@@ -188,8 +197,8 @@ class Handle:
         cplx = _is_complex(A, complex)
         name = "cuMpSGEMM_%sgemm_%s" % ("c" if cplx else "s", "Mx2x2" if long_is_m else "2xNx2")
         a, b = _scalar(alpha, cplx), _scalar(beta, cplx)
-        st = getattr(self._lib, name)(self._h, op_A, op_B, length, C.cast(a, C.c_void_p), _ptr(A),
-                                      lda, stridea, _ptr(B), ldb, strideb, C.cast(b, C.c_void_p),
+        st = getattr(self._lib, name)(self._h, op_A, op_B, length, a, _ptr(A),
+                                      lda, stridea, _ptr(B), ldb, strideb, b,
                                       _ptr(Cmat), ldc, stridec, batch_count)
         if check and st != CUBLAS_STATUS_SUCCESS:
             raise CuMpSGEMMError(st, name)
@@ -201,8 +210,8 @@ class Handle:
         a, b = _scalar(alpha, False), _scalar(beta, False)
         mod = C.c_uint(0xFFFFFFFF)
         st = self._lib.cuMpSGEMM_sgemm_module(self._h, op_A, op_B, m, n, k,
-                                              C.cast(a, C.c_void_p), _ptr(A), lda, _ptr(B), ldb,
-                                              C.cast(b, C.c_void_p), _ptr(Cmat), ldc, int(mode),
+                                              a, _ptr(A), lda, _ptr(B), ldb,
+                                              b, _ptr(Cmat), ldc, int(mode),
                                               C.byref(mod))
         return st, mod.value
 
@@ -396,8 +405,8 @@ def sgemm_static_scratch(stream, op_A: int, op_B: int, m: int, n: int, k: int, a
     s = 0 if stream is None else getattr(stream, "cuda_stream", stream)
     a, b = _scalar(alpha, False), _scalar(beta, False)
     return lib.cuMpSGEMM_sgemm_static_scratch(C.c_void_p(int(s)), op_A, op_B, m, n, k,
-                                              C.cast(a, C.c_void_p), _ptr(A), lda, _ptr(B), ldb,
-                                              C.cast(b, C.c_void_p), _ptr(Cmat), ldc, int(mode))
+                                              a, _ptr(A), lda, _ptr(B), ldb,
+                                              b, _ptr(Cmat), ldc, int(mode))
 
 
 # ---------------------------------------------------------------------- convenience

@@ -434,12 +434,20 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
   const std::uint64_t m_exp = m * fpe; // rows of the expanded real problem
   const std::uint64_t k_exp = k * fpe;
 
+  // A single wave of 128 x 64 tiles and at most 12 units of K: that tile has the smallest constant and
+  // the smallest slope of all estimates then, so a small call, whose time is mostly the host's,
+  // does not work the others out.
+  const bool small = ec && batch < 8 && k_exp <= 768 && m_exp + n <= 4096 &&
+                     h->tuning.untouched() &&
+                     ((m_exp + 127) / 128) * ((n + 63) / 64) * batch <= h->num_sms;
+
   // ---- the pre-split path's tile or K slices, and what it would take
   const bool auto_kind = want_fp16 && want_tf32;
   const StreamKind stream_kind = auto_kind ? StreamKind::device
                                  : want_fp16 ? StreamKind::fp16 : StreamKind::tf32;
-  PresplitChoice pre = choose_presplit(h, m_exp, n, k_exp, batch, ec, want_tf32, !ptr_arrays);
-  if (auto_kind)
+  PresplitChoice pre = {{64, false, 0.0}, 1, 0.0};
+  if (!small) pre = choose_presplit(h, m_exp, n, k_exp, batch, ec, want_tf32, !ptr_arrays);
+  if (auto_kind && !small)
     pre.us = 0.5 * (pre.us + choose_presplit(h, m_exp, n, k_exp, batch, ec, false, !ptr_arrays).us);
 
   // ---- one launch on CTA pairs, operands split between TMA and the tensor core
@@ -447,10 +455,10 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
   // (batches of matrices with at most 128 rows would leave one CTA of every pair idle: the kernel
   // below serves those it can, 2048 x 128^3 82 us against 95-110 here)
   FusedGemmArgs fa;
-  const bool fused = mode == CUMPSGEMM_FP16TCEC && !ptr_arrays &&
+  const bool fused = !small && mode == CUMPSGEMM_FP16TCEC && !ptr_arrays &&
                      fused_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch,
                                    &fa);
-  if (ec && !ptr_arrays && !(fused && batch >= 8 && m_exp <= 128 && h->tuning.stream == -1) &&
+  if (!small && ec && !ptr_arrays && !(fused && batch >= 8 && m_exp <= 128 && h->tuning.stream == -1) &&
       stream_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, stream_kind,
                      pre.us, &ga)) {
     bool room = true;

@@ -85,6 +85,9 @@ struct Tuning {
   int tail_split = -1; // CUMPSGEMM_TAIL_SPLIT: 0 = never, -1 = by rule, n > 1 = at most n slices
   int stream = -1;     // CUMPSGEMM_STREAM: 0 / 1 the pair kernel that splits its operands off / on
                        // wherever it is applicable, 256 / 128 on with that tile width, -1 by rule
+  bool untouched() const {
+    return stream == -1 && split_k == -1 && tail_split == -1 && !others_forced();
+  }
   // a switch of one of the other kernels or of their schedules is set
   bool others_forced() const {
     return tile_n != 0 || pair != -1 || drain_chunk != 0 || first_chunk != 0 || pace != 1 ||
