@@ -13,12 +13,13 @@
 //   * The array is kStaticScratchBytes (32 MiB) per GPU, resident from library load to
 //     process exit on every GPU that loads the library.  The panels of a call need
 //     2 * (round_up(m, tile_m) + round_up(n, tile_n)) * round_up(k,64) * elem bytes
-//     (elem = 2 for FP16TCEC, 4 for TF32TCEC; tile_m x tile_n is the tile the library's one
-//     tile rule picks for the shape: 256 x 256 when the CTA-pair kernel runs, else 128 x
-//     256 / 128 / 64; the environment overrides CUMPSGEMM_TILE_N and CUMPSGEMM_PAIR apply
-//     here as everywhere).  The bound that holds for every tile choice is
-//     2 * (round_up(m,256) + round_up(n,256)) * round_up(k,64) * elem <= 32 MiB; e.g.
-//     FP16TCEC m=n=k=2048 fits exactly.  Larger problems are rejected with
+//     (elem = 2 for FP16TCEC, 4 for TF32TCEC).  tile_m x tile_n is the tile the library's one
+//     tile rule picks for the shape (256 x 256 when the CTA-pair kernel runs, else 128 x 256 /
+//     128 / 64) if its panels fit, else the widest narrower single-CTA tile whose panels do; so
+//     every problem with
+//     2 * (round_up(m,128) + round_up(n,64)) * round_up(k,64) * elem <= 32 MiB is computed, e.g.
+//     FP16TCEC m=n=k=2048, which fits exactly.  A tile forced with CUMPSGEMM_TILE_N or
+//     CUMPSGEMM_PAIR is kept.  Larger problems are rejected with
 //     CUBLAS_STATUS_INVALID_VALUE and an error line; nothing is launched.
 //   * The first call on each device looks up the device address of the array
 //     (cudaGetSymbolAddress) and sets the kernels' shared-memory attribute.  Make that first
@@ -107,16 +108,29 @@ extern "C" cublasStatus_t cuMpSGEMM_sgemm_static_scratch(
   const Tuning tuning = read_tuning_env(); // no handle to cache them in
   const TileChoice choice = pick_tile(tuning, static_cast<unsigned>(pd->num_sms), m, n, k, 1, true,
                                       kind == SplitKind::tf32, false);
-  const int tile_n = choice.tile_n;
-  const bool use_pair = choice.pair;
-  const std::uint64_t rows_pad_a = round_up(m, use_pair ? 256 : 128);
-  const std::uint64_t rows_pad_b = round_up(n, tile_n);
+  int tile_n = choice.tile_n;
+  bool use_pair = choice.pair;
   const std::uint64_t k_pad = round_up(k, 64);
-  // Each factor is below 2^31, so the row sum times k_pad stays below 2^63 / 8 only after this
-  // first test; the byte counts are formed afterwards and cannot wrap.
+  std::uint64_t rows_pad_a = 0, rows_pad_b = 0;
+  // Each factor is below 2^31, so the row sum times k_pad stays below 2^63 / 8 only after the
+  // first two tests; the byte counts are formed afterwards and cannot wrap.
   const std::uint64_t max_elems = kStaticScratchBytes / (2 * es);
-  const bool fits = (rows_pad_a + rows_pad_b) <= max_elems && k_pad <= max_elems &&
-                    (rows_pad_a + rows_pad_b) * k_pad <= max_elems;
+  auto panels_fit = [&]() {
+    rows_pad_a = round_up(m, use_pair ? 256 : 128);
+    rows_pad_b = round_up(n, tile_n);
+    return (rows_pad_a + rows_pad_b) <= max_elems && k_pad <= max_elems &&
+           (rows_pad_a + rows_pad_b) * k_pad <= max_elems;
+  };
+  bool fits = panels_fit();
+  // The fastest tile is often not the one with the least padding: where its panels do not fit the
+  // array, the narrower single-CTA tiles are tried before the call is refused (a caller without a
+  // way to allocate has nothing to fall back on), unless a tuning variable forces the tile.
+  const bool forced = tuning.tile_n != 0 || tuning.pair == 1;
+  while (!fits && !forced && (use_pair || tile_n > 64)) {
+    if (use_pair) use_pair = false;
+    else tile_n /= 2;
+    fits = panels_fit();
+  }
   const std::uint64_t bytes_a = fits ? 2 * rows_pad_a * k_pad * es : 0;
   const std::uint64_t bytes_b = fits ? 2 * rows_pad_b * k_pad * es : 0;
   if (!fits) {

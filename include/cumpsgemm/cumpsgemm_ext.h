@@ -300,10 +300,10 @@ cublasStatus_t cuMpSGEMM_cgemm_2xNx2(cuMpSGEMM_handle_t handle, cublasOperation_
  *   - Problems whose panels exceed 32 MiB return CUBLAS_STATUS_INVALID_VALUE with an error
  *     line and launch nothing.  FP16TCEC panels take 4*(round_up(m,tile_m)+round_up(n,tile_n))*
  *     round_up(k,64) bytes, TF32TCEC twice that, where tile_m x tile_n is the tile the library
- *     picks for the shape (256 x 256 with the CTA-pair kernel, else 128 x 256/128/64; the
- *     CUMPSGEMM_TILE_N / CUMPSGEMM_PAIR overrides count).  Whatever the tile,
- *     4*(round_up(m,256)+round_up(n,256))*round_up(k,64) <= 32 MiB always fits (FP16TCEC;
- *     m=n=k=2048 fits exactly).
+ *     picks for the shape (256 x 256 with the CTA-pair kernel, else 128 x 256/128/64), or a
+ *     narrower one where that does not fit: whatever has
+ *     4*(round_up(m,128)+round_up(n,64))*round_up(k,64) <= 32 MiB is computed (FP16TCEC;
+ *     m=n=k=2048 fits exactly).  A tile forced with CUMPSGEMM_TILE_N / CUMPSGEMM_PAIR is kept.
  *   - The first call on a device resolves the array's device address and configures the
  *     kernels; issue it before any stream capture on that device.
  *   - The array is shared by all calls on a GPU: calls that overlap in time on one GPU race.
