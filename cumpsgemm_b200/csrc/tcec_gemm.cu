@@ -67,9 +67,6 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
   constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, BM, BN);
   constexpr int CPT = BN / 2; // accumulator columns per epilogue thread
 
-  // Gated launch: leave at once when the device-side decision picked the other kind.
-  if (p.dyn != nullptr && p.dyn->gemm_mode != MY_MODE) return;
-
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -130,7 +127,18 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
   const bool dbg = (p.debug != nullptr);
   unsigned long long dbg_wait = 0, dbg_wait2 = 0;
 
-  if (warp == 0) {
+  // Gated launch: nothing to do when the device-side decision picked the other kind.  The
+  // decision is written by a kernel in front of the split pass.  That the split pass has waited
+  // for it says that the write is done; that this grid sees it, the wait here says.
+  bool mine = true;
+  if (p.dyn != nullptr) {
+    ptx::griddep_wait();
+    mine = p.dyn->gemm_mode == MY_MODE;
+  }
+
+  if (!mine) {
+    // straight to the teardown
+  } else if (warp == 0) {
     // ================================================================ TMA producer
     if (ptx::elect_one()) {
       // launched with programmatic serialization behind the split pass: everything up to here
@@ -219,6 +227,9 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
     const uint32_t lane_addr = (quarter * 32u) << 16;
     const uint32_t col_base = half * CPT;
 
+    // C and the scaling constants belong to earlier work on the stream; nothing is lost, the first
+    // finished chunk comes after the panels
+    ptx::griddep_wait();
     float acc[CPT];
 #pragma unroll
     for (int i = 0; i < CPT; ++i) acc[i] = 0.f;
@@ -304,6 +315,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                           const __grid_constant__ CUtensorMap map_b16, const KernelParams p16,
                           const __grid_constant__ CUtensorMap map_a32,
                           const __grid_constant__ CUtensorMap map_b32, const KernelParams p32) {
+  ptx::griddep_wait(); // the decision is written by an earlier kernel of the call
   if (p16.dyn->gemm_mode == CUMPSGEMM_TF32TCEC)
     tcec_gemm_body<1, BN, true>(map_a32, map_b32, p32);
   else

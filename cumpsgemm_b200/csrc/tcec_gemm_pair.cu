@@ -97,8 +97,6 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
   constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, 2 * BM_CTA, BN_PAIR);
   constexpr int CPT = BN_PAIR / 2;
 
-  if (p.dyn != nullptr && p.dyn->gemm_mode != MY_MODE) return; // uniform over the cluster
-
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -148,7 +146,19 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
   const bool dbg = (p.debug != nullptr);
   unsigned long long dbg_wait = 0, dbg_wait2 = 0;
 
-  if (warp == 0) {
+  // Gated launch: nothing to do when the device-side decision picked the other kind (uniform
+  // over the grid).  The decision is written by a kernel in front of the split pass.  That the
+  // split pass has waited for it says that the write is done; that this grid sees it, the wait
+  // here says.
+  bool mine = true;
+  if (p.dyn != nullptr) {
+    ptx::griddep_wait();
+    mine = p.dyn->gemm_mode == MY_MODE;
+  }
+
+  if (!mine) {
+    // straight to the teardown
+  } else if (warp == 0) {
     // ================================================================ TMA producer (both CTAs)
     if (ptx::elect_one()) {
       // launched with programmatic serialization behind the split pass, which also zeroes the
@@ -427,6 +437,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
                                const __grid_constant__ CUtensorMap map_a32,
                                const __grid_constant__ CUtensorMap map_b32,
                                const GemmKernelParams p32, const PairPlan plan) {
+  ptx::griddep_wait(); // the decision is written by an earlier kernel of the call
   if (p16.dyn->gemm_mode == CUMPSGEMM_TF32TCEC) {
     pair_body<1>(map_a32, map_b32, p32, plan);
   } else {
