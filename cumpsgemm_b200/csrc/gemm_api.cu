@@ -25,8 +25,11 @@ inline std::uint64_t round_up(std::uint64_t x, std::uint64_t a) { return (x + a 
 
 bool ensure_workspace(cuMpSGEMM_handle *h, std::size_t bytes) {
   if (h->workspace_bytes >= bytes) return true;
-  // cudaFree waits for work that may still read the old buffer.
-  if (h->workspace != nullptr) cudaFree(h->workspace);
+  if (h->workspace != nullptr) {
+    if (h->workspace_in_graph) h->graph_workspaces.push_back(h->workspace);
+    else cudaFree(h->workspace); // waits for work that may still read the old buffer
+  }
+  h->workspace_in_graph = false;
   h->workspace = nullptr;
   h->workspace_bytes = 0;
   if (cudaMalloc(&h->workspace, bytes) != cudaSuccess) {

@@ -135,6 +135,7 @@ extern "C" cublasStatus_t cuMpSGEMM_destroy(cuMpSGEMM_handle_t handle) {
   cudaFree(handle->dev_dyn_params);
   cudaFree(handle->dev_status);
   cudaFree(handle->workspace);
+  for (void *w : handle->graph_workspaces) cudaFree(w);
   if (handle->order_event != nullptr) cudaEventDestroy(handle->order_event);
   delete handle;
   return CUBLAS_STATUS_SUCCESS;

@@ -145,6 +145,11 @@ struct cuMpSGEMM_handle {
   void *workspace = nullptr;
   std::size_t workspace_bytes = 0;
   std::size_t workspace_limit_bytes = 0; // 0 = derive from free memory
+  // A call was captured into a graph while the handle had this workspace: the graph writes to it on
+  // every replay, so when a later call needs a larger one it is kept (here) until the handle is
+  // destroyed instead of being freed.
+  bool workspace_in_graph = false;
+  std::vector<void *> graph_workspaces;
 
   cumpsgemm_b200::Tuning tuning;
 
@@ -176,8 +181,9 @@ struct cuMpSGEMM_handle {
 namespace cumpsgemm_b200 {
 
 // Record the handle's ordering event behind the work just enqueued (see cuMpSGEMM_handle).
-// Skipped while the stream is being captured into a graph: a captured event cannot order
-// work outside the capture, and a graph replays as one unit of its launch stream anyway.
+// Not while the stream is being captured into a graph: a captured event cannot order work outside
+// the capture, and a graph replays as one unit of its launch stream anyway.  What is noted then is
+// that a graph may hold the address of the workspace.
 inline void mark_stream_work(cuMpSGEMM_handle *h) {
   if (h->order_event == nullptr) return;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -185,7 +191,10 @@ inline void mark_stream_work(cuMpSGEMM_handle *h) {
     cudaGetLastError();
     return;
   }
-  if (cap != cudaStreamCaptureStatusNone) return;
+  if (cap != cudaStreamCaptureStatusNone) {
+    h->workspace_in_graph = h->workspace != nullptr;
+    return;
+  }
   if (cudaEventRecord(h->order_event, h->cuda_stream) == cudaSuccess)
     h->order_event_recorded = true;
   else

@@ -1,0 +1,82 @@
+"""The handle's workspace: who may free it, and when it may grow."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from cumpsgemm_b200 import api  # noqa: E402
+
+N, T = api.CUBLAS_OP_N, api.CUBLAS_OP_T
+FP16TCEC, TF32TCEC = api.ComputeMode.FP16TCEC, api.ComputeMode.TF32TCEC
+SLACK = 4 << 20                                   # granularity of cudaMalloc
+
+
+def _free_bytes():
+    import torch
+
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_a_graph_keeps_the_workspace_it_was_captured_with(oracle):
+    """64 products of 512 x 512 x 1024 are 256 pair tiles; the 34 left over from the whole waves are
+    cut along K and their sums go through the workspace.  A graph captured from such a call has to
+    stay valid when a larger call makes the handle's workspace grow: the memory it writes to must not
+    be given back.  (That is asserted on the free memory before the graph is replayed.)"""
+    import torch
+
+    batch, m, n, k = 64, 512, 512, 1024
+    big = 4096
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    a = torch.rand(batch * m * k, device="cuda", generator=g) * 2 - 1
+    b = torch.rand(batch * k * n, device="cuda", generator=g) * 2 - 1
+    c = torch.zeros(batch * m * n, device="cuda")
+    x, y = torch.ones(big * big, device="cuda"), torch.zeros(big * big, device="cuda")
+
+    def small_call(h):
+        h.use_current_torch_stream()
+        h.gemm_strided_batch(N, N, m, n, k, 1.0, a, m, m * k, b, k, k * n, 0.0, c, m, m * n, batch,
+                             FP16TCEC)
+
+    def big_call(h):
+        h.use_current_torch_stream()
+        h.gemm(N, N, big, big, big, 1.0, x, big, x, big, 0.0, y, big, TF32TCEC)
+
+    with api.Handle() as h:                       # loads the kernels
+        small_call(h)
+        big_call(h)
+        torch.cuda.synchronize()
+    with api.Handle() as h:                       # what the larger call takes by itself
+        before = _free_bytes()
+        big_call(h)
+        alone = before - _free_bytes()
+    with api.Handle() as h:                       # without a graph the outgrown block goes back
+        before = _free_bytes()
+        small_call(h)
+        pieces = before - _free_bytes()
+        assert 4 * SLACK < pieces < 64 << 20
+        big_call(h)
+        assert before - _free_bytes() <= alone + SLACK
+    with api.Handle() as h:
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            small_call(h)
+        side.synchronize()
+        want = c.clone()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            small_call(h)
+        torch.cuda.synchronize()
+        before = _free_bytes()
+        big_call(h)
+        assert before - _free_bytes() >= alone - SLACK
+        c.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(c, want)
+        del graph
+        assert h.kernel_status() == 0
+    ah, bh, ch = (t.cpu().numpy() for t in (a, b, want))
+    i = batch - 1                                 # one of the cut tiles
+    truth = oracle.gemm_f64(N, N, m, n, k, 1.0, ah[i * m * k:], m, bh[i * k * n:], k, 0.0, None, m)
+    assert oracle.residual(truth, ch[i * m * n:], m) < oracle.error_threshold(True, k)
