@@ -23,8 +23,22 @@ constexpr std::size_t kDefaultWorkspaceLimit = 8ull << 30;
 
 inline std::uint64_t round_up(std::uint64_t x, std::uint64_t a) { return (x + a - 1) / a * a; }
 
+// Whether memory may be allocated and freed now: not while the stream is being captured into a
+// graph, where either would end the capture.
+bool may_allocate(const cuMpSGEMM_handle *h) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->cuda_stream, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return cap == cudaStreamCaptureStatusNone;
+}
+
+// Makes the workspace hold `bytes`.  Returns false, with the old workspace untouched, while the
+// stream is being captured, and false without a workspace if there is no memory.
 bool ensure_workspace(cuMpSGEMM_handle *h, std::size_t bytes) {
   if (h->workspace_bytes >= bytes) return true;
+  if (!may_allocate(h)) return false;
   if (h->workspace != nullptr) {
     if (h->workspace_in_graph) h->graph_workspaces.push_back(h->workspace);
     else cudaFree(h->workspace); // waits for work that may still read the old buffer
@@ -38,17 +52,6 @@ bool ensure_workspace(cuMpSGEMM_handle *h, std::size_t bytes) {
   }
   h->workspace_bytes = bytes;
   return true;
-}
-
-// Whether the workspace can be grown now: not while the stream is being captured into a graph,
-// where an allocation would end the capture.
-bool may_allocate(const cuMpSGEMM_handle *h) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(h->cuda_stream, &cap) != cudaSuccess) {
-    cudaGetLastError();
-    return true;
-  }
-  return cap == cudaStreamCaptureStatusNone;
 }
 
 __global__ void dyn_params_from_flag_kernel(DynParams *out, const int *flag) {
@@ -612,7 +615,9 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
       h->workspace_bytes >= bytes_panels && !may_allocate(h))
     bytes_tail = 0; // captured with a workspace that only holds the panels: no pieces
   if (!ensure_workspace(h, bytes_panels + bytes_tail)) {
-    log_error("failed to allocate the operand workspace");
+    log_error(may_allocate(h) ? "failed to allocate the operand workspace"
+                              : "the operand workspace cannot grow while the stream is captured; "
+                                "make one call of this size before the capture");
     return CUBLAS_STATUS_ALLOC_FAILED;
   }
   char *ws_a = reinterpret_cast<char *>(h->workspace);

@@ -80,3 +80,40 @@ def test_a_graph_keeps_the_workspace_it_was_captured_with(oracle):
     i = batch - 1                                 # one of the cut tiles
     truth = oracle.gemm_f64(N, N, m, n, k, 1.0, ah[i * m * k:], m, bh[i * k * n:], k, 0.0, None, m)
     assert oracle.residual(truth, ch[i * m * n:], m) < oracle.error_threshold(True, k)
+
+
+@pytest.mark.parametrize("mode,shape,fits", [(FP16TCEC, (256, 256, 8192), True),    # K slices, on the fly
+                                             (TF32TCEC, (700, 520, 900), False)])   # panels
+def test_nothing_is_allocated_during_a_capture(oracle, monkeypatch, mode, shape, fits):
+    """A handle without a workspace, captured.  K slices of the on-the-fly kernel are left out (the
+    call needs no memory then); a call that cannot do without panels is refused.  Neither may
+    allocate or free, which would end the capture."""
+    import torch
+
+    m, n, k = shape
+    a, b = oracle.gen_uniform(1, m * k), oracle.gen_uniform(2, k * n)
+    da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    c, d = torch.zeros(m * n, device="cuda"), torch.zeros(4, device="cuda")
+    monkeypatch.setenv("CUMPSGEMM_STREAM", "0")
+    with api.Handle() as h:                       # loads the kernels
+        h.use_current_torch_stream()
+        h.gemm(N, N, m, n, k, 1.0, da, m, db, k, 0.0, c, m, mode)
+        torch.cuda.synchronize()
+    with api.Handle() as h:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            h.use_current_torch_stream()
+            st = h.gemm(N, N, m, n, k, 1.0, da, m, db, k, 0.0, c, m, mode, check=False)
+            d.add_(1.0)                           # the capture goes on
+        assert st == (api.CUBLAS_STATUS_SUCCESS if fits else 3)
+        c.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert d[0].item() == 1.0
+        if fits:
+            truth = oracle.gemm_f64(N, N, m, n, k, 1.0, a, m, b, k, 0.0, None, m)
+            assert oracle.residual(truth, c.cpu().numpy(), m) < oracle.error_threshold(True, k)
+        else:
+            assert torch.count_nonzero(c).item() == 0
+        del graph
+        assert h.kernel_status() == 0
