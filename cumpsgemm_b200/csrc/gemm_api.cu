@@ -289,7 +289,7 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
   if (batch > 0x3fffffffull || n > 0x3fffffffull) return false; // (TMA coordinates are 32-bit)
   const int tile_n = (t.stream == 128 || t.stream == 256) ? t.stream : (n <= 128 ? 128 : 256);
   int clusters = 0;
-  if (stream_max_clusters(tile_n, &clusters) != cudaSuccess) {
+  if (stream_max_clusters(kind, tile_n, &clusters) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -467,60 +467,55 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
   if (!small && ec && !ptr_arrays && !(fused && batch >= 8 && m_exp <= 128 && h->tuning.stream == -1) &&
       stream_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, stream_kind,
                      pre.us, &ga)) {
-    bool room = true;
     if (ga.plan.piece_clusters > 0) {
       const std::size_t bytes = stream_scratch_bytes(ga.plan);
       const std::size_t limit =
           h->workspace_limit_bytes ? h->workspace_limit_bytes : kDefaultWorkspaceLimit;
-      if (h->workspace_bytes < bytes && (bytes > limit || !may_allocate(h))) {
+      if (bytes > limit || !ensure_workspace(h, bytes)) {
         // no room for the pieces' sums: whole tiles only, which need no memory
         ga.plan.whole_tiles = ga.plan.total_tiles;
         ga.plan.piece_clusters = 0;
         ga.plan.slices = 0;
-      } else {
-        room = ensure_workspace(h, bytes);
       }
     }
-    if (room) {
-      ga.c = reinterpret_cast<float *>(c);
-      ga.ldc = ldc * fpe;
-      ga.stride_c = stridec * fpe;
-      ga.alpha_r = Scalar<T>::re(alpha);
-      ga.alpha_i = Scalar<T>::im(alpha);
-      ga.beta_r = Scalar<T>::re(beta);
-      ga.beta_i = Scalar<T>::im(beta);
-      ga.dyn = dyn;
-      ga.dev_status = h->dev_status;
-      ga.debug = h->debug_buffer;
-      ga.partial = reinterpret_cast<float *>(h->workspace);
-      if (used_kernel_module_id != nullptr) {
-        *used_kernel_module_id = (ga.plan.slices > 1) ? 100u : tile_class(pre.tile.tile_n);
+    ga.c = reinterpret_cast<float *>(c);
+    ga.ldc = ldc * fpe;
+    ga.stride_c = stridec * fpe;
+    ga.alpha_r = Scalar<T>::re(alpha);
+    ga.alpha_i = Scalar<T>::im(alpha);
+    ga.beta_r = Scalar<T>::re(beta);
+    ga.beta_i = Scalar<T>::im(beta);
+    ga.dyn = dyn;
+    ga.dev_status = h->dev_status;
+    ga.debug = h->debug_buffer;
+    ga.partial = reinterpret_cast<float *>(h->workspace);
+    if (used_kernel_module_id != nullptr) {
+      *used_kernel_module_id = (ga.plan.slices > 1) ? 100u : tile_class(pre.tile.tile_n);
+    }
+    const bool prof = h->exp_stats.profiling_enabled;
+    if (prof) h->exp_stats.profiler.start("gemm_kernel", h->cuda_stream);
+    cuMpSGEMM_handle::TimingTriple tt{};
+    if (h->kernel_timing) {
+      for (auto &e : tt.e) cudaEventCreate(&e);
+      cudaEventRecord(tt.e[0], h->cuda_stream);
+      cudaEventRecord(tt.e[1], h->cuda_stream);
+    }
+    cudaError_t gerr = launch_tcec_gemm_stream(ga, h->cuda_stream);
+    const bool addressable = gerr != cudaErrorNotSupported;
+    if (h->kernel_timing && addressable) {
+      cudaEventRecord(tt.e[2], h->cuda_stream);
+      h->timing_events.push_back(tt);
+    } else if (h->kernel_timing) {
+      for (auto &e : tt.e) cudaEventDestroy(e);
+    }
+    if (prof) h->exp_stats.profiler.stop("gemm_kernel", h->cuda_stream);
+    if (addressable) {
+      mark_stream_work(h);
+      if (gerr != cudaSuccess) {
+        log_error(std::string("kernel launch failed: ") + cudaGetErrorString(gerr));
+        return CUBLAS_STATUS_EXECUTION_FAILED;
       }
-      const bool prof = h->exp_stats.profiling_enabled;
-      if (prof) h->exp_stats.profiler.start("gemm_kernel", h->cuda_stream);
-      cuMpSGEMM_handle::TimingTriple tt{};
-      if (h->kernel_timing) {
-        for (auto &e : tt.e) cudaEventCreate(&e);
-        cudaEventRecord(tt.e[0], h->cuda_stream);
-        cudaEventRecord(tt.e[1], h->cuda_stream);
-      }
-      cudaError_t gerr = launch_tcec_gemm_stream(ga, h->cuda_stream);
-      const bool addressable = gerr != cudaErrorNotSupported;
-      if (h->kernel_timing && addressable) {
-        cudaEventRecord(tt.e[2], h->cuda_stream);
-        h->timing_events.push_back(tt);
-      } else if (h->kernel_timing) {
-        for (auto &e : tt.e) cudaEventDestroy(e);
-      }
-      if (prof) h->exp_stats.profiler.stop("gemm_kernel", h->cuda_stream);
-      if (addressable) {
-        mark_stream_work(h);
-        if (gerr != cudaSuccess) {
-          log_error(std::string("kernel launch failed: ") + cudaGetErrorString(gerr));
-          return CUBLAS_STATUS_EXECUTION_FAILED;
-        }
-        return CUBLAS_STATUS_SUCCESS;
-      }
+      return CUBLAS_STATUS_SUCCESS;
     }
   }
 

@@ -386,7 +386,8 @@ struct StreamGemmArgs {
   float *partial; // stream_scratch_bytes() bytes when the plan cuts tiles along K
 };
 std::size_t stream_scratch_bytes(const StreamPlan &plan);
-cudaError_t stream_max_clusters(int tile_n, int *clusters); // of the current device
+// CTA pairs of one of its kernels the current device keeps resident; an error if it cannot run there
+cudaError_t stream_max_clusters(StreamKind kind, int tile_n, int *clusters);
 cudaError_t launch_tcec_gemm_stream(const StreamGemmArgs &a, cudaStream_t stream);
 // Self-test of the bounded mbarrier wait (see cuMpSGEMM_selftest_bounded_wait).
 cudaError_t launch_bounded_wait_selftest(int *dev_status, unsigned long long limit_ns,

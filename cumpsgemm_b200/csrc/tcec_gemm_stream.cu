@@ -902,8 +902,15 @@ cudaError_t launch_tcec_gemm_stream(const StreamGemmArgs &a, cudaStream_t stream
   return cudaErrorInvalidValue;
 }
 
-cudaError_t stream_max_clusters(int tile_n, int *clusters) {
-  return tile_n == 256 ? stream_setup<0, 256>(clusters) : stream_setup<0, 128>(clusters);
+cudaError_t stream_max_clusters(StreamKind kind, int tile_n, int *clusters) {
+  switch (kind) {
+  case StreamKind::fp16:
+    return tile_n == 256 ? stream_setup<0, 256>(clusters) : stream_setup<0, 128>(clusters);
+  case StreamKind::tf32:
+    return tile_n == 256 ? stream_setup<1, 256>(clusters) : stream_setup<1, 128>(clusters);
+  default:
+    return tile_n == 256 ? stream_setup<2, 256>(clusters) : stream_setup<2, 128>(clusters);
+  }
 }
 
 } // namespace cumpsgemm_b200

@@ -117,3 +117,34 @@ def test_nothing_is_allocated_during_a_capture(oracle, monkeypatch, mode, shape,
             assert torch.count_nonzero(c).item() == 0
         del graph
         assert h.kernel_status() == 0
+
+
+def test_the_limit_decides_about_pieces_and_not_the_history(oracle):
+    """K pieces that would go beyond the workspace limit are left out, and the tiles stay whole: with
+    the same bits whether or not an earlier call has left a large workspace on the handle."""
+    import torch
+
+    batch, m, n, k = 10, 520, 300, 1500
+    a, b = oracle.gen_uniform(1, batch * m * k), oracle.gen_uniform(2, batch * k * n)
+    da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+
+    def call(h, limit):
+        h.set_workspace_limit(limit)
+        c = torch.zeros(batch * m * n, device="cuda")
+        h.gemm_strided_batch(T, N, m, n, k, 1.0, da, k, m * k, db, k, k * n, 0.0, c, m, m * n, batch,
+                             TF32TCEC)
+        return c
+
+    with api.Handle() as h:
+        h.use_current_torch_stream()
+        fresh = call(h, 1 << 20)
+        cut = call(h, 0)
+        after = call(h, 1 << 20)
+        assert torch.equal(fresh, after)
+        assert not torch.equal(fresh, cut)
+        for c in (fresh, cut):
+            res = c.cpu().numpy()
+            for i in (0, batch - 1):
+                truth = oracle.gemm_f64(T, N, m, n, k, 1.0, a[i * m * k:], k, b[i * k * n:], k, 0.0, None, m)
+                assert oracle.residual(truth, res[i * m * n:(i + 1) * m * n], m) < oracle.error_threshold(True, k)
+        assert h.kernel_status() == 0
