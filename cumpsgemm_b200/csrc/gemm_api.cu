@@ -372,6 +372,16 @@ PresplitChoice choose_presplit(const cuMpSGEMM_handle *h, std::uint64_t m_exp, s
   return c;
 }
 
+// Whether a launch of the pair kernel on `batch` products cuts any tile along K, given memory.
+bool pair_cuts(const Tuning &t, bool tf32, std::uint64_t m_exp, std::uint64_t n, std::uint32_t k_pad,
+               std::uint64_t batch, int clusters) {
+  const std::uint64_t tiles = ((m_exp + 255) / 256) * ((n + 255) / 256) * batch;
+  return tiles <= 0x7fffffffull &&
+         plan_pair(t, tf32, true, static_cast<std::uint32_t>(tiles), k_pad / 64,
+                   static_cast<std::uint32_t>(clusters))
+                 .piece_clusters > 0;
+}
+
 // The reference's module ids name tile classes.
 inline unsigned tile_class(int tile_n) { return (tile_n == 256) ? 0u : (tile_n == 128) ? 1u : 2u; }
 
@@ -600,16 +610,28 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
   // split-K partial sums: k_slices blocks of m x n floats per batch entry, behind the panels
   const std::size_t bytes_p_1 =
       (k_slices > 1) ? static_cast<std::size_t>(k_slices) * m_exp * n * sizeof(float) : 0;
-  // scratch for the K pieces of pair tiles (once per call, behind everything else)
-  std::size_t bytes_tail = use_pair ? pair_tail_scratch_bytes(h->num_sms) : 0;
   std::uint64_t chunk = std::max<std::uint64_t>(1, limit / (bytes_a_1 + bytes_b_1 + bytes_p_1));
   chunk = std::min<std::uint64_t>(chunk, batch);
   chunk = std::min<std::uint64_t>(chunk, 32768); // planes of a tensor map, tiles of a launch
   const std::size_t bytes_panels = chunk * (bytes_a_1 + bytes_b_1 + bytes_p_1);
-  if (bytes_tail > 0 && h->workspace_bytes < bytes_panels + bytes_tail &&
-      h->workspace_bytes >= bytes_panels && !may_allocate(h))
-    bytes_tail = 0; // captured with a workspace that only holds the panels: no pieces
-  if (!ensure_workspace(h, bytes_panels + bytes_tail)) {
+  // Scratch for the K pieces of pair tiles (once per call, behind everything else), if any launch
+  // of the call cuts one.  It never takes a call over a limit that the panels keep; and where it
+  // cannot be had (the workspace of a captured call only holds the panels, no memory) the tiles
+  // stay whole.
+  std::size_t bytes_tail = 0;
+  if (use_pair) {
+    int clusters = 1;
+    const bool cuts =
+        pair_max_clusters(stream_kind, &clusters) == cudaSuccess &&
+        (pair_cuts(h->tuning, !want_fp16, m_exp, n, k_pad, chunk, clusters) ||
+         (batch % chunk != 0 &&
+          pair_cuts(h->tuning, !want_fp16, m_exp, n, k_pad, batch % chunk, clusters)));
+    const std::size_t bytes = cuts ? pair_tail_scratch_bytes(h->num_sms) : 0;
+    if ((bytes_panels + bytes <= limit || bytes_panels > limit) &&
+        ensure_workspace(h, bytes_panels + bytes))
+      bytes_tail = bytes;
+  }
+  if (!ensure_workspace(h, bytes_panels)) {
     log_error(may_allocate(h) ? "failed to allocate the operand workspace"
                               : "the operand workspace cannot grow while the stream is captured; "
                                 "make one call of this size before the capture");

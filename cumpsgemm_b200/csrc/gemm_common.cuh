@@ -82,5 +82,7 @@ cudaError_t launch_piece_fixup(const PieceFixupArgs &a, const WorkPlan &w, cudaS
 // CTA-pair kernel (tcec_gemm_pair.cu): 256 x 256 tile per cluster of two CTAs.
 cudaError_t launch_tcec_gemm_pair(const TcecGemmArgs &a, cudaStream_t stream);
 cudaError_t launch_tcec_gemm_pair_auto(const TcecGemmArgs &a, cudaStream_t stream);
+// CTA pairs of the kernel of that kind the current device keeps resident.
+cudaError_t pair_max_clusters(StreamKind kind, int *clusters);
 
 } // namespace cumpsgemm_b200

@@ -624,6 +624,17 @@ template <int KIND> cudaError_t launch_pair(const TcecGemmArgs &a, cudaStream_t 
 
 } // namespace
 
+cudaError_t pair_max_clusters(StreamKind kind, int *clusters) {
+  switch (kind) {
+  case StreamKind::fp16:
+    return pair_setup<0>(tcec_gemm_pair_kernel<0>, clusters);
+  case StreamKind::tf32:
+    return pair_setup<1>(tcec_gemm_pair_kernel<1>, clusters);
+  default:
+    return pair_setup<2>(tcec_gemm_pair_auto_kernel, clusters);
+  }
+}
+
 cudaError_t launch_tcec_gemm_pair(const TcecGemmArgs &a, cudaStream_t stream) {
   if (!a.error_correction) return cudaErrorInvalidValue;
   return (a.kind == SplitKind::fp16) ? launch_pair<0>(a, stream) : launch_pair<1>(a, stream);

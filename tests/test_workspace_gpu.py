@@ -148,3 +148,44 @@ def test_the_limit_decides_about_pieces_and_not_the_history(oracle):
                 truth = oracle.gemm_f64(T, N, m, n, k, 1.0, a[i * m * k:], k, b[i * k * n:], k, 0.0, None, m)
                 assert oracle.residual(truth, res[i * m * n:(i + 1) * m * n], m) < oracle.error_threshold(True, k)
         assert h.kernel_status() == 0
+
+
+def test_pair_scratch_is_taken_when_needed_and_within_the_limit(oracle, monkeypatch):
+    """The pair kernel's scratch for K pieces: none for a launch that cuts no tile (148 tiles are two
+    whole waves), none where it would go beyond a workspace limit that the panels keep."""
+    import torch
+
+    def used(h, m, n, k, limit, out):
+        x = torch.ones(1, device="cuda")          # (the caching allocator's first block)
+        a, b = (torch.rand(s, device="cuda", generator=torch.Generator("cuda").manual_seed(9)) * 2 - 1
+                for s in (m * k, k * n))
+        c = torch.zeros(m * n, device="cuda")
+        h.use_current_torch_stream()
+        h.set_workspace_limit(limit)
+        before = _free_bytes()
+        h.gemm(N, N, m, n, k, 1.0, a, m, b, k, 0.0, c, m, FP16TCEC)
+        taken = before - _free_bytes()
+        out.append(c)
+        del x
+        return taken
+
+    whole, cut = (9472, 1024, 512), (4096, 4096, 2048)
+    panels = lambda m, n, k: 4 * (m + n) * k      # noqa: E731
+    outs = []
+    for shape in (whole, cut):                    # loads the kernels
+        with api.Handle() as h:
+            used(h, *shape, 0, outs)
+    del outs[:]
+    with api.Handle() as h:
+        assert used(h, *whole, 0, outs) <= panels(*whole) + SLACK
+    with api.Handle() as h:
+        assert used(h, *cut, 0, outs) > panels(*cut) + 4 * SLACK
+    limit = panels(*cut) + 2 * SLACK
+    with api.Handle() as h:
+        assert used(h, *cut, limit, outs) <= limit
+        assert h.kernel_status() == 0
+    monkeypatch.setenv("CUMPSGEMM_TAIL_SPLIT", "0")
+    with api.Handle() as h:
+        used(h, *cut, 0, outs)
+    _, with_pieces, limited, uncut = outs
+    assert torch.equal(limited, uncut) and not torch.equal(limited, with_pieces)
