@@ -225,7 +225,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
       constexpr uint16_t BOTH = 0x3;
       bool ok = true;
       const long long dbg_t0 = clock64();
-      const uint32_t chunk = p.drain_chunk;
+      const uint32_t chunk = p.drain_chunk, first = p.first_chunk;
       const uint64_t desc0 = ptx::make_kmajor_desc<ROW_BYTES>(ptx::smem_u32(smem));
       constexpr uint64_t kStage = STAGE_BYTES >> 4, kTile = TILE_BYTES >> 4;
       uint32_t s = 0, ph = 0, d0_ph = 1, d1_ph = 1;
@@ -236,7 +236,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
         uint32_t chunk_end = 0; // first stage after the current chunk
         for (uint32_t kb = 0; kb < kbn; ++kb) {
           const bool first_in_chunk = (kb == chunk_end);
-          if (first_in_chunk) chunk_end = min(kb + chunk, kbn);
+          if (first_in_chunk) chunk_end = min(kb + (kb == 0 ? first : chunk), kbn);
           ok = ptx::mbar_wait_timed(ptx::smem_u32(&full_bar[s]), ph, abort_flag, p.status,
                                     ptx::kErrWaitFull, dbg, &dbg_wait);
           if (!ok) break;
@@ -309,7 +309,11 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
     WorkList list(plan.w, cluster_id, num_clusters);
     WorkItem x;
     while (ok && list.next(plan.w, x)) {
-      const uint32_t n_chunks = (x.un * STAGES_PER_UNIT + p.drain_chunk - 1u) / p.drain_chunk;
+      const uint32_t stages = x.un * STAGES_PER_UNIT;
+      const uint32_t n_chunks =
+          1u + (stages > p.first_chunk
+                    ? (stages - p.first_chunk + p.drain_chunk - 1u) / p.drain_chunk
+                    : 0u);
       const uint32_t prefetch_at =
           ((p.beta_r == 0.f && p.beta_i == 0.f) || x.un != plan.w.units) ? n_chunks
           : (n_chunks > C_PREFETCH_LEAD) ? n_chunks - C_PREFETCH_LEAD
@@ -517,7 +521,12 @@ bool pair_prepare(const TcecGemmArgs &a, SplitKind kind, int max_clusters, CUten
     const uint32_t pairs = static_cast<uint32_t>(max_clusters);
     const uint32_t dflt = (static_cast<uint64_t>(p.tiles_m) * p.tiles_n * a.batch > pairs) ? 2 : 1;
     p.drain_chunk = static_cast<uint16_t>((v >= 1) ? (v > 0xffff ? 0xffff : v) : dflt);
-    p.first_chunk = p.drain_chunk; // (the fused kernel's field)
+    // The first chunk of a tile may be longer (the epilogue warps are still storing the previous
+    // tile then), but by default it is not: 512 FP16 k values in it cost accuracy and, with the
+    // rolled epilogue, bought no time.
+    const int fv = a.tuning.first_chunk;
+    p.first_chunk = static_cast<uint16_t>((fv >= 1) ? (fv > 0xffff ? 0xffff : fv) : p.drain_chunk);
+    if (p.first_chunk < p.drain_chunk) p.first_chunk = p.drain_chunk;
   }
   const uint64_t total = static_cast<uint64_t>(p.tiles_m) * p.tiles_n * a.batch;
   if (total == 0 || total > 0x7fffffffull) return false;

@@ -96,3 +96,24 @@ def test_capture_without_room_for_pieces(oracle):
             assert oracle.residual(want, res[i * m * n:(i + 1) * m * n], m) < oracle.error_threshold(True, k)
         assert h.kernel_status() == 0
         del g
+
+
+def test_the_first_chunk_of_the_pair_kernel_can_be_lengthened(handle, oracle, monkeypatch):
+    """CUMPSGEMM_FIRST_CHUNK sets how many stages the pair kernel sums up before it drains its
+    accumulator for the first time in a tile: another rounding, the same result within tolerance; a
+    value below the drain chunk changes nothing."""
+    args = (handle, oracle, False, N, N, 520, 300, 1500, FP16TCEC, 0.5, 0)
+    monkeypatch.setenv("CUMPSGEMM_PAIR", "1")
+    monkeypatch.setenv("CUMPSGEMM_TAIL_SPLIT", "0")
+    monkeypatch.setenv("CUMPSGEMM_DRAIN_CHUNK", "2")
+    outs = {}
+    for first in ("0", "1", "7", "1000"):         # default, below the drain chunk, odd, whole K loop
+        monkeypatch.setenv("CUMPSGEMM_FIRST_CHUNK", first)
+        handle.reload_tuning_env()
+        outs[first] = _run(*args).view(np.uint32)
+    for name in ("PAIR", "TAIL_SPLIT", "DRAIN_CHUNK", "FIRST_CHUNK"):
+        monkeypatch.delenv("CUMPSGEMM_" + name)
+    handle.reload_tuning_env()
+    np.testing.assert_array_equal(outs["0"], outs["1"])
+    assert not np.array_equal(outs["0"], outs["7"])
+    assert not np.array_equal(outs["7"], outs["1000"])
