@@ -76,15 +76,17 @@ __device__ __forceinline__ void add_corrections_in_tmem(uint32_t taddr, const fl
   ptx::tmem_st_wait();
 }
 
-// C(row, col) = alpha * acc for columns [col0, col0 + CPT), straight from the registers
+// C(row, col) = alpha * acc for columns [col0, col0 + CPT), straight from the registers.  A complex
+// alpha is multiplied out whatever its imaginary part, as in store_loop: an infinite sum gives the
+// same NaN in the other component on every path.
 template <int CPT>
 __device__ __forceinline__ void store_registers(const float (&acc)[CPT], float *cbase, uint64_t ldc,
                                                 uint32_t col0, uint32_t n, bool row_ok, float ar,
-                                                float ai) {
+                                                float ai, bool is_complex) {
   if (col0 >= n) return; // uniform over the warp
   const uint32_t cols = n - col0;
   float *cp = cbase + static_cast<uint64_t>(col0) * ldc;
-  if (ai == 0.f) {
+  if (!is_complex) {
 #pragma unroll
     for (int i = 0; i < CPT; ++i) {
       if (row_ok && static_cast<uint32_t>(i) < cols) __stcs(cp, ar * acc[i]);

@@ -622,7 +622,8 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
                               static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2) * CPT;
         const float unscale = (p.dyn != nullptr) ? p.dyn->unscale_c : 1.f;
         store_registers<CPT>(acc, p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row, p.ldc,
-                             col0, p.n, row < p.m, p.alpha_r * unscale, p.alpha_i * unscale);
+                             col0, p.n, row < p.m, p.alpha_r * unscale, p.alpha_i * unscale,
+                             (p.flags & kIsComplex) != 0);
         continue;
       }
       // the finished sums stay in the D1 columns; from here on they are read from there, and what
