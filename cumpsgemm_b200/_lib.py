@@ -92,6 +92,8 @@ PROTOTYPES = {
     "cuMpSGEMM_reload_tuning_env": (None, [vp]),
     "cuMpSGEMM_plan_stream": (i32, [u64, u64, u64, u64, i32, u32, C.POINTER(u32), C.POINTER(u32),
                                     C.POINTER(u32), C.POINTER(u32), C.POINTER(u32)]),
+    "cuMpSGEMM_plan_pair": (i32, [u32, u32, u32, i32, C.POINTER(u32), C.POINTER(u32), C.POINTER(u32),
+                                  C.POINTER(u32), C.POINTER(u32)]),
     "cuMpSGEMM_plan_pair_tail": (i32, [u32, u32, u32, i32, C.POINTER(u32), C.POINTER(u32),
                                        C.POINTER(u32), C.POINTER(u32)]),
     "cuMpSGEMM_set_debug_buffer": (None, [vp, vp]),

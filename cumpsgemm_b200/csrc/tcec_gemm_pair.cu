@@ -687,3 +687,20 @@ extern "C" int cuMpSGEMM_plan_pair_tail(unsigned total_tiles, unsigned clusters,
   *work_items = sliced ? t.whole_tiles + t.piece_clusters : total_tiles;
   return 0;
 }
+
+extern "C" int cuMpSGEMM_plan_pair(unsigned total_tiles, unsigned clusters, unsigned k_pad, int tf32,
+                                   unsigned *units, unsigned *whole_tiles, unsigned *piece_clusters,
+                                   unsigned *slices, unsigned *slice_units) {
+  using namespace cumpsgemm_b200;
+  if (total_tiles == 0 || clusters == 0 || k_pad == 0 || k_pad % 64 != 0 || units == nullptr ||
+      whole_tiles == nullptr || piece_clusters == nullptr || slices == nullptr ||
+      slice_units == nullptr)
+    return 1;
+  const WorkPlan t = plan_pair(Tuning{}, tf32 != 0, true, total_tiles, k_pad / 64, clusters);
+  *units = t.units;
+  *whole_tiles = t.whole_tiles;
+  *piece_clusters = t.piece_clusters;
+  *slices = t.slices;
+  *slice_units = t.slice_units;
+  return 0;
+}

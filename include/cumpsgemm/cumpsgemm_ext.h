@@ -151,17 +151,27 @@ void cuMpSGEMM_set_count_tail_padding(cuMpSGEMM_handle_t handle, int enable);
  * CUMPSGEMM_TAIL_SPLIT, CUMPSGEMM_STREAM) once, when it is created, so that a GEMM call does not query the
  * environment; this reads them again. */
 void cuMpSGEMM_reload_tuning_env(cuMpSGEMM_handle_t handle);
-/* Host-only query (no GPU needed): how the CTA-pair kernel would schedule `total_tiles` tiles
- * of 256 x 256 with a K loop of k_pad values (a multiple of 64; tf32 != 0 for the TF32 kinds) on
- * `clusters` CTA pairs.  Tiles [0, *split_begin) run whole; each later tile (the last, partly
- * filled wave) is cut into *slices K slices of *slice_k values, *work_items work items in
- * all.  *slices == 1: nothing is cut into slices (a last wave that is more than half full may
- * instead be shared by all pairs in K pieces of equal length).  Returns 0, or 1 for invalid arguments.  No counterpart
- * in the reference (its atomic split-K kernel, src/cumpsgemm.cu:272-304, is the nearest
+/* Host-only query (no GPU needed): the K slices of the CTA-pair kernel's last, partly filled wave,
+ * for `total_tiles` tiles of 256 x 256 with a K loop of k_pad values (a multiple of 64; tf32 != 0
+ * for the TF32 kinds) on `clusters` CTA pairs.  Tiles [0, *split_begin) are not sliced; each later
+ * tile is cut into *slices K slices of *slice_k values, *work_items work items in all.
+ * *slices == 1: no tile is cut into slices of its own.  That includes a last wave that is more
+ * than half full and is shared by all pairs in pieces of equal length, which this query cannot
+ * express: cuMpSGEMM_plan_pair reports the whole plan.  Returns 0, or 1 for invalid arguments.  No
+ * counterpart in the reference (its atomic split-K kernel, src/cumpsgemm.cu:272-304, is the nearest
  * relative). */
 int cuMpSGEMM_plan_pair_tail(unsigned total_tiles, unsigned clusters, unsigned k_pad, int tf32,
                              unsigned *split_begin, unsigned *slices, unsigned *slice_k,
                              unsigned *work_items);
+/* Host-only query (no GPU needed): how the CTA-pair kernel deals the same tiles.  *units is the K
+ * loop in units of 64 values; tiles [0, *whole_tiles) run whole; the K loops of the others, laid end
+ * to end (u units in all), are shared by *piece_clusters pairs (0: every tile is whole).
+ * *slice_units > 0: every such tile is cut into *slices slices of that many units (the last may be
+ * shorter), one pair each; *slice_units == 0: pair c takes units [c * u / p, (c + 1) * u / p) for
+ * p = *piece_clusters.  A second kernel adds the pieces.  Returns 0, or 1 for invalid arguments. */
+int cuMpSGEMM_plan_pair(unsigned total_tiles, unsigned clusters, unsigned k_pad, int tf32,
+                        unsigned *units, unsigned *whole_tiles, unsigned *piece_clusters,
+                        unsigned *slices, unsigned *slice_units);
 /* Host-only query (no GPU needed): how the kernel that splits its operands between TMA and the
  * tensor core would deal an m x n x k x batch problem (sizes of the real, expanded problem) in
  * 256 x tile_n pair tiles (tile_n 256 or 128) to `clusters` CTA pairs.  *units is the K loop in
