@@ -53,6 +53,10 @@ class CuMpSGEMMError(RuntimeError):
         self.status = status
 
 
+# Handle.last_route (cuMpSGEMM_get_last_route)
+(ROUTE_NONE, ROUTE_PRESPLIT_SINGLE, ROUTE_PRESPLIT_PAIR, ROUTE_STREAMING,
+ ROUTE_ON_THE_FLY) = range(5)
+
 DevPtr = Union[int, "torch.Tensor"]  # noqa: F821
 
 
@@ -227,6 +231,12 @@ class Handle:
 
     def set_workspace_limit(self, nbytes: int) -> None:
         self._lib.cuMpSGEMM_set_workspace_limit(self._h, nbytes)
+
+    def last_route(self) -> tuple[int, bool]:
+        """Which kernels the last GEMM call launched (ROUTE_*), and whether it cut a tile along K."""
+        cut = C.c_int(0)
+        route = self._lib.cuMpSGEMM_get_last_route(self._h, C.byref(cut))
+        return route, bool(cut.value)
 
     def reload_tuning_env(self) -> None:
         """Read the CUMPSGEMM_TILE_N / PAIR / DRAIN_CHUNK / FIRST_CHUNK / PACE / FUSED / STREAM variables

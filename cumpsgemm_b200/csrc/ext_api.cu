@@ -219,6 +219,11 @@ void cuMpSGEMM_set_workspace_limit(cuMpSGEMM_handle_t h, size_t bytes) {
   h->workspace_limit_bytes = bytes;
 }
 
+int cuMpSGEMM_get_last_route(cuMpSGEMM_handle_t h, int *cut_along_k) {
+  if (h == nullptr) return CUMPSGEMM_ROUTE_NONE;
+  if (cut_along_k != nullptr) *cut_along_k = h->last_cut_along_k ? 1 : 0;
+  return h->last_route;
+}
 void cuMpSGEMM_reload_tuning_env(cuMpSGEMM_handle_t h) { h->tuning = read_tuning_env(); }
 
 void cuMpSGEMM_set_count_tail_padding(cuMpSGEMM_handle_t h, int enable) {

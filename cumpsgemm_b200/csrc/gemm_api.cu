@@ -12,6 +12,8 @@
 #include "gemm_common.cuh"
 #include "work_list.cuh"
 
+#include <cumpsgemm/cumpsgemm_ext.h>
+
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -399,6 +401,8 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
   constexpr bool is_complex = std::is_same<T, cuComplex>::value;
   if (h == nullptr) return CUBLAS_STATUS_NOT_INITIALIZED;
   if (mode == CUMPSGEMM_DRY_RUN) return CUBLAS_STATUS_SUCCESS;
+  h->last_route = CUMPSGEMM_ROUTE_NONE;
+  h->last_cut_along_k = false;
   const bool ptr_arrays = (a_array != nullptr) || (b_array != nullptr) || (c_array != nullptr);
   if (ptr_arrays && (a_array == nullptr || b_array == nullptr || c_array == nullptr))
     return CUBLAS_STATUS_INVALID_VALUE;
@@ -525,6 +529,8 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
         log_error(std::string("kernel launch failed: ") + cudaGetErrorString(gerr));
         return CUBLAS_STATUS_EXECUTION_FAILED;
       }
+      h->last_route = CUMPSGEMM_ROUTE_STREAMING;
+      h->last_cut_along_k = ga.plan.piece_clusters > 0;
       return CUBLAS_STATUS_SUCCESS;
     }
   }
@@ -587,6 +593,8 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
       log_error(std::string("kernel launch failed: ") + cudaGetErrorString(ferr));
       return CUBLAS_STATUS_EXECUTION_FAILED;
     }
+    h->last_route = CUMPSGEMM_ROUTE_ON_THE_FLY;
+    h->last_cut_along_k = fa.k_slices > 1;
     return CUBLAS_STATUS_SUCCESS;
   }
 
@@ -737,6 +745,8 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
     log_error(std::string("kernel launch failed: ") + cudaGetErrorString(err));
     return CUBLAS_STATUS_EXECUTION_FAILED;
   }
+  h->last_route = use_pair ? CUMPSGEMM_ROUTE_PRESPLIT_PAIR : CUMPSGEMM_ROUTE_PRESPLIT_SINGLE;
+  h->last_cut_along_k = k_slices > 1 || bytes_tail > 0; // (the scratch is only there to be used)
   return CUBLAS_STATUS_SUCCESS;
 }
 
@@ -750,6 +760,7 @@ cublasStatus_t gemm_with_statistics(cuMpSGEMM_handle *h, cublasOperation_t op_A,
                                     cuMpSGEMM_compute_mode_t mode, unsigned *stats_id_a_out,
                                     unsigned *stats_id_b_out, unsigned *flag_id_out) {
   if (h == nullptr) return CUBLAS_STATUS_NOT_INITIALIZED;
+  h->last_route = CUMPSGEMM_ROUTE_NONE;
   if (mode != CUMPSGEMM_AUTO && mode != CUMPSGEMM_FP16TCEC_SCALING)
     return CUBLAS_STATUS_INVALID_VALUE;
   if (m == 0 || n == 0 || k == 0 || batch == 0 || a == nullptr || b == nullptr)

@@ -153,6 +153,10 @@ struct cuMpSGEMM_handle {
 
   cumpsgemm_b200::Tuning tuning;
 
+  // What the last GEMM call launched (see cuMpSGEMM_get_last_route).
+  int last_route = 0;
+  bool last_cut_along_k = false;
+
   // Device status word the GEMM kernel writes when a bounded wait gives up.
   int *dev_status = nullptr; // [0] kernel status word, [1] wave counter of the pair kernel
 

@@ -128,6 +128,17 @@ cublasStatus_t cuMpSGEMM_sgemm_module(
  * epilogue for an accumulator, 6 = bad launch, 8 = the epilogue warps of a CTA for one another
  * (tail split of the CTA-pair kernel). */
 int cuMpSGEMM_get_kernel_status(cuMpSGEMM_handle_t handle);
+/* Which kernels the handle's last GEMM call launched, and in *cut_along_k (nullable) whether any of
+ * its tiles was cut along K; host state only, nothing is synchronised.  CUMPSGEMM_ROUTE_NONE: no call
+ * yet, or the last one was refused or failed. */
+enum {
+  CUMPSGEMM_ROUTE_NONE = 0,
+  CUMPSGEMM_ROUTE_PRESPLIT_SINGLE = 1, /* split pass, then one CTA per tile */
+  CUMPSGEMM_ROUTE_PRESPLIT_PAIR = 2,   /* split pass, then one CTA pair per tile */
+  CUMPSGEMM_ROUTE_STREAMING = 3,       /* CTA pairs, operands split between TMA and the tensor core */
+  CUMPSGEMM_ROUTE_ON_THE_FLY = 4       /* single CTAs that load and split the operands themselves */
+};
+int cuMpSGEMM_get_last_route(cuMpSGEMM_handle_t handle, int *cut_along_k);
 /* Self-test of the bounded wait: a one-CTA kernel waits, with the same routine the GEMM kernels
  * use, on a barrier that nothing signals; after limit_ms it must give up, record its code and
  * return normally.  Returns the status word (expected: 2, the "waited for operands" code) and

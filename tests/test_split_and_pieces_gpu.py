@@ -72,7 +72,7 @@ def test_capture_without_room_for_pieces(oracle):
     none: no allocation may happen, so the tiles stay whole, and the replay is right."""
     import torch
 
-    batch, m, n, k = 10, 520, 300, 1500
+    batch, m, n, k = 13, 520, 300, 1500           # 78 tiles on 74 pairs: the last four would be cut
     a, b = oracle.gen_uniform(1, batch * m * k), oracle.gen_uniform(2, batch * k * n)
     da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
     dc = torch.zeros(batch * m * n, device="cuda")
@@ -88,12 +88,17 @@ def test_capture_without_room_for_pieces(oracle):
         with torch.cuda.graph(g, stream=s):
             h.gemm_strided_batch(T, N, m, n, k, 1.0, da, k, m * k, db, k, k * n, 0.0, dc, m, m * n,
                                  batch, FP16TCEC)
+            assert h.last_route() == (api.ROUTE_STREAMING, False)
         g.replay()
         torch.cuda.synchronize()
         res = dc.cpu().numpy()
         for i in (0, batch - 1):
             want = oracle.gemm_f64(T, N, m, n, k, 1.0, a[i * m * k:], k, b[i * k * n:], k, 0.0, None, m)
             assert oracle.residual(want, res[i * m * n:(i + 1) * m * n], m) < oracle.error_threshold(True, k)
+        with torch.cuda.stream(s):                # (with memory to be had they are)
+            h.gemm_strided_batch(T, N, m, n, k, 1.0, da, k, m * k, db, k, k * n, 0.0, dc, m, m * n,
+                                 batch, FP16TCEC)
+            assert h.last_route() == (api.ROUTE_STREAMING, True)
         assert h.kernel_status() == 0
         del g
 

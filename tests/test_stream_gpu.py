@@ -37,7 +37,7 @@ def _gen(oracle, cplx, seed, count, scale=1.0):
 
 
 def _check(handle, oracle, width, cplx, op_a, op_b, m, n, k, mode, batch=1, beta=0.0, scale=1.0,
-           pad=0, shared_b=False, reps=1):
+           pad=0, shared_b=False, reps=1, cut=None):
     import torch
 
     q = 2 if cplx else 4                          # elements per 16 bytes
@@ -59,6 +59,9 @@ def _check(handle, oracle, width, cplx, op_a, op_b, m, n, k, mode, batch=1, beta
             dc = torch.from_numpy(c0.copy()).cuda()
             handle.gemm_strided_batch(op_a, op_b, m, n, k, alpha, da, lda, lda * an, db, ldb, sb,
                                       beta, dc, ldc, ldc * n, batch, mode)
+            route, was_cut = handle.last_route()
+            assert route == api.ROUTE_STREAMING   # and not a route the call has fallen back to
+            assert cut is None or was_cut == cut
             outs.append(dc.cpu().numpy())
     for o in outs[1:]:
         np.testing.assert_array_equal(o.view(np.uint32), outs[0].view(np.uint32))
@@ -97,13 +100,51 @@ def test_smallest_and_edge_sizes(handle, oracle, width, shape):
 
 
 @pytest.mark.parametrize("width", [256, 128])
-@pytest.mark.parametrize("shape,batch", [((256, 256, 4096), 1),    # slices and the reduction kernel
-                                         ((520, 300, 1500), 10),   # pieces that end inside tiles
-                                         ((256, 250, 192), 76)])   # whole wave plus a few tiles
+@pytest.mark.parametrize("shape,batch,cut", [
+    ((256, 256, 4096), 1, {256: True, 128: True}),     # slices, added by the piece kernel
+    ((520, 300, 1500), 13, {256: True, 128: True}),    # pieces that end inside tiles
+    ((520, 300, 1500), 10, {256: False, 128: True}),   # 60 (too many left over) and 90 tiles
+    ((256, 250, 192), 76, {256: False, 128: False})])  # a whole wave plus a few tiles too short to cut
 @pytest.mark.parametrize("mode", [FP16TCEC, TF32TCEC])
-def test_k_pieces_and_slices(handle, oracle, width, shape, batch, mode):
+def test_k_pieces_and_slices(handle, oracle, width, shape, batch, cut, mode):
     """Cut tiles: right, and bit-identical from run to run."""
-    _check(handle, oracle, width, False, T, N, *shape, mode, batch=batch, beta=-0.5, reps=3)
+    _check(handle, oracle, width, False, T, N, *shape, mode, batch=batch, beta=-0.5, reps=3,
+           cut=cut[width])
+
+
+@pytest.mark.parametrize("cplx,op_a,op_b", [(False, N, N), (False, T, T), (True, N, N), (True, Cj, T)])
+@pytest.mark.parametrize("mode", [FP16TCEC, TF32TCEC])
+def test_interleaved_batches_have_the_bits_of_contiguous_ones(handle, oracle, cplx, op_a, op_b, mode):
+    """Matrices of a batch interleaved column by column (batch stride = one column, leading dimension =
+    batch columns), and overlapping ones (stride of one 16-byte group): the same bits as from copies
+    laid out one behind the other."""
+    import torch
+
+    m, n, k, batch = 132, 72, 52, 12
+    q = 2 if cplx else 4
+    am, an = (m, k) if op_a == N else (k, m)
+    bm, bn = (k, n) if op_b == N else (n, k)
+    a = torch.from_numpy(_gen(oracle, cplx, 1, am * an * batch)).cuda()
+    b = torch.from_numpy(_gen(oracle, cplx, 2, bm * bn * batch)).cuda()
+
+    def run(da, lda, sa, db, ldb, sb):
+        c = torch.zeros(batch * m * n, dtype=a.dtype, device="cuda")
+        with _Stream(handle, 1):
+            handle.gemm_strided_batch(op_a, op_b, m, n, k, 1.0, da, lda, sa, db, ldb, sb, 0.0, c, m, m * n,
+                                      batch, mode)
+        assert handle.last_route()[0] == api.ROUTE_STREAMING
+        return c
+
+    # the storage read as [column][batch][row], and copied to [batch][column][row]
+    flat = lambda x, cols, rows: x.view(cols, batch, rows).permute(1, 0, 2).contiguous().view(-1)  # noqa: E731
+    got = run(a, am * batch, am, b, bm * batch, bm)
+    want = run(flat(a, an, am), am, am * an, flat(b, bn, bm), bm, bm * bn)
+    assert torch.equal(got, want)
+    # overlapping: matrix i starts q elements after matrix i - 1
+    got = run(a, am, q, b, bm, q)
+    shifted = lambda x, size: torch.cat([x[i * q:i * q + size] for i in range(batch)])             # noqa: E731
+    want = run(shifted(a, am * an), am, am * an, shifted(b, bm * bn), bm, bm * bn)
+    assert torch.equal(got, want)
 
 
 @pytest.mark.parametrize("width", [256, 128])
@@ -131,6 +172,7 @@ def test_auto_decides_on_the_device(handle, oracle, wide):
         ia, ib = handle.exp_stats_ext(m, k, da, m), handle.exp_stats_ext(k, n, db, k)
         handle.gemm_strided_batch_with_stats(N, N, m, n, k, 1.0, da, m, 0, db, k, 0, 0.0, dc, m, 0, 1,
                                              AUTO, ia, ib)
+        assert handle.last_route()[0] == api.ROUTE_STREAMING
     if wide:
         assert handle.get_exp_stats_compute_mode_level(ia) == TF32TCEC
     truth = oracle.gemm_f64(N, N, m, n, k, 1.0, a, m, b, k, 0.0, None, m)
@@ -149,7 +191,9 @@ def test_calls_tma_cannot_address_take_another_path(handle, oracle):
     with _Stream(handle, 1):
         c = torch.zeros(m * n, device="cuda")
         handle.gemm(N, N, m, n, k, 1.0, da, m + 1, db, k + 3, 0.0, c, m, FP16TCEC)
+        assert handle.last_route()[0] == api.ROUTE_PRESPLIT_SINGLE
         assert oracle.residual(truth, c.cpu().numpy(), m) < oracle.error_threshold(True, k)
         c = torch.zeros(128 * n, device="cuda")
         handle.gemm(N, N, 128, n, 64, 1.0, da[1:], 128, db, k + 3, 0.0, c, 128, TF32TCEC)
+        assert handle.last_route()[0] == api.ROUTE_PRESPLIT_SINGLE
         assert oracle.residual(off, c.cpu().numpy(), 128) < oracle.error_threshold(True, 64)
