@@ -276,6 +276,52 @@ def test_pointer_array_batched_entry_points(oracle):
         lib.cuMpSGEMM_hijack_unset_compute_mode()
 
 
+@pytest.mark.parametrize("cplx", [False, True])
+def test_pointer_array_with_cut_tiles(cplx):
+    """A pointer-array batch of 256 pair tiles, the last 34 of which are cut along K: the kernel that
+    adds the pieces finds every C through the array, and the bits are those of the strided call."""
+    torch, lib = _setup()
+    blas = torch.cuda.current_blas_handle()
+    batch, m, n, k = (2, 1024, 4096, 1024) if cplx else (2, 2048, 4096, 2048)
+    out = [C.c_uint32() for _ in range(5)]
+    assert lib.cuMpSGEMM_plan_pair(256, 74, 2048, 0, *map(C.byref, out)) == 0 and out[2].value > 0
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    a, b, c0 = (torch.randn(batch * s, device="cuda", generator=g,
+                            dtype=torch.complex64 if cplx else torch.float32)
+                for s in (m * k, k * n, m * n))
+    alpha, beta = ((C.c_float * 2)(1.0, -0.5), (C.c_float * 2)(0.5, 0.25)) if cplx else (
+        C.c_float(1.5), C.c_float(0.5))
+    strided = lib.cublasCgemmStridedBatched if cplx else lib.cublasSgemmStridedBatched
+    arrays = lib.cublasCgemmBatched if cplx else lib.cublasSgemmBatched
+
+    def scattered(x, size):
+        """Copies of the batch's matrices, allocated last one first, and the array of their addresses."""
+        mats = [x[i * size:(i + 1) * size].clone() for i in reversed(range(batch))][::-1]
+        return mats, torch.tensor([t.data_ptr() for t in mats], dtype=torch.int64, device="cuda")
+
+    try:
+        lib.cuMpSGEMM_hijack_set_compute_mode(1)
+        want = c0.clone()
+        assert strided(blas, 0, 0, m, n, k, C.byref(alpha), a.data_ptr(), m, m * k, b.data_ptr(), k, k * n,
+                       C.byref(beta), want.data_ptr(), m, m * n, batch) == 0
+        (ma, pa), (mb, pb), (mc, pc) = scattered(a, m * k), scattered(b, k * n), scattered(c0, m * n)
+        assert arrays(blas, 0, 0, m, n, k, C.byref(alpha), pa.data_ptr(), m, pb.data_ptr(), k, C.byref(beta),
+                      pc.data_ptr(), m, batch) == 0
+        torch.cuda.synchronize()
+        got = torch.cat(mc)
+        assert torch.equal(got, want)
+    finally:
+        lib.cuMpSGEMM_hijack_unset_compute_mode()
+    wide = torch.complex128 if cplx else torch.float64
+    al, be = (1 - 0.5j, 0.5 + 0.25j) if cplx else (1.5, 0.5)
+    for i in range(batch):                        # column-major products: the transposes, row-major
+        x, y, z, r = (t.view(batch, rows, cols)[i].to(wide) for t, rows, cols in
+                      ((a, k, m), (b, n, k), (c0, n, m), (got, n, m)))
+        truth = al * (y @ x) + be * z
+        assert float((r - truth).norm() / truth.norm()) < 2.0 ** -23 * (2 * k if cplx else k) ** 0.5
+
+
 TORCH_CLIENT = r"""
 import torch
 torch.backends.cuda.matmul.allow_tf32 = False
