@@ -5,10 +5,12 @@
 // (:549-605) and the AUTO / FP16TCEC_SCALING orchestration of the
 // interception layer (src/cumpsgemm_cublas.cu:445-577, :829-961).
 //
-// One call = split op(A) -> split op(B) -> tcgen05 GEMM, all on the handle's
-// stream.  The reference's module table (364 instantiations per arch,
-// src/instance_sm80.cu) collapses to three tile widths because op N/T/C,
-// leading dimensions and edges are absorbed by the split pass.
+// A call takes one of three routes, all on the handle's stream: split pass -> tcgen05 GEMM on the
+// panels (tcec_gemm.cu, tcec_gemm_pair.cu), one kernel on CTA pairs that splits its operands behind
+// TMA (tcec_gemm_stream.cu), or one on single CTAs that loads and splits them itself
+// (tcec_gemm_fused.cu); tiles cut along K are added by one more launch.  The reference's module
+// table (364 instantiations per arch, src/instance_sm80.cu) collapses to a few tile widths because
+// op N/T/C, leading dimensions and edges are absorbed where the operands are split.
 #include "gemm_common.cuh"
 #include "work_list.cuh"
 
@@ -77,13 +79,18 @@ template <> struct Scalar<cuComplex> {
 
 // ---------------------------------------------------------------- which kernel
 //
-// Estimated time of a call on each path, in microseconds.  A call is one or more waves of tiles,
+// Estimated time of a call on the pre-split and the streaming paths, in microseconds.  (The
+// on-the-fly kernel is not among them: it has rules of its own, see fused_args, and where they let
+// it in it is taken whenever streaming is not, whatever the pre-split path is estimated to take.)  A
+// call is one or more waves of tiles,
 // each as long as its K loop; what the paths trade is idle SMs against operand traffic, the split
 // pass against converting every operand element once per tile that uses it, and cutting tiles
 // along K against adding the pieces.  The constants are least-squares fits to 104 problems of
 // 1-80 pair tiles and k = 128-8192 with every path forced in turn (B200, mean error 5-9 %);
 // taking the path with the smallest estimate was 0.5 % slower on average than the best path of
-// each problem, the fixed rule it replaces 7 %.  Examples, us per call (K slices of 128 x 256
+// each problem, the fixed rule it replaces 7 %.  Beyond that range of k an estimate only has to put
+// the paths in the right order: operands that come from DRAM at a long row pitch are not modelled
+// (256 x 256 x 65536 streams in 48 us, estimated 33).  Examples, us per call (K slices of 128 x 256
 // tiles / 128 x 128 tiles / pairs in K pieces / streaming):
 //   2048 x 1024 x 2048     43 / 30 / 37 / 40        464 x 3256 x 7240      113 / 102 / 98 / 80
 //   1536 x 1536 x 4096     69 / 58 / 63 / 62        512 x 4096 x 4096       77 / 64 / 67 / 62
@@ -456,7 +463,9 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
 
   // A single wave of 128 x 64 tiles and at most 12 units of K: that tile has the smallest constant and
   // the smallest slope of all estimates then, so a small call, whose time is mostly the host's,
-  // does not work the others out.
+  // does not work the others out.  (Only streaming has no split pass to pay for: 4096 rows of 768 k
+  // values are 25 MB of split traffic, 38 in TF32TCEC, at 0.073 us a MB 1.8 and 2.8 us, about the 2.1
+  // and 2.8 by which its constant is larger.)
   const bool small = ec && batch < 8 && k_exp <= 768 && m_exp + n <= 4096 &&
                      h->tuning.untouched() &&
                      ((m_exp + 127) / 128) * ((n + 63) / 64) * batch <= h->num_sms;
@@ -472,8 +481,12 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
 
   // ---- one launch on CTA pairs, operands split between TMA and the tensor core
   StreamGemmArgs ga;
-  // (batches of matrices with at most 128 rows would leave one CTA of every pair idle: the kernel
-  // below serves those it can, 2048 x 128^3 82 us against 95-110 here)
+  // (Batches of matrices with at most 128 rows would leave one CTA of every pair idle, and go to the
+  // kernel below where it can take them.  Measured, on the fly / streaming, us: 2048 x 128^3 82 / 110,
+  // 2048 x 128 x 64 x 64 47 / 75, 512 x 128 x 512 x 128 86 / 100, 2048 x complex 64 x 128 x 128
+  // 132 / 166; but 512 x 128 x 256 x 256 78 / 73, 512 x 128 x 128 x 512 95 / 81, 512 x 64 x 256 x 256
+  // 79 / 65, 64 x 64 x 512 x 1024 70 / 56, 64 x 128 x 128 x 128 12.6 / 11.0: the rule is right for
+  // large batches of short products and gives up to a quarter away elsewhere.)
   FusedGemmArgs fa;
   const bool fused = !small && mode == CUMPSGEMM_FP16TCEC && !ptr_arrays &&
                      fused_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch,

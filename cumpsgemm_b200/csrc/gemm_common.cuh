@@ -43,7 +43,7 @@ struct GemmKernelParams {
   uint16_t k_slices;
   // Stages whose hi*hi products accumulate in TMEM before one drain (pair kernel; 1 or 2).
   uint16_t drain_chunk;
-  // Stages in the first chunk of every tile (pair kernel; >= drain_chunk).
+  // Stages in the first chunk of every tile (pair and on-the-fly kernels; >= drain_chunk).
   uint16_t first_chunk;
   uint16_t is_complex;
 };

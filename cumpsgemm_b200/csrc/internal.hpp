@@ -70,10 +70,11 @@ struct Profiler {
 // (cuMpSGEMM_reload_tuning_env reads them again); entry points without a handle read them per
 // call.  CUMPSGEMM_TILE_N = 256 / 128 / 64 forces the tile width, CUMPSGEMM_PAIR = 0 / 1 the
 // CTA-pair kernel off / on, CUMPSGEMM_DRAIN_CHUNK and CUMPSGEMM_FIRST_CHUNK the number of
-// K stages per accumulator drain (pair kernel), CUMPSGEMM_PACE = 0 the wave pacing off,
-// CUMPSGEMM_FUSED = 0 / 1 the kernel that splits operands on the fly off / on wherever it is
-// applicable, CUMPSGEMM_SPLIT_K = 0 / n the K-slicing of problems with few tiles off / to n
-// slices.
+// K stages per accumulator drain and in the first one of a tile (pair and on-the-fly kernels),
+// CUMPSGEMM_PACE = 0 the wave pacing off, CUMPSGEMM_FUSED = 0 / 1 the kernel that splits operands
+// on the fly off / on wherever it is applicable, CUMPSGEMM_SPLIT_K = 0 / n the K-slicing of
+// problems with few tiles off / to n slices.  A switch of one kernel keeps the streaming kernel off,
+// unless CUMPSGEMM_STREAM says otherwise, so that it reaches the kernel it is meant for.
 struct Tuning {
   int tile_n = 0;      // 0 = by rule
   int pair = -1;       // -1 = by rule

@@ -103,8 +103,7 @@ enum : int {
   kErrWaitD0Full = 4,  // epilogue waited for a chunk's main accumulator
   kErrWaitD1Full = 5,  // epilogue waited for the correction accumulator
   kErrBadLaunch = 6,
-  kErrWaitD1Empty = 7, // MMA issuer waited for the epilogue to read the correction accumulator
-  kErrWaitTail = 8     // epilogue warps of a CTA waited for one another (tail split of the pair kernel)
+  kErrWaitD1Empty = 7  // MMA issuer waited for the epilogue to give the correction accumulator back
 };
 
 constexpr uint64_t kWaitLimitNs = 1000ull * 1000ull * 1000ull; // 1 s

@@ -9,12 +9,13 @@
 // K-major layout a UMMA shared-memory descriptor reads.  Per stage the tensor core then forms
 // the three products hi*hi, hi*lo and lo*hi; every chunk of stages the accumulators are
 // drained and added to an FP32 running sum with round-to-nearest adds outside the tensor core
-// (hi*hi as it is, the two corrections times 2^-11), and the alpha / beta epilogue is the one
-// of tcec_gemm_pair.cu.
+// (hi*hi as it is, the two corrections times 2^-11), and the alpha / beta epilogue stores from the
+// registers (many short tiles per launch: see epilogue.cuh on the rolled one of the other kernels).
 //
 // It pays where the split pass of the two-kernel path costs as much as the GEMM: short K and
-// many small problems (strided batches of a few hundred rows), where writing the panels to HBM
-// and reading them back is most of the traffic.  It loses for long K on large matrices, where
+// many small problems (strided batches of at most 128 rows, where a CTA pair of
+// tcec_gemm_stream.cu would leave one CTA idle), where writing the panels to HBM and reading them
+// back is most of the traffic.  It loses for long K on large matrices, where
 // every operand element is converted once per tile that uses it (n / BN times for A, m / 128
 // times for B) and the converter warps, not the tensor core, set the pace; the dispatch keeps
 // the pre-split path there.  A second regime is a handful of tiles with a very long K loop:
@@ -608,9 +609,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) tcec_gemm_fused_kernel(const F
           const uint64_t a_lo = a_hi + kALo, b_hi = a_hi + kBHi;
           // Every tcgen05.mma reads its A tile from shared memory anew, and a 128 x 128 x 16
           // product is as long as that read.  The B_hi and B_lo tiles of a stage are adjacent in
-          // shared memory, so A_hi x [B_hi; B_lo] is ONE instruction of twice the width that yields hi*hi (columns 0..BN) and hi*lo
-          // (columns BN..2BN); lo*hi is added onto the second half.  Eight instructions per
-          // stage instead of twelve, and all three products of a chunk leave TMEM together.
+          // shared memory, so A_hi x [B_hi; B_lo] is ONE instruction of twice the width that
+          // yields hi*hi (columns 0..BN) and hi*lo (columns BN..2BN); lo*hi is added onto the
+          // second half.  Eight instructions per stage instead of twelve, and all three products
+          // of a chunk leave TMEM together.
 #pragma unroll
           for (int ks = 0; ks < K_STEPS; ++ks) {
             ptx::mma_f16_ss(acc_hh, a_hi + 2 * ks, b_hi + 2 * ks, IDESC2,
@@ -800,8 +802,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) tcec_gemm_fused_kernel(const F
         }
         continue;
       }
-      // general case; loads of a group of columns are all issued before its first store
-      // (see tcec_gemm_pair.cu)
+      // general case; loads of a group of columns are all issued before its first store (the
+      // compiler must assume that a store aliases the next load)
       constexpr int EPI_BATCH = 8;
 #pragma unroll
       for (int i0 = 0; i0 < CPT; i0 += EPI_BATCH) {
@@ -916,9 +918,9 @@ cudaError_t launch_fused_variant(const FusedGemmArgs &a, cudaStream_t stream) {
   p.status = a.dev_status;
   p.debug = nullptr;
   p.wave_counter = nullptr;
-  // drain every two stages (128 k values); the first chunk of a tile follows the accuracy rule
-  // of the pair kernel (tcec_gemm_pair.cu): it may be longer while the epilogue warps still
-  // store the previous tile
+  // drain every two stages (128 k values); the first chunk of a tile may be longer, the epilogue
+  // warps are still storing the previous tile then: 512 k values where K is long enough for that
+  // not to show in the error (8192 and more), 256 from 2048 on
   p.drain_chunk = (a.tuning.drain_chunk >= 1) ? static_cast<uint32_t>(a.tuning.drain_chunk) : 2u;
   const uint32_t k_total = p.k_blocks * KS;
   const uint32_t first_k = (k_total >= 8192u) ? 512u : (k_total >= 2048u ? 256u : 128u);

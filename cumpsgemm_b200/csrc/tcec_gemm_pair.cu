@@ -12,13 +12,12 @@
 // walks the tiles  t = cluster, cluster + #clusters, ...  The producer and the MMA issuer run
 // ahead into the next tile while the epilogue warps still write the previous one: the next
 // tile's operands are loaded and its hi*hi products start as soon as the last drain of D0 is
-// done; its correction products wait only until the epilogue has copied D1 into registers.
-// Three schedule details came out of measurements and are explained where they are coded:
+// done; its correction products wait until the epilogue gives D1 back, which is after the stores:
+// the finished sums are kept in the D1 columns and stored from there (epilogue.cuh).
+// Two schedule details came out of measurements and are explained where they are coded:
 // clusters announce every tile start on a device counter and wait for their wave (keeps
 // clusters that share panel rows at the same k, so the rows are fetched from DRAM once per
-// wave); the first drain chunk of a tile is longer than the others (the epilogue warps are
-// still storing the previous tile then); with beta != 0 the C tile is prefetched into L2 and
-// read in groups of columns.
+// wave); with beta != 0 the C tile is prefetched into L2 and read in groups of columns.
 //
 // Barriers (one set per CTA at identical shared-memory offsets; "leader" = cluster rank 0):
 //   full[s]   leader's only: 1 arrival (leader's producer, expect_tx of both CTAs' bytes);
@@ -27,7 +26,7 @@
 //   d0_full   in both CTAs: commit multicast after the hi*hi products of a chunk of stages
 //   d0_empty  leader's only: 16 arrivals = 8 drain warps of each CTA (remote mbarrier arrive)
 //   d1_full   in both CTAs: commit multicast after the last stage of a tile
-//   d1_empty  leader's only: 16 arrivals, after the epilogue warps have read D1
+//   d1_empty  leader's only: 16 arrivals, after the epilogue warps have stored the tile from D1
 // Every wait is bounded; no TMA multicast is used.
 #include "epilogue.cuh"
 #include "gemm_common.cuh"
@@ -522,8 +521,8 @@ bool pair_prepare(const TcecGemmArgs &a, SplitKind kind, int max_clusters, CUten
     const uint32_t dflt = (static_cast<uint64_t>(p.tiles_m) * p.tiles_n * a.batch > pairs) ? 2 : 1;
     p.drain_chunk = static_cast<uint16_t>((v >= 1) ? (v > 0xffff ? 0xffff : v) : dflt);
     // The first chunk of a tile may be longer (the epilogue warps are still storing the previous
-    // tile then), but by default it is not: 512 FP16 k values in it cost accuracy and, with the
-    // rolled epilogue, bought no time.
+    // tile then).  By default it is not: accuracy falls with the length of a chunk, and time hardly
+    // does (4096^3, beta = 0.5, us per call with a first chunk of 2 / 4 / 8 stages: 336 / 337 / 328).
     const int fv = a.tuning.first_chunk;
     p.first_chunk = static_cast<uint16_t>((fv >= 1) ? (fv > 0xffff ? 0xffff : fv) : p.drain_chunk);
     if (p.first_chunk < p.drain_chunk) p.first_chunk = p.drain_chunk;

@@ -23,10 +23,13 @@
 // What bounds it: shared-memory traffic.  Per stage of 64 k values an SM's shared memory takes 64 KiB
 // from TMA, gives 64 KiB to the converters, takes 64 KiB of hi / lo tiles back and feeds 96 KiB
 // to the tensor core: 2304 cycles at 128 bytes per cycle, against 1536 of tensor-core work.
-// Measured 2450 cycles per stage (m = n = k = 2048), and with short tiles about 4,500 per tile for
-// the hand-over of D1 on top.  Measured per call, paths that applied before / here (us): 512 x
-// complex 256^3 FP16TCEC_SCALING (one third of it the scan) 558 / 374, 512 x 256^3 123 / 80,
-// TF32TCEC 512 x 256^3 262 / 104, 256 x 256 x 65536 68.7 / 48.7.  Errors against 64-bit products
+// Measured 2570 cycles per stage at m = n = k = 2048 (the issuer's counters, see
+// cuMpSGEMM_set_debug_buffer; 260 of them waiting for accumulators), and with short tiles 8,000 to
+// 9,400 cycles per tile of waiting at D0 and D1: the epilogue gives D1 back only after the last
+// column is stored (512 x complex 256^3: 3230 cycles per stage, eight stages a tile).  Measured per
+// call, paths that applied before / here (us): 512 x complex 256^3 FP16TCEC_SCALING (a quarter of it
+// the scan) 574 / 377, 512 x 256^3 123 / 80-90, TF32TCEC 512 x 256^3 262 / 104-125, 256 x 256 x 65536
+// 69.6 / 48.3.  Errors against 64-bit products
 // are equal or smaller (those two: 2.1e-7 -> 1.5e-7 and 4.1e-7 -> 2.1e-7), because D0 is drained
 // every 64 FP16 / 32 TF32 values.
 //
@@ -818,8 +821,12 @@ template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, 
   p.w.slice_units = 0;
   p.w.piece_clusters = static_cast<uint16_t>(plan.piece_clusters);
   p.w.slices = static_cast<uint16_t>(plan.slices);
-  // direct stores: at least three waves of whole tiles of a short K loop, beta = 0 (with 256 columns
-  // the sums leave too few registers for it)
+  // Direct stores: at least three waves of whole tiles of a short K loop, beta = 0 (with 256 columns
+  // the sums leave too few registers for it).  What they save is a tile's hand-over, so the gain
+  // shrinks with the K loop.  Batches of 256 x 128 x 64u, looped / direct stores, us, three and eight
+  // waves (medians of runs in turn): FP16TCEC u = 1 15.6 / 15.2 and 31.9 / 31.1, u = 4 28.3 / 27.4 and
+  // 59.8 / 59.4, u = 8 44.6 / 44.3 and 103.4 / 102.9; TF32TCEC u = 2 30.6 / 29.9 and 58.3 / 57.4, u = 8
+  // 58.1 / 57.9.  At u = 16 and above, and at one wave, the two sides differ by less than their runs.
   if (BN == 128 && plan.piece_clusters == 0 && plan.whole_tiles >= 3u * static_cast<uint32_t>(max_clusters) &&
       plan.units <= 16 && a.beta_r == 0.f && a.beta_i == 0.f)
     p.flags |= kDirectStores;

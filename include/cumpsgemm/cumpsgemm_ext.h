@@ -125,8 +125,7 @@ cublasStatus_t cuMpSGEMM_sgemm_module(
  * code in a device word.  This call synchronises the handle's stream, returns the word and
  * clears it.  0 = no error; 1 = a producer / converter waited for a free stage, 2 = the MMA
  * issuer for operands, 3 / 7 = the MMA issuer for the drain of an accumulator, 4 / 5 = the
- * epilogue for an accumulator, 6 = bad launch, 8 = the epilogue warps of a CTA for one another
- * (tail split of the CTA-pair kernel). */
+ * epilogue for an accumulator, 6 = bad launch. */
 int cuMpSGEMM_get_kernel_status(cuMpSGEMM_handle_t handle);
 /* Which kernels the handle's last GEMM call launched, and in *cut_along_k (nullable) whether any of
  * its tiles was cut along K; host state only, nothing is synchronised.  CUMPSGEMM_ROUTE_NONE: no call
@@ -145,8 +144,10 @@ int cuMpSGEMM_get_last_route(cuMpSGEMM_handle_t handle, int *cut_along_k);
  * the time the wait took.  The context stays usable; nothing faults. */
 int cuMpSGEMM_selftest_bounded_wait(cuMpSGEMM_handle_t handle, unsigned limit_ms,
                                     double *waited_ms);
-/* Cap (bytes) for the operand workspace a strided-batch call may use at once; batches beyond
- * it are processed in chunks.  0 restores the default (8 GiB). */
+/* Cap (bytes) for the workspace a call may use at once: the panels of a strided batch beyond it are
+ * (with the sums of K slices, where the pre-split route cuts K) are processed in chunks of at least
+ * one matrix, and sums of K pieces that would go beyond it are left out (the tiles stay whole then).
+ * 0 restores the default (8 GiB). */
 void cuMpSGEMM_set_workspace_limit(cuMpSGEMM_handle_t handle, size_t bytes);
 /* Compatibility switch for the exponent statistics (off by default; also set by the
  * environment variable CUMPSGEMM_COUNT_TAIL_PADDING=1 at handle creation).  The reference's
@@ -159,8 +160,8 @@ void cuMpSGEMM_set_workspace_limit(cuMpSGEMM_handle_t handle, size_t bytes);
 void cuMpSGEMM_set_count_tail_padding(cuMpSGEMM_handle_t handle, int enable);
 /* A handle reads the tuning variables (CUMPSGEMM_TILE_N, CUMPSGEMM_PAIR, CUMPSGEMM_DRAIN_CHUNK,
  * CUMPSGEMM_FIRST_CHUNK, CUMPSGEMM_PACE, CUMPSGEMM_FUSED, CUMPSGEMM_SPLIT_K,
- * CUMPSGEMM_TAIL_SPLIT, CUMPSGEMM_STREAM) once, when it is created, so that a GEMM call does not query the
- * environment; this reads them again. */
+ * CUMPSGEMM_TAIL_SPLIT, CUMPSGEMM_STREAM) once, when it is created, so that a GEMM call does not
+ * query the environment; this reads them again. */
 void cuMpSGEMM_reload_tuning_env(cuMpSGEMM_handle_t handle);
 /* Host-only query (no GPU needed): the K slices of the CTA-pair kernel's last, partly filled wave,
  * for `total_tiles` tiles of 256 x 256 with a K loop of k_pad values (a multiple of 64; tf32 != 0

@@ -54,7 +54,7 @@ def test_every_unit_of_every_tile_is_done_once(clib, tile_n, clusters):
             assert sum(p[1] for p in parts) == units
         for tile, parts in pieces_of.items():
             # ascending k is ascending cluster, without gaps, and every piece but the first is its
-            # cluster's first item: what the summing CTA relies on
+            # cluster's first item: what the kernel that adds them relies on
             parts.sort()
             cs = [p[1] for p in parts]
             assert cs == list(range(cs[0], cs[0] + len(cs)))
