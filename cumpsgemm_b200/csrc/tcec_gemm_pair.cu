@@ -87,51 +87,48 @@ struct PairPlan {
   WorkPlan w;
 };
 
-template <int KIND>
-__device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtensorMap &map_b,
-                                          const GemmKernelParams &p, const PairPlan &plan) {
-  constexpr int K_STEPS = ROW_BYTES / 32;
-  constexpr uint32_t STAGES_PER_UNIT = (KIND == 0) ? 1 : 2; // a unit is 64 k values
-  constexpr int MY_MODE = (KIND == 0) ? CUMPSGEMM_FP16TCEC : CUMPSGEMM_TF32TCEC;
-  constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, 2 * BM_CTA, BN_PAIR);
-  constexpr int CPT = BN_PAIR / 2;
+// Where a CTA's stages, barriers and flags are in shared memory.
+struct SharedLayout {
+  uint8_t *smem;
+  uint64_t *full_bar, *empty_bar, *d0_full, *d0_empty, *d1_full, *d1_empty;
+  uint32_t *tmem_base_ptr;
+  volatile int *abort_flag;
+  __device__ __forceinline__ SharedLayout() {
+    extern __shared__ uint8_t smem_raw[];
+    smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                       ~static_cast<uintptr_t>(1023));
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES);
+    full_bar = bars;
+    empty_bar = bars + STAGES;
+    d0_full = bars + 2 * STAGES;
+    d0_empty = bars + 2 * STAGES + 1;
+    d1_full = bars + 2 * STAGES + 2;
+    d1_empty = bars + 2 * STAGES + 3;
+    tmem_base_ptr = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
+    abort_flag = reinterpret_cast<volatile int *>(tmem_base_ptr + 1);
+  }
+};
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t *smem = reinterpret_cast<uint8_t *>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES);
-  uint64_t *full_bar = bars;
-  uint64_t *empty_bar = bars + STAGES;
-  uint64_t *d0_full = bars + 2 * STAGES;
-  uint64_t *d0_empty = bars + 2 * STAGES + 1;
-  uint64_t *d1_full = bars + 2 * STAGES + 2;
-  uint64_t *d1_empty = bars + 2 * STAGES + 3;
-  uint32_t *tmem_base_ptr = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_base_ptr + 1);
-
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const uint32_t rank = ptx::cluster_ctarank();
-  const bool leader = (rank == 0);
-  const uint32_t cluster_id = blockIdx.x >> 1;
-  const uint32_t num_clusters = gridDim.x >> 1;
-
+// Barriers, TMEM, tensor maps, and the peer's: what a CTA does before it needs anything of an earlier
+// kernel, the same for both kinds.  Returns the TMEM address.
+__device__ __forceinline__ uint32_t set_up(const CUtensorMap &map_a, const CUtensorMap &map_b) {
+  const SharedLayout sm;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      ptx::mbar_init(ptx::smem_u32(&full_bar[s]), 1);
-      ptx::mbar_init(ptx::smem_u32(&empty_bar[s]), 1);
+      ptx::mbar_init(ptx::smem_u32(&sm.full_bar[s]), 1);
+      ptx::mbar_init(ptx::smem_u32(&sm.empty_bar[s]), 1);
     }
-    ptx::mbar_init(ptx::smem_u32(d0_full), 1);
-    ptx::mbar_init(ptx::smem_u32(d0_empty), 2 * NUM_EPI_WARPS);
-    ptx::mbar_init(ptx::smem_u32(d1_full), 1);
-    ptx::mbar_init(ptx::smem_u32(d1_empty), 2 * NUM_EPI_WARPS);
-    *abort_flag = 0;
+    ptx::mbar_init(ptx::smem_u32(sm.d0_full), 1);
+    ptx::mbar_init(ptx::smem_u32(sm.d0_empty), 2 * NUM_EPI_WARPS);
+    ptx::mbar_init(ptx::smem_u32(sm.d1_full), 1);
+    ptx::mbar_init(ptx::smem_u32(sm.d1_empty), 2 * NUM_EPI_WARPS);
+    *sm.abort_flag = 0;
     ptx::mbar_init_fence();
     ptx::prefetch_tensormap(&map_a);
     ptx::prefetch_tensormap(&map_b);
   }
-  if (warp == 1) {
-    ptx::tmem_alloc_pair(ptx::smem_u32(tmem_base_ptr), TMEM_COLS);
+  if ((threadIdx.x >> 5) == 1) {
+    ptx::tmem_alloc_pair(ptx::smem_u32(sm.tmem_base_ptr), TMEM_COLS);
     ptx::tmem_relinquish_pair();
   }
   ptx::tc_fence_before();
@@ -140,7 +137,34 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
   ptx::cluster_arrive();
   ptx::cluster_wait();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *tmem_base_ptr;
+  return *sm.tmem_base_ptr;
+}
+
+// SET_UP = false: the caller has called set_up.
+template <int KIND, bool SET_UP = true>
+__device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtensorMap &map_b,
+                                          const GemmKernelParams &p, const PairPlan &plan) {
+  constexpr int K_STEPS = ROW_BYTES / 32;
+  constexpr uint32_t STAGES_PER_UNIT = (KIND == 0) ? 1 : 2; // a unit is 64 k values
+  constexpr int MY_MODE = (KIND == 0) ? CUMPSGEMM_FP16TCEC : CUMPSGEMM_TF32TCEC;
+  constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, 2 * BM_CTA, BN_PAIR);
+  constexpr int CPT = BN_PAIR / 2;
+
+  const SharedLayout sm;
+  uint8_t *smem = sm.smem;
+  uint64_t *full_bar = sm.full_bar, *empty_bar = sm.empty_bar;
+  uint64_t *d0_full = sm.d0_full, *d0_empty = sm.d0_empty;
+  uint64_t *d1_full = sm.d1_full, *d1_empty = sm.d1_empty;
+  volatile int *abort_flag = sm.abort_flag;
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = ptx::cluster_ctarank();
+  const bool leader = (rank == 0);
+  const uint32_t cluster_id = blockIdx.x >> 1;
+  const uint32_t num_clusters = gridDim.x >> 1;
+
+  const uint32_t tmem_base = SET_UP ? set_up(map_a, map_b) : *sm.tmem_base_ptr;
   const uint32_t k_blocks = p.k_blocks;
   const bool dbg = (p.debug != nullptr);
   unsigned long long dbg_wait = 0, dbg_wait2 = 0;
@@ -440,11 +464,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
                                const __grid_constant__ CUtensorMap map_a32,
                                const __grid_constant__ CUtensorMap map_b32,
                                const GemmKernelParams p32, const PairPlan plan) {
+  set_up(map_a16, map_b16);
   ptx::griddep_wait(); // the decision is written by an earlier kernel of the call
   if (p16.dyn->gemm_mode == CUMPSGEMM_TF32TCEC) {
-    pair_body<1>(map_a32, map_b32, p32, plan);
+    pair_body<1, false>(map_a32, map_b32, p32, plan);
   } else {
-    pair_body<0>(map_a16, map_b16, p16, plan);
+    pair_body<0, false>(map_a16, map_b16, p16, plan);
   }
 }
 
