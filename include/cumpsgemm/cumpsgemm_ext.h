@@ -146,7 +146,8 @@ int cuMpSGEMM_selftest_bounded_wait(cuMpSGEMM_handle_t handle, unsigned limit_ms
                                     double *waited_ms);
 /* Cap (bytes) for the workspace a call may use at once: the panels of a strided batch beyond it are
  * (with the sums of K slices, where the pre-split route cuts K) are processed in chunks of at least
- * one matrix, and sums of K pieces that would go beyond it are left out (the tiles stay whole then).
+ * one matrix, and sums of K pieces that would take a call beyond a limit it otherwise keeps are left
+ * out (the tiles stay whole then).
  * 0 restores the default (8 GiB). */
 void cuMpSGEMM_set_workspace_limit(cuMpSGEMM_handle_t handle, size_t bytes);
 /* Compatibility switch for the exponent statistics (off by default; also set by the
