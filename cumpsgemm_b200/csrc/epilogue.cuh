@@ -46,6 +46,47 @@ template <int CPT> __device__ __forceinline__ void drain_sums(uint32_t taddr, fl
   }
 }
 
+// The same on pairs of sums, one packed instruction per two columns.
+__device__ __forceinline__ void add_pair(unsigned long long &acc, uint32_t x, uint32_t y) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(x), "r"(y));
+  asm volatile("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(v));
+}
+__device__ __forceinline__ void scale_pair(unsigned long long &acc, float s) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(s));
+  asm volatile("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(v));
+}
+template <int CPT>
+__device__ __forceinline__ void drain_pairs(uint32_t taddr, unsigned long long (&acc)[CPT / 2]) {
+#pragma unroll
+  for (int c = 0; c < CPT; c += 16) {
+    uint32_t v[16];
+    ptx::tmem_ld_32x32b_x16(taddr + c, v);
+    ptx::tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) add_pair(acc[c / 2 + i], v[2 * i], v[2 * i + 1]);
+  }
+}
+// acc + TMEM columns, left in the columns
+template <int CPT>
+__device__ __forceinline__ void finish_pairs_in_tmem(uint32_t taddr,
+                                                     unsigned long long (&acc)[CPT / 2]) {
+#pragma unroll
+  for (int c = 0; c < CPT; c += 16) {
+    uint32_t v[16];
+    ptx::tmem_ld_32x32b_x16(taddr + c, v);
+    ptx::tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      add_pair(acc[c / 2 + i], v[2 * i], v[2 * i + 1]);
+      asm("mov.b64 {%0, %1}, %2;" : "=r"(v[2 * i]), "=r"(v[2 * i + 1]) : "l"(acc[c / 2 + i]));
+    }
+    ptx::tmem_st_32x32b_x16(taddr + c, v);
+  }
+  ptx::tmem_st_wait();
+}
+
 // acc -> TMEM columns [taddr, taddr + CPT) of this warp's lanes
 template <int CPT> __device__ __forceinline__ void sums_to_tmem(uint32_t taddr, const float (&acc)[CPT]) {
 #pragma unroll

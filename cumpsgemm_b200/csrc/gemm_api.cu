@@ -90,7 +90,7 @@ template <> struct Scalar<cuComplex> {
 // taking the path with the smallest estimate was 0.5 % slower on average than the best path of
 // each problem, the fixed rule it replaces 7 %.  Beyond that range of k an estimate only has to put
 // the paths in the right order: operands that come from DRAM at a long row pitch are not modelled
-// (256 x 256 x 65536 streams in 48 us, estimated 33).  Examples, us per call (K slices of 128 x 256
+// (256 x 256 x 65536 streams in 46 us, estimated 33).  Examples, us per call (K slices of 128 x 256
 // tiles / 128 x 128 tiles / pairs in K pieces / streaming):
 //   2048 x 1024 x 2048     43 / 30 / 37 / 40        464 x 3256 x 7240      113 / 102 / 98 / 80
 //   1536 x 1536 x 4096     69 / 58 / 63 / 62        512 x 4096 x 4096       77 / 64 / 67 / 62
@@ -133,15 +133,18 @@ struct PathModel {
     return 2.0 + 0.15 * split + 1.32 * std::ceil(stages / slices) +
            0.69e-6 * 4 * static_cast<double>(m) * n * batch * slices;
   }
-  double stream(const StreamPlan &pl) const { // tcec_gemm_stream.cu
+  // tcec_gemm_stream.cu.  (Fitted to 35 problems of 1-110 tiles and k = 96-32768 in each kind, mean
+  // error 5-9 %.  Examples, us, 256 / 128 columns: 2048 x 1024 x 2048 FP16TCEC 48 / 41, complex
+  // 1280 x 960 x 1500 61 / 66, 256 x 256 x 8192 23 / 18; TF32TCEC 4096 x 1024 x 2048 86 / 115.)
+  double stream(const StreamPlan &pl) const {
     const bool tf32 = stages > units, wide = pl.tile_n == 256;
-    double length = waves(pl.whole_tiles, pairs) * units, t = tf32 ? 8.5 : 7.8;
+    double length = waves(pl.whole_tiles, pairs) * units, t = 9.0;
     if (pl.piece_clusters > 0) {
       const double left = pl.total_tiles - pl.whole_tiles;
       length += std::ceil(left * units / pl.piece_clusters);
-      t += (tf32 ? 4.9 : 2.9) + 0.19 * left;
+      t += 4.9 + (wide ? 0.17 * left : 0.0);
     }
-    return t + length * (tf32 ? (wide ? 2.33 : 1.85) : (wide ? 1.56 : 1.35));
+    return t + length * (tf32 ? (wide ? 2.43 : 1.62) : (wide ? 1.34 : 0.90));
   }
 };
 
@@ -296,28 +299,40 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
     return false;
   const std::uint64_t m_exp = m * fpe, k_exp = k * fpe;
   if (batch > 0x3fffffffull || n > 0x3fffffffull) return false; // (TMA coordinates are 32-bit)
-  const int tile_n = (t.stream == 128 || t.stream == 256) ? t.stream : (n <= 128 ? 128 : 256);
-  int clusters = 0;
-  if (stream_max_clusters(kind, tile_n, &clusters) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  const StreamPlan plan = plan_stream(t, tile_n, m_exp, n, k_exp, batch,
+  // The width: forced, or 128 for narrow products, or the one estimated to be faster (batches of small
+  // matrices, which the estimates are not fitted to: 256).
+  StreamPlan plan = {};
+  double best = presplit_us;
+  for (const int tile_n : {256, 128}) {
+    if ((t.stream == 128 || t.stream == 256) ? tile_n != t.stream : (n <= 128 && tile_n == 256)) continue;
+    int clusters = 0;
+    if (stream_max_clusters(kind, tile_n, &clusters) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    const StreamPlan pl = plan_stream(t, tile_n, m_exp, n, k_exp, batch,
                                       static_cast<std::uint32_t>(clusters));
-  if (plan.total_tiles == 0) return false;
-  if (t.stream == -1 && !small_matrix_batch(plan, m_exp, n, batch, clusters)) {
-    // beyond one and a half waves the operands are reused by too many tiles to convert them again
-    // for each (4096^3 TF32TCEC: 600 us against 560), and the model is not fitted to it
-    if (2ull * plan.total_tiles > 3ull * static_cast<std::uint64_t>(clusters)) return false;
+    if (pl.total_tiles == 0) continue;
+    if (t.stream != -1 || small_matrix_batch(pl, m_exp, n, batch, clusters)) {
+      plan = pl;
+      break;
+    }
+    // beyond one and a half waves of wide tiles the operands are reused by too many tiles to convert
+    // them again for each (4096 x 4096 x 1024: 102 us against 91), and the model is not fitted to it
+    if (2ull * pl.total_tiles > 3ull * (256 / tile_n) * static_cast<std::uint64_t>(clusters)) continue;
     // (the kind of an AUTO call is not known here: the mean of both)
     double us = 0.0;
     if (kind != StreamKind::tf32)
-      us += PathModel(h->num_sms, m_exp, n, k_exp, batch, false).stream(plan);
+      us += PathModel(h->num_sms, m_exp, n, k_exp, batch, false).stream(pl);
     if (kind != StreamKind::fp16)
-      us += PathModel(h->num_sms, m_exp, n, k_exp, batch, true).stream(plan);
+      us += PathModel(h->num_sms, m_exp, n, k_exp, batch, true).stream(pl);
     if (kind == StreamKind::device) us *= 0.5;
-    if (us >= presplit_us) return false;
+    if (us < best) {
+      best = us;
+      plan = pl;
+    }
   }
+  if (plan.total_tiles == 0) return false;
   *out = StreamGemmArgs{};
   out->kind = kind;
   out->a = StreamOperand{reinterpret_cast<const float *>(a), lda * fpe, sa};

@@ -135,8 +135,9 @@ cudaError_t launch_piece_fixup(const PieceFixupArgs &a, const WorkPlan &w, cudaS
   //   16 tiles in 64        (1024 x 1024 x 4096)          89  63  54  39  38  37
   //   16 of 90 tiles        (256 x 256 x 1536, batch 90)  128 101  94  79  79  80
   //   32 of 106 tiles       (the same, batch 106)         235 157 139  99  91  93
-  // So one group is right from about six tiles on, where the first line still gives four.
-  if (w.piece_clusters >= 8u * tiles) {
+  // So one group is right from about six tiles on (768 x 768 x 3072, nine tiles in 72: 36 us with
+  // four groups).
+  if (tiles < 6u && w.piece_clusters >= 8u * tiles) {
     if (tiles == 1) return launch<1, 4>(p, tiles, stream);
     if (tiles == 2) return launch<2, 4>(p, tiles, stream);
     return launch<4, 4>(p, tiles, stream);

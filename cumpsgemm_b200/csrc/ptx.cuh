@@ -186,6 +186,27 @@ __device__ __forceinline__ bool mbar_wait_timed(uint32_t bar, uint32_t parity,
   return ok;
 }
 
+// mbar_wait for code that is short of registers: the abort flag by its shared-memory address.
+__device__ __forceinline__ bool mbar_wait_s(uint32_t bar, uint32_t parity, uint32_t abort_smem,
+                                            int *status_gmem, int code) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const uint64_t t0 = globaltimer_ns();
+  uint32_t spins = 0;
+  while (true) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((++spins & 0x3f) == 0) {
+      int aborted;
+      asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(aborted) : "r"(abort_smem));
+      if (aborted) return false;
+      if (globaltimer_ns() - t0 > kWaitLimitNs) {
+        asm volatile("st.volatile.shared.s32 [%0], 1;" ::"r"(abort_smem) : "memory");
+        if (status_gmem != nullptr) atomicCAS(status_gmem, 0, code);
+        return false;
+      }
+    }
+  }
+}
+
 // Programmatic dependent launch.  A kernel launched with the programmatic-serialization
 // attribute may start while the kernel before it in the stream still runs; griddep_wait()
 // returns once that kernel has completed and its writes are visible (a no-op for a kernel
@@ -320,6 +341,21 @@ __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_
         "r"(r[14]), "r"(r[15])
       : "memory");
 }
+// same, 8 columns
+__device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               :
+               : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]),
+                 "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+// same, 4 columns
+__device__ __forceinline__ void tmem_st_32x32b_x4(uint32_t taddr, const uint32_t (&r)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};"
+               :
+               : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+               : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
@@ -408,6 +444,48 @@ __device__ __forceinline__ void mma_tf32_ss_pair(uint32_t d_tmem, uint64_t a_des
       "}\n"
       :
       : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// The same with A in tensor memory: lane = row (each CTA of the pair holds its own 128), a 32-bit
+// column = two consecutive FP16 or one TF32 value of K.
+__device__ __forceinline__ void mma_f16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                                uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mma_tf32_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                                 uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::tf32 [%0], [%1], %2, %3, p;\n\t"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// D[tmem] = A * B + D * 2^-SHIFT; kind::f16, A in tensor memory
+template <int SHIFT>
+__device__ __forceinline__ void mma_f16_ts_pair_scaled(uint32_t d_tmem, uint32_t a_tmem,
+                                                       uint64_t b_desc, uint32_t idesc) {
+  static_assert(SHIFT >= 0 && SHIFT <= 15, "range of scale-input-d");
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(SHIFT)
       : "memory");
 }
 

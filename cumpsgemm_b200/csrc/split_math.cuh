@@ -24,6 +24,27 @@ __device__ __forceinline__ void split2(float v0, float v1, uint32_t &hi, uint32_
   lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
+// The same values with v - hi already scaled: fma(hi, -2^11, v * 2^11) is exact, and taking hi as FP16
+// saves the conversion back.
+__device__ __forceinline__ void split2_mixed(float v0, float v1, uint32_t &hi, uint32_t &lo) {
+  unsigned long long v, w;
+  float w0, w1, d0, d1;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(v0), "f"(v1));
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(w) : "l"(v), "l"(0x4500000045000000ull)); // 2^11, twice
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(w0), "=f"(w1) : "l"(w));
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(v1), "f"(v0));
+  asm("{\n\t"
+      ".reg .b16 h0, h1, c;\n\t"
+      "mov.b32 {h0, h1}, %2;\n\t"
+      "mov.b16 c, 0xE800;\n\t" // -2^11
+      "fma.rn.f32.f16 %0, h0, c, %3;\n\t"
+      "fma.rn.f32.f16 %1, h1, c, %4;\n\t"
+      "}"
+      : "=f"(d0), "=f"(d1)
+      : "r"(hi), "f"(w0), "f"(w1));
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(d1), "f"(d0));
+}
+
 // hi = RNA_tf32(v), lo = RNA_tf32(v - hi)
 __device__ __forceinline__ void split_tf32(float v, uint32_t &hi, uint32_t &lo) {
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(v));

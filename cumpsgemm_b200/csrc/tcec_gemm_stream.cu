@@ -7,49 +7,54 @@
 //   * fetches its own 128 rows of op(A) and its own BN / 2 rows of op(B) as plain FP32 through TMA
 //     into a ring of raw slots (32 k values each; edges are zero filled by TMA, so no thread
 //     tests bounds),
-//   * has eight converter warps split the raw values into hi / lo (same bits as split_kernels.cu)
-//     and write them as 128-byte-swizzled K-major tiles into a ring of operand stages,
-//   * and holds its 128 rows of the two TMEM accumulators (D0 = hi*hi, drained every stage into
-//     FP32 registers; D1 = lo*hi + hi*lo, drained once per tile), which its eight epilogue warps
-//     drain.
+//   * has two teams of eight converter warps, which take the raw slots in turn and split the values
+//     into hi / lo (same bits as split_kernels.cu): A goes to tensor memory, lane = row, B to
+//     128-byte-swizzled K-major tiles in shared memory,
+//   * and holds its 128 rows of the accumulators in tensor memory, which its eight epilogue warps
+//     drain after every stage (64 FP16 / 32 TF32 values of k) into FP32 running sums in registers.
 // The even CTA's single issuing thread drives the tensor cores of both SMs (cta_group::2).
 //
-// Why pairs, and why raw slots in shared memory.  Per SM and 64 k values a 256 x 256 pair tile
-// converts 128 + 128 rows for a 128 x 256 share of C, half of what a 128 x 128 tile of
-// tcec_gemm_fused.cu converts per product.  Letting TMA run three slots ahead takes the
-// global-memory latency off the converter warps, which was a third of their time when they loaded
-// for themselves.
+// One accumulator per half of the tile's columns takes all three products of a stage: first the
+// corrections lo*hi + hi*lo, then hi*hi, whose first instruction scales what is there by 2^-11
+// (scale-input-d; TF32's lo is not scaled).  With accumulators of their own for the corrections and A
+// in shared memory, tensor memory was full and the tensor core read A three times and B three times
+// per stage through the shared-memory port, on top of TMA's and the converters' traffic: 2304 of the
+// 2570 cycles a stage of 64 k values took.  Now the port has 1664 to do, the corrections no longer hold
+// the next tile up, and three accumulators (BN = 128: four) of half a tile rotate.  Where K fits
+// one unit of 64 the corrections keep an accumulator of their own (kSeparate): adding them inside the
+// tensor core would truncate the one sum there is, 1.6e-7 instead of 6e-8 for k = 1.
 //
-// What bounds it: shared-memory traffic.  Per stage of 64 k values an SM's shared memory takes 64 KiB
-// from TMA, gives 64 KiB to the converters, takes 64 KiB of hi / lo tiles back and feeds 96 KiB
-// to the tensor core: 2304 cycles at 128 bytes per cycle, against 1536 of tensor-core work.
-// Measured 2570 cycles per stage at m = n = k = 2048 (the issuer's counters, see
-// cuMpSGEMM_set_debug_buffer; 260 of them waiting for accumulators), and with short tiles 8,000 to
-// 9,400 cycles per tile of waiting at D0 and D1: the epilogue gives D1 back only after the last
-// column is stored (512 x complex 256^3: 3230 cycles per stage, eight stages a tile).  Measured per
-// call, paths that applied before / here (us): 512 x complex 256^3 FP16TCEC_SCALING (a quarter of it
-// the scan) 574 / 377, 512 x 256^3 123 / 80-90, TF32TCEC 512 x 256^3 262 / 104-125, 256 x 256 x 65536
-// 69.6 / 48.3.  Errors against 64-bit products
-// are equal or smaller (those two: 2.1e-7 -> 1.5e-7 and 4.1e-7 -> 2.1e-7), because D0 is drained
-// every 64 FP16 / 32 TF32 values.
+// What bounds it: the instructions of the converters and the epilogue, and the power.  Cycles per stage of
+// 64 k values, m = n = k = 2048, 256 columns: 2570 before, 2100 now (1536 are tensor-core work; of
+// the issuer's 2100 it waits 860 for operands and 420 for accumulators); 128 columns 2310 -> 1520.
+// That took, each alone worth little and together the difference: the second converter team, the
+// epilogue's adds two at a time, a split in six instead of eight instructions per pair, and loops that
+// keep few enough registers not to spill.  Measured per call, before / now (us): 2048 x 1024 x 2048 with
+// 128 columns 47.8 / 34.2, complex 1280 x 960 x 1500 66 / 59, 2048^3 53.3 / 49.4, 512 x complex 256^3
+// 241 / 225 (beta = 0.5 328 / 289), 512 x 256^3 82 / 76, TF32TCEC 512 x 256^3 112 / 104, 256 x 256 x
+// 65536 50.0 / 47.6.  Errors against 64-bit products are equal or smaller (k = 96 ... 65536: 1.13e-7 ->
+// 1.11e-7, 2048: 1.598e-7 -> 1.581e-7; k <= 64: the same).
 //
 // Work distribution: work_list.cuh.  What is left over from whole waves (total mod clusters, or
 // everything when there are fewer tiles than clusters) can be cut along K; piece_fixup.cu then
 // adds the pieces and runs their epilogue.
 //
-// Threads: 640 = warp 0 TMA producer, warp 1 TMEM allocation + MMA issue (even CTA), warps 2-3
-// idle, warps 4-11 drain / epilogue, warps 12-19 converters.  Launched with 96 registers per
-// thread = 61440; setmaxnreg gives the epilogue warps 160 (they hold 128 running sums each), the
-// converters 56 and the rest 48: 256*160 + 256*56 + 128*48 = 61440, so the increase can always be
-// served.
+// Threads: 896 = warp 0 TMA producer, warp 1 TMEM allocation + MMA issue (even CTA), warps 2-3
+// idle, warps 4-11 drain / epilogue, warps 12-27 converters.  Launched with 72 registers per
+// thread = 64512, which setmaxnreg deals out again (StreamCfg); the sum is the same, so the increase
+// can always be served.
 //
 // Barriers (per CTA, same shared-memory offsets; "leader" = even CTA):
 //   raw_full[r]    1 arrival (producer, expect_tx) + TMA bytes      own CTA
-//   raw_empty[r]   8 arrivals, one per converter warp               own CTA
-//   full[s]        leader's only: 16 arrivals, 8 converter warps of each CTA
+//   raw_empty[r]   8 arrivals, one per warp of the slot's team      own CTA
+//   full[s]        leader's only: the converter warps of both CTAs
 //   empty[s]       tcgen05.commit multicast from the leader         both CTAs
-//   d0_full, d0_empty, d1_full, d1_empty: as in tcec_gemm_pair.cu
-// Every wait is bounded; no TMA multicast is used.
+//   d_full[b]      the same, after the products of one half of the columns
+//   d_empty[b]     leader's only: 8 arrivals, the epilogue warps of that half in both CTAs
+// Waits tell phases apart by one bit, so a waiter may be at most one phase behind: the number of raw
+// slots is even, because copies complete in any order and a slot that both teams used could show one
+// team the phase before the other's.  (Commits complete in order.)  Every wait is bounded; no TMA
+// multicast is used.
 #include "epilogue.cuh"
 #include "gemm_common.cuh"
 #include "ptx.cuh"
@@ -64,13 +69,10 @@ namespace {
 constexpr int BM_CTA = 128;
 constexpr int ROW_BYTES = kGemmRowBytes;
 constexpr int SLOT_K = 32; // k values of a raw slot (128 bytes of FP32)
-constexpr int NUM_THREADS = 640;
+constexpr int NUM_THREADS = 896;
 constexpr int FIRST_EPI_WARP = 4, NUM_EPI_WARPS = 8;
-constexpr int FIRST_CVT_WARP = 12, NUM_CVT_WARPS = 8;
-constexpr int LAUNCH_REGS = 96;
-constexpr int REGS_EPI = 160, REGS_CVT = 56, REGS_REST = 48;
-static_assert(256 * REGS_EPI + 256 * REGS_CVT + 128 * REGS_REST <= NUM_THREADS * LAUNCH_REGS,
-              "register re-allocation must fit what the CTA was launched with");
+constexpr int FIRST_CVT_WARP = 12, CVT_TEAMS = 2, TEAM_WARPS = 8;
+constexpr int LAUNCH_REGS = 72;
 constexpr uint32_t C_PREFETCH_LEAD = 8; // stages between the L2 prefetch of C and its use
 
 // Raw layouts a converter can read (values of StreamGemmArgs::layout_a / layout_b).
@@ -98,21 +100,40 @@ struct StreamParams {
 };
 static_assert(sizeof(StreamParams) <= 128, "kernel parameter structs stay within 128 bytes");
 constexpr uint32_t kIsComplex = 1, kConjA = 2, kConjB = 4, kBatchA = 8, kBatchB = 16,
-                   kDirectStores = 32;
+                   kDirectStores = 32, kSeparate = 64;
 
 template <int BN> struct StreamCfg {
-  static constexpr int B_ROWS = BN / 2; // rows of op(B) per CTA
-  static constexpr int A_TILE = BM_CTA * ROW_BYTES;
+  static constexpr int B_ROWS = BN / 2;     // rows of op(B) per CTA: two blocks of HALF_ROWS, one
+  static constexpr int HALF_ROWS = BN / 4;  // for each half of the tile's columns
   static constexpr int B_TILE = B_ROWS * ROW_BYTES;
-  static constexpr int STAGE_BYTES = 2 * (A_TILE + B_TILE);
-  static constexpr int STAGES = (BN == 256) ? 2 : 3;
+  static constexpr int STAGE_BYTES = 2 * B_TILE; // hi, lo
+  static constexpr int STAGES = (BN == 256) ? 2 : 4;
   static constexpr int RAW_A = BM_CTA * SLOT_K * 4;
-  static constexpr int RAW_BYTES = RAW_A + B_ROWS * SLOT_K * 4;
-  static constexpr int RAW_SLOTS = 3;
+  static constexpr int RAW_HALF_B = HALF_ROWS * SLOT_K * 4;
+  static constexpr int RAW_BYTES = RAW_A + 2 * RAW_HALF_B;
+  static constexpr int RAW_SLOTS = (BN == 256) ? 4 : 6;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + RAW_SLOTS * RAW_BYTES + 1024 + 256;
-  static constexpr uint32_t TMEM_COLS = 2 * BN;
+  // Tensor memory: accumulators of half a tile's columns each, then A, 64 columns per stage (hi, lo)
+  static constexpr uint32_t D_BUFS = (BN == 256) ? 3 : 4;
+  static constexpr uint32_t A_COL = D_BUFS * (BN / 2);
+  static constexpr int REGS_EPI = (BN == 256) ? 152 : 112;
+  static constexpr int REGS_CVT = (BN == 256) ? 40 : 48;
+  static constexpr int REGS_REST = (BN == 256) ? 40 : 72;
+  static_assert(256 * REGS_EPI + 512 * REGS_CVT + 128 * REGS_REST <= NUM_THREADS * LAUNCH_REGS,
+                "register re-allocation must fit what the CTA was launched with");
+  static_assert(REGS_EPI >= LAUNCH_REGS && REGS_CVT <= LAUNCH_REGS && REGS_REST <= LAUNCH_REGS,
+                "setmaxnreg.inc goes up, setmaxnreg.dec down: anything else is an illegal instruction");
+  // Barriers behind the raw slots, as byte offsets: eight bytes each
+  static constexpr uint32_t RAW_FULL = 0, RAW_EMPTY = 8 * RAW_SLOTS, FULL = RAW_EMPTY + 8 * RAW_SLOTS,
+                            EMPTY = FULL + 8 * STAGES, D_FULL = EMPTY + 8 * STAGES,
+                            D_EMPTY = D_FULL + 8 * D_BUFS, TMEM_PTR = D_EMPTY + 8 * D_BUFS,
+                            ABORT = TMEM_PTR + 4;
+  static_assert(ABORT + 4 <= 256, "barriers");
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
+  static_assert(RAW_SLOTS % CVT_TEAMS == 0, "a raw slot belongs to one team");
+  static_assert(A_COL + STAGES * 64 <= 512, "tensor memory");
 };
+constexpr uint32_t A_STAGE_COLS = 64, A_LO_COLS = 32, TMEM_COLS = 512;
 
 struct TileCoord {
   uint32_t batch;
@@ -132,12 +153,12 @@ __device__ __forceinline__ TileCoord tile_coord(uint32_t tile, const StreamParam
 }
 
 template <int KIND>
-__device__ __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+__device__ __forceinline__ void mma_pair(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc,
                                          uint32_t acc) {
   if constexpr (KIND == 0) {
-    ptx::mma_f16_ss_pair(d, a, b, idesc, acc);
+    ptx::mma_f16_ts_pair(d, a, b, idesc, acc);
   } else {
-    ptx::mma_tf32_ss_pair(d, a, b, idesc, acc);
+    ptx::mma_tf32_ts_pair(d, a, b, idesc, acc);
   }
 }
 
@@ -151,18 +172,17 @@ __device__ __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uin
 // ones are read 4 or 8 bytes per lane along the row.  Row r's 16-byte chunk q of a swizzled
 // tile is at r * 128 + ((q ^ (r & 7)) << 4), i.e. at (r * 128 + ((r & 7) << 4)) ^ (q << 4).
 struct ConverterState {
-  uint64_t *raw_full, *raw_empty, *empty;
-  uint32_t full_leader; // shared::cluster address of full[0] in the leader
-  uint32_t raw, dst;    // shared addresses of slot 0's raw tile and stage 0's hi tile of the operand
-  uint32_t lo_delta;
-  uint32_t row;         // this lane's row of the tile
+  uint32_t bars;        // shared address of this CTA's barriers
+  uint32_t bars_leader; // shared::cluster address of the leader's
+  uint32_t raw;         // shared address of slot 0's raw tile
+  uint32_t row;         // this lane's row of the raw tile
+  uint32_t dst;         // stage 0's hi values of the lane's row: shared address of the (swizzled) row
+                        // for B, the warp's tensor-memory address for A
+  uint32_t team;
   uint32_t group0;      // first of the warp's 8-k groups in a slot
   float scale;
   uint32_t conj_mask;   // sign bit if the operand is conjugated, else 0
-  volatile int *abort_flag;
   int *status;
-  bool timed;
-  unsigned long long wait_raw, wait_empty;
 };
 
 __device__ __forceinline__ float flip_sign(float x, uint32_t mask) {
@@ -212,34 +232,44 @@ __device__ __forceinline__ void load_raw8(uint32_t lane_addr, uint32_t g, const 
   }
 }
 
-// Splits eight consecutive k values and stores them at 8-k group kc of the stage.
-template <int KIND>
-__device__ __forceinline__ void split_store8(const float (&v)[8], uint32_t lane_dst,
-                                             uint32_t lo_delta, uint32_t kc) {
-  if constexpr (KIND == 0) {
+// Splits eight consecutive k values and stores them at 8-k group kc of the stage: A in tensor
+// memory, B in shared memory.
+template <int KIND, int BN, bool IS_A>
+__device__ __forceinline__ void split_store8(const float (&v)[8], uint32_t dst, uint32_t kc) {
+  if constexpr (IS_A && KIND == 1) {
+    uint32_t h[8], l[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) split_tf32(v[t], h[t], l[t]);
+    ptx::tmem_st_32x32b_x8(dst + 8u * kc, h);
+    ptx::tmem_st_32x32b_x8(dst + A_LO_COLS + 8u * kc, l);
+    return;
+  }
+  constexpr int VECS = (KIND == 0) ? 1 : 2; // vectors of four 32-bit words
+#pragma unroll
+  for (uint32_t g = 0; g < VECS; ++g) {
     uint32_t h[4], l[4];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) split2(v[2 * t], v[2 * t + 1], h[t], l[t]);
-    const uint32_t addr = lane_dst ^ (kc << 4);
-    st_shared_v4(addr, h[0], h[1], h[2], h[3]);
-    st_shared_v4(addr + lo_delta, l[0], l[1], l[2], l[3]);
-  } else {
-#pragma unroll
-    for (uint32_t g = 0; g < 2; ++g) {
-      uint32_t h[4], l[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) split_tf32(v[4 * g + t], h[t], l[t]);
-      const uint32_t addr = lane_dst ^ ((2u * kc + g) << 4);
+    for (int t = 0; t < 4; ++t) {
+      if constexpr (KIND == 0) split2_mixed(v[2 * t], v[2 * t + 1], h[t], l[t]);
+      else split_tf32(v[4 * g + t], h[t], l[t]);
+    }
+    const uint32_t q = VECS * kc + g;
+    if constexpr (IS_A) {
+      ptx::tmem_st_32x32b_x4(dst + 4u * q, h);
+      ptx::tmem_st_32x32b_x4(dst + A_LO_COLS + 4u * q, l);
+    } else {
+      const uint32_t addr = dst ^ (q << 4);
       st_shared_v4(addr, h[0], h[1], h[2], h[3]);
-      st_shared_v4(addr + lo_delta, l[0], l[1], l[2], l[3]);
+      st_shared_v4(addr + StreamCfg<BN>::B_TILE, l[0], l[1], l[2], l[3]);
     }
   }
 }
 
-template <int KIND, int BN, int LAYOUT, int ROWS, int JOBS>
+template <int KIND, int BN, int LAYOUT, int ROWS, int JOBS, bool IS_A>
 __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterState &st) {
   using Cfg = StreamCfg<BN>;
   constexpr uint32_t SLOTS_PER_STAGE = (KIND == 0) ? 2 : 1;
+  constexpr uint32_t STAGE_STEP = 2 / SLOTS_PER_STAGE; // stages from a team's slot to its next
   const uint32_t r = st.row;
   const int lane = static_cast<int>(threadIdx.x & 31);
   uint32_t lane_raw;
@@ -248,52 +278,63 @@ __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterSta
   else if constexpr (LAYOUT == kRawCplxBR) lane_raw = st.raw + r * 8u;
   else if constexpr (LAYOUT == kRawCplxAR) lane_raw = st.raw + (r >> 1) * 8u;
   else lane_raw = st.raw + (r >> 1) * 128u + (((r >> 1) & 7u) << 4);
-  const uint32_t lane_dst = st.dst + r * 128u + ((r & 7u) << 4);
   const bool scaled = st.scale != 1.f;
-  uint32_t rs = 0, rph = 0, s = 0, ph = 0;
+  uint32_t rs = st.team, rph = 0;
+  uint32_t s = (KIND == 0) ? 0u : st.team, ph = 0;
+  const uint32_t kc0 = st.group0 + ((KIND == 0) ? 4u * st.team : 0u);
 #pragma unroll 1
-  for (uint32_t i = 0; i < total_stages; ++i) {
-#pragma unroll 1
-    for (uint32_t half = 0; half < SLOTS_PER_STAGE; ++half) {
-      if (!ptx::mbar_wait_timed(ptx::smem_u32(&st.raw_full[rs]), rph, st.abort_flag, st.status,
-                                ptx::kErrWaitFull, st.timed, &st.wait_raw))
-        return;
-      if (half == 0) {
-        if (!ptx::mbar_wait_timed(ptx::smem_u32(&st.empty[s]), ph ^ 1u, st.abort_flag, st.status,
-                                  ptx::kErrWaitEmpty, st.timed, &st.wait_empty))
-          return;
-      }
-      // two groups at a time: enough independent arithmetic, and no spills at this register count
-      const uint32_t raw_addr = lane_raw + rs * Cfg::RAW_BYTES;
-      const uint32_t dst_addr = lane_dst + s * Cfg::STAGE_BYTES;
-#pragma unroll
-      for (int j = 0; j < JOBS; j += 2) {
-        float v[2][8];
-        load_raw8<LAYOUT, ROWS>(raw_addr, st.group0 + j, st, v[0]);
-        load_raw8<LAYOUT, ROWS>(raw_addr, st.group0 + j + 1, st, v[1]);
-        if (scaled) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            v[0][e] *= st.scale;
-            v[1][e] *= st.scale;
-          }
-        }
-        split_store8<KIND>(v[0], dst_addr, st.lo_delta, 4u * half + st.group0 + j);
-        split_store8<KIND>(v[1], dst_addr, st.lo_delta, 4u * half + st.group0 + j + 1);
-      }
-      // every value of the slot has been read: it may be refilled
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&st.raw_empty[rs]));
-      if (++rs == Cfg::RAW_SLOTS) {
-        rs = 0;
-        rph ^= 1u;
-      }
-    }
-    fence_proxy_async_shared();
+  for (uint32_t i = (KIND == 0) ? 0u : st.team; i < total_stages; i += STAGE_STEP) {
+    if (!ptx::mbar_wait_s(st.bars + Cfg::RAW_FULL + 8u * rs, rph, st.bars + Cfg::ABORT, st.status,
+                          ptx::kErrWaitFull))
+      return;
+    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * s, ph ^ 1u, st.bars + Cfg::ABORT, st.status,
+                          ptx::kErrWaitEmpty))
+      return;
     __syncwarp();
-    if (lane == 0) ptx::mbar_arrive_cluster(st.full_leader + 8u * s);
-    if (++s == Cfg::STAGES) {
-      s = 0;
+    if constexpr (IS_A) ptx::tc_fence_after();
+    const uint32_t raw_addr = lane_raw + rs * Cfg::RAW_BYTES;
+    const uint32_t dst = st.dst + s * (IS_A ? A_STAGE_COLS : static_cast<uint32_t>(Cfg::STAGE_BYTES));
+#pragma unroll
+    for (int j = 0; j < JOBS; ++j) {
+      float v[8];
+      load_raw8<LAYOUT, ROWS>(raw_addr, st.group0 + j, st, v);
+      if (scaled) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] *= st.scale;
+      }
+      split_store8<KIND, BN, IS_A>(v, dst, kc0 + j);
+    }
+    if constexpr (IS_A) {
+      ptx::tmem_st_wait();
+      ptx::tc_fence_before();
+    } else {
+      fence_proxy_async_shared();
+    }
+    // every value of the slot has been read: it may be refilled
+    __syncwarp();
+    if (lane == 0) {
+      ptx::mbar_arrive(st.bars + Cfg::RAW_EMPTY + 8u * rs);
+      ptx::mbar_arrive_cluster(st.bars_leader + Cfg::FULL + 8u * s);
+    }
+    rs += CVT_TEAMS;
+    if (rs >= Cfg::RAW_SLOTS) {
+      rs -= Cfg::RAW_SLOTS;
+      rph ^= 1u;
+    }
+    s += STAGE_STEP;
+    if (s >= Cfg::STAGES) {
+      s -= Cfg::STAGES;
+      ph ^= 1u;
+    }
+  }
+  // the issuer's last commits arrive on this CTA's barriers: it must not be gone by then
+  for (uint32_t i = 0; i < Cfg::STAGES; i += STAGE_STEP) {
+    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * s, ph ^ 1u, st.bars + Cfg::ABORT, st.status,
+                          ptx::kErrWaitEmpty))
+      return;
+    s += STAGE_STEP;
+    if (s >= Cfg::STAGES) {
+      s -= Cfg::STAGES;
       ph ^= 1u;
     }
   }
@@ -307,26 +348,15 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   constexpr int K_STEPS = ROW_BYTES / 32;
   constexpr uint32_t SLOTS_PER_STAGE = (KIND == 0) ? 2 : 1;
   constexpr uint32_t STAGES_PER_UNIT = (KIND == 0) ? 1 : 2;
-  constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, 2 * BM_CTA, BN);
-  constexpr float LO_SCALE_INV = (KIND == 0) ? (1.f / 2048.f) : 1.f;
-  constexpr uint32_t D1_COL = BN;
+  constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, 2 * BM_CTA, BN / 2);
   constexpr int CPT = BN / 2; // accumulator columns per epilogue thread
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t *raw_smem = smem + STAGES * Cfg::STAGE_BYTES;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(raw_smem + RAW_SLOTS * Cfg::RAW_BYTES);
-  uint64_t *raw_full = bars;
-  uint64_t *raw_empty = raw_full + RAW_SLOTS;
-  uint64_t *full_bar = raw_empty + RAW_SLOTS;
-  uint64_t *empty_bar = full_bar + STAGES;
-  uint64_t *d0_full = empty_bar + STAGES;
-  uint64_t *d0_empty = d0_full + 1;
-  uint64_t *d1_full = d0_full + 2;
-  uint64_t *d1_empty = d0_full + 3;
-  uint32_t *tmem_base_ptr = reinterpret_cast<uint32_t *>(d0_full + 4);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_base_ptr + 1);
+  const uint32_t bars = ptx::smem_u32(raw_smem + RAW_SLOTS * Cfg::RAW_BYTES);
+  const uint32_t abort_flag = bars + Cfg::ABORT;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -336,25 +366,25 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   const uint32_t num_clusters = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < RAW_SLOTS; ++s) {
-      ptx::mbar_init(ptx::smem_u32(&raw_full[s]), 1);
-      ptx::mbar_init(ptx::smem_u32(&raw_empty[s]), NUM_CVT_WARPS);
+    for (uint32_t r = 0; r < RAW_SLOTS; ++r) {
+      ptx::mbar_init(bars + Cfg::RAW_FULL + 8u * r, 1);
+      ptx::mbar_init(bars + Cfg::RAW_EMPTY + 8u * r, TEAM_WARPS);
     }
-    for (int s = 0; s < STAGES; ++s) {
-      ptx::mbar_init(ptx::smem_u32(&full_bar[s]), 2 * NUM_CVT_WARPS);
-      ptx::mbar_init(ptx::smem_u32(&empty_bar[s]), 1);
+    for (uint32_t s = 0; s < STAGES; ++s) {
+      ptx::mbar_init(bars + Cfg::FULL + 8u * s, 2 * SLOTS_PER_STAGE * TEAM_WARPS);
+      ptx::mbar_init(bars + Cfg::EMPTY + 8u * s, 1);
     }
-    ptx::mbar_init(ptx::smem_u32(d0_full), 1);
-    ptx::mbar_init(ptx::smem_u32(d0_empty), 2 * NUM_EPI_WARPS);
-    ptx::mbar_init(ptx::smem_u32(d1_full), 1);
-    ptx::mbar_init(ptx::smem_u32(d1_empty), 2 * NUM_EPI_WARPS);
-    *abort_flag = 0;
+    for (uint32_t b = 0; b < Cfg::D_BUFS; ++b) {
+      ptx::mbar_init(bars + Cfg::D_FULL + 8u * b, 1);
+      ptx::mbar_init(bars + Cfg::D_EMPTY + 8u * b, NUM_EPI_WARPS); // half of them, in both CTAs
+    }
+    st_shared_u32(abort_flag, 0u);
     ptx::mbar_init_fence();
     ptx::prefetch_tensormap(&map_a);
     ptx::prefetch_tensormap(&map_b);
   }
   if (warp == 1) {
-    ptx::tmem_alloc_pair(ptx::smem_u32(tmem_base_ptr), Cfg::TMEM_COLS);
+    ptx::tmem_alloc_pair(bars + Cfg::TMEM_PTR, TMEM_COLS);
     ptx::tmem_relinquish_pair();
   }
   ptx::tc_fence_before();
@@ -363,15 +393,14 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   ptx::cluster_arrive();
   ptx::cluster_wait();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *tmem_base_ptr;
+  constexpr uint32_t tmem_base = 0; // all of tensor memory
   // launched behind the previous kernel of the stream (programmatic serialization): from here
   // on global memory is read and written
   ptx::griddep_wait();
   const bool dbg = (p.debug != nullptr);
-  unsigned long long dbg_wait = 0, dbg_wait2 = 0;
 
   if (warp < FIRST_EPI_WARP) {
-    ptx::setmaxnreg_dec<REGS_REST>();
+    ptx::setmaxnreg_dec<Cfg::REGS_REST>();
     if (warp == 0) {
       if (ptx::elect_one()) {
         // ============================================================== TMA producer (both CTAs)
@@ -390,23 +419,27 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
         WorkItem x;
         while (ok && list.next(p.w, x)) {
           const TileCoord tc = tile_coord<BN>(x.tile, p, rank);
-          const int b_row = tc.n0 + static_cast<int>(rank) * Cfg::B_ROWS;
+          const int b_row = tc.n0 + static_cast<int>(rank) * Cfg::HALF_ROWS;
           const int t0 = static_cast<int>(2u * x.u0);
           int ax = a_k ? t0 * SLOT_K : tc.m0;
           int ay = a_k ? (a_cplx ? tc.m0 >> 1 : tc.m0) : t0 * a_dy;
           int bx = b_k ? t0 * SLOT_K : (b_cplx ? 2 * b_row : b_row);
           int by = b_k ? b_row : t0 * b_dy;
+          // the rows for the second half of the tile's columns
+          const int bx2 = b_k ? 0 : (b_cplx ? BN : BN / 2), by2 = b_k ? BN / 2 : 0;
           const int az = (p.flags & kBatchA) ? static_cast<int>(tc.batch) : 0;
           const int bz = (p.flags & kBatchB) ? static_cast<int>(tc.batch) : 0;
           for (uint32_t t = 0; t < 2u * x.un; ++t) {
-            ok = ptx::mbar_wait(ptx::smem_u32(&raw_empty[s]), ph ^ 1u, abort_flag, p.status,
+            ok = ptx::mbar_wait_s(bars + Cfg::RAW_EMPTY + 8u * s, ph ^ 1u, abort_flag, p.status,
                                 ptx::kErrWaitEmpty);
             if (!ok) break;
-            const uint32_t fb = ptx::smem_u32(&raw_full[s]);
+            const uint32_t fb = bars + Cfg::RAW_FULL + 8u * s;
             ptx::mbar_arrive_expect_tx(fb, bytes);
             const uint32_t dst = ptx::smem_u32(raw_smem + s * Cfg::RAW_BYTES);
             ptx::tma_load_3d(dst, &map_a, fb, ax, ay, az);
             ptx::tma_load_3d(dst + Cfg::RAW_A, &map_b, fb, bx, by, bz);
+            ptx::tma_load_3d(dst + Cfg::RAW_A + Cfg::RAW_HALF_B, &map_b, fb, bx + bx2,
+                             by + by2, bz);
             if (a_k) ax += SLOT_K;
             else ay += a_dy;
             if (b_k) bx += SLOT_K;
@@ -421,66 +454,95 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     } else if (warp == 1 && leader) {
       if (ptx::elect_one()) {
         // ============================================================== MMA issuer (leader only)
-        const uint32_t d0 = tmem_base, d1 = tmem_base + D1_COL;
         constexpr uint16_t BOTH = 0x3;
         const uint64_t desc0 = ptx::make_kmajor_desc<ROW_BYTES>(ptx::smem_u32(smem));
-        constexpr uint64_t kStage = Cfg::STAGE_BYTES >> 4;
-        constexpr uint64_t kALo = Cfg::A_TILE >> 4, kBHi = (2 * Cfg::A_TILE) >> 4,
-                           kBLo = (2 * Cfg::A_TILE + Cfg::B_TILE) >> 4;
-        uint32_t s = 0, ph = 0, d0_ph = 1, d1_ph = 1;
+        constexpr uint64_t kStage = Cfg::STAGE_BYTES >> 4, kLo = Cfg::B_TILE >> 4,
+                           kHalf = (Cfg::HALF_ROWS * ROW_BYTES) >> 4;
+        uint32_t s = 0, ph = 0, b = 0, d_ph = 1;
         bool ok = true;
-        const long long dbg_t0 = clock64();
+        const bool separate = (p.flags & kSeparate) != 0;
+        auto wait_timed = [&](uint32_t bar, uint32_t parity, int code, uint32_t &cycles) {
+          const uint32_t t0 = dbg ? static_cast<uint32_t>(clock()) : 0u;
+          const bool r = ptx::mbar_wait_s(bar, parity, abort_flag, p.status, code);
+          if (dbg) cycles += static_cast<uint32_t>(clock()) - t0;
+          return r;
+        };
+        uint32_t dbg_wait = 0, dbg_wait2 = 0;
+        const long long dbg_t0 = dbg ? clock64() : 0;
         WorkList list(p.w, cluster_id, num_clusters);
         WorkItem x;
         while (ok && list.next(p.w, x)) {
           const uint32_t kbn = x.un * STAGES_PER_UNIT;
           for (uint32_t kb = 0; kb < kbn; ++kb) {
-            ok = ptx::mbar_wait_timed(ptx::smem_u32(&full_bar[s]), ph, abort_flag, p.status,
-                                      ptx::kErrWaitFull, dbg, &dbg_wait);
+            ok = wait_timed(bars + Cfg::FULL + 8u * s, ph, ptx::kErrWaitFull, dbg_wait);
             if (!ok) break;
-            ptx::tc_fence_after();
-            const uint64_t a_hi = desc0 + s * kStage;
-            const uint64_t a_lo = a_hi + kALo, b_hi = a_hi + kBHi, b_lo = a_hi + kBLo;
-            auto corrections = [&](uint32_t acc_first) {
-#pragma unroll
-              for (int ks = 0; ks < K_STEPS; ++ks)
-                mma_pair<KIND>(d1, a_lo + 2 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : acc_first);
-#pragma unroll
-              for (int ks = 0; ks < K_STEPS; ++ks)
-                mma_pair<KIND>(d1, a_hi + 2 * ks, b_lo + 2 * ks, IDESC, 1u);
-            };
-            // D0 is drained every stage.  The corrections come before the hi*hi products, so that
-            // the drain of the previous stage's D0 hides behind them; in the first stage of an
-            // item they come after, because they have to wait until the epilogue has given D1 back.
-            if (kb > 0) corrections(1u);
-            ok = ptx::mbar_wait_timed(ptx::smem_u32(d0_empty), d0_ph, abort_flag, p.status,
-                                      ptx::kErrWaitD0Empty, dbg, &dbg_wait2);
-            if (!ok) break;
-            d0_ph ^= 1u;
-            ptx::tc_fence_after();
-#pragma unroll
-            for (int ks = 0; ks < K_STEPS; ++ks)
-              mma_pair<KIND>(d0, a_hi + 2 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : 0u);
-            ptx::tc_commit_pair(ptx::smem_u32(d0_full), BOTH);
-            if (kb == 0) {
-              ok = ptx::mbar_wait_timed(ptx::smem_u32(d1_empty), d1_ph, abort_flag, p.status,
-                                        ptx::kErrWaitD1Empty, dbg, &dbg_wait2);
-              if (!ok) break;
-              d1_ph ^= 1u;
+            const uint32_t a_hi = tmem_base + Cfg::A_COL + s * A_STAGE_COLS, a_lo = a_hi + A_LO_COLS;
+            // the previous sums of these columns must have been drained (at the end of an item:
+            // stored)
+            auto next_buffer = [&]() {
+              ok = ok && wait_timed(bars + Cfg::D_EMPTY + 8u * b, d_ph, ptx::kErrWaitD0Empty, dbg_wait2);
               ptx::tc_fence_after();
-              corrections(0u);
+              return tmem_base + b * CPT;
+            };
+            auto filled = [&]() {
+              ptx::tc_commit_pair(bars + Cfg::D_FULL + 8u * b, BOTH);
+              if (++b == Cfg::D_BUFS) {
+                b = 0;
+                d_ph ^= 1u;
+              }
+            };
+            const uint64_t b_hi0 = desc0 + s * kStage;
+            auto corrections = [&](uint32_t d, uint64_t b_hi) {
+#pragma unroll
+              for (int ks = 0; ks < K_STEPS; ++ks)
+                mma_pair<KIND>(d, a_lo + 8 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : 0u);
+#pragma unroll
+              for (int ks = 0; ks < K_STEPS; ++ks)
+                mma_pair<KIND>(d, a_hi + 8 * ks, b_hi + kLo + 2 * ks, IDESC, 1u);
+            };
+            if (!separate) {
+              // per half of the columns: corrections, then hi*hi on top of them
+#pragma unroll
+              for (uint32_t g = 0; g < 2; ++g) {
+                const uint32_t d = next_buffer();
+                if (!ok) break;
+                const uint64_t b_hi = b_hi0 + g * kHalf;
+                corrections(d, b_hi);
+                if constexpr (KIND == 0) ptx::mma_f16_ts_pair_scaled<11>(d, a_hi, b_hi, IDESC);
+                else mma_pair<KIND>(d, a_hi, b_hi, IDESC, 1u);
+#pragma unroll
+                for (int ks = 1; ks < K_STEPS; ++ks)
+                  mma_pair<KIND>(d, a_hi + 8 * ks, b_hi + 2 * ks, IDESC, 1u);
+                filled();
+              }
+            } else {
+              // the corrections of both halves, then hi*hi of both, in accumulators of their own
+#pragma unroll 1
+              for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t d = next_buffer();
+                if (!ok) break;
+                const uint64_t b_hi = b_hi0 + (q & 1u) * kHalf;
+                if (q < 2) {
+                  corrections(d, b_hi);
+                } else {
+#pragma unroll
+                  for (int ks = 0; ks < K_STEPS; ++ks)
+                    mma_pair<KIND>(d, a_hi + 8 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : 0u);
+                }
+                filled();
+              }
             }
-            ptx::tc_commit_pair(ptx::smem_u32(&empty_bar[s]), BOTH);
+            if (!ok) break;
+            ptx::tc_commit_pair(bars + Cfg::EMPTY + 8u * s, BOTH);
             if (++s == STAGES) {
               s = 0;
               ph ^= 1u;
             }
           }
-          if (ok) ptx::tc_commit_pair(ptx::smem_u32(d1_full), BOTH);
         }
         if (dbg) {
-          atomicAdd(p.debug + 0, dbg_wait);
-          atomicAdd(p.debug + 1, dbg_wait2);
+          atomicAdd(p.debug + 0, static_cast<unsigned long long>(dbg_wait));
+          atomicAdd(p.debug + 1, static_cast<unsigned long long>(dbg_wait2));
           atomicAdd(p.debug + 4, static_cast<unsigned long long>(clock64() - dbg_t0));
           atomicAdd(p.debug + 5, 1ull);
         }
@@ -488,11 +550,12 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     }
   } else if (warp >= FIRST_CVT_WARP) {
     // ================================================================ converters (both CTAs)
-    ptx::setmaxnreg_dec<REGS_CVT>();
-    // warps 0-3: the four 32-row blocks of A; warps 4-7: those of B (BN = 128: two warps to each
-    // of its two blocks, half of a slot's groups each)
+    ptx::setmaxnreg_dec<Cfg::REGS_CVT>();
+    // Two teams of eight warps take the raw slots in turn.  In a team warps 0-3 convert the four
+    // 32-row blocks of A, warps 4-7 those of B (BN = 128: two warps to each of its two blocks, half
+    // of a slot's groups each).
     constexpr int B_JOBS = (BN == 256) ? 4 : 2;
-    const uint32_t cw = static_cast<uint32_t>(warp - FIRST_CVT_WARP);
+    const uint32_t cw = static_cast<uint32_t>(warp - FIRST_CVT_WARP) & 7u;
     const bool for_a = cw < 4;
     // the converters see a plain stream of stages; only its length depends on the work items
     uint32_t total_stages = 0;
@@ -502,136 +565,142 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
       while (list.next(p.w, x)) total_stages += x.un * STAGES_PER_UNIT;
     }
     ConverterState st;
-    st.raw_full = raw_full;
-    st.raw_empty = raw_empty;
-    st.empty = empty_bar;
-    st.full_leader = ptx::map_to_cta(ptx::smem_u32(full_bar), 0);
-    st.raw = ptx::smem_u32(raw_smem) + (for_a ? 0u : Cfg::RAW_A);
-    st.dst = ptx::smem_u32(smem) + (for_a ? 0u : 2u * Cfg::A_TILE);
-    st.lo_delta = for_a ? Cfg::A_TILE : Cfg::B_TILE;
-    st.row = (for_a ? cw : (BN == 256 ? cw - 4u : (cw - 4u) >> 1)) * 32u + lane;
-    st.group0 = (for_a || BN == 256) ? 0u : 2u * (cw & 1u);
+    st.bars = bars;
+    st.bars_leader = ptx::map_to_cta(bars, 0);
+    st.team = static_cast<uint32_t>(warp - FIRST_CVT_WARP) >> 3;
+    st.raw = ptx::smem_u32(raw_smem);
+    if (for_a) {
+      st.row = cw * 32u + lane;
+      st.group0 = 0;
+      st.dst = tmem_base + Cfg::A_COL + ((cw * 32u) << 16);
+    } else {
+      const uint32_t half = (cw - 4u) >> 1; // of the tile's columns
+      st.row = (BN == 256 ? (cw & 1u) * 32u : 0u) + lane;
+      st.group0 = (BN == 256) ? 0u : 2u * (cw & 1u);
+      st.raw += Cfg::RAW_A + half * Cfg::RAW_HALF_B;
+      const uint32_t r = half * Cfg::HALF_ROWS + st.row;
+      st.dst = ptx::smem_u32(smem) + r * 128u + ((r & 7u) << 4);
+    }
     st.scale = 1.f;
     if (p.dyn != nullptr) st.scale = for_a ? p.dyn->scale_a : p.dyn->scale_b;
     st.conj_mask = (p.flags & (for_a ? kConjA : kConjB)) ? 0x80000000u : 0u;
-    st.abort_flag = abort_flag;
     st.status = p.status;
-    st.timed = dbg;
-    st.wait_raw = st.wait_empty = 0;
     if (for_a) {
       switch (p.layout_a) {
       case kRawK:
-        convert_loop<KIND, BN, kRawK, BM_CTA, 4>(total_stages, st);
+        convert_loop<KIND, BN, kRawK, BM_CTA, 4, true>(total_stages, st);
         break;
       case kRawR:
-        convert_loop<KIND, BN, kRawR, BM_CTA, 4>(total_stages, st);
+        convert_loop<KIND, BN, kRawR, BM_CTA, 4, true>(total_stages, st);
         break;
       case kRawCplxAR:
-        convert_loop<KIND, BN, kRawCplxAR, BM_CTA, 4>(total_stages, st);
+        convert_loop<KIND, BN, kRawCplxAR, BM_CTA, 4, true>(total_stages, st);
         break;
       default:
-        convert_loop<KIND, BN, kRawCplxAK, BM_CTA, 4>(total_stages, st);
+        convert_loop<KIND, BN, kRawCplxAK, BM_CTA, 4, true>(total_stages, st);
         break;
       }
     } else {
       switch (p.layout_b) {
       case kRawK:
-        convert_loop<KIND, BN, kRawK, Cfg::B_ROWS, B_JOBS>(total_stages, st);
+        convert_loop<KIND, BN, kRawK, Cfg::HALF_ROWS, B_JOBS, false>(total_stages, st);
         break;
       case kRawR:
-        convert_loop<KIND, BN, kRawR, Cfg::B_ROWS, B_JOBS>(total_stages, st);
+        convert_loop<KIND, BN, kRawR, Cfg::HALF_ROWS, B_JOBS, false>(total_stages, st);
         break;
       default:
-        convert_loop<KIND, BN, kRawCplxBR, Cfg::B_ROWS, B_JOBS>(total_stages, st);
+        convert_loop<KIND, BN, kRawCplxBR, Cfg::HALF_ROWS, B_JOBS, false>(total_stages, st);
         break;
       }
     }
-    if (dbg && cw == 0 && lane == 0) {
-      atomicAdd(p.debug + 2, st.wait_raw);
-      atomicAdd(p.debug + 3, st.wait_empty);
-    }
   } else {
     // ================================================================ drain + epilogue (both CTAs)
-    ptx::setmaxnreg_inc<REGS_EPI>();
-    const uint32_t t_base = tmem_base + ((static_cast<uint32_t>(warp & 3) * 32u) << 16) +
-                            static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2) * CPT;
-    const uint32_t d0_empty_leader = ptx::map_to_cta(ptx::smem_u32(d0_empty), 0);
+    ptx::setmaxnreg_inc<Cfg::REGS_EPI>();
+    // Few registers are left beside the running sums: what the loop over the stages keeps is little,
+    // and the rest is worked out where it is needed.
+    const uint32_t half = static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2); // of the columns
+    const uint32_t t_base = tmem_base + ((static_cast<uint32_t>(warp & 3) * 32u) << 16);
 
-    uint32_t d0_ph = 0, d1_ph = 0;
+    uint32_t b = half, d_ph = 0; // accumulator and parity of the next stage
+    auto give_back = [&]() {
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (ptx::elect_one()) ptx::mbar_arrive_cluster(ptx::map_to_cta(bars + Cfg::D_EMPTY + 8u * b, 0));
+      __syncwarp();
+      b += 2u;
+      if (b >= Cfg::D_BUFS) {
+        b -= Cfg::D_BUFS;
+        d_ph ^= 1u;
+      }
+    };
+    // beta != 0: pull this warp's part of a C tile into L2 before the epilogue reads it
+    auto prefetch_c = [&](uint32_t tile) {
+      const TileCoord tc = tile_coord<BN>(opaque(tile), p, rank);
+      const uint32_t row = static_cast<uint32_t>(tc.m0) + static_cast<uint32_t>(warp & 3) * 32u;
+      const float *cp = p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row;
+#pragma unroll 1
+      for (int q = 0; q < CPT / 32; ++q) {
+        const uint32_t col =
+            static_cast<uint32_t>(tc.n0) +
+            static_cast<uint32_t>(((warp - FIRST_EPI_WARP) >> 2) * CPT + q * 32 + lane);
+        if (col < p.n && row < p.m) ptx::prefetch_l2(cp + static_cast<uint64_t>(col) * p.ldc);
+      }
+    };
     bool ok = true;
     WorkList list(p.w, cluster_id, num_clusters);
     WorkItem x;
     while (ok && list.next(p.w, x)) {
-      const uint32_t drains = x.un * STAGES_PER_UNIT;
-      const uint32_t prefetch_at = (p.beta_r == 0.f && p.beta_i == 0.f) ? drains
-                                   : (drains > C_PREFETCH_LEAD)         ? drains - C_PREFETCH_LEAD
-                                                                        : 0u;
-      float acc[CPT];
+      const bool separate = (p.flags & kSeparate) != 0;
+      uint32_t left = x.un * (separate ? 2u * STAGES_PER_UNIT : STAGES_PER_UNIT); // stages to drain
+      if (left < C_PREFETCH_LEAD && (p.beta_r != 0.f || p.beta_i != 0.f)) prefetch_c(x.tile);
+      unsigned long long acc[CPT / 2];
 #pragma unroll
-      for (int i = 0; i < CPT; ++i) acc[i] = 0.f;
+      for (int i = 0; i < CPT / 2; ++i) acc[i] = 0ull;
 
 #pragma unroll 1
-      for (uint32_t c = 0; c < drains; ++c) {
-        if (c == prefetch_at) {
-          // beta != 0: pull this warp's part of the C tile into L2 before the epilogue reads it
-          const TileCoord tc = tile_coord<BN>(opaque(x.tile), p, rank);
-          const uint32_t row = static_cast<uint32_t>(tc.m0) + static_cast<uint32_t>(warp & 3) * 32u;
-          const float *cp = p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row;
-#pragma unroll 1
-          for (int q = 0; q < CPT / 32; ++q) {
-            const uint32_t col =
-                static_cast<uint32_t>(tc.n0) +
-                static_cast<uint32_t>(((warp - FIRST_EPI_WARP) >> 2) * CPT + q * 32 + lane);
-            if (col < p.n && row < p.m) ptx::prefetch_l2(cp + static_cast<uint64_t>(col) * p.ldc);
-          }
-        }
-        ok = ptx::mbar_wait(ptx::smem_u32(d0_full), d0_ph, abort_flag, p.status, ptx::kErrWaitD0Full);
+      while (true) {
+        if (left == C_PREFETCH_LEAD && (p.beta_r != 0.f || p.beta_i != 0.f)) prefetch_c(x.tile);
+        ok = ptx::mbar_wait_s(bars + Cfg::D_FULL + 8u * b, d_ph, abort_flag, p.status,
+                              ptx::kErrWaitD0Full);
         if (!ok) break;
-        d0_ph ^= 1u;
-        ptx::tc_fence_after();
-        drain_sums<CPT>(t_base, acc);
-        ptx::tc_fence_before();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive_cluster(d0_empty_leader);
+        ptx::tc_fence_after();
+        if (--left == 0) break; // the last ones are added below
+        drain_pairs<CPT>(t_base + b * CPT, acc);
+        // (corrections in an accumulator of their own come first, and nothing else is in acc then
+        // but, in TF32, finished sums, whose corrections are not scaled)
+        if (KIND == 0 && separate) {
+#pragma unroll
+          for (int i = 0; i < CPT / 2; ++i) scale_pair(acc[i], 1.f / 2048.f);
+        }
+        give_back();
       }
       if (!ok) break;
-
-      ok = ptx::mbar_wait(ptx::smem_u32(d1_full), d1_ph, abort_flag, p.status, ptx::kErrWaitD1Full);
-      if (!ok) break;
-      d1_ph ^= 1u;
-      ptx::tc_fence_after();
-      const uint32_t t_sums = t_base + D1_COL;
+      const uint32_t t_sums = t_base + b * CPT;
       if (BN == 128 && (p.flags & kDirectStores)) {
         // Many short tiles per cluster, C not read: stores straight from the registers.  That is
         // long code, but it stays in the instruction cache from tile to tile, and D1 goes back to
         // the issuer before the stores instead of after them.
+        drain_pairs<CPT>(t_sums, acc);
+        give_back();
+        float sums[CPT];
 #pragma unroll
-        for (int c = 0; c < CPT; c += 16) {
-          uint32_t v[16];
-          ptx::tmem_ld_32x32b_x16(t_sums + c, v);
-          ptx::tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i)
-            acc[c + i] = fmaf(__uint_as_float(v[i]), LO_SCALE_INV, acc[c + i]);
-        }
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0)
-          ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(d1_empty), 0));
+        for (int i = 0; i < CPT / 2; ++i)
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(sums[2 * i]), "=f"(sums[2 * i + 1]) : "l"(acc[i]));
         const TileCoord tc = tile_coord<BN>(opaque(x.tile), p, rank);
         const uint32_t row = static_cast<uint32_t>(tc.m0) + static_cast<uint32_t>(warp & 3) * 32u +
                              static_cast<uint32_t>(lane);
         const uint32_t col0 = static_cast<uint32_t>(tc.n0) +
                               static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2) * CPT;
         const float unscale = (p.dyn != nullptr) ? p.dyn->unscale_c : 1.f;
-        store_registers<CPT>(acc, p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row, p.ldc,
+        store_registers<CPT>(sums, p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row, p.ldc,
                              col0, p.n, row < p.m, p.alpha_r * unscale, p.alpha_i * unscale,
                              (p.flags & kIsComplex) != 0);
         continue;
       }
       // the finished sums stay in the D1 columns; from here on they are read from there, and what
       // the epilogue needs to know of the tile is worked out only now (epilogue.cuh)
-      add_corrections_in_tmem<CPT>(t_sums, acc, LO_SCALE_INV);
+      finish_pairs_in_tmem<CPT>(t_sums, acc);
       const bool part = x.un != p.w.units; // this item is a piece of a tile
       const TileCoord tc = tile_coord<BN>(opaque(x.tile), p, rank);
       const uint32_t quarter = static_cast<uint32_t>(warp & 3);
@@ -639,13 +708,6 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
       const uint32_t row =
           static_cast<uint32_t>(tc.m0) + quarter * 32u + static_cast<uint32_t>(lane);
       float *cbase = p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row;
-      const uint32_t d1_empty_leader = ptx::map_to_cta(ptx::smem_u32(d1_empty), 0);
-      auto release_d1 = [&]() {
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive_cluster(d1_empty_leader);
-      };
-
       if (part) {
         // park the partial sums for the kernel that adds the pieces
         constexpr uint32_t HALF = BN * BM_CTA; // floats of one CTA's half of a tile
@@ -661,7 +723,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
           for (int i = 0; i < kEpiGroup; ++i)
             __stcg(mine + (c + i) * BM_CTA, __uint_as_float(v[i]));
         }
-        release_d1();
+        give_back();
         continue;
       }
 
@@ -669,7 +731,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
       store_tile<CPT>(t_sums, cbase, p.ldc, static_cast<uint32_t>(tc.n0) + col_base, p.n, row < p.m,
                       p.alpha_r * unscale, p.alpha_i * unscale, p.beta_r, p.beta_i,
                       (p.flags & kIsComplex) != 0);
-      release_d1();
+      give_back();
     }
   }
 
@@ -679,7 +741,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   __syncthreads();
   ptx::cluster_arrive();
   ptx::cluster_wait();
-  if (*abort_flag) {
+  if (*reinterpret_cast<volatile int *>(raw_smem + RAW_SLOTS * Cfg::RAW_BYTES + Cfg::ABORT)) {
     // a wait gave up: let copies and tensor-core work still in flight land
     const uint64_t t0 = ptx::globaltimer_ns();
     while (ptx::globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
@@ -687,7 +749,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   }
   if (warp == 1) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
+    ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
 }
 
@@ -787,7 +849,7 @@ template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, 
   if (se != cudaSuccess) return se;
   CUtensorMap map_a, map_b;
   if (!raw_map(&map_a, a.a, a.layout_a, a.m, a.k, a.batch, BM_CTA) ||
-      !raw_map(&map_b, a.b, a.layout_b, a.n, a.k, a.batch, BN / 2))
+      !raw_map(&map_b, a.b, a.layout_b, a.n, a.k, a.batch, StreamCfg<BN>::HALF_ROWS))
     return cudaErrorNotSupported; // an extent TMA cannot address: the caller takes another path
   StreamParams p;
   p.c = a.c;
@@ -811,6 +873,7 @@ template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, 
                                  (a.conj_b ? kConjB : 0) |
                                  (a.batch > 1 && a.a.stride != 0 ? kBatchA : 0) |
                                  (a.batch > 1 && a.b.stride != 0 ? kBatchB : 0));
+  if (a.k <= 64) p.flags |= kSeparate;
   const StreamPlan &plan = a.plan;
   if (plan.tile_n != BN || plan.total_tiles != p.tiles_m * p.tiles_n * a.batch ||
       plan.units != (a.k + 63) / 64)
