@@ -301,8 +301,10 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
   if (batch > 0x3fffffffull || n > 0x3fffffffull) return false; // (TMA coordinates are 32-bit)
   // The width: forced, or 128 for narrow products, or the one estimated to be faster (batches of small
   // matrices, which the estimates are not fitted to: 256).
+  // (Near equal estimates the pre-split path is as fast: 2048^3, estimated 51.9 and 52.0, takes 63.6 us
+  // here and 63.1 there, beta = 0.5.)
   StreamPlan plan = {};
-  double best = presplit_us;
+  double best = 0.97 * presplit_us;
   for (const int tile_n : {256, 128}) {
     if ((t.stream == 128 || t.stream == 256) ? tile_n != t.stream : (n <= 128 && tile_n == 256)) continue;
     int clusters = 0;
