@@ -19,6 +19,16 @@
 // While the tensor core runs the two correction products of a stage the
 // epilogue warps drain D0 of the same stage, so D0 needs no double buffering
 // and the two accumulators fill the 512 TMEM columns at BN = 256.
+//
+// The narrowest tiles (BN = 64) are bound by the shared-memory port: per stage of 128 x 64 TMA writes
+// 48 KiB and twelve products read 6 KiB of operands each, 960 cycles at 128 bytes a cycle for 384 of
+// tensor-core work; 940 were measured at 1024^3.  The B_hi and B_lo tiles of a stage lie next to each
+// other, so Ahi * [Bhi; Blo] is one product of width 128 that reads Ahi once: 832 cycles.  It leaves hi*hi
+// and hi*lo side by side, lo*hi is added to the second half, both are drained every stage into sums of
+// their own, and two such accumulators alternate.  us per call, before / now: 1024^3 15.4 / 14.5
+// (TF32TCEC 24.7 / 22.9), 768^3 12.3 / 11.7 (18.3 / 16.8), 896 x 1152 x 1400 19.4 / 17.7.  With 128 columns
+// the port has 1152 instead of 1280 cycles to do, but twice the sums to drain and none to spare: 1536^3
+// 24.8 / 25.9, so they stay as they were.
 #include "epilogue.cuh"
 #include "gemm_common.cuh"
 #include "ptx.cuh"
@@ -43,6 +53,8 @@ template <int BN, bool EC> struct TileCfg {
   static constexpr int STAGES_RAW = (SMEM_LIMIT - 2048) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
+  static constexpr bool MERGED = EC && BN == 64; // hi*hi and hi*lo from one product, see above
+  static constexpr uint32_t D_COLS = 2 * BN;      // MERGED: columns of an accumulator
   static_assert(STAGES >= 2, "need at least two stages");
 };
 
@@ -60,7 +72,7 @@ template <int KIND> __device__ __forceinline__ void mma_ss(uint32_t d, uint64_t 
 // Where a CTA's stages, barriers and flags are in shared memory.
 template <int BN, bool EC> struct SharedLayout {
   uint8_t *smem;
-  uint64_t *full_bar, *empty_bar, *d0_full, *d0_empty, *d1_full;
+  uint64_t *full_bar, *empty_bar, *d0_full, *d0_empty, *d1_full; // MERGED: d0_full[2], d0_empty[2]
   uint32_t *tmem_base_ptr;
   volatile int *abort_flag;
   __device__ __forceinline__ SharedLayout() {
@@ -73,9 +85,9 @@ template <int BN, bool EC> struct SharedLayout {
     full_bar = bars;
     empty_bar = bars + STAGES;
     d0_full = bars + 2 * STAGES;
-    d0_empty = bars + 2 * STAGES + 1;
-    d1_full = bars + 2 * STAGES + 2;
-    tmem_base_ptr = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 3);
+    d0_empty = bars + 2 * STAGES + 2;
+    d1_full = bars + 2 * STAGES + 4;
+    tmem_base_ptr = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 5);
     abort_flag = reinterpret_cast<volatile int *>(tmem_base_ptr + 1);
   }
 };
@@ -91,8 +103,10 @@ __device__ __forceinline__ uint32_t set_up(const CUtensorMap &map_a, const CUten
       ptx::mbar_init(ptx::smem_u32(&sm.full_bar[s]), 1);
       ptx::mbar_init(ptx::smem_u32(&sm.empty_bar[s]), 1);
     }
-    ptx::mbar_init(ptx::smem_u32(sm.d0_full), 1);
-    ptx::mbar_init(ptx::smem_u32(sm.d0_empty), NUM_EPI_WARPS);
+    for (int b = 0; b < 2; ++b) {
+      ptx::mbar_init(ptx::smem_u32(&sm.d0_full[b]), 1);
+      ptx::mbar_init(ptx::smem_u32(&sm.d0_empty[b]), NUM_EPI_WARPS);
+    }
     ptx::mbar_init(ptx::smem_u32(sm.d1_full), 1);
     *sm.abort_flag = 0;
     ptx::mbar_init_fence();
@@ -201,6 +215,7 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
     if (ptx::elect_one()) {
       const uint32_t d0 = tmem_base;
       const uint32_t d1 = tmem_base + D1_COL;
+      const uint64_t desc0 = ptx::make_kmajor_desc<ROW_BYTES>(ptx::smem_u32(smem));
       bool ok = true;
       const long long dbg_t0 = clock64();
       for (uint32_t kb = 0; kb < k_blocks && ok; ++kb) {
@@ -209,6 +224,26 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
         ok = ptx::mbar_wait_timed(ptx::smem_u32(&full_bar[s]), ph, abort_flag, p.status,
                                   ptx::kErrWaitFull, dbg, &dbg_wait);
         if (!ok) break;
+        if constexpr (Cfg::MERGED) {
+          constexpr uint32_t IDESC2 = ptx::make_idesc(KIND == 0 ? 0 : 2, BM, 2 * BN);
+          const uint32_t b = kb & 1u;
+          ok = ptx::mbar_wait_timed(ptx::smem_u32(&d0_empty[b]), ((kb >> 1) & 1u) ^ 1u, abort_flag,
+                                    p.status, ptx::kErrWaitD0Empty, dbg, &dbg_wait2);
+          if (!ok) break;
+          ptx::tc_fence_after();
+          const uint64_t a_hi = desc0 + s * static_cast<uint64_t>(Cfg::STAGE_BYTES >> 4);
+          const uint64_t a_lo = a_hi + (Cfg::A_TILE >> 4), b_hi = a_hi + ((2 * Cfg::A_TILE) >> 4);
+          const uint32_t d = tmem_base + b * Cfg::D_COLS;
+#pragma unroll
+          for (int ks = 0; ks < K_STEPS; ++ks)
+            mma_ss<KIND>(d, a_hi + 2 * ks, b_hi + 2 * ks, IDESC2, ks > 0 ? 1u : 0u);
+#pragma unroll
+          for (int ks = 0; ks < K_STEPS; ++ks)
+            mma_ss<KIND>(d + BN, a_lo + 2 * ks, b_hi + 2 * ks, IDESC, 1u);
+          ptx::tc_commit(ptx::smem_u32(&empty_bar[s]));
+          ptx::tc_commit(ptx::smem_u32(&d0_full[b]));
+          continue;
+        }
         // D0 of the previous stage must have been drained before it is overwritten.
         ok = ptx::mbar_wait_timed(ptx::smem_u32(d0_empty), (kb & 1u) ^ 1u, abort_flag, p.status,
                                   ptx::kErrWaitD0Empty, dbg, &dbg_wait2);
@@ -239,7 +274,7 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
         }
         ptx::tc_commit(ptx::smem_u32(&empty_bar[s]));
       }
-      if (ok) ptx::tc_commit(ptx::smem_u32(d1_full));
+      if (ok && !Cfg::MERGED) ptx::tc_commit(ptx::smem_u32(d1_full));
       if (dbg) {
         atomicAdd(p.debug + 0, dbg_wait);
         atomicAdd(p.debug + 1, dbg_wait2);
@@ -262,26 +297,52 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
     for (int i = 0; i < CPT; ++i) acc[i] = 0.f;
 
     bool ok = true;
-    for (uint32_t kb = 0; kb < k_blocks; ++kb) {
-      ok = ptx::mbar_wait_timed(ptx::smem_u32(d0_full), kb & 1u, abort_flag, p.status,
-                                ptx::kErrWaitD0Full, dbg, &dbg_wait);
-      if (!ok) break;
-      ptx::tc_fence_after();
+    // (MERGED: the sums of the corrections; the finished sums end up in the D1 columns either way)
+    float cor[Cfg::MERGED ? CPT : 1];
+    if constexpr (Cfg::MERGED) {
 #pragma unroll
-      for (int pc = 0; pc < CPT / 32; ++pc) {
-        uint32_t v[32];
-        ptx::tmem_ld_32x32b_x32(tmem_base + lane_addr + col_base + pc * 32, v);
-        ptx::tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[pc * 32 + i] += __uint_as_float(v[i]);
+      for (int i = 0; i < CPT; ++i) cor[i] = 0.f;
+      for (uint32_t kb = 0; kb < k_blocks; ++kb) {
+        const uint32_t b = kb & 1u;
+        ok = ptx::mbar_wait_timed(ptx::smem_u32(&d0_full[b]), (kb >> 1) & 1u, abort_flag, p.status,
+                                  ptx::kErrWaitD0Full, dbg, &dbg_wait);
+        if (!ok) break;
+        ptx::tc_fence_after();
+        const uint32_t t = tmem_base + lane_addr + b * Cfg::D_COLS + col_base;
+        drain_sums<CPT>(t, acc);
+        drain_sums<CPT>(t + BN, cor);
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&d0_empty[b]));
       }
-      ptx::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(d0_empty));
+    } else {
+      for (uint32_t kb = 0; kb < k_blocks; ++kb) {
+        ok = ptx::mbar_wait_timed(ptx::smem_u32(d0_full), kb & 1u, abort_flag, p.status,
+                                  ptx::kErrWaitD0Full, dbg, &dbg_wait);
+        if (!ok) break;
+        ptx::tc_fence_after();
+#pragma unroll
+        for (int pc = 0; pc < CPT / 32; ++pc) {
+          uint32_t v[32];
+          ptx::tmem_ld_32x32b_x32(tmem_base + lane_addr + col_base + pc * 32, v);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) acc[pc * 32 + i] += __uint_as_float(v[i]);
+        }
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(d0_empty));
+      }
     }
 
     if (dbg && warp == 4 && lane == 0) atomicAdd(p.debug + 3, dbg_wait);
-    if (ok && EC) {
+    if (ok && Cfg::MERGED) {
+      if constexpr (Cfg::MERGED) {
+#pragma unroll
+        for (int i = 0; i < CPT; ++i) acc[i] = fmaf(cor[i], p.lo_scale_inv, acc[i]);
+      }
+      sums_to_tmem<CPT>(tmem_base + D1_COL + lane_addr + col_base, acc);
+    } else if (ok && EC) {
       ok = ptx::mbar_wait(ptx::smem_u32(d1_full), 0u, abort_flag, p.status, ptx::kErrWaitD1Full);
       if (ok) {
         ptx::tc_fence_after();
