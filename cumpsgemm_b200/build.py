@@ -35,6 +35,7 @@ CUDA_SOURCES = [
     "tcec_gemm_pair.cu",
     "tcec_gemm_fused.cu",
     "tcec_gemm_stream.cu",
+    "tcec_gemm_small.cu",
     "piece_fixup.cu",
     "gemm_api.cu",
     "ext_api.cu",

@@ -487,6 +487,69 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
                      h->tuning.untouched() &&
                      ((m_exp + 127) / 128) * ((n + 63) / 64) * batch <= h->num_sms;
 
+  // ---- one launch for what is mostly fixed costs.  A chunk of K (64 values in FP16TCEC, 32 in TF32TCEC)
+  // takes this kernel 0.9 to 1.2 us and the pre-split GEMM 0.5, whose second launch costs 2.4 us of
+  // host time.  Measured in loops, pre-split / one launch, us: 64^3 8.9 / 6.2, 128^3 8.8 / 6.5, 512 x 512 x
+  // 128 8.8 / 6.0 (TF32TCEC, four chunks: 8.5 / 6.6), complex 128^3 (four) 9.3 / 6.7, 256^3 (four) 8.9 /
+  // 7.8, 251 x 864 x 300 (five) 8.8 / 10; 1024 x 1024 x 128, 256 tiles, 8.7 / 9.2.  With statistics in
+  // front the GPU's time counts and not the host's: 251 x 864 x 300 FP16TCEC_SCALING 14.8 / 16.4.
+  const std::uint64_t small_chunks = (k_exp + (want_tf32 ? 31 : 63)) / (want_tf32 ? 32 : 64);
+  const std::uint64_t small_tiles = ((m_exp + 127) / 128) * ((n + 31) / 32) * batch;
+  if (small && small_tiles <= h->num_sms && small_chunks <= (dyn == nullptr ? 4u : 2u) &&
+      lda * fpe <= 0xffffffffull && ldb * fpe <= 0xffffffffull && ldc * fpe <= 0xffffffffull) {
+    SmallGemmArgs sa;
+    sa.kind = (want_fp16 && want_tf32) ? StreamKind::device
+              : want_fp16              ? StreamKind::fp16
+                                       : StreamKind::tf32;
+    sa.pointers = ptr_arrays;
+    sa.a = ptr_arrays ? static_cast<const void *>(a_array) : a;
+    sa.b = ptr_arrays ? static_cast<const void *>(b_array) : b;
+    sa.c = ptr_arrays ? const_cast<void *>(static_cast<const void *>(c_array)) : c;
+    sa.lda = static_cast<std::uint32_t>(lda * fpe);
+    sa.ldb = static_cast<std::uint32_t>(ldb * fpe);
+    sa.ldc = static_cast<std::uint32_t>(ldc * fpe);
+    sa.stride_a = stridea * fpe;
+    sa.stride_b = strideb * fpe;
+    sa.stride_c = stridec * fpe;
+    sa.m = static_cast<std::uint32_t>(m_exp);
+    sa.n = static_cast<std::uint32_t>(n);
+    sa.k = static_cast<std::uint32_t>(k_exp);
+    sa.batch = static_cast<std::uint32_t>(batch);
+    sa.a_k_contig = !a_n;
+    sa.b_k_contig = b_n;
+    sa.is_complex = is_complex;
+    sa.conj_a = is_complex && op_A == CUBLAS_OP_C;
+    sa.conj_b = is_complex && op_B == CUBLAS_OP_C;
+    sa.alpha_r = Scalar<T>::re(alpha);
+    sa.alpha_i = Scalar<T>::im(alpha);
+    sa.beta_r = Scalar<T>::re(beta);
+    sa.beta_i = Scalar<T>::im(beta);
+    sa.dyn = dyn;
+    sa.dev_status = h->dev_status;
+    if (used_kernel_module_id != nullptr) *used_kernel_module_id = tile_class(64);
+    const bool prof = h->exp_stats.profiling_enabled;
+    if (prof) h->exp_stats.profiler.start("gemm_kernel", h->cuda_stream);
+    cuMpSGEMM_handle::TimingTriple tt{};
+    if (h->kernel_timing) {
+      for (auto &e : tt.e) cudaEventCreate(&e);
+      cudaEventRecord(tt.e[0], h->cuda_stream);
+      cudaEventRecord(tt.e[1], h->cuda_stream);
+    }
+    const cudaError_t serr = launch_tcec_gemm_small(sa, h->cuda_stream);
+    if (h->kernel_timing) {
+      cudaEventRecord(tt.e[2], h->cuda_stream);
+      h->timing_events.push_back(tt);
+    }
+    if (prof) h->exp_stats.profiler.stop("gemm_kernel", h->cuda_stream);
+    mark_stream_work(h);
+    if (serr != cudaSuccess) {
+      log_error(std::string("kernel launch failed: ") + cudaGetErrorString(serr));
+      return CUBLAS_STATUS_EXECUTION_FAILED;
+    }
+    h->last_route = CUMPSGEMM_ROUTE_ON_THE_FLY;
+    return CUBLAS_STATUS_SUCCESS;
+  }
+
   // ---- the pre-split path's tile or K slices, and what it would take
   const bool auto_kind = want_fp16 && want_tf32;
   const StreamKind stream_kind = auto_kind ? StreamKind::device

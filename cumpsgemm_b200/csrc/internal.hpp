@@ -364,6 +364,23 @@ struct StreamOperand {
   const float *src;
   std::uint64_t ld, stride; // multiples of 4 (TMA: 16 bytes); stride 0: one matrix for all batches
 };
+// One-launch GEMM for small products (tcec_gemm_small.cu): no workspace, error-corrected kinds only,
+// any operand.  Sizes are those of the real (expanded) problem, leading dimensions and strides in floats.
+struct SmallGemmArgs {
+  StreamKind kind;
+  const void *a, *b; // or, with `pointers`, device arrays of one pointer per batch entry
+  void *c;
+  bool pointers;
+  std::uint32_t lda, ldb, ldc;
+  std::uint64_t stride_a, stride_b, stride_c;
+  std::uint32_t m, n, k, batch;
+  bool a_k_contig, b_k_contig; // as stored: op(A) row by row, op(B) column by column
+  bool is_complex, conj_a, conj_b;
+  float alpha_r, alpha_i, beta_r, beta_i;
+  const DynParams *dyn; // nullable
+  int *dev_status;
+};
+cudaError_t launch_tcec_gemm_small(const SmallGemmArgs &a, cudaStream_t stream);
 // How the tiles of a launch are dealt to the CTA pairs; see tcec_gemm_stream.cu.
 struct StreamPlan {
   int tile_n;                    // 256 or 128 columns per pair tile (256 rows)
