@@ -133,6 +133,10 @@ struct PathModel {
     return 2.0 + 0.15 * split + 1.32 * std::ceil(stages / slices) +
            0.69e-6 * 4 * static_cast<double>(m) * n * batch * slices;
   }
+  // tcec_gemm_stream.cu on single CTAs, 128 x 128 tiles (16 x 128 x 128 x 4096 65 us, estimated 67)
+  double stream_solo(const StreamPlan &pl) const {
+    return 9.0 + waves(pl.total_tiles, sms) * units * (stages > units ? 1.62 : 0.90);
+  }
   // tcec_gemm_stream.cu.  (Fitted to 35 problems of 1-110 tiles and k = 96-32768 in each kind, mean
   // error 5-9 %.  Examples, us, 256 / 128 columns: 2048 x 1024 x 2048 FP16TCEC 48 / 41, complex
   // 1280 x 960 x 1500 61 / 66, 256 x 256 x 8192 23 / 18; TF32TCEC 4096 x 1024 x 2048 86 / 115.)
@@ -174,7 +178,11 @@ TileChoice pick_tile(const Tuning &tuning, unsigned num_sms, std::uint64_t m_exp
     const WorkPlan w = plan_pair(tuning, tf32, can_cut, static_cast<std::uint32_t>(pair_tiles),
                                  static_cast<std::uint32_t>(model.units), num_sms / 2);
     const double t = model.pair(w);
-    if (tuning.pair == 1 || pair_tiles > num_sms / 2 || t < best.us) best = {256, true, t};
+    // Pieces laid end to end leave every pair two to park.  That is 0.4 us per left-over tile more (complex
+    // 1280 x 960 x 1500: 71 us, 56 without it); no other tile is better there, but streaming is.
+    const double parked =
+        w.piece_clusters > 0 && w.slice_units == 0 ? 0.4 * (w.total_tiles - w.whole_tiles) : 0.0;
+    if (tuning.pair == 1 || pair_tiles > num_sms / 2 || t < best.us) best = {256, true, t + parked};
   }
   return best;
 }
@@ -301,10 +309,32 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
   if (batch > 0x3fffffffull || n > 0x3fffffffull) return false; // (TMA coordinates are 32-bit)
   // The width: forced, or 128 for narrow products, or the one estimated to be faster (batches of small
   // matrices, which the estimates are not fitted to: 256).
-  // (Near equal estimates the pre-split path is as fast: 2048^3, estimated 51.9 and 52.0, takes 63.6 us
-  // here and 63.1 there, beta = 0.5.)
+  // (At equal estimates the pre-split path is as fast: 2048^3, estimated 51.9 here and 52.2 there, takes
+  // 62.2 and 62.3 us, beta = 0.5.)
   StreamPlan plan = {};
-  double best = 0.97 * presplit_us;
+  double best = 0.99 * presplit_us;
+  const auto estimate = [&](const StreamPlan &pl) {
+    // (the kind of an AUTO call is not known here: the mean of both)
+    double us = 0.0;
+    for (const bool tf32 : {false, true}) {
+      if (kind == (tf32 ? StreamKind::fp16 : StreamKind::tf32)) continue;
+      const PathModel model(h->num_sms, m_exp, n, k_exp, batch, tf32);
+      us += pl.tile_m == 128 ? model.stream_solo(pl) : model.stream(pl);
+    }
+    return kind == StreamKind::device ? 0.5 * us : us;
+  };
+  // Batches of matrices with at most 128 rows would leave one CTA of every pair idle: single CTAs, but
+  // for a few tiles with a long K loop, which pairs can cut.  Measured (us per call; the kernel that took
+  // the call before / pairs / single CTAs), FP16TCEC: 2048 x 128^3 76.5 / 108 / 66.8, 2048 x 128 x 64 x 64
+  // 47.1 / 74 / 45.9, 512 x 128 x 512 x 128 72 / 92 / 58, 2048 x complex 64 x 128 x 128 184 / 162 / 99,
+  // 512 x 128 x 256 x 256 72 / 71 / 51, 1000 x 32^3 37 / 37 / 22, 64 x 128^3 10.5 / 10.7 / 8.5; 16 x 128 x
+  // 128 x 4096 31 / 31 / 65, 8 x 48 x 104 x 960 25 / 14 / 18.  TF32TCEC, pairs / single CTAs: 2048 x 128^3
+  // 146 / 80, 512 x 128 x 128 x 512 120 / 74, 400 x 100 x 300 x 200 150 / 91.
+  const bool few_rows = t.stream <= 1 && batch >= 8 && m_exp <= 128 && n <= 1024;
+  if (few_rows) {
+    plan = plan_stream_solo(m_exp, n, k_exp, batch);
+    if (plan.total_tiles != 0) best = estimate(plan);
+  }
   for (const int tile_n : {256, 128}) {
     if ((t.stream == 128 || t.stream == 256) ? tile_n != t.stream : (n <= 128 && tile_n == 256)) continue;
     int clusters = 0;
@@ -315,21 +345,17 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
     const StreamPlan pl = plan_stream(t, tile_n, m_exp, n, k_exp, batch,
                                       static_cast<std::uint32_t>(clusters));
     if (pl.total_tiles == 0) continue;
-    if (t.stream != -1 || small_matrix_batch(pl, m_exp, n, batch, clusters)) {
+    if (!few_rows && (t.stream != -1 || small_matrix_batch(pl, m_exp, n, batch, clusters))) {
       plan = pl;
       break;
     }
     // beyond one and a half waves of wide tiles the operands are reused by too many tiles to convert
     // them again for each (4096 x 4096 x 1024: 102 us against 91), and the model is not fitted to it
     if (2ull * pl.total_tiles > 3ull * (256 / tile_n) * static_cast<std::uint64_t>(clusters)) continue;
-    // (the kind of an AUTO call is not known here: the mean of both)
-    double us = 0.0;
-    if (kind != StreamKind::tf32)
-      us += PathModel(h->num_sms, m_exp, n, k_exp, batch, false).stream(pl);
-    if (kind != StreamKind::fp16)
-      us += PathModel(h->num_sms, m_exp, n, k_exp, batch, true).stream(pl);
-    if (kind == StreamKind::device) us *= 0.5;
-    if (us < best) {
+    const double us = estimate(pl);
+    // (128 columns instead of 256 only for a clear gain: 96 x 342 x 23008, estimated 27.4 and 27.6, takes
+    // 35 and 30 us)
+    if (us < best * (plan.tile_n == 256 ? 0.93 : 1.0)) {
       best = us;
       plan = pl;
     }
@@ -561,17 +587,11 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
 
   // ---- one launch on CTA pairs, operands split between TMA and the tensor core
   StreamGemmArgs ga;
-  // (Batches of matrices with at most 128 rows would leave one CTA of every pair idle, and go to the
-  // kernel below where it can take them.  Measured, on the fly / streaming, us: 2048 x 128^3 82 / 110,
-  // 2048 x 128 x 64 x 64 47 / 75, 512 x 128 x 512 x 128 86 / 100, 2048 x complex 64 x 128 x 128
-  // 132 / 166; but 512 x 128 x 256 x 256 78 / 73, 512 x 128 x 128 x 512 95 / 81, 512 x 64 x 256 x 256
-  // 79 / 65, 64 x 64 x 512 x 1024 70 / 56, 64 x 128 x 128 x 128 12.6 / 11.0: the rule is right for
-  // large batches of short products and gives up to a quarter away elsewhere.)
   FusedGemmArgs fa;
   const bool fused = !small && mode == CUMPSGEMM_FP16TCEC && !ptr_arrays &&
                      fused_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch,
                                    &fa);
-  if (!small && ec && !ptr_arrays && !(fused && batch >= 8 && m_exp <= 128 && h->tuning.stream == -1) &&
+  if (!small && ec && !ptr_arrays &&
       stream_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, stream_kind,
                      pre.us, &ga)) {
     if (ga.plan.piece_clusters > 0) {

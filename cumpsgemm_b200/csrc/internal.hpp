@@ -383,7 +383,8 @@ struct SmallGemmArgs {
 cudaError_t launch_tcec_gemm_small(const SmallGemmArgs &a, cudaStream_t stream);
 // How the tiles of a launch are dealt to the CTA pairs; see tcec_gemm_stream.cu.
 struct StreamPlan {
-  int tile_n;                    // 256 or 128 columns per pair tile (256 rows)
+  int tile_m;                    // 256 rows: CTA pairs; 128: single CTAs
+  int tile_n;                    // 256 or 128 columns per tile
   std::uint32_t total_tiles;
   std::uint32_t units;           // K loop in units of 64 k values
   std::uint32_t whole_tiles;     // dealt whole, in waves
@@ -392,6 +393,8 @@ struct StreamPlan {
 };
 StreamPlan plan_stream(const Tuning &tuning, int tile_n, std::uint64_t m, std::uint64_t n,
                        std::uint64_t k, std::uint64_t batch, std::uint32_t clusters);
+// 128 x 128 tiles on single CTAs, none of them cut.
+StreamPlan plan_stream_solo(std::uint64_t m, std::uint64_t n, std::uint64_t k, std::uint64_t batch);
 struct StreamGemmArgs {
   StreamKind kind;
   StreamOperand a, b;

@@ -456,45 +456,47 @@ __device__ __forceinline__ void mma_tf32_ss_pair(uint32_t d_tmem, uint64_t a_des
       : "memory");
 }
 
-// The same with A in tensor memory: lane = row (each CTA of the pair holds its own 128), a 32-bit
-// column = two consecutive FP16 or one TF32 value of K.
-__device__ __forceinline__ void mma_f16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                                uint32_t idesc, uint32_t accumulate) {
+// The same with A in tensor memory, for one CTA (CG = 1) or a pair (2): lane = row (each CTA holds its
+// own 128), a 32-bit column = two consecutive FP16 or one TF32 value of K.
+template <int CG>
+__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                           uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "tcgen05.mma.cta_group::%5.kind::f16 [%0], [%1], %2, %3, p;\n\t"
       "}\n"
       :
-      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(CG)
       : "memory");
 }
-__device__ __forceinline__ void mma_tf32_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                                 uint32_t idesc, uint32_t accumulate) {
+template <int CG>
+__device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                            uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::tf32 [%0], [%1], %2, %3, p;\n\t"
+      "tcgen05.mma.cta_group::%5.kind::tf32 [%0], [%1], %2, %3, p;\n\t"
       "}\n"
       :
-      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(CG)
       : "memory");
 }
 // D[tmem] = A * B + D * 2^-SHIFT; kind::f16, A in tensor memory
-template <int SHIFT>
-__device__ __forceinline__ void mma_f16_ts_pair_scaled(uint32_t d_tmem, uint32_t a_tmem,
-                                                       uint64_t b_desc, uint32_t idesc) {
+template <int CG, int SHIFT>
+__device__ __forceinline__ void mma_f16_ts_scaled(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                                  uint32_t idesc) {
   static_assert(SHIFT >= 0 && SHIFT <= 15, "range of scale-input-d");
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
       "setp.eq.b32 p, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t"
+      "tcgen05.mma.cta_group::%5.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t"
       "}\n"
       :
-      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(SHIFT)
+      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(SHIFT), "n"(CG)
       : "memory");
 }
 

@@ -102,16 +102,17 @@ static_assert(sizeof(StreamParams) <= 128, "kernel parameter structs stay within
 constexpr uint32_t kIsComplex = 1, kConjA = 2, kConjB = 4, kBatchA = 8, kBatchB = 16,
                    kDirectStores = 32, kSeparate = 64;
 
-template <int BN> struct StreamCfg {
-  static constexpr int B_ROWS = BN / 2;     // rows of op(B) per CTA: two blocks of HALF_ROWS, one
-  static constexpr int HALF_ROWS = BN / 4;  // for each half of the tile's columns
+// CG: CTAs of a cluster, 2 (a pair shares a 256-row tile) or 1 (128 rows).
+template <int BN, int CG> struct StreamCfg {
+  static constexpr int B_ROWS = BN / CG;         // rows of op(B) per CTA: two blocks of HALF_ROWS,
+  static constexpr int HALF_ROWS = BN / 2 / CG;  // one for each half of the tile's columns
   static constexpr int B_TILE = B_ROWS * ROW_BYTES;
   static constexpr int STAGE_BYTES = 2 * B_TILE; // hi, lo
-  static constexpr int STAGES = (BN == 256) ? 2 : 4;
+  static constexpr int STAGES = (BN == 256) ? 2 : (CG == 1) ? 3 : 4;
   static constexpr int RAW_A = BM_CTA * SLOT_K * 4;
   static constexpr int RAW_HALF_B = HALF_ROWS * SLOT_K * 4;
   static constexpr int RAW_BYTES = RAW_A + 2 * RAW_HALF_B;
-  static constexpr int RAW_SLOTS = (BN == 256) ? 4 : 6;
+  static constexpr int RAW_SLOTS = (B_ROWS == 128) ? 4 : 6;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + RAW_SLOTS * RAW_BYTES + 1024 + 256;
   // Tensor memory: accumulators of half a tile's columns each, then A, 64 columns per stage (hi, lo)
   static constexpr uint32_t D_BUFS = (BN == 256) ? 3 : 4;
@@ -141,25 +142,26 @@ struct TileCoord {
   int n0; // first column of the pair's BN columns
 };
 
-template <int BN>
+template <int BN, int CG>
 __device__ __forceinline__ TileCoord tile_coord(uint32_t tile, const StreamParams &p,
                                                 uint32_t rank) {
   const TilePos t = tile_raster(tile, p.tiles_m, p.tiles_n);
   TileCoord c;
   c.batch = t.batch;
-  c.m0 = static_cast<int>(t.tm * 2 * BM_CTA + rank * BM_CTA);
+  c.m0 = static_cast<int>((t.tm * CG + rank) * BM_CTA);
   c.n0 = static_cast<int>(t.tn * BN);
   return c;
 }
 
-template <int KIND>
-__device__ __forceinline__ void mma_pair(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc,
-                                         uint32_t acc) {
-  if constexpr (KIND == 0) {
-    ptx::mma_f16_ts_pair(d, a, b, idesc, acc);
-  } else {
-    ptx::mma_tf32_ts_pair(d, a, b, idesc, acc);
-  }
+template <int KIND, int CG>
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc,
+                                       uint32_t acc) {
+  if constexpr (KIND == 0) ptx::mma_f16_ts<CG>(d, a, b, idesc, acc);
+  else ptx::mma_tf32_ts<CG>(d, a, b, idesc, acc);
+}
+template <int CG> __device__ __forceinline__ void commit(uint32_t bar) {
+  if constexpr (CG == 2) ptx::tc_commit_pair(bar, 0x3);
+  else ptx::tc_commit(bar);
 }
 
 // ---------------------------------------------------------------- converters
@@ -234,7 +236,7 @@ __device__ __forceinline__ void load_raw8(uint32_t lane_addr, uint32_t g, const 
 
 // Splits eight consecutive k values and stores them at 8-k group kc of the stage: A in tensor
 // memory, B in shared memory.
-template <int KIND, int BN, bool IS_A>
+template <int KIND, int BN, int CG, bool IS_A>
 __device__ __forceinline__ void split_store8(const float (&v)[8], uint32_t dst, uint32_t kc) {
   if constexpr (IS_A && KIND == 1) {
     uint32_t h[8], l[8];
@@ -260,14 +262,14 @@ __device__ __forceinline__ void split_store8(const float (&v)[8], uint32_t dst, 
     } else {
       const uint32_t addr = dst ^ (q << 4);
       st_shared_v4(addr, h[0], h[1], h[2], h[3]);
-      st_shared_v4(addr + StreamCfg<BN>::B_TILE, l[0], l[1], l[2], l[3]);
+      st_shared_v4(addr + StreamCfg<BN, CG>::B_TILE, l[0], l[1], l[2], l[3]);
     }
   }
 }
 
-template <int KIND, int BN, int LAYOUT, int ROWS, int JOBS, bool IS_A>
+template <int KIND, int BN, int CG, int LAYOUT, int ROWS, int JOBS, bool IS_A>
 __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterState &st) {
-  using Cfg = StreamCfg<BN>;
+  using Cfg = StreamCfg<BN, CG>;
   constexpr uint32_t SLOTS_PER_STAGE = (KIND == 0) ? 2 : 1;
   constexpr uint32_t STAGE_STEP = 2 / SLOTS_PER_STAGE; // stages from a team's slot to its next
   const uint32_t r = st.row;
@@ -302,7 +304,7 @@ __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterSta
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] *= st.scale;
       }
-      split_store8<KIND, BN, IS_A>(v, dst, kc0 + j);
+      split_store8<KIND, BN, CG, IS_A>(v, dst, kc0 + j);
     }
     if constexpr (IS_A) {
       ptx::tmem_st_wait();
@@ -328,27 +330,23 @@ __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterSta
     }
   }
   // the issuer's last commits arrive on this CTA's barriers: it must not be gone by then
-  for (uint32_t i = 0; i < Cfg::STAGES; i += STAGE_STEP) {
-    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * s, ph ^ 1u, st.bars + Cfg::ABORT, st.status,
-                          ptx::kErrWaitEmpty))
+  for (uint32_t i = total_stages; i < total_stages + Cfg::STAGES; ++i) {
+    if (i < Cfg::STAGES) continue; // (nothing was in it)
+    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * (i % Cfg::STAGES), (i / Cfg::STAGES - 1u) & 1u,
+                          st.bars + Cfg::ABORT, st.status, ptx::kErrWaitEmpty))
       return;
-    s += STAGE_STEP;
-    if (s >= Cfg::STAGES) {
-      s -= Cfg::STAGES;
-      ph ^= 1u;
-    }
   }
 }
 
-template <int KIND, int BN>
+template <int KIND, int BN, int CG>
 __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUtensorMap &map_b,
                                             const StreamParams &p) {
-  using Cfg = StreamCfg<BN>;
+  using Cfg = StreamCfg<BN, CG>;
   constexpr int STAGES = Cfg::STAGES, RAW_SLOTS = Cfg::RAW_SLOTS;
   constexpr int K_STEPS = ROW_BYTES / 32;
   constexpr uint32_t SLOTS_PER_STAGE = (KIND == 0) ? 2 : 1;
   constexpr uint32_t STAGES_PER_UNIT = (KIND == 0) ? 1 : 2;
-  constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, 2 * BM_CTA, BN / 2);
+  constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, CG * BM_CTA, BN / 2);
   constexpr int CPT = BN / 2; // accumulator columns per epilogue thread
 
   extern __shared__ uint8_t smem_raw[];
@@ -360,10 +358,10 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = ptx::cluster_ctarank();
+  const uint32_t rank = (CG == 2) ? ptx::cluster_ctarank() : 0u;
   const bool leader = (rank == 0);
-  const uint32_t cluster_id = blockIdx.x >> 1;
-  const uint32_t num_clusters = gridDim.x >> 1;
+  const uint32_t cluster_id = blockIdx.x / CG;
+  const uint32_t num_clusters = gridDim.x / CG;
 
   if (threadIdx.x == 0) {
     for (uint32_t r = 0; r < RAW_SLOTS; ++r) {
@@ -371,12 +369,12 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
       ptx::mbar_init(bars + Cfg::RAW_EMPTY + 8u * r, TEAM_WARPS);
     }
     for (uint32_t s = 0; s < STAGES; ++s) {
-      ptx::mbar_init(bars + Cfg::FULL + 8u * s, 2 * SLOTS_PER_STAGE * TEAM_WARPS);
+      ptx::mbar_init(bars + Cfg::FULL + 8u * s, CG * SLOTS_PER_STAGE * TEAM_WARPS);
       ptx::mbar_init(bars + Cfg::EMPTY + 8u * s, 1);
     }
     for (uint32_t b = 0; b < Cfg::D_BUFS; ++b) {
       ptx::mbar_init(bars + Cfg::D_FULL + 8u * b, 1);
-      ptx::mbar_init(bars + Cfg::D_EMPTY + 8u * b, NUM_EPI_WARPS); // half of them, in both CTAs
+      ptx::mbar_init(bars + Cfg::D_EMPTY + 8u * b, CG * NUM_EPI_WARPS / 2);
     }
     st_shared_u32(abort_flag, 0u);
     ptx::mbar_init_fence();
@@ -384,14 +382,20 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     ptx::prefetch_tensormap(&map_b);
   }
   if (warp == 1) {
-    ptx::tmem_alloc_pair(bars + Cfg::TMEM_PTR, TMEM_COLS);
-    ptx::tmem_relinquish_pair();
+    if constexpr (CG == 2) {
+      ptx::tmem_alloc_pair(bars + Cfg::TMEM_PTR, TMEM_COLS);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(bars + Cfg::TMEM_PTR, TMEM_COLS);
+      ptx::tmem_relinquish();
+    }
   }
   ptx::tc_fence_before();
   __syncthreads();
-  // both CTAs' barriers must exist before any remote arrive
-  ptx::cluster_arrive();
-  ptx::cluster_wait();
+  if constexpr (CG == 2) { // both CTAs' barriers must exist before any remote arrive
+    ptx::cluster_arrive();
+    ptx::cluster_wait();
+  }
   ptx::tc_fence_after();
   constexpr uint32_t tmem_base = 0; // all of tensor memory
   // launched behind the previous kernel of the stream (programmatic serialization): from here
@@ -418,7 +422,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
         WorkList list(p.w, cluster_id, num_clusters);
         WorkItem x;
         while (ok && list.next(p.w, x)) {
-          const TileCoord tc = tile_coord<BN>(x.tile, p, rank);
+          const TileCoord tc = tile_coord<BN, CG>(x.tile, p, rank);
           const int b_row = tc.n0 + static_cast<int>(rank) * Cfg::HALF_ROWS;
           const int t0 = static_cast<int>(2u * x.u0);
           int ax = a_k ? t0 * SLOT_K : tc.m0;
@@ -454,7 +458,6 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     } else if (warp == 1 && leader) {
       if (ptx::elect_one()) {
         // ============================================================== MMA issuer (leader only)
-        constexpr uint16_t BOTH = 0x3;
         const uint64_t desc0 = ptx::make_kmajor_desc<ROW_BYTES>(ptx::smem_u32(smem));
         constexpr uint64_t kStage = Cfg::STAGE_BYTES >> 4, kLo = Cfg::B_TILE >> 4,
                            kHalf = (Cfg::HALF_ROWS * ROW_BYTES) >> 4;
@@ -485,7 +488,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
               return tmem_base + b * CPT;
             };
             auto filled = [&]() {
-              ptx::tc_commit_pair(bars + Cfg::D_FULL + 8u * b, BOTH);
+              commit<CG>(bars + Cfg::D_FULL + 8u * b);
               if (++b == Cfg::D_BUFS) {
                 b = 0;
                 d_ph ^= 1u;
@@ -495,10 +498,10 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
             auto corrections = [&](uint32_t d, uint64_t b_hi) {
 #pragma unroll
               for (int ks = 0; ks < K_STEPS; ++ks)
-                mma_pair<KIND>(d, a_lo + 8 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : 0u);
+                mma_ts<KIND, CG>(d, a_lo + 8 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : 0u);
 #pragma unroll
               for (int ks = 0; ks < K_STEPS; ++ks)
-                mma_pair<KIND>(d, a_hi + 8 * ks, b_hi + kLo + 2 * ks, IDESC, 1u);
+                mma_ts<KIND, CG>(d, a_hi + 8 * ks, b_hi + kLo + 2 * ks, IDESC, 1u);
             };
             if (!separate) {
               // per half of the columns: corrections, then hi*hi on top of them
@@ -508,11 +511,11 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
                 if (!ok) break;
                 const uint64_t b_hi = b_hi0 + g * kHalf;
                 corrections(d, b_hi);
-                if constexpr (KIND == 0) ptx::mma_f16_ts_pair_scaled<11>(d, a_hi, b_hi, IDESC);
-                else mma_pair<KIND>(d, a_hi, b_hi, IDESC, 1u);
+                if constexpr (KIND == 0) ptx::mma_f16_ts_scaled<CG, 11>(d, a_hi, b_hi, IDESC);
+                else mma_ts<KIND, CG>(d, a_hi, b_hi, IDESC, 1u);
 #pragma unroll
                 for (int ks = 1; ks < K_STEPS; ++ks)
-                  mma_pair<KIND>(d, a_hi + 8 * ks, b_hi + 2 * ks, IDESC, 1u);
+                  mma_ts<KIND, CG>(d, a_hi + 8 * ks, b_hi + 2 * ks, IDESC, 1u);
                 filled();
               }
             } else {
@@ -527,13 +530,13 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
                 } else {
 #pragma unroll
                   for (int ks = 0; ks < K_STEPS; ++ks)
-                    mma_pair<KIND>(d, a_hi + 8 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : 0u);
+                    mma_ts<KIND, CG>(d, a_hi + 8 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : 0u);
                 }
                 filled();
               }
             }
             if (!ok) break;
-            ptx::tc_commit_pair(bars + Cfg::EMPTY + 8u * s, BOTH);
+            commit<CG>(bars + Cfg::EMPTY + 8u * s);
             if (++s == STAGES) {
               s = 0;
               ph ^= 1u;
@@ -552,9 +555,9 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     // ================================================================ converters (both CTAs)
     ptx::setmaxnreg_dec<Cfg::REGS_CVT>();
     // Two teams of eight warps take the raw slots in turn.  In a team warps 0-3 convert the four
-    // 32-row blocks of A, warps 4-7 those of B (BN = 128: two warps to each of its two blocks, half
-    // of a slot's groups each).
-    constexpr int B_JOBS = (BN == 256) ? 4 : 2;
+    // 32-row blocks of A, warps 4-7 those of B (64 rows: two warps to each of its two blocks,
+    // half of a slot's groups each).
+    constexpr int B_JOBS = (Cfg::B_ROWS == 128) ? 4 : 2;
     const uint32_t cw = static_cast<uint32_t>(warp - FIRST_CVT_WARP) & 7u;
     const bool for_a = cw < 4;
     // the converters see a plain stream of stages; only its length depends on the work items
@@ -575,8 +578,8 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
       st.dst = tmem_base + Cfg::A_COL + ((cw * 32u) << 16);
     } else {
       const uint32_t half = (cw - 4u) >> 1; // of the tile's columns
-      st.row = (BN == 256 ? (cw & 1u) * 32u : 0u) + lane;
-      st.group0 = (BN == 256) ? 0u : 2u * (cw & 1u);
+      st.row = (Cfg::B_ROWS == 128 ? (cw & 1u) * 32u : 0u) + lane;
+      st.group0 = (Cfg::B_ROWS == 128) ? 0u : 2u * (cw & 1u);
       st.raw += Cfg::RAW_A + half * Cfg::RAW_HALF_B;
       const uint32_t r = half * Cfg::HALF_ROWS + st.row;
       st.dst = ptx::smem_u32(smem) + r * 128u + ((r & 7u) << 4);
@@ -588,28 +591,28 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     if (for_a) {
       switch (p.layout_a) {
       case kRawK:
-        convert_loop<KIND, BN, kRawK, BM_CTA, 4, true>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawK, BM_CTA, 4, true>(total_stages, st);
         break;
       case kRawR:
-        convert_loop<KIND, BN, kRawR, BM_CTA, 4, true>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawR, BM_CTA, 4, true>(total_stages, st);
         break;
       case kRawCplxAR:
-        convert_loop<KIND, BN, kRawCplxAR, BM_CTA, 4, true>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawCplxAR, BM_CTA, 4, true>(total_stages, st);
         break;
       default:
-        convert_loop<KIND, BN, kRawCplxAK, BM_CTA, 4, true>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawCplxAK, BM_CTA, 4, true>(total_stages, st);
         break;
       }
     } else {
       switch (p.layout_b) {
       case kRawK:
-        convert_loop<KIND, BN, kRawK, Cfg::HALF_ROWS, B_JOBS, false>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawK, Cfg::HALF_ROWS, B_JOBS, false>(total_stages, st);
         break;
       case kRawR:
-        convert_loop<KIND, BN, kRawR, Cfg::HALF_ROWS, B_JOBS, false>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawR, Cfg::HALF_ROWS, B_JOBS, false>(total_stages, st);
         break;
       default:
-        convert_loop<KIND, BN, kRawCplxBR, Cfg::HALF_ROWS, B_JOBS, false>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawCplxBR, Cfg::HALF_ROWS, B_JOBS, false>(total_stages, st);
         break;
       }
     }
@@ -635,7 +638,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     };
     // beta != 0: pull this warp's part of a C tile into L2 before the epilogue reads it
     auto prefetch_c = [&](uint32_t tile) {
-      const TileCoord tc = tile_coord<BN>(opaque(tile), p, rank);
+      const TileCoord tc = tile_coord<BN, CG>(opaque(tile), p, rank);
       const uint32_t row = static_cast<uint32_t>(tc.m0) + static_cast<uint32_t>(warp & 3) * 32u;
       const float *cp = p.c + static_cast<uint64_t>(tc.batch) * p.stride_c + row;
 #pragma unroll 1
@@ -687,7 +690,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
 #pragma unroll
         for (int i = 0; i < CPT / 2; ++i)
           asm("mov.b64 {%0, %1}, %2;" : "=f"(sums[2 * i]), "=f"(sums[2 * i + 1]) : "l"(acc[i]));
-        const TileCoord tc = tile_coord<BN>(opaque(x.tile), p, rank);
+        const TileCoord tc = tile_coord<BN, CG>(opaque(x.tile), p, rank);
         const uint32_t row = static_cast<uint32_t>(tc.m0) + static_cast<uint32_t>(warp & 3) * 32u +
                              static_cast<uint32_t>(lane);
         const uint32_t col0 = static_cast<uint32_t>(tc.n0) +
@@ -702,7 +705,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
       // the epilogue needs to know of the tile is worked out only now (epilogue.cuh)
       finish_pairs_in_tmem<CPT>(t_sums, acc);
       const bool part = x.un != p.w.units; // this item is a piece of a tile
-      const TileCoord tc = tile_coord<BN>(opaque(x.tile), p, rank);
+      const TileCoord tc = tile_coord<BN, CG>(opaque(x.tile), p, rank);
       const uint32_t quarter = static_cast<uint32_t>(warp & 3);
       const uint32_t col_base = static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2) * CPT;
       const uint32_t row =
@@ -739,8 +742,10 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   // neither CTA leaves while the other still uses its shared memory or TMEM
   ptx::tc_fence_before();
   __syncthreads();
-  ptx::cluster_arrive();
-  ptx::cluster_wait();
+  if constexpr (CG == 2) {
+    ptx::cluster_arrive();
+    ptx::cluster_wait();
+  }
   if (*reinterpret_cast<volatile int *>(raw_smem + RAW_SLOTS * Cfg::RAW_BYTES + Cfg::ABORT)) {
     // a wait gave up: let copies and tensor-core work still in flight land
     const uint64_t t0 = ptx::globaltimer_ns();
@@ -749,7 +754,8 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   }
   if (warp == 1) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    if constexpr (CG == 2) ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else ptx::tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
@@ -761,25 +767,46 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
   if constexpr (KIND == 2) {
     ptx::griddep_wait(); // the decision is written by an earlier kernel of the call
     if (p.dyn->gemm_mode == CUMPSGEMM_TF32TCEC)
-      stream_body<1, BN>(map_a, map_b, p);
+      stream_body<1, BN, 2>(map_a, map_b, p);
     else
-      stream_body<0, BN>(map_a, map_b, p);
+      stream_body<0, BN, 2>(map_a, map_b, p);
   } else {
-    stream_body<KIND, BN>(map_a, map_b, p);
+    stream_body<KIND, BN, 2>(map_a, map_b, p);
   }
 }
 
+// The same on single CTAs, 128 x 128 tiles: batches of matrices with at most 128 rows.
+template <int KIND>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+    tcec_gemm_stream_solo_kernel(const __grid_constant__ CUtensorMap map_a,
+                                 const __grid_constant__ CUtensorMap map_b, const StreamParams p) {
+  if constexpr (KIND == 2) {
+    ptx::griddep_wait();
+    if (p.dyn->gemm_mode == CUMPSGEMM_TF32TCEC)
+      stream_body<1, 128, 1>(map_a, map_b, p);
+    else
+      stream_body<0, 128, 1>(map_a, map_b, p);
+  } else {
+    stream_body<KIND, 128, 1>(map_a, map_b, p);
+  }
+}
+
+template <int KIND, int BN, int CG> constexpr auto stream_kernel() {
+  if constexpr (CG == 2) return &tcec_gemm_stream_kernel<KIND, BN>;
+  else return &tcec_gemm_stream_solo_kernel<KIND>;
+}
+
 // Per device and kernel, once: shared-memory attribute, register count, resident clusters.
-template <int KIND, int BN> cudaError_t stream_setup(int *clusters_out) {
+template <int KIND, int BN, int CG> cudaError_t stream_setup(int *clusters_out) {
   static std::once_flag once[64];
   static cudaError_t setup_error[64];
   static int max_clusters[64];
-  auto kernel = tcec_gemm_stream_kernel<KIND, BN>;
+  auto kernel = stream_kernel<KIND, BN, CG>();
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   std::call_once(once[dev], [&]() {
-    constexpr int smem = StreamCfg<BN>::SMEM_BYTES;
+    constexpr int smem = StreamCfg<BN, CG>::SMEM_BYTES;
     setup_error[dev] =
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     // the register re-allocation inside the kernel draws on what the CTA was launched with: an
@@ -792,13 +819,13 @@ template <int KIND, int BN> cudaError_t stream_setup(int *clusters_out) {
     }
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int clusters = sms / 2;
+    int clusters = sms / CG;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(2 * clusters));
     cfg.blockDim = dim3(NUM_THREADS);
     cfg.dynamicSmemBytes = smem;
     int active = 0;
-    if (setup_error[dev] == cudaSuccess &&
+    if (CG == 2 && setup_error[dev] == cudaSuccess &&
         cudaOccupancyMaxActiveClusters(&active, kernel, &cfg) == cudaSuccess) {
       if (active > 0 && active < clusters) clusters = active;
     } else {
@@ -843,13 +870,14 @@ bool raw_map(CUtensorMap *map, const StreamOperand &o, int layout, uint64_t rows
   return make_float_map(map, o.src, dims, strides, box, swizzle);
 }
 
-template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, cudaStream_t stream) {
+template <int KIND, int BN, int CG>
+cudaError_t launch_variant(const StreamGemmArgs &a, cudaStream_t stream) {
   int max_clusters = 1;
-  const cudaError_t se = stream_setup<KIND, BN>(&max_clusters);
+  const cudaError_t se = stream_setup<KIND, BN, CG>(&max_clusters);
   if (se != cudaSuccess) return se;
   CUtensorMap map_a, map_b;
   if (!raw_map(&map_a, a.a, a.layout_a, a.m, a.k, a.batch, BM_CTA) ||
-      !raw_map(&map_b, a.b, a.layout_b, a.n, a.k, a.batch, StreamCfg<BN>::HALF_ROWS))
+      !raw_map(&map_b, a.b, a.layout_b, a.n, a.k, a.batch, StreamCfg<BN, CG>::HALF_ROWS))
     return cudaErrorNotSupported; // an extent TMA cannot address: the caller takes another path
   StreamParams p;
   p.c = a.c;
@@ -861,7 +889,7 @@ template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, 
   p.stride_c = a.stride_c;
   p.m = a.m;
   p.n = a.n;
-  p.tiles_m = (a.m + 2 * BM_CTA - 1) / (2 * BM_CTA);
+  p.tiles_m = (a.m + CG * BM_CTA - 1) / (CG * BM_CTA);
   p.tiles_n = (a.n + BN - 1) / BN;
   p.alpha_r = a.alpha_r;
   p.alpha_i = a.alpha_i;
@@ -875,7 +903,7 @@ template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, 
                                  (a.batch > 1 && a.b.stride != 0 ? kBatchB : 0));
   if (a.k <= 64) p.flags |= kSeparate;
   const StreamPlan &plan = a.plan;
-  if (plan.tile_n != BN || plan.total_tiles != p.tiles_m * p.tiles_n * a.batch ||
+  if (plan.tile_n != BN || plan.tile_m != CG * BM_CTA || plan.total_tiles != p.tiles_m * p.tiles_n * a.batch ||
       plan.units != (a.k + 63) / 64)
     return cudaErrorInvalidValue;
   p.w.total_tiles = plan.total_tiles;
@@ -896,8 +924,8 @@ template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, 
   uint32_t clusters = plan.whole_tiles > plan.piece_clusters ? plan.whole_tiles : plan.piece_clusters;
   if (clusters > static_cast<uint32_t>(max_clusters)) clusters = static_cast<uint32_t>(max_clusters);
   if (clusters == 0 || plan.piece_clusters > clusters) return cudaErrorInvalidValue;
-  const cudaError_t e = launch_chained(tcec_gemm_stream_kernel<KIND, BN>, 2 * clusters, NUM_THREADS,
-                                       StreamCfg<BN>::SMEM_BYTES, stream, map_a, map_b, p);
+  const cudaError_t e = launch_chained(stream_kernel<KIND, BN, CG>(), CG * clusters, NUM_THREADS,
+                                       StreamCfg<BN, CG>::SMEM_BYTES, stream, map_a, map_b, p);
   if (e != cudaSuccess || plan.piece_clusters == 0) return e;
   const PieceFixupArgs f = {a.partial,  a.c,       nullptr,   a.dyn,     a.ldc,
                             a.stride_c, a.m,       a.n,       p.tiles_m, p.tiles_n,
@@ -906,14 +934,14 @@ template <int KIND, int BN> cudaError_t launch_variant(const StreamGemmArgs &a, 
   return launch_piece_fixup(f, p.w, stream);
 }
 
-template <int BN> cudaError_t launch_by_kind(const StreamGemmArgs &a, cudaStream_t stream) {
+template <int BN, int CG> cudaError_t launch_by_kind(const StreamGemmArgs &a, cudaStream_t stream) {
   switch (a.kind) {
   case StreamKind::fp16:
-    return launch_variant<0, BN>(a, stream);
+    return launch_variant<0, BN, CG>(a, stream);
   case StreamKind::tf32:
-    return launch_variant<1, BN>(a, stream);
+    return launch_variant<1, BN, CG>(a, stream);
   default:
-    return a.dyn != nullptr ? launch_variant<2, BN>(a, stream) : cudaErrorInvalidValue;
+    return a.dyn != nullptr ? launch_variant<2, BN, CG>(a, stream) : cudaErrorInvalidValue;
   }
 }
 
@@ -924,6 +952,7 @@ template <int BN> cudaError_t launch_by_kind(const StreamGemmArgs &a, cudaStream
 StreamPlan plan_stream(const Tuning &tuning, int tile_n, uint64_t m, uint64_t n, uint64_t k,
                        uint64_t batch, uint32_t clusters) {
   StreamPlan pl = {};
+  pl.tile_m = 2 * BM_CTA;
   pl.tile_n = tile_n;
   const uint64_t total =
       ((m + 2 * BM_CTA - 1) / (2 * BM_CTA)) * ((n + tile_n - 1) / tile_n) * batch;
@@ -962,25 +991,38 @@ StreamPlan plan_stream(const Tuning &tuning, int tile_n, uint64_t m, uint64_t n,
   return pl;
 }
 
+StreamPlan plan_stream_solo(uint64_t m, uint64_t n, uint64_t k, uint64_t batch) {
+  StreamPlan pl = {};
+  const uint64_t total = ((m + BM_CTA - 1) / BM_CTA) * ((n + 127) / 128) * batch;
+  const uint64_t units = (k + 63) / 64;
+  if (total == 0 || total > 0x3fffffffull || units == 0 || units > 0x3fffffull) return pl;
+  pl.tile_m = BM_CTA;
+  pl.tile_n = 128;
+  pl.total_tiles = pl.whole_tiles = static_cast<uint32_t>(total);
+  pl.units = static_cast<uint32_t>(units);
+  return pl;
+}
+
 std::size_t stream_scratch_bytes(const StreamPlan &plan) {
   return static_cast<std::size_t>(plan.piece_clusters) * 2u * 2u * BM_CTA *
          static_cast<std::size_t>(plan.tile_n) * sizeof(float);
 }
 
 cudaError_t launch_tcec_gemm_stream(const StreamGemmArgs &a, cudaStream_t stream) {
-  if (a.plan.tile_n == 256) return launch_by_kind<256>(a, stream);
-  if (a.plan.tile_n == 128) return launch_by_kind<128>(a, stream);
+  if (a.plan.tile_m == BM_CTA) return launch_by_kind<128, 1>(a, stream);
+  if (a.plan.tile_n == 256) return launch_by_kind<256, 2>(a, stream);
+  if (a.plan.tile_n == 128) return launch_by_kind<128, 2>(a, stream);
   return cudaErrorInvalidValue;
 }
 
 cudaError_t stream_max_clusters(StreamKind kind, int tile_n, int *clusters) {
   switch (kind) {
   case StreamKind::fp16:
-    return tile_n == 256 ? stream_setup<0, 256>(clusters) : stream_setup<0, 128>(clusters);
+    return tile_n == 256 ? stream_setup<0, 256, 2>(clusters) : stream_setup<0, 128, 2>(clusters);
   case StreamKind::tf32:
-    return tile_n == 256 ? stream_setup<1, 256>(clusters) : stream_setup<1, 128>(clusters);
+    return tile_n == 256 ? stream_setup<1, 256, 2>(clusters) : stream_setup<1, 128, 2>(clusters);
   default:
-    return tile_n == 256 ? stream_setup<2, 256>(clusters) : stream_setup<2, 128>(clusters);
+    return tile_n == 256 ? stream_setup<2, 256, 2>(clusters) : stream_setup<2, 128, 2>(clusters);
   }
 }
 
