@@ -353,9 +353,7 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
     // them again for each (4096 x 4096 x 1024: 102 us against 91), and the model is not fitted to it
     if (2ull * pl.total_tiles > 3ull * (256 / tile_n) * static_cast<std::uint64_t>(clusters)) continue;
     const double us = estimate(pl);
-    // (128 columns instead of 256 only for a clear gain: 96 x 342 x 23008, estimated 27.4 and 27.6, takes
-    // 35 and 30 us)
-    if (us < best * (plan.tile_n == 256 ? 0.93 : 1.0)) {
+    if (us < best) {
       best = us;
       plan = pl;
     }
@@ -587,13 +585,17 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
 
   // ---- one launch on CTA pairs, operands split between TMA and the tensor core
   StreamGemmArgs ga;
+  // (Where the on-the-fly kernel would take the call, that is what streaming stands against, and it is faster
+  // in all that was measured, us: 256 x 256 x 8192 23.4 / 16.8, 384 x 384 x 32768 73 / 48, 96 x 342 x 23008
+  // 35 / 25, 9 x 300 x 300 x 900 44 / 20, 8 x 200 x 500 x 1000 38 / 22, and the batches in stream_args.)
+  constexpr double kNoEstimate = 1e30;
   FusedGemmArgs fa;
   const bool fused = !small && mode == CUMPSGEMM_FP16TCEC && !ptr_arrays &&
                      fused_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch,
                                    &fa);
   if (!small && ec && !ptr_arrays &&
       stream_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, stream_kind,
-                     pre.us, &ga)) {
+                     fused ? kNoEstimate : pre.us, &ga)) {
     if (ga.plan.piece_clusters > 0) {
       const std::size_t bytes = stream_scratch_bytes(ga.plan);
       const std::size_t limit =
