@@ -48,13 +48,15 @@
 //   raw_full[r]    1 arrival (producer, expect_tx) + TMA bytes      own CTA
 //   raw_empty[r]   8 arrivals, one per warp of the slot's team      own CTA
 //   full[s]        leader's only: the converter warps of both CTAs
-//   empty[s]       tcgen05.commit multicast from the leader         both CTAs
-//   d_full[b]      the same, after the products of one half of the columns
+//   empty[e]       tcgen05.commit multicast from the leader         both CTAs
+//   d_full[f]      the same, after the products of one half of the columns
 //   d_empty[b]     leader's only: 8 arrivals, the epilogue warps of that half in both CTAs
-// Waits tell phases apart by one bit, so a waiter may be at most one phase behind: the number of raw
-// slots is even, because copies complete in any order and a slot that both teams used could show one
-// team the phase before the other's.  (Commits complete in order.)  Every wait is bounded; no TMA
-// multicast is used.
+// A wait tells phases apart by one bit, so whoever waits on a barrier looks at each of its phases, and
+// before the next one can end: one that passed over a phase could take the phase before it for the one
+// it wants, and nothing says that arrivals on different barriers are seen in the order they were sent.
+// So the number of raw slots is even (a slot belongs to one team), either half of the columns has
+// d_full barriers of its own, and where the teams share an odd number of stages in turn (TF32TCEC on
+// single CTAs) each has empty barriers of its own.  Every wait is bounded; no TMA multicast is used.
 #include "epilogue.cuh"
 #include "gemm_common.cuh"
 #include "ptx.cuh"
@@ -116,6 +118,10 @@ template <int BN, int CG> struct StreamCfg {
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + RAW_SLOTS * RAW_BYTES + 1024 + 256;
   // Tensor memory: accumulators of half a tile's columns each, then A, 64 columns per stage (hi, lo)
   static constexpr uint32_t D_BUFS = (BN == 256) ? 3 : 4;
+  // An accumulator that serves both halves of the columns in turn has a d_full barrier for each, and
+  // a stage that both teams use in turn has two empty barriers, committed to in turn.
+  static constexpr uint32_t D_FULL_BARS = (D_BUFS % 2 == 0) ? D_BUFS : 2 * D_BUFS;
+  static constexpr uint32_t EMPTY_BARS = (STAGES % 2 == 0) ? STAGES : 2 * STAGES;
   static constexpr uint32_t A_COL = D_BUFS * (BN / 2);
   static constexpr int REGS_EPI = (BN == 256) ? 152 : 112;
   static constexpr int REGS_CVT = (BN == 256) ? 40 : 48;
@@ -126,8 +132,8 @@ template <int BN, int CG> struct StreamCfg {
                 "setmaxnreg.inc goes up, setmaxnreg.dec down: anything else is an illegal instruction");
   // Barriers behind the raw slots, as byte offsets: eight bytes each
   static constexpr uint32_t RAW_FULL = 0, RAW_EMPTY = 8 * RAW_SLOTS, FULL = RAW_EMPTY + 8 * RAW_SLOTS,
-                            EMPTY = FULL + 8 * STAGES, D_FULL = EMPTY + 8 * STAGES,
-                            D_EMPTY = D_FULL + 8 * D_BUFS, TMEM_PTR = D_EMPTY + 8 * D_BUFS,
+                            EMPTY = FULL + 8 * STAGES, D_FULL = EMPTY + 8 * EMPTY_BARS,
+                            D_EMPTY = D_FULL + 8 * D_FULL_BARS, TMEM_PTR = D_EMPTY + 8 * D_BUFS,
                             ABORT = TMEM_PTR + 4;
   static_assert(ABORT + 4 <= 256, "barriers");
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
@@ -282,14 +288,25 @@ __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterSta
   else lane_raw = st.raw + (r >> 1) * 128u + (((r >> 1) & 7u) << 4);
   const bool scaled = st.scale != 1.f;
   uint32_t rs = st.team, rph = 0;
-  uint32_t s = (KIND == 0) ? 0u : st.team, ph = 0;
+  // index in the stream of stages; barrier and parity of the release of the stage's previous use
+  uint32_t i = (KIND == 0) ? 0u : st.team;
+  uint32_t e = (i + Cfg::STAGES) % Cfg::EMPTY_BARS, e_ph = 1;
+  auto next = [&]() {
+    i += STAGE_STEP;
+    e += STAGE_STEP;
+    if (e >= Cfg::EMPTY_BARS) {
+      e -= Cfg::EMPTY_BARS;
+      e_ph ^= 1u;
+    }
+  };
   const uint32_t kc0 = st.group0 + ((KIND == 0) ? 4u * st.team : 0u);
 #pragma unroll 1
-  for (uint32_t i = (KIND == 0) ? 0u : st.team; i < total_stages; i += STAGE_STEP) {
+  for (; i < total_stages; next()) {
+    const uint32_t s = (Cfg::EMPTY_BARS > Cfg::STAGES && e >= Cfg::STAGES) ? e - Cfg::STAGES : e;
     if (!ptx::mbar_wait_s(st.bars + Cfg::RAW_FULL + 8u * rs, rph, st.bars + Cfg::ABORT, st.status,
                           ptx::kErrWaitFull))
       return;
-    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * s, ph ^ 1u, st.bars + Cfg::ABORT, st.status,
+    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * e, e_ph, st.bars + Cfg::ABORT, st.status,
                           ptx::kErrWaitEmpty))
       return;
     __syncwarp();
@@ -302,7 +319,7 @@ __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterSta
       load_raw8<LAYOUT, ROWS>(raw_addr, st.group0 + j, st, v);
       if (scaled) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] *= st.scale;
+        for (int t = 0; t < 8; ++t) v[t] *= st.scale;
       }
       split_store8<KIND, BN, CG, IS_A>(v, dst, kc0 + j);
     }
@@ -323,17 +340,13 @@ __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterSta
       rs -= Cfg::RAW_SLOTS;
       rph ^= 1u;
     }
-    s += STAGE_STEP;
-    if (s >= Cfg::STAGES) {
-      s -= Cfg::STAGES;
-      ph ^= 1u;
-    }
   }
-  // the issuer's last commits arrive on this CTA's barriers: it must not be gone by then
-  for (uint32_t i = total_stages; i < total_stages + Cfg::STAGES; ++i) {
+  // the issuer's last commits arrive on this CTA's barriers: it must not be gone by then (TF32TCEC:
+  // each team waits for those that it would go on with)
+  for (; i < total_stages + Cfg::STAGES; next()) {
     if (i < Cfg::STAGES) continue; // (nothing was in it)
-    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * (i % Cfg::STAGES), (i / Cfg::STAGES - 1u) & 1u,
-                          st.bars + Cfg::ABORT, st.status, ptx::kErrWaitEmpty))
+    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * e, e_ph, st.bars + Cfg::ABORT, st.status,
+                          ptx::kErrWaitEmpty))
       return;
   }
 }
@@ -370,10 +383,10 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     }
     for (uint32_t s = 0; s < STAGES; ++s) {
       ptx::mbar_init(bars + Cfg::FULL + 8u * s, CG * SLOTS_PER_STAGE * TEAM_WARPS);
-      ptx::mbar_init(bars + Cfg::EMPTY + 8u * s, 1);
     }
+    for (uint32_t e = 0; e < Cfg::EMPTY_BARS; ++e) ptx::mbar_init(bars + Cfg::EMPTY + 8u * e, 1);
+    for (uint32_t f = 0; f < Cfg::D_FULL_BARS; ++f) ptx::mbar_init(bars + Cfg::D_FULL + 8u * f, 1);
     for (uint32_t b = 0; b < Cfg::D_BUFS; ++b) {
-      ptx::mbar_init(bars + Cfg::D_FULL + 8u * b, 1);
       ptx::mbar_init(bars + Cfg::D_EMPTY + 8u * b, CG * NUM_EPI_WARPS / 2);
     }
     st_shared_u32(abort_flag, 0u);
@@ -462,6 +475,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
         constexpr uint64_t kStage = Cfg::STAGE_BYTES >> 4, kLo = Cfg::B_TILE >> 4,
                            kHalf = (Cfg::HALF_ROWS * ROW_BYTES) >> 4;
         uint32_t s = 0, ph = 0, b = 0, d_ph = 1;
+        uint32_t e = 0, f = 0; // the next empty and d_full barriers to commit to
         bool ok = true;
         const bool separate = (p.flags & kSeparate) != 0;
         auto wait_timed = [&](uint32_t bar, uint32_t parity, int code, uint32_t &cycles) {
@@ -488,7 +502,8 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
               return tmem_base + b * CPT;
             };
             auto filled = [&]() {
-              commit<CG>(bars + Cfg::D_FULL + 8u * b);
+              commit<CG>(bars + Cfg::D_FULL + 8u * (Cfg::D_FULL_BARS == Cfg::D_BUFS ? b : f));
+              if (++f == Cfg::D_FULL_BARS) f = 0;
               if (++b == Cfg::D_BUFS) {
                 b = 0;
                 d_ph ^= 1u;
@@ -536,7 +551,8 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
               }
             }
             if (!ok) break;
-            commit<CG>(bars + Cfg::EMPTY + 8u * s);
+            commit<CG>(bars + Cfg::EMPTY + 8u * (Cfg::EMPTY_BARS == STAGES ? s : e));
+            if (++e == Cfg::EMPTY_BARS) e = 0;
             if (++s == STAGES) {
               s = 0;
               ph ^= 1u;
@@ -624,15 +640,18 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     const uint32_t half = static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2); // of the columns
     const uint32_t t_base = tmem_base + ((static_cast<uint32_t>(warp & 3) * 32u) << 16);
 
-    uint32_t b = half, d_ph = 0; // accumulator and parity of the next stage
+    uint32_t f = half, d_ph = 0; // d_full barrier and parity of the next stage
+    auto buffer = [&]() { // its accumulator
+      return (Cfg::D_FULL_BARS > Cfg::D_BUFS && f >= Cfg::D_BUFS) ? f - Cfg::D_BUFS : f;
+    };
     auto give_back = [&]() {
       ptx::tc_fence_before();
       __syncwarp();
-      if (ptx::elect_one()) ptx::mbar_arrive_cluster(ptx::map_to_cta(bars + Cfg::D_EMPTY + 8u * b, 0));
+      if (ptx::elect_one()) ptx::mbar_arrive_cluster(ptx::map_to_cta(bars + Cfg::D_EMPTY + 8u * buffer(), 0));
       __syncwarp();
-      b += 2u;
-      if (b >= Cfg::D_BUFS) {
-        b -= Cfg::D_BUFS;
+      f += 2u;
+      if (f >= Cfg::D_FULL_BARS) {
+        f -= Cfg::D_FULL_BARS;
         d_ph ^= 1u;
       }
     };
@@ -663,13 +682,13 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
 #pragma unroll 1
       while (true) {
         if (left == C_PREFETCH_LEAD && (p.beta_r != 0.f || p.beta_i != 0.f)) prefetch_c(x.tile);
-        ok = ptx::mbar_wait_s(bars + Cfg::D_FULL + 8u * b, d_ph, abort_flag, p.status,
+        ok = ptx::mbar_wait_s(bars + Cfg::D_FULL + 8u * f, d_ph, abort_flag, p.status,
                               ptx::kErrWaitD0Full);
         if (!ok) break;
         __syncwarp();
         ptx::tc_fence_after();
         if (--left == 0) break; // the last ones are added below
-        drain_pairs<CPT>(t_base + b * CPT, acc);
+        drain_pairs<CPT>(t_base + buffer() * CPT, acc);
         // (corrections in an accumulator of their own come first, and nothing else is in acc then
         // but, in TF32, finished sums, whose corrections are not scaled)
         if (KIND == 0 && separate) {
@@ -679,7 +698,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
         give_back();
       }
       if (!ok) break;
-      const uint32_t t_sums = t_base + b * CPT;
+      const uint32_t t_sums = t_base + buffer() * CPT;
       if (BN == 128 && (p.flags & kDirectStores)) {
         // Many short tiles per cluster, C not read: stores straight from the registers.  That is
         // long code, but it stays in the instruction cache from tile to tile, and D1 goes back to
