@@ -131,6 +131,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
   }
 }
 
+// A bounded wait gives up lane by lane.  Where a whole warp waits and goes on to warp-wide instructions
+// (tcgen05.ld / st, shuffles), all of its lanes have to go on or none: a lane that gave up alone would
+// leave the others waiting for it without a limit.
+__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
+
 // Bounded wait for roles that can afford a little extra latency: between polls the thread
 // sleeps, so a waiting warp leaves the issue slots of its scheduler to the warps that work.
 __device__ __forceinline__ bool mbar_wait_backoff(uint32_t bar, uint32_t parity,

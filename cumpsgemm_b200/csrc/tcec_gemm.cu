@@ -304,8 +304,8 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
       for (int i = 0; i < CPT; ++i) cor[i] = 0.f;
       for (uint32_t kb = 0; kb < k_blocks; ++kb) {
         const uint32_t b = kb & 1u;
-        ok = ptx::mbar_wait_timed(ptx::smem_u32(&d0_full[b]), (kb >> 1) & 1u, abort_flag, p.status,
-                                  ptx::kErrWaitD0Full, dbg, &dbg_wait);
+        ok = ptx::warp_agrees(ptx::mbar_wait_timed(ptx::smem_u32(&d0_full[b]), (kb >> 1) & 1u, abort_flag,
+                                                   p.status, ptx::kErrWaitD0Full, dbg, &dbg_wait));
         if (!ok) break;
         ptx::tc_fence_after();
         const uint32_t t = tmem_base + lane_addr + b * Cfg::D_COLS + col_base;
@@ -317,8 +317,8 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
       }
     } else {
       for (uint32_t kb = 0; kb < k_blocks; ++kb) {
-        ok = ptx::mbar_wait_timed(ptx::smem_u32(d0_full), kb & 1u, abort_flag, p.status,
-                                  ptx::kErrWaitD0Full, dbg, &dbg_wait);
+        ok = ptx::warp_agrees(ptx::mbar_wait_timed(ptx::smem_u32(d0_full), kb & 1u, abort_flag,
+                                                   p.status, ptx::kErrWaitD0Full, dbg, &dbg_wait));
         if (!ok) break;
         ptx::tc_fence_after();
 #pragma unroll
@@ -343,7 +343,8 @@ __device__ __forceinline__ void tcec_gemm_body(const CUtensorMap &map_a, const C
       }
       sums_to_tmem<CPT>(tmem_base + D1_COL + lane_addr + col_base, acc);
     } else if (ok && EC) {
-      ok = ptx::mbar_wait(ptx::smem_u32(d1_full), 0u, abort_flag, p.status, ptx::kErrWaitD1Full);
+      ok = ptx::warp_agrees(ptx::mbar_wait(ptx::smem_u32(d1_full), 0u, abort_flag, p.status,
+                                           ptx::kErrWaitD1Full));
       if (ok) {
         ptx::tc_fence_after();
         add_corrections_in_tmem<CPT>(tmem_base + D1_COL + lane_addr + col_base, acc,

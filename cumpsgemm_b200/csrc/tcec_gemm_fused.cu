@@ -765,8 +765,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) tcec_gemm_fused_kernel(const F
 
       for (uint32_t c = 0; c < n_chunks; ++c, ++chunk_idx) {
         const uint32_t b0 = chunk_idx & 1u;
-        ok = ptx::mbar_wait_backoff(ptx::smem_u32(&d0_full[b0]), (chunk_idx >> 1) & 1u, abort_flag,
-                                    p.status, ptx::kErrWaitD0Full, 64);
+        ok = ptx::warp_agrees(ptx::mbar_wait_backoff(ptx::smem_u32(&d0_full[b0]), (chunk_idx >> 1) & 1u,
+                                                     abort_flag, p.status, ptx::kErrWaitD0Full, 64));
         if (!ok) break;
         ptx::tc_fence_after();
         // running sum += hi*hi + (hi*lo + lo*hi) * 2^-11, both FP32 round-to-nearest adds

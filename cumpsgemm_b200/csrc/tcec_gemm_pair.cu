@@ -362,7 +362,8 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
             if (col < p.n && row < p.m) ptx::prefetch_l2(cp + static_cast<uint64_t>(col) * p.ldc);
           }
         }
-        ok = ptx::mbar_wait(ptx::smem_u32(d0_full), d0_ph, abort_flag, p.status, ptx::kErrWaitD0Full);
+        ok = ptx::warp_agrees(ptx::mbar_wait(ptx::smem_u32(d0_full), d0_ph, abort_flag, p.status,
+                                             ptx::kErrWaitD0Full));
         if (!ok) break;
         d0_ph ^= 1u;
         ptx::tc_fence_after();
@@ -373,7 +374,8 @@ __device__ __forceinline__ void pair_body(const CUtensorMap &map_a, const CUtens
       }
       if (!ok) break;
 
-      ok = ptx::mbar_wait(ptx::smem_u32(d1_full), d1_ph, abort_flag, p.status, ptx::kErrWaitD1Full);
+      ok = ptx::warp_agrees(ptx::mbar_wait(ptx::smem_u32(d1_full), d1_ph, abort_flag, p.status,
+                                           ptx::kErrWaitD1Full));
       if (!ok) break;
       d1_ph ^= 1u;
       ptx::tc_fence_after();

@@ -253,9 +253,8 @@ __device__ __forceinline__ void small_body(const SmallParams &p, uint32_t tiles,
   bool ok = true;
   // adds chunk c's products, which were committed on done[c & 1]
   auto drain = [&](uint32_t c2) {
-    ok = ok && ptx::mbar_wait(done + 8u * (c2 & 1u), (c2 >> 1) & 1u, abort_flag, p.status,
-                              ptx::kErrWaitD0Full);
-    __syncwarp();
+    ok = ptx::warp_agrees(ok && ptx::mbar_wait(done + 8u * (c2 & 1u), (c2 >> 1) & 1u, abort_flag,
+                                               p.status, ptx::kErrWaitD0Full));
     if (!ok) return;
     ptx::tc_fence_after();
     uint32_t v[COLS], w[COLS];

@@ -303,13 +303,11 @@ __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterSta
 #pragma unroll 1
   for (; i < total_stages; next()) {
     const uint32_t s = (Cfg::EMPTY_BARS > Cfg::STAGES && e >= Cfg::STAGES) ? e - Cfg::STAGES : e;
-    if (!ptx::mbar_wait_s(st.bars + Cfg::RAW_FULL + 8u * rs, rph, st.bars + Cfg::ABORT, st.status,
-                          ptx::kErrWaitFull))
+    if (!ptx::warp_agrees(ptx::mbar_wait_s(st.bars + Cfg::RAW_FULL + 8u * rs, rph,
+                                           st.bars + Cfg::ABORT, st.status, ptx::kErrWaitFull) &&
+                          ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * e, e_ph, st.bars + Cfg::ABORT,
+                                           st.status, ptx::kErrWaitEmpty)))
       return;
-    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * e, e_ph, st.bars + Cfg::ABORT, st.status,
-                          ptx::kErrWaitEmpty))
-      return;
-    __syncwarp();
     if constexpr (IS_A) ptx::tc_fence_after();
     const uint32_t raw_addr = lane_raw + rs * Cfg::RAW_BYTES;
     const uint32_t dst = st.dst + s * (IS_A ? A_STAGE_COLS : static_cast<uint32_t>(Cfg::STAGE_BYTES));
@@ -682,10 +680,9 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
 #pragma unroll 1
       while (true) {
         if (left == C_PREFETCH_LEAD && (p.beta_r != 0.f || p.beta_i != 0.f)) prefetch_c(x.tile);
-        ok = ptx::mbar_wait_s(bars + Cfg::D_FULL + 8u * f, d_ph, abort_flag, p.status,
-                              ptx::kErrWaitD0Full);
+        ok = ptx::warp_agrees(ptx::mbar_wait_s(bars + Cfg::D_FULL + 8u * f, d_ph, abort_flag, p.status,
+                                               ptx::kErrWaitD0Full));
         if (!ok) break;
-        __syncwarp();
         ptx::tc_fence_after();
         if (--left == 0) break; // the last ones are added below
         drain_pairs<CPT>(t_base + buffer() * CPT, acc);

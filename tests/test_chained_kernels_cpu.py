@@ -40,3 +40,18 @@ def test_device_decision_is_read_behind_the_wait(source, functions):
         assert "dyn->" in body, name
         assert "griddep_wait()" in body, name
         assert body.index("griddep_wait()") < body.index("dyn->"), name
+
+
+@pytest.mark.parametrize("source", ["tcec_gemm.cu", "tcec_gemm_pair.cu", "tcec_gemm_fused.cu",
+                                    "tcec_gemm_small.cu", "tcec_gemm_stream.cu"])
+def test_a_warp_that_waits_for_an_accumulator_goes_on_as_a_whole(source):
+    """A bounded wait gives up lane by lane; the loads from tensor memory that follow need the whole
+    warp, so its lanes agree on the result (likewise converters that write to tensor memory)."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / source).read_text())
+    waits = [s for s in re.findall(r"[^;{}]*ptx::mbar_wait[^;]*;", text)
+             if "kErrWaitD0Full" in s or "kErrWaitD1Full" in s]
+    assert waits
+    if source == "tcec_gemm_stream.cu":
+        waits += re.findall(r"[^;{}]*ptx::mbar_wait[^;{}]*;", _body(text, "convert_loop"))[:1]
+    for s in waits:
+        assert "warp_agrees(" in s, s
