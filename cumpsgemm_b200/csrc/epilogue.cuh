@@ -52,11 +52,6 @@ __device__ __forceinline__ void add_pair(unsigned long long &acc, uint32_t x, ui
   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(x), "r"(y));
   asm volatile("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(v));
 }
-__device__ __forceinline__ void scale_pair(unsigned long long &acc, float s) {
-  unsigned long long v;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(s));
-  asm volatile("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(v));
-}
 template <int CPT>
 __device__ __forceinline__ void drain_pairs(uint32_t taddr, unsigned long long (&acc)[CPT / 2]) {
 #pragma unroll
@@ -68,18 +63,45 @@ __device__ __forceinline__ void drain_pairs(uint32_t taddr, unsigned long long (
     for (int i = 0; i < 8; ++i) add_pair(acc[c / 2 + i], v[2 * i], v[2 * i + 1]);
   }
 }
-// acc + TMEM columns, left in the columns
-template <int CPT>
-__device__ __forceinline__ void finish_pairs_in_tmem(uint32_t taddr,
-                                                     unsigned long long (&acc)[CPT / 2]) {
+// acc += s * TMEM columns, which lie in runs of RUN, a run every STEP columns
+template <int CPT, int RUN, int STEP>
+__device__ __forceinline__ void add_corrections_to_pairs(uint32_t taddr,
+                                                         unsigned long long (&acc)[CPT / 2], float s) {
+  unsigned long long s2;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(s2) : "f"(s));
+#pragma unroll
+  for (int c = 0; c < CPT; c += 16) {
+    uint32_t v[16];
+    ptx::tmem_ld_32x32b_x16(taddr + c / RUN * STEP + c % RUN, v);
+    ptx::tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      unsigned long long x;
+      asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "r"(v[2 * i]), "r"(v[2 * i + 1]));
+      asm volatile("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[c / 2 + i]) : "l"(x), "l"(s2));
+    }
+  }
+}
+// acc + TMEM columns + s * corrections, left in the columns (the corrections as above)
+template <int CPT, int RUN, int STEP>
+__device__ __forceinline__ void finish_pairs_in_tmem(uint32_t taddr, uint32_t t_cor,
+                                                     unsigned long long (&acc)[CPT / 2], float s) {
+  unsigned long long s2;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(s2) : "f"(s));
 #pragma unroll
   for (int c = 0; c < CPT; c += 16) {
     uint32_t v[16];
     ptx::tmem_ld_32x32b_x16(taddr + c, v);
     ptx::tmem_ld_wait();
 #pragma unroll
+    for (int i = 0; i < 8; ++i) add_pair(acc[c / 2 + i], v[2 * i], v[2 * i + 1]);
+    ptx::tmem_ld_32x32b_x16(t_cor + c / RUN * STEP + c % RUN, v);
+    ptx::tmem_ld_wait();
+#pragma unroll
     for (int i = 0; i < 8; ++i) {
-      add_pair(acc[c / 2 + i], v[2 * i], v[2 * i + 1]);
+      unsigned long long x;
+      asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "r"(v[2 * i]), "r"(v[2 * i + 1]));
+      asm volatile("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[c / 2 + i]) : "l"(x), "l"(s2));
       asm("mov.b64 {%0, %1}, %2;" : "=r"(v[2 * i]), "=r"(v[2 * i + 1]) : "l"(acc[c / 2 + i]));
     }
     ptx::tmem_st_32x32b_x16(taddr + c, v);

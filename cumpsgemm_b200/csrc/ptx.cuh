@@ -489,22 +489,6 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, ui
       : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "n"(CG)
       : "memory");
 }
-// D[tmem] = A * B + D * 2^-SHIFT; kind::f16, A in tensor memory
-template <int CG, int SHIFT>
-__device__ __forceinline__ void mma_f16_ts_scaled(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                                  uint32_t idesc) {
-  static_assert(SHIFT >= 0 && SHIFT <= 15, "range of scale-input-d");
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.eq.b32 p, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::%5.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t"
-      "}\n"
-      :
-      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(SHIFT), "n"(CG)
-      : "memory");
-}
-
 // ---------------------------------------------------------------- descriptors
 // Shared-memory matrix descriptor for a K-major operand tile whose rows are
 // `SWIZZLE_BYTES` long (one swizzle atom wide) and stored densely, 8-row

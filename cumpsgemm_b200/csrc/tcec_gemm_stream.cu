@@ -7,33 +7,36 @@
 //   * fetches its own 128 rows of op(A) and its own BN / 2 rows of op(B) as plain FP32 through TMA
 //     into a ring of raw slots (32 k values each; edges are zero filled by TMA, so no thread
 //     tests bounds),
-//   * has two teams of eight converter warps, which take the raw slots in turn and split the values
-//     into hi / lo (same bits as split_kernels.cu): A goes to tensor memory, lane = row, B to
-//     128-byte-swizzled K-major tiles in shared memory,
-//   * and holds its 128 rows of the accumulators in tensor memory, which its eight epilogue warps
-//     drain after every stage (64 FP16 / 32 TF32 values of k) into FP32 running sums in registers.
+//   * has sixteen converter warps, which split the raw values into hi / lo (same bits as
+//     split_kernels.cu) and write them as 128-byte-swizzled K-major tiles in shared memory, with 128
+//     columns A's to tensor memory instead, lane = row,
+//   * and holds its 128 rows of the accumulators in tensor memory: those of hi*hi, one per half of the
+//     tile's columns, which its eight epilogue warps drain after every stage (64 FP16 / 32 TF32 values
+//     of k) into FP32 running sums in registers, and those of the corrections lo*hi + hi*lo, which are
+//     read once, at the end of the tile.
 // The even CTA's single issuing thread drives the tensor cores of both SMs (cta_group::2).
 //
-// One accumulator per half of the tile's columns takes all three products of a stage: first the
-// corrections lo*hi + hi*lo, then hi*hi, whose first instruction scales what is there by 2^-11
-// (scale-input-d; TF32's lo is not scaled).  With accumulators of their own for the corrections and A
-// in shared memory, tensor memory was full and the tensor core read A three times and B three times
-// per stage through the shared-memory port, on top of TMA's and the converters' traffic: 2304 of the
-// 2570 cycles a stage of 64 k values took.  Now the port has 1664 to do, the corrections no longer hold
-// the next tile up, and three accumulators (BN = 128: four) of half a tile rotate.  Where K fits
-// one unit of 64 the corrections keep an accumulator of their own (kSeparate): adding them inside the
-// tensor core would truncate the one sum there is, 1.6e-7 instead of 6e-8 for k = 1.
+// The corrections have accumulators of their own because the tensor core truncates what it adds, and
+// aligns the products of FP16 numbers below 2^-14 as if they were larger.  Added to hi*hi there (scaled by
+// 2^-11 on the way, which would leave room for A in tensor memory with 256 columns too) they
+// cost 2 to 6 % less time and lost bits wherever few products make up a sum: with one non-zero per row of
+// A the mean of the relative errors was -3.5e-8 instead of 0, and with small elements in B
+// the largest one 4e-6 instead of 4.5e-7.  (Draining both kinds every stage instead takes 1.5 times as long.)
+// The issue order hides the drain of one stage behind the corrections of the next; a finished tile's
+// corrections are given back before its stores.
 //
-// What bounds it: the instructions of the converters and the epilogue, and the power.  Cycles per stage of
-// 64 k values, m = n = k = 2048, 256 columns: 2570 before, 2100 now (1536 are tensor-core work; of
-// the issuer's 2100 it waits 860 for operands and 420 for accumulators); 128 columns 2310 -> 1520.
-// That took, each alone worth little and together the difference: the second converter team, the
-// epilogue's adds two at a time, a split in six instead of eight instructions per pair, and loops that
-// keep few enough registers not to spill.  Measured per call, before / now (us): 2048 x 1024 x 2048 with
-// 128 columns 47.8 / 34.2, complex 1280 x 960 x 1500 66 / 59, 2048^3 53.3 / 49.4, 512 x complex 256^3
-// 241 / 225 (beta = 0.5 328 / 289), 512 x 256^3 82 / 76, TF32TCEC 512 x 256^3 112 / 104, 256 x 256 x
-// 65536 50.0 / 47.6.  Errors against 64-bit products are equal or smaller (k = 96 ... 65536: 1.13e-7 ->
-// 1.11e-7, 2048: 1.598e-7 -> 1.581e-7; k <= 64: the same).
+// What bounds it: with 256 columns shared memory.  Per stage of 64 k values it takes 64 KiB from TMA,
+// gives 64 KiB to the converters, takes 64 KiB of hi / lo tiles back and feeds 112 KiB to the tensor
+// core (A_hi once more for either half): 2432 cycles at 128 bytes a cycle, for 1536 of tensor-core work.
+// With 128 columns the instructions of the converters and the epilogue (with A in tensor memory the port
+// has 1088 cycles to do, and the tensor core 768).  Two rules of the code below matter as much:
+// sums are added two at a time (packed), and whatever is live in the loop over the stages besides the 128
+// sums is little; a variant that kept all sums in registers up to the end of the tile spilled some
+// of them and took 81 us for 2048^3 instead of 53.  Measured per call (us, 256 columns / 128): 2048^3
+// 52.8 / 61.0, 2048 x 1024 x 2048 40.9 / 34.1, complex 1280 x 960 x 1500 57.8 / 63.1, 512 x complex 256^3
+// 234 / 339 (beta = 0.5 309 / 420), 512 x 256^3 83 / 105, TF32TCEC 107 / 147, 256 x 256 x 65536 51 / 49.
+// One team of eight converter warps, A in shared memory and sums added one by one took 53.3 and
+// 47.8 us for the first two in their better width.
 //
 // Work distribution: work_list.cuh.  What is left over from whole waves (total mod clusters, or
 // everything when there are fewer tiles than clusters) can be cut along K; piece_fixup.cu then
@@ -46,17 +49,18 @@
 //
 // Barriers (per CTA, same shared-memory offsets; "leader" = even CTA):
 //   raw_full[r]    1 arrival (producer, expect_tx) + TMA bytes      own CTA
-//   raw_empty[r]   8 arrivals, one per warp of the slot's team      own CTA
+//   raw_empty[r]   8 or 16 arrivals, the slot's converter warps    own CTA
 //   full[s]        leader's only: the converter warps of both CTAs
-//   empty[e]       tcgen05.commit multicast from the leader         both CTAs
-//   d_full[f]      the same, after the products of one half of the columns
+//   empty[s]       tcgen05.commit multicast from the leader         both CTAs
+//   d_full[b]      the same, after hi*hi of one half of the columns
 //   d_empty[b]     leader's only: 8 arrivals, the epilogue warps of that half in both CTAs
+//   d1_empty       leader's only: 16 arrivals, the epilogue warps of both CTAs
 // A wait tells phases apart by one bit, so whoever waits on a barrier looks at each of its phases, and
 // before the next one can end: one that passed over a phase could take the phase before it for the one
 // it wants, and nothing says that arrivals on different barriers are seen in the order they were sent.
-// So the number of raw slots is even (a slot belongs to one team), either half of the columns has
-// d_full barriers of its own, and where the teams share an odd number of stages in turn (TF32TCEC on
-// single CTAs) each has empty barriers of its own.  Every wait is bounded; no TMA multicast is used.
+// So the numbers of stages and accumulators are even (each belongs to one team, one half of the columns),
+// and where the number of raw slots is not, every converter warp has a share of each slot.  Every
+// wait is bounded; no TMA multicast is used.
 #include "epilogue.cuh"
 #include "gemm_common.cuh"
 #include "ptx.cuh"
@@ -102,27 +106,31 @@ struct StreamParams {
 };
 static_assert(sizeof(StreamParams) <= 128, "kernel parameter structs stay within 128 bytes");
 constexpr uint32_t kIsComplex = 1, kConjA = 2, kConjB = 4, kBatchA = 8, kBatchB = 16,
-                   kDirectStores = 32, kSeparate = 64;
+                   kDirectStores = 32;
 
 // CG: CTAs of a cluster, 2 (a pair shares a 256-row tile) or 1 (128 rows).
 template <int BN, int CG> struct StreamCfg {
   static constexpr int B_ROWS = BN / CG;         // rows of op(B) per CTA: two blocks of HALF_ROWS,
   static constexpr int HALF_ROWS = BN / 2 / CG;  // one for each half of the tile's columns
-  static constexpr int B_TILE = B_ROWS * ROW_BYTES;
-  static constexpr int STAGE_BYTES = 2 * B_TILE; // hi, lo
-  static constexpr int STAGES = (BN == 256) ? 2 : (CG == 1) ? 3 : 4;
+  // 128 columns: A in tensor memory.  256: the accumulators take all of it, and A is in shared memory.
+  static constexpr bool A_IN_TMEM = BN == 128;
+  static constexpr int A_TILE = BM_CTA * ROW_BYTES, B_TILE = B_ROWS * ROW_BYTES;
+  static constexpr int A_BYTES = A_IN_TMEM ? 0 : 2 * A_TILE; // of a stage: hi, lo; those of B behind it
+  static constexpr int STAGE_BYTES = A_BYTES + 2 * B_TILE;
+  static constexpr int STAGES = 2;
   static constexpr int RAW_A = BM_CTA * SLOT_K * 4;
   static constexpr int RAW_HALF_B = HALF_ROWS * SLOT_K * 4;
   static constexpr int RAW_BYTES = RAW_A + 2 * RAW_HALF_B;
-  static constexpr int RAW_SLOTS = (B_ROWS == 128) ? 4 : 6;
+  static constexpr int RAW_SLOTS = (BN == 256) ? 3 : (CG == 1) ? 4 : 6;
+  // An even number of slots: the two converter teams take them in turn; otherwise every warp has a
+  // share of each.
+  static constexpr int SLOT_TEAMS = (RAW_SLOTS % 2 == 0) ? 2 : 1;
+  static constexpr int SLOT_WARPS = CVT_TEAMS / SLOT_TEAMS * TEAM_WARPS;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + RAW_SLOTS * RAW_BYTES + 1024 + 256;
-  // Tensor memory: accumulators of half a tile's columns each, then A, 64 columns per stage (hi, lo)
-  static constexpr uint32_t D_BUFS = (BN == 256) ? 3 : 4;
-  // An accumulator that serves both halves of the columns in turn has a d_full barrier for each, and
-  // a stage that both teams use in turn has two empty barriers, committed to in turn.
-  static constexpr uint32_t D_FULL_BARS = (D_BUFS % 2 == 0) ? D_BUFS : 2 * D_BUFS;
-  static constexpr uint32_t EMPTY_BARS = (STAGES % 2 == 0) ? STAGES : 2 * STAGES;
-  static constexpr uint32_t A_COL = D_BUFS * (BN / 2);
+  // Tensor memory: accumulators for hi*hi of half a tile's columns each, the corrections of the whole
+  // tile, then A, 64 columns per stage (hi, lo)
+  static constexpr uint32_t D_BUFS = (BN == 256) ? 2 : 4;
+  static constexpr uint32_t D1_COL = D_BUFS * (BN / 2), A_COL = D1_COL + BN;
   static constexpr int REGS_EPI = (BN == 256) ? 152 : 112;
   static constexpr int REGS_CVT = (BN == 256) ? 40 : 48;
   static constexpr int REGS_REST = (BN == 256) ? 40 : 72;
@@ -132,13 +140,13 @@ template <int BN, int CG> struct StreamCfg {
                 "setmaxnreg.inc goes up, setmaxnreg.dec down: anything else is an illegal instruction");
   // Barriers behind the raw slots, as byte offsets: eight bytes each
   static constexpr uint32_t RAW_FULL = 0, RAW_EMPTY = 8 * RAW_SLOTS, FULL = RAW_EMPTY + 8 * RAW_SLOTS,
-                            EMPTY = FULL + 8 * STAGES, D_FULL = EMPTY + 8 * EMPTY_BARS,
-                            D_EMPTY = D_FULL + 8 * D_FULL_BARS, TMEM_PTR = D_EMPTY + 8 * D_BUFS,
-                            ABORT = TMEM_PTR + 4;
+                            EMPTY = FULL + 8 * STAGES, D_FULL = EMPTY + 8 * STAGES,
+                            D_EMPTY = D_FULL + 8 * D_BUFS, D1_EMPTY = D_EMPTY + 8 * D_BUFS,
+                            TMEM_PTR = D1_EMPTY + 8, ABORT = TMEM_PTR + 4;
   static_assert(ABORT + 4 <= 256, "barriers");
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
-  static_assert(RAW_SLOTS % CVT_TEAMS == 0, "a raw slot belongs to one team");
-  static_assert(A_COL + STAGES * 64 <= 512, "tensor memory");
+  static_assert(STAGES % 2 == 0 && D_BUFS % 2 == 0, "a stage belongs to one team, a buffer to one half");
+  static_assert(A_COL + (A_IN_TMEM ? STAGES * 64 : 0) <= 512, "tensor memory");
 };
 constexpr uint32_t A_STAGE_COLS = 64, A_LO_COLS = 32, TMEM_COLS = 512;
 
@@ -159,11 +167,18 @@ __device__ __forceinline__ TileCoord tile_coord(uint32_t tile, const StreamParam
   return c;
 }
 
-template <int KIND, int CG>
-__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc,
-                                       uint32_t acc) {
-  if constexpr (KIND == 0) ptx::mma_f16_ts<CG>(d, a, b, idesc, acc);
-  else ptx::mma_tf32_ts<CG>(d, a, b, idesc, acc);
+// One product over 32 bytes of K: step ks of the 128 bytes that `a` and `b` begin (a: a tensor-memory
+// address or, like b, a descriptor).
+template <int KIND, int CG, typename A>
+__device__ __forceinline__ void mma(uint32_t d, A a, uint64_t b, int ks, uint32_t idesc, uint32_t acc) {
+  if constexpr (sizeof(A) == 4) {
+    if constexpr (KIND == 0) ptx::mma_f16_ts<CG>(d, a + 8 * ks, b + 2 * ks, idesc, acc);
+    else ptx::mma_tf32_ts<CG>(d, a + 8 * ks, b + 2 * ks, idesc, acc);
+  } else {
+    static_assert(CG == 2, "A in shared memory: pairs only");
+    if constexpr (KIND == 0) ptx::mma_f16_ss_pair(d, a + 2 * ks, b + 2 * ks, idesc, acc);
+    else ptx::mma_tf32_ss_pair(d, a + 2 * ks, b + 2 * ks, idesc, acc);
+  }
 }
 template <int CG> __device__ __forceinline__ void commit(uint32_t bar) {
   if constexpr (CG == 2) ptx::tc_commit_pair(bar, 0x3);
@@ -184,8 +199,8 @@ struct ConverterState {
   uint32_t bars_leader; // shared::cluster address of the leader's
   uint32_t raw;         // shared address of slot 0's raw tile
   uint32_t row;         // this lane's row of the raw tile
-  uint32_t dst;         // stage 0's hi values of the lane's row: shared address of the (swizzled) row
-                        // for B, the warp's tensor-memory address for A
+  uint32_t dst;         // stage 0's hi values of the lane's row: shared address of the (swizzled) row,
+                        // or the warp's tensor-memory address
   uint32_t team;
   uint32_t group0;      // first of the warp's 8-k groups in a slot
   float scale;
@@ -241,10 +256,10 @@ __device__ __forceinline__ void load_raw8(uint32_t lane_addr, uint32_t g, const 
 }
 
 // Splits eight consecutive k values and stores them at 8-k group kc of the stage: A in tensor
-// memory, B in shared memory.
-template <int KIND, int BN, int CG, bool IS_A>
+// memory where it goes there, else in shared memory.
+template <int KIND, int LO_DELTA, bool TO_TMEM>
 __device__ __forceinline__ void split_store8(const float (&v)[8], uint32_t dst, uint32_t kc) {
-  if constexpr (IS_A && KIND == 1) {
+  if constexpr (TO_TMEM && KIND == 1) {
     uint32_t h[8], l[8];
 #pragma unroll
     for (int t = 0; t < 8; ++t) split_tf32(v[t], h[t], l[t]);
@@ -262,13 +277,13 @@ __device__ __forceinline__ void split_store8(const float (&v)[8], uint32_t dst, 
       else split_tf32(v[4 * g + t], h[t], l[t]);
     }
     const uint32_t q = VECS * kc + g;
-    if constexpr (IS_A) {
+    if constexpr (TO_TMEM) {
       ptx::tmem_st_32x32b_x4(dst + 4u * q, h);
       ptx::tmem_st_32x32b_x4(dst + A_LO_COLS + 4u * q, l);
     } else {
       const uint32_t addr = dst ^ (q << 4);
       st_shared_v4(addr, h[0], h[1], h[2], h[3]);
-      st_shared_v4(addr + StreamCfg<BN, CG>::B_TILE, l[0], l[1], l[2], l[3]);
+      st_shared_v4(addr + LO_DELTA, l[0], l[1], l[2], l[3]);
     }
   }
 }
@@ -277,7 +292,10 @@ template <int KIND, int BN, int CG, int LAYOUT, int ROWS, int JOBS, bool IS_A>
 __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterState &st) {
   using Cfg = StreamCfg<BN, CG>;
   constexpr uint32_t SLOTS_PER_STAGE = (KIND == 0) ? 2 : 1;
-  constexpr uint32_t STAGE_STEP = 2 / SLOTS_PER_STAGE; // stages from a team's slot to its next
+  constexpr bool TO_TMEM = IS_A && Cfg::A_IN_TMEM;
+  constexpr bool IN_TURN = Cfg::SLOT_TEAMS == 2;
+  // stages from a warp's slot to its next one (in turn: a team's); a stage of two slots is passed in two
+  constexpr uint32_t STAGE_STEP = IN_TURN ? 2 / SLOTS_PER_STAGE : 1;
   const uint32_t r = st.row;
   const int lane = static_cast<int>(threadIdx.x & 31);
   uint32_t lane_raw;
@@ -287,30 +305,29 @@ __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterSta
   else if constexpr (LAYOUT == kRawCplxAR) lane_raw = st.raw + (r >> 1) * 8u;
   else lane_raw = st.raw + (r >> 1) * 128u + (((r >> 1) & 7u) << 4);
   const bool scaled = st.scale != 1.f;
-  uint32_t rs = st.team, rph = 0;
-  // index in the stream of stages; barrier and parity of the release of the stage's previous use
-  uint32_t i = (KIND == 0) ? 0u : st.team;
-  uint32_t e = (i + Cfg::STAGES) % Cfg::EMPTY_BARS, e_ph = 1;
+  uint32_t rs = IN_TURN ? st.team : 0u, rph = 0;
+  // index in the stream of stages; the stage, and parity of the release of its previous use
+  uint32_t i = (KIND == 1 && IN_TURN) ? st.team : 0u;
+  uint32_t s = i, e_ph = 1;
   auto next = [&]() {
     i += STAGE_STEP;
-    e += STAGE_STEP;
-    if (e >= Cfg::EMPTY_BARS) {
-      e -= Cfg::EMPTY_BARS;
+    s += STAGE_STEP;
+    if (s >= Cfg::STAGES) {
+      s -= Cfg::STAGES;
       e_ph ^= 1u;
     }
   };
-  const uint32_t kc0 = st.group0 + ((KIND == 0) ? 4u * st.team : 0u);
+  uint32_t second = (KIND == 0 && IN_TURN) ? st.team : 0u; // the slot is the second of its stage
 #pragma unroll 1
-  for (; i < total_stages; next()) {
-    const uint32_t s = (Cfg::EMPTY_BARS > Cfg::STAGES && e >= Cfg::STAGES) ? e - Cfg::STAGES : e;
+  while (i < total_stages) {
     if (!ptx::warp_agrees(ptx::mbar_wait_s(st.bars + Cfg::RAW_FULL + 8u * rs, rph,
                                            st.bars + Cfg::ABORT, st.status, ptx::kErrWaitFull) &&
-                          ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * e, e_ph, st.bars + Cfg::ABORT,
+                          ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * s, e_ph, st.bars + Cfg::ABORT,
                                            st.status, ptx::kErrWaitEmpty)))
       return;
-    if constexpr (IS_A) ptx::tc_fence_after();
+    if constexpr (TO_TMEM) ptx::tc_fence_after();
     const uint32_t raw_addr = lane_raw + rs * Cfg::RAW_BYTES;
-    const uint32_t dst = st.dst + s * (IS_A ? A_STAGE_COLS : static_cast<uint32_t>(Cfg::STAGE_BYTES));
+    const uint32_t dst = st.dst + s * (TO_TMEM ? A_STAGE_COLS : static_cast<uint32_t>(Cfg::STAGE_BYTES));
 #pragma unroll
     for (int j = 0; j < JOBS; ++j) {
       float v[8];
@@ -319,9 +336,9 @@ __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterSta
 #pragma unroll
         for (int t = 0; t < 8; ++t) v[t] *= st.scale;
       }
-      split_store8<KIND, BN, CG, IS_A>(v, dst, kc0 + j);
+      split_store8<KIND, IS_A ? Cfg::A_TILE : Cfg::B_TILE, TO_TMEM>(v, dst, 4u * second + st.group0 + j);
     }
-    if constexpr (IS_A) {
+    if constexpr (TO_TMEM) {
       ptx::tmem_st_wait();
       ptx::tc_fence_before();
     } else {
@@ -333,17 +350,22 @@ __device__ __forceinline__ void convert_loop(uint32_t total_stages, ConverterSta
       ptx::mbar_arrive(st.bars + Cfg::RAW_EMPTY + 8u * rs);
       ptx::mbar_arrive_cluster(st.bars_leader + Cfg::FULL + 8u * s);
     }
-    rs += CVT_TEAMS;
+    rs += Cfg::SLOT_TEAMS;
     if (rs >= Cfg::RAW_SLOTS) {
       rs -= Cfg::RAW_SLOTS;
       rph ^= 1u;
     }
+    if (KIND == 0 && !IN_TURN) {
+      second ^= 1u;
+      if (second != 0) continue;
+    }
+    next();
   }
   // the issuer's last commits arrive on this CTA's barriers: it must not be gone by then (TF32TCEC:
   // each team waits for those that it would go on with)
   for (; i < total_stages + Cfg::STAGES; next()) {
     if (i < Cfg::STAGES) continue; // (nothing was in it)
-    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * e, e_ph, st.bars + Cfg::ABORT, st.status,
+    if (!ptx::mbar_wait_s(st.bars + Cfg::EMPTY + 8u * s, e_ph, st.bars + Cfg::ABORT, st.status,
                           ptx::kErrWaitEmpty))
       return;
   }
@@ -357,7 +379,9 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   constexpr int K_STEPS = ROW_BYTES / 32;
   constexpr uint32_t SLOTS_PER_STAGE = (KIND == 0) ? 2 : 1;
   constexpr uint32_t STAGES_PER_UNIT = (KIND == 0) ? 1 : 2;
-  constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, CG * BM_CTA, BN / 2);
+  constexpr uint32_t IDESC = ptx::make_idesc(KIND == 0 ? 0 : 2, CG * BM_CTA, BN),
+                     IDESC_HALF = ptx::make_idesc(KIND == 0 ? 0 : 2, CG * BM_CTA, BN / 2);
+  constexpr float LO_SCALE_INV = (KIND == 0) ? (1.f / 2048.f) : 1.f;
   constexpr int CPT = BN / 2; // accumulator columns per epilogue thread
 
   extern __shared__ uint8_t smem_raw[];
@@ -377,16 +401,17 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   if (threadIdx.x == 0) {
     for (uint32_t r = 0; r < RAW_SLOTS; ++r) {
       ptx::mbar_init(bars + Cfg::RAW_FULL + 8u * r, 1);
-      ptx::mbar_init(bars + Cfg::RAW_EMPTY + 8u * r, TEAM_WARPS);
+      ptx::mbar_init(bars + Cfg::RAW_EMPTY + 8u * r, Cfg::SLOT_WARPS);
     }
     for (uint32_t s = 0; s < STAGES; ++s) {
-      ptx::mbar_init(bars + Cfg::FULL + 8u * s, CG * SLOTS_PER_STAGE * TEAM_WARPS);
+      ptx::mbar_init(bars + Cfg::FULL + 8u * s, CG * SLOTS_PER_STAGE * Cfg::SLOT_WARPS);
+      ptx::mbar_init(bars + Cfg::EMPTY + 8u * s, 1);
     }
-    for (uint32_t e = 0; e < Cfg::EMPTY_BARS; ++e) ptx::mbar_init(bars + Cfg::EMPTY + 8u * e, 1);
-    for (uint32_t f = 0; f < Cfg::D_FULL_BARS; ++f) ptx::mbar_init(bars + Cfg::D_FULL + 8u * f, 1);
     for (uint32_t b = 0; b < Cfg::D_BUFS; ++b) {
+      ptx::mbar_init(bars + Cfg::D_FULL + 8u * b, 1);
       ptx::mbar_init(bars + Cfg::D_EMPTY + 8u * b, CG * NUM_EPI_WARPS / 2);
     }
+    ptx::mbar_init(bars + Cfg::D1_EMPTY, CG * NUM_EPI_WARPS);
     st_shared_u32(abort_flag, 0u);
     ptx::mbar_init_fence();
     ptx::prefetch_tensormap(&map_a);
@@ -472,10 +497,8 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
         const uint64_t desc0 = ptx::make_kmajor_desc<ROW_BYTES>(ptx::smem_u32(smem));
         constexpr uint64_t kStage = Cfg::STAGE_BYTES >> 4, kLo = Cfg::B_TILE >> 4,
                            kHalf = (Cfg::HALF_ROWS * ROW_BYTES) >> 4;
-        uint32_t s = 0, ph = 0, b = 0, d_ph = 1;
-        uint32_t e = 0, f = 0; // the next empty and d_full barriers to commit to
+        uint32_t s = 0, ph = 0, b = 0, d_ph = 1, d1_ph = 1;
         bool ok = true;
-        const bool separate = (p.flags & kSeparate) != 0;
         auto wait_timed = [&](uint32_t bar, uint32_t parity, int code, uint32_t &cycles) {
           const uint32_t t0 = dbg ? static_cast<uint32_t>(clock()) : 0u;
           const bool r = ptx::mbar_wait_s(bar, parity, abort_flag, p.status, code);
@@ -491,7 +514,25 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
           for (uint32_t kb = 0; kb < kbn; ++kb) {
             ok = wait_timed(bars + Cfg::FULL + 8u * s, ph, ptx::kErrWaitFull, dbg_wait);
             if (!ok) break;
-            const uint32_t a_hi = tmem_base + Cfg::A_COL + s * A_STAGE_COLS, a_lo = a_hi + A_LO_COLS;
+            // (the item before this one: its corrections must have been read)
+            if (kb == 0)
+              ok = wait_timed(bars + Cfg::D1_EMPTY, d1_ph, ptx::kErrWaitD1Empty, dbg_wait2);
+            if (!ok) break;
+            ptx::tc_fence_after();
+            const uint64_t stage = desc0 + s * kStage;
+            const uint64_t b_hi = stage + (Cfg::A_BYTES >> 4), b_lo = b_hi + kLo;
+            const auto a_hi = [&]() {
+              if constexpr (Cfg::A_IN_TMEM) return tmem_base + Cfg::A_COL + s * A_STAGE_COLS;
+              else return stage;
+            }();
+            const auto a_lo = a_hi + (Cfg::A_IN_TMEM ? A_LO_COLS : Cfg::A_TILE >> 4);
+            // The corrections come first: behind them the sums of the stage before are drained.
+#pragma unroll
+            for (int ks = 0; ks < K_STEPS; ++ks)
+              mma<KIND, CG>(tmem_base + Cfg::D1_COL, a_lo, b_hi, ks, IDESC, (ks > 0 || kb > 0) ? 1u : 0u);
+#pragma unroll
+            for (int ks = 0; ks < K_STEPS; ++ks)
+              mma<KIND, CG>(tmem_base + Cfg::D1_COL, a_hi, b_lo, ks, IDESC, 1u);
             // the previous sums of these columns must have been drained (at the end of an item:
             // stored)
             auto next_buffer = [&]() {
@@ -500,62 +541,29 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
               return tmem_base + b * CPT;
             };
             auto filled = [&]() {
-              commit<CG>(bars + Cfg::D_FULL + 8u * (Cfg::D_FULL_BARS == Cfg::D_BUFS ? b : f));
-              if (++f == Cfg::D_FULL_BARS) f = 0;
+              commit<CG>(bars + Cfg::D_FULL + 8u * b);
               if (++b == Cfg::D_BUFS) {
                 b = 0;
                 d_ph ^= 1u;
               }
             };
-            const uint64_t b_hi0 = desc0 + s * kStage;
-            auto corrections = [&](uint32_t d, uint64_t b_hi) {
+#pragma unroll
+            for (uint32_t g = 0; g < 2; ++g) {
+              const uint32_t d = next_buffer();
+              if (!ok) break;
 #pragma unroll
               for (int ks = 0; ks < K_STEPS; ++ks)
-                mma_ts<KIND, CG>(d, a_lo + 8 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : 0u);
-#pragma unroll
-              for (int ks = 0; ks < K_STEPS; ++ks)
-                mma_ts<KIND, CG>(d, a_hi + 8 * ks, b_hi + kLo + 2 * ks, IDESC, 1u);
-            };
-            if (!separate) {
-              // per half of the columns: corrections, then hi*hi on top of them
-#pragma unroll
-              for (uint32_t g = 0; g < 2; ++g) {
-                const uint32_t d = next_buffer();
-                if (!ok) break;
-                const uint64_t b_hi = b_hi0 + g * kHalf;
-                corrections(d, b_hi);
-                if constexpr (KIND == 0) ptx::mma_f16_ts_scaled<CG, 11>(d, a_hi, b_hi, IDESC);
-                else mma_ts<KIND, CG>(d, a_hi, b_hi, IDESC, 1u);
-#pragma unroll
-                for (int ks = 1; ks < K_STEPS; ++ks)
-                  mma_ts<KIND, CG>(d, a_hi + 8 * ks, b_hi + 2 * ks, IDESC, 1u);
-                filled();
-              }
-            } else {
-              // the corrections of both halves, then hi*hi of both, in accumulators of their own
-#pragma unroll 1
-              for (uint32_t q = 0; q < 4; ++q) {
-                const uint32_t d = next_buffer();
-                if (!ok) break;
-                const uint64_t b_hi = b_hi0 + (q & 1u) * kHalf;
-                if (q < 2) {
-                  corrections(d, b_hi);
-                } else {
-#pragma unroll
-                  for (int ks = 0; ks < K_STEPS; ++ks)
-                    mma_ts<KIND, CG>(d, a_hi + 8 * ks, b_hi + 2 * ks, IDESC, ks > 0 ? 1u : 0u);
-                }
-                filled();
-              }
+                mma<KIND, CG>(d, a_hi, b_hi + g * kHalf, ks, IDESC_HALF, ks > 0 ? 1u : 0u);
+              filled(); // (behind an item's last products this tells of its corrections too)
             }
             if (!ok) break;
-            commit<CG>(bars + Cfg::EMPTY + 8u * (Cfg::EMPTY_BARS == STAGES ? s : e));
-            if (++e == Cfg::EMPTY_BARS) e = 0;
+            commit<CG>(bars + Cfg::EMPTY + 8u * s);
             if (++s == STAGES) {
               s = 0;
               ph ^= 1u;
             }
           }
+          d1_ph ^= 1u;
         }
         if (dbg) {
           atomicAdd(p.debug + 0, static_cast<unsigned long long>(dbg_wait));
@@ -568,10 +576,12 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
   } else if (warp >= FIRST_CVT_WARP) {
     // ================================================================ converters (both CTAs)
     ptx::setmaxnreg_dec<Cfg::REGS_CVT>();
-    // Two teams of eight warps take the raw slots in turn.  In a team warps 0-3 convert the four
-    // 32-row blocks of A, warps 4-7 those of B (64 rows: two warps to each of its two blocks,
-    // half of a slot's groups each).
-    constexpr int B_JOBS = (Cfg::B_ROWS == 128) ? 4 : 2;
+    // Two teams of eight warps take the raw slots in turn, or (three slots) half of each slot's groups.
+    // In a team warps 0-3 convert the four 32-row blocks of A, warps 4-7 those of B (64 rows: two
+    // warps to each of its two blocks, half of a slot's groups each).
+    constexpr int A_JOBS = (Cfg::SLOT_TEAMS == 2) ? 4 : 2;
+    constexpr int B_JOBS = (Cfg::B_ROWS == 128) ? A_JOBS : 2;
+    static_assert(Cfg::B_ROWS == 128 || Cfg::SLOT_TEAMS == 2, "who converts what");
     const uint32_t cw = static_cast<uint32_t>(warp - FIRST_CVT_WARP) & 7u;
     const bool for_a = cw < 4;
     // the converters see a plain stream of stages; only its length depends on the work items
@@ -589,15 +599,17 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     if (for_a) {
       st.row = cw * 32u + lane;
       st.group0 = 0;
-      st.dst = tmem_base + Cfg::A_COL + ((cw * 32u) << 16);
+      if constexpr (Cfg::A_IN_TMEM) st.dst = tmem_base + Cfg::A_COL + ((cw * 32u) << 16);
+      else st.dst = ptx::smem_u32(smem) + st.row * 128u + ((st.row & 7u) << 4);
     } else {
       const uint32_t half = (cw - 4u) >> 1; // of the tile's columns
       st.row = (Cfg::B_ROWS == 128 ? (cw & 1u) * 32u : 0u) + lane;
       st.group0 = (Cfg::B_ROWS == 128) ? 0u : 2u * (cw & 1u);
       st.raw += Cfg::RAW_A + half * Cfg::RAW_HALF_B;
       const uint32_t r = half * Cfg::HALF_ROWS + st.row;
-      st.dst = ptx::smem_u32(smem) + r * 128u + ((r & 7u) << 4);
+      st.dst = ptx::smem_u32(smem) + Cfg::A_BYTES + r * 128u + ((r & 7u) << 4);
     }
+    if (Cfg::SLOT_TEAMS == 1) st.group0 = 2u * st.team;
     st.scale = 1.f;
     if (p.dyn != nullptr) st.scale = for_a ? p.dyn->scale_a : p.dyn->scale_b;
     st.conj_mask = (p.flags & (for_a ? kConjA : kConjB)) ? 0x80000000u : 0u;
@@ -605,16 +617,16 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     if (for_a) {
       switch (p.layout_a) {
       case kRawK:
-        convert_loop<KIND, BN, CG, kRawK, BM_CTA, 4, true>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawK, BM_CTA, A_JOBS, true>(total_stages, st);
         break;
       case kRawR:
-        convert_loop<KIND, BN, CG, kRawR, BM_CTA, 4, true>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawR, BM_CTA, A_JOBS, true>(total_stages, st);
         break;
       case kRawCplxAR:
-        convert_loop<KIND, BN, CG, kRawCplxAR, BM_CTA, 4, true>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawCplxAR, BM_CTA, A_JOBS, true>(total_stages, st);
         break;
       default:
-        convert_loop<KIND, BN, CG, kRawCplxAK, BM_CTA, 4, true>(total_stages, st);
+        convert_loop<KIND, BN, CG, kRawCplxAK, BM_CTA, A_JOBS, true>(total_stages, st);
         break;
       }
     } else {
@@ -638,18 +650,18 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     const uint32_t half = static_cast<uint32_t>((warp - FIRST_EPI_WARP) >> 2); // of the columns
     const uint32_t t_base = tmem_base + ((static_cast<uint32_t>(warp & 3) * 32u) << 16);
 
-    uint32_t f = half, d_ph = 0; // d_full barrier and parity of the next stage
-    auto buffer = [&]() { // its accumulator
-      return (Cfg::D_FULL_BARS > Cfg::D_BUFS && f >= Cfg::D_BUFS) ? f - Cfg::D_BUFS : f;
-    };
-    auto give_back = [&]() {
+    uint32_t b = half, d_ph = 0; // accumulator and parity of the next stage
+    auto arrive = [&](uint32_t bar) { // at the leader
       ptx::tc_fence_before();
       __syncwarp();
-      if (ptx::elect_one()) ptx::mbar_arrive_cluster(ptx::map_to_cta(bars + Cfg::D_EMPTY + 8u * buffer(), 0));
+      if (ptx::elect_one()) ptx::mbar_arrive_cluster(ptx::map_to_cta(bars + bar, 0));
       __syncwarp();
-      f += 2u;
-      if (f >= Cfg::D_FULL_BARS) {
-        f -= Cfg::D_FULL_BARS;
+    };
+    auto give_back = [&]() {
+      arrive(Cfg::D_EMPTY + 8u * b);
+      b += 2u;
+      if (b >= Cfg::D_BUFS) {
+        b -= Cfg::D_BUFS;
         d_ph ^= 1u;
       }
     };
@@ -670,8 +682,7 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
     WorkList list(p.w, cluster_id, num_clusters);
     WorkItem x;
     while (ok && list.next(p.w, x)) {
-      const bool separate = (p.flags & kSeparate) != 0;
-      uint32_t left = x.un * (separate ? 2u * STAGES_PER_UNIT : STAGES_PER_UNIT); // stages to drain
+      uint32_t left = x.un * STAGES_PER_UNIT; // stages to drain
       if (left < C_PREFETCH_LEAD && (p.beta_r != 0.f || p.beta_i != 0.f)) prefetch_c(x.tile);
       unsigned long long acc[CPT / 2];
 #pragma unroll
@@ -680,27 +691,25 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
 #pragma unroll 1
       while (true) {
         if (left == C_PREFETCH_LEAD && (p.beta_r != 0.f || p.beta_i != 0.f)) prefetch_c(x.tile);
-        ok = ptx::warp_agrees(ptx::mbar_wait_s(bars + Cfg::D_FULL + 8u * f, d_ph, abort_flag, p.status,
+        ok = ptx::warp_agrees(ptx::mbar_wait_s(bars + Cfg::D_FULL + 8u * b, d_ph, abort_flag, p.status,
                                                ptx::kErrWaitD0Full));
         if (!ok) break;
         ptx::tc_fence_after();
         if (--left == 0) break; // the last ones are added below
-        drain_pairs<CPT>(t_base + buffer() * CPT, acc);
-        // (corrections in an accumulator of their own come first, and nothing else is in acc then
-        // but, in TF32, finished sums, whose corrections are not scaled)
-        if (KIND == 0 && separate) {
-#pragma unroll
-          for (int i = 0; i < CPT / 2; ++i) scale_pair(acc[i], 1.f / 2048.f);
-        }
+        drain_pairs<CPT>(t_base + b * CPT, acc);
         give_back();
       }
       if (!ok) break;
-      const uint32_t t_sums = t_base + buffer() * CPT;
+      // (a pair's columns come half from one CTA's rows of op(B), half from the other's)
+      const uint32_t t_cor = t_base + Cfg::D1_COL + half * Cfg::HALF_ROWS;
+      const uint32_t t_sums = t_base + b * CPT;
       if (BN == 128 && (p.flags & kDirectStores)) {
         // Many short tiles per cluster, C not read: stores straight from the registers.  That is
-        // long code, but it stays in the instruction cache from tile to tile, and D1 goes back to
+        // long code, but it stays in the instruction cache from tile to tile, and the columns go back to
         // the issuer before the stores instead of after them.
         drain_pairs<CPT>(t_sums, acc);
+        add_corrections_to_pairs<CPT, Cfg::HALF_ROWS, Cfg::B_ROWS>(t_cor, acc, LO_SCALE_INV);
+        arrive(Cfg::D1_EMPTY);
         give_back();
         float sums[CPT];
 #pragma unroll
@@ -717,9 +726,10 @@ __device__ __forceinline__ void stream_body(const CUtensorMap &map_a, const CUte
                              (p.flags & kIsComplex) != 0);
         continue;
       }
-      // the finished sums stay in the D1 columns; from here on they are read from there, and what
-      // the epilogue needs to know of the tile is worked out only now (epilogue.cuh)
-      finish_pairs_in_tmem<CPT>(t_sums, acc);
+      // the finished sums go back to the columns of the last ones; from here on they are read from
+      // there, and what the epilogue needs to know of the tile is worked out only now (epilogue.cuh)
+      finish_pairs_in_tmem<CPT, Cfg::HALF_ROWS, Cfg::B_ROWS>(t_sums, t_cor, acc, LO_SCALE_INV);
+      arrive(Cfg::D1_EMPTY);
       const bool part = x.un != p.w.units; // this item is a piece of a tile
       const TileCoord tc = tile_coord<BN, CG>(opaque(x.tile), p, rank);
       const uint32_t quarter = static_cast<uint32_t>(warp & 3);
@@ -917,7 +927,6 @@ cudaError_t launch_variant(const StreamGemmArgs &a, cudaStream_t stream) {
                                  (a.conj_b ? kConjB : 0) |
                                  (a.batch > 1 && a.a.stride != 0 ? kBatchA : 0) |
                                  (a.batch > 1 && a.b.stride != 0 ? kBatchB : 0));
-  if (a.k <= 64) p.flags |= kSeparate;
   const StreamPlan &plan = a.plan;
   if (plan.tile_n != BN || plan.tile_m != CG * BM_CTA || plan.total_tiles != p.tiles_m * p.tiles_n * a.batch ||
       plan.units != (a.k + 63) / 64)

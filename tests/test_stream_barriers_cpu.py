@@ -18,8 +18,9 @@ def _constants(bn, cg):
     """StreamCfg's integer constants for one pair of template arguments."""
     body = SOURCE[SOURCE.index("struct StreamCfg {"):]
     body = re.sub(r"//[^\n]*", "", body[:body.index("\n};")])
-    known = {"BN": bn, "CG": cg, "BM_CTA": 128, "ROW_BYTES": 128, "SLOT_K": 32}
-    for name, expr in re.findall(r"static constexpr (?:int|uint32_t) (\w+) = ([^;,]+);", body):
+    known = {"BN": bn, "CG": cg, "BM_CTA": 128, "ROW_BYTES": 128, "SLOT_K": 32, "CVT_TEAMS": 2,
+             "TEAM_WARPS": 8}
+    for name, expr in re.findall(r"static constexpr (?:int|uint32_t|bool) (\w+) = ([^;,]+);", body):
         expr = expr.replace("/", "//")
         while "?" in expr:                        # C's conditional, innermost last
             cond, rest = expr.split("?", 1)
@@ -67,7 +68,8 @@ def test_epilogue_halves_tell_the_phases_of_their_accumulators_apart(bn, cg):
 def test_converter_teams_tell_the_phases_of_their_stages_apart(bn, cg, kind):
     c = _constants(bn, cg)
     stages, bars = c["STAGES"], c.get("EMPTY_BARS", c["STAGES"])
-    step = 1 if kind == "fp16" else 2             # FP16: both teams fill a stage, TF32: in turn
+    # all warps fill every stage; or, TF32 with slots that the teams take in turn, one of two teams does
+    step = 1 if kind == "fp16" or c["SLOT_TEAMS"] == 1 else 2
     for total in ([1, 2, 3, 64, 65] if kind == "fp16" else [2, 4, 6, 8, 64]):
         last = set()
         for team in (0, 1):
@@ -81,5 +83,10 @@ def test_converter_teams_tell_the_phases_of_their_stages_apart(bn, cg, kind):
 
 
 @pytest.mark.parametrize("bn,cg", CONFIGS)
-def test_a_raw_slot_belongs_to_one_team(bn, cg):
-    assert _constants(bn, cg)["RAW_SLOTS"] % 2 == 0
+def test_a_raw_slot_belongs_to_one_team_or_to_all_warps(bn, cg):
+    c = _constants(bn, cg)
+    assert c["SLOT_TEAMS"] in (1, 2) and c["RAW_SLOTS"] % c["SLOT_TEAMS"] == 0
+    # slot u of the stream is refilled once its u-th use has been given back: each of its phases is seen
+    for team in range(c["SLOT_TEAMS"]):
+        uses = range(team, 64, c["SLOT_TEAMS"])
+        assert _phases_are_told_apart([(u, u + c["RAW_SLOTS"]) for u in uses], c["RAW_SLOTS"])
