@@ -792,7 +792,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) tcec_gemm_fused_kernel(const F
       // C(row, col) = alpha * acc + beta * C(row, col)
       float *cp = cbase + static_cast<uint64_t>(tc.n0 + col_base) * p.ldc;
       const bool plain = (ai == 0.f) && !read_c; // real scalar, C not read
-      if (plain && row_ok && tc.n0 + col_base + CPT <= p.n) {
+      // (the whole warp goes one way: the other one exchanges values between its lanes)
+      if (plain && __all_sync(0xffffffffu, row_ok) && tc.n0 + col_base + CPT <= p.n) {
         // the common case, kept as short as possible: the epilogue warps are the slowest
         // role of a short-K tile
 #pragma unroll

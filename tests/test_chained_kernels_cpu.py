@@ -55,3 +55,12 @@ def test_a_warp_that_waits_for_an_accumulator_goes_on_as_a_whole(source):
         waits += re.findall(r"[^;{}]*ptx::mbar_wait[^;{}]*;", _body(text, "convert_loop"))[:1]
     for s in waits:
         assert "warp_agrees(" in s, s
+
+
+def test_the_on_the_fly_kernel_chooses_its_stores_warp_by_warp():
+    """Its general epilogue exchanges values between the lanes of a warp: no lane may take the short one
+    by itself (a warp that holds the last rows of a matrix would wait for it without a limit)."""
+    body = _body((CSRC / "tcec_gemm_fused.cu").read_text(), "tcec_gemm_fused_kernel")
+    short = re.search(r"if \(plain\b([^{]*)\{", body).group(1)
+    assert "__shfl_xor_sync(0xffffffffu" in body and "__all_sync(0xffffffffu, row_ok)" in short
+    assert "row_ok" not in short.replace("__all_sync(0xffffffffu, row_ok)", "")
