@@ -5,10 +5,11 @@
 // (:549-605) and the AUTO / FP16TCEC_SCALING orchestration of the
 // interception layer (src/cumpsgemm_cublas.cu:445-577, :829-961).
 //
-// A call takes one of three routes, all on the handle's stream: split pass -> tcgen05 GEMM on the
-// panels (tcec_gemm.cu, tcec_gemm_pair.cu), one kernel on CTA pairs that splits its operands behind
-// TMA (tcec_gemm_stream.cu), or one on single CTAs that loads and splits them itself
-// (tcec_gemm_fused.cu); tiles cut along K are added by one more launch.  The reference's module
+// A call takes one of these routes, all on the handle's stream: split pass -> tcgen05 GEMM on the
+// panels, on single CTAs (tcec_gemm.cu) or pairs (tcec_gemm_pair.cu); one kernel on CTA pairs or single
+// CTAs that splits its operands behind TMA (tcec_gemm_stream.cu); for small products one that loads
+// and splits them itself (tcec_gemm_small.cu).  Tiles cut along K are added by one more launch.  (A fifth
+// kernel, tcec_gemm_fused.cu, runs only where a switch asks for it.)  The reference's module
 // table (364 instantiations per arch, src/instance_sm80.cu) collapses to a few tile widths because
 // op N/T/C, leading dimensions and edges are absorbed where the operands are split.
 #include "gemm_common.cuh"
@@ -79,33 +80,33 @@ template <> struct Scalar<cuComplex> {
 
 // ---------------------------------------------------------------- which kernel
 //
-// Estimated time of a call on the pre-split and the streaming paths, in microseconds.  (The
-// on-the-fly kernel is not among them: it has rules of its own, see fused_args, and where they let
-// it in it is taken whenever streaming is not, whatever the pre-split path is estimated to take.)  A
-// call is one or more waves of tiles,
-// each as long as its K loop; what the paths trade is idle SMs against operand traffic, the split
-// pass against converting every operand element once per tile that uses it, and cutting tiles
-// along K against adding the pieces.  The constants are least-squares fits to 104 problems of
-// 1-80 pair tiles and k = 128-8192 with every path forced in turn (B200, mean error 5-9 %);
-// taking the path with the smallest estimate was 0.5 % slower on average than the best path of
-// each problem, the fixed rule it replaces 7 %.  Beyond that range of k an estimate only has to put
-// the paths in the right order: operands that come from DRAM at a long row pitch are not modelled
-// (256 x 256 x 65536 streams in 46 us, estimated 33).  Examples, us per call (K slices of 128 x 256
-// tiles / 128 x 128 tiles / pairs in K pieces / streaming):
-//   2048 x 1024 x 2048     43 / 30 / 37 / 40        464 x 3256 x 7240      113 / 102 / 98 / 80
-//   1536 x 1536 x 4096     69 / 58 / 63 / 62        512 x 4096 x 4096       77 / 64 / 67 / 62
-//   complex 1280 x 960 x 1500  - / 75 / 65 / 70     TF32TCEC 4096 x 1024 x 2048  - / 104 / 95 / 82
+// Estimated time of a call on the pre-split and the streaming paths, in microseconds.  A call is
+// one or more waves of tiles, each as long as its K loop; what the paths trade is idle SMs against
+// operand traffic, the split pass against converting every operand element once per tile that
+// uses it, and cutting tiles along K against adding the pieces.
+//
+// Two steps.  single(), pair() and split_k() choose the tile of the pre-split path; they are fits to 104
+// problems of 1-80 pair tiles and k = 128-8192 (B200, mean error 5-9 %), and leave out what all tiles
+// have in common.  presplit_call() adds that, and the call goes where it is estimated to end first.
+// What it adds, and the estimates of streaming, are fits to 580 random problems in each of FP16TCEC and TF32TCEC
+// with every path forced in turn: single products of 1-111 pair tiles (m, n 32-4096, k 128-131072)
+// and batches of 8-2048 (m, n 16-1024, k 32-2048), real and complex, every op, beta = 0 and 0.5,
+// operands on 16 bytes; the GPU's time in runs of twelve calls.  Mean error on as many others: 10 % pre-split, 5-7 %
+// streaming.  On 1150 calls drawn once more, choosing by these estimates was 0.5 % slower than the best
+// path of each (largest 1.38); the constants before, fitted to fewer sizes and to no batches, lost 1 to 10 %
+// by kind of problem there (10 % in batches of 8-48 matrices of at most 128 rows, largest 1.9).
 // A unit of 64 k values is one stage in FP16TCEC and two in TF32TCEC, for all paths alike.
 struct PathModel {
   double units, stages, sms, pairs;
-  double split; // megabytes the split pass reads and writes
-  std::uint64_t m, n, batch;
+  double split; // megabytes the split pass reads and writes, without padding
+  double c_passes; // over C: 2 if it is read too
+  std::uint64_t m, n, k, batch;
 
   static double waves(std::uint64_t tiles, double slots) { return std::ceil(tiles / slots); }
-  PathModel(unsigned num_sms, std::uint64_t m_, std::uint64_t n_, std::uint64_t k,
-            std::uint64_t batch_, bool tf32)
-      : units(static_cast<double>((k + 63) / 64)), stages(tf32 ? 2 * units : units), sms(num_sms),
-        pairs(num_sms / 2), m(m_), n(n_), batch(batch_) {
+  PathModel(unsigned num_sms, std::uint64_t m_, std::uint64_t n_, std::uint64_t k_,
+            std::uint64_t batch_, bool tf32, bool reads_c = false)
+      : units(static_cast<double>((k_ + 63) / 64)), stages(tf32 ? 2 * units : units), sms(num_sms),
+        pairs(num_sms / 2), c_passes(reads_c ? 2.0 : 1.0), m(m_), n(n_), k(k_), batch(batch_) {
     split = 1e-6 * static_cast<double>(m + n) * k * batch * (tf32 ? 12 : 8);
   }
   std::uint64_t tiles(std::uint64_t bm, std::uint64_t bn) const {
@@ -133,22 +134,35 @@ struct PathModel {
     return 2.0 + 0.15 * split + 1.32 * std::ceil(stages / slices) +
            0.69e-6 * 4 * static_cast<double>(m) * n * batch * slices;
   }
-  // tcec_gemm_stream.cu on single CTAs, 128 x 128 tiles (16 x 128 x 128 x 4096 65 us, estimated 67)
-  double stream_solo(const StreamPlan &pl) const {
-    return 9.0 + waves(pl.total_tiles, sms) * units * (stages > units ? 1.62 : 0.90);
+  // The whole call, `t` being the estimate its tile (tile_m x tile_n) was chosen by.  Beyond that: the rows and k
+  // values that pad the panels, the stores of every wave, and where pieces of pair tiles are laid end to end, two
+  // to park for every pair instead of one.
+  double presplit_call(double t, int tile_m, int tile_n, double waves_of_tiles, double parked) const {
+    const auto up = [](std::uint64_t v, std::uint64_t q) { return static_cast<double>((v + q - 1) / q * q); };
+    const double lo_hi = stages > units ? 8e-6 : 4e-6;
+    const double padding = lo_hi * batch * ((up(m, tile_m) + up(n, tile_n)) * up(k, 64) -
+                                            static_cast<double>(m + n) * static_cast<double>(k));
+    return t + 0.2 * padding + 0.8 * c_passes * waves_of_tiles * (tile_n / 128.0) + 0.3 * parked;
   }
-  // tcec_gemm_stream.cu.  (Fitted to 35 problems of 1-110 tiles and k = 96-32768 in each kind, mean
-  // error 5-9 %.  Examples, us, 256 / 128 columns: 2048 x 1024 x 2048 FP16TCEC 48 / 41, complex
-  // 1280 x 960 x 1500 61 / 66, 256 x 256 x 8192 23 / 18; TF32TCEC 4096 x 1024 x 2048 86 / 115.)
+  // tcec_gemm_stream.cu on single CTAs, 128 x 128 tiles
+  double stream_solo(const StreamPlan &pl) const {
+    const double busy = std::min(1.0, pl.total_tiles / sms), a = stages > units ? 1.62 : 0.83;
+    return 4.0 + waves(pl.total_tiles, sms) * (units * (a + 0.24 * busy) + 1.7 * c_passes);
+  }
+  // tcec_gemm_stream.cu on pairs
   double stream(const StreamPlan &pl) const {
     const bool tf32 = stages > units, wide = pl.tile_n == 256;
-    double length = waves(pl.whole_tiles, pairs) * units, t = 9.0;
+    const double busy =
+        std::min(1.0, std::max<double>(pl.whole_tiles, pl.piece_clusters) / pairs);
+    const double unit = wide ? (tf32 ? 1.90 + 0.63 * busy : 0.96 + 0.52 * busy)
+                             : (tf32 ? 1.39 + 0.39 * busy : 0.62 + 0.30 * busy);
+    const double w = waves(pl.whole_tiles, pairs);
+    double t = (wide ? 6.5 : 6.0) + w * (units * unit + (wide ? 2.2 : 1.55) * c_passes);
     if (pl.piece_clusters > 0) {
       const double left = pl.total_tiles - pl.whole_tiles;
-      length += std::ceil(left * units / pl.piece_clusters);
-      t += 4.9 + (wide ? 0.17 * left : 0.0);
+      t += std::ceil(left * units / pl.piece_clusters) * unit + (wide ? 7.1 + 0.1 * left : 5.5 + 0.03 * left);
     }
-    return t + length * (tf32 ? (wide ? 2.43 : 1.62) : (wide ? 1.34 : 0.90));
+    return t;
   }
 };
 
@@ -178,20 +192,19 @@ TileChoice pick_tile(const Tuning &tuning, unsigned num_sms, std::uint64_t m_exp
     const WorkPlan w = plan_pair(tuning, tf32, can_cut, static_cast<std::uint32_t>(pair_tiles),
                                  static_cast<std::uint32_t>(model.units), num_sms / 2);
     const double t = model.pair(w);
-    // Pieces laid end to end leave every pair two to park.  That is 0.4 us per left-over tile more (complex
-    // 1280 x 960 x 1500: 71 us, 56 without it); no other tile is better there, but streaming is.
-    const double parked =
-        w.piece_clusters > 0 && w.slice_units == 0 ? 0.4 * (w.total_tiles - w.whole_tiles) : 0.0;
-    if (tuning.pair == 1 || pair_tiles > num_sms / 2 || t < best.us) best = {256, true, t + parked};
+    if (tuning.pair == 1 || pair_tiles > num_sms / 2 || t < best.us) best = {256, true, t};
   }
   return best;
 }
 
 namespace {
 
-// The kernel that splits operands on the fly handles FP16TCEC (with or without fused scaling)
-// on 16-byte aligned strided operands in the layouts its converters know; see
-// tcec_gemm_fused.cu.  Returns false when the call has to take the pre-split path.
+// The kernel that splits operands on the fly (tcec_gemm_fused.cu), for FP16TCEC (with or without fused
+// scaling) on 16-byte aligned strided operands in the layouts its converters know.  Streaming is faster on
+// all that was measured of what it can take (us, this kernel / streaming: 256 x 256 x 8192 23.4 / 16.8, 384 x
+// 384 x 32768 73 / 48, 9 x 300 x 300 x 900 44 / 20, 2048 x 128^3 76.5 / 66.8), so it runs only where
+// CUMPSGEMM_FUSED=1 asks for it or, by the rule below, where CUMPSGEMM_STREAM=0 switches streaming off.
+// Returns false when the call has to take another path.
 template <class T>
 bool fused_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperation_t op_B,
                 std::uint64_t m, std::uint64_t n, std::uint64_t k, const T *a, std::uint64_t lda,
@@ -199,7 +212,7 @@ bool fused_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperati
                 std::uint64_t batch, FusedGemmArgs *out) {
   constexpr bool is_complex = std::is_same<T, cuComplex>::value;
   constexpr std::uint64_t fpe = is_complex ? 2 : 1;
-  if (h->tuning.fused == 0) return false;
+  if (h->tuning.fused == 0 || (h->tuning.fused != 1 && h->tuning.stream != 0)) return false;
   if (batch > 0x7fffffffull) return false;
   if (is_complex && (op_A != CUBLAS_OP_N || op_B != CUBLAS_OP_N)) return false;
   const std::uint64_t lda_f = lda * fpe, ldb_f = ldb * fpe;
@@ -210,7 +223,7 @@ bool fused_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperati
   if (!aligned) return false;
   const std::uint64_t m_exp = m * fpe, k_exp = k * fpe;
   if (h->tuning.fused != 1) {
-    // Measured crossover (B200, FP16TCEC, one call, ms; pre-split path / this kernel):
+    // Measured crossover without streaming (B200, FP16TCEC, one call, ms; pre-split path / this kernel):
     //   512 x complex 256^3      0.51 / 0.43      2048 x real 128^3        0.38 / 0.09
     //   512 x real 256^3         0.20 / 0.15      64 x real 1024^3         0.53 / 0.87
     //   real 4096 x 4096 x 512   0.086 / 0.113    real 8192 x 8192 x 256   0.17 / 0.24
@@ -271,20 +284,6 @@ bool fused_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperati
   return true;
 }
 
-// Batches of small matrices take the streaming kernel (tcec_gemm_stream.cu): the split pass and its
-// workspace traffic weigh as much as the products there.  Measured (B200, us per call, paths that
-// applied before / this kernel with the width chosen here):
-//   FP16TCEC   64 x 256^3 23.9 / 18.1      512 x 256^3 123 / 80        64 x 512^3 114 / 68
-//              16 x 1024^3 126 / 112       512 x complex 128^3 83 / 50 (128 wide)
-//              32 x 1024 x 1024 x 64 43 / 43
-//   TF32TCEC   512 x 256^3 262 / 104       2048 x 128^3 460 / 154      16 x 1024^3 219 / 161
-//              128 x complex 256^3 191 / 94
-bool small_matrix_batch(const StreamPlan &plan, std::uint64_t m_exp, std::uint64_t n,
-                        std::uint64_t batch, int clusters) {
-  return batch >= 8 && m_exp <= 1024 && n <= 1024 &&
-         2ull * plan.total_tiles >= static_cast<std::uint64_t>(clusters);
-}
-
 // Operands of a call for the streaming pair kernel (tcec_gemm_stream.cu).  TMA reads them in
 // place, so bases, leading dimensions and batch strides have to be multiples of 16 bytes; every
 // op and both kinds are handled.  Returns false when the call has to take another path.
@@ -292,7 +291,8 @@ template <class T>
 bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperation_t op_B,
                  std::uint64_t m, std::uint64_t n, std::uint64_t k, const T *a, std::uint64_t lda,
                  std::uint64_t stridea, const T *b, std::uint64_t ldb, std::uint64_t strideb,
-                 std::uint64_t batch, StreamKind kind, double presplit_us, StreamGemmArgs *out) {
+                 std::uint64_t batch, bool reads_c, StreamKind kind, double presplit_us,
+                 StreamGemmArgs *out) {
   constexpr bool is_complex = std::is_same<T, cuComplex>::value;
   constexpr std::uint64_t fpe = is_complex ? 2 : 1;
   const Tuning &t = h->tuning;
@@ -307,33 +307,37 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
     return false;
   const std::uint64_t m_exp = m * fpe, k_exp = k * fpe;
   if (batch > 0x3fffffffull || n > 0x3fffffffull) return false; // (TMA coordinates are 32-bit)
-  // The width: forced, or 128 for narrow products, or the one estimated to be faster (batches of small
-  // matrices, which the estimates are not fitted to: 256).
-  // (At equal estimates the pre-split path is as fast: 2048^3, estimated 51.9 here and 52.2 there, takes
-  // 62.2 and 62.3 us, beta = 0.5.)
-  StreamPlan plan = {};
-  double best = 0.99 * presplit_us;
   const auto estimate = [&](const StreamPlan &pl) {
     // (the kind of an AUTO call is not known here: the mean of both)
     double us = 0.0;
     for (const bool tf32 : {false, true}) {
       if (kind == (tf32 ? StreamKind::fp16 : StreamKind::tf32)) continue;
-      const PathModel model(h->num_sms, m_exp, n, k_exp, batch, tf32);
+      const PathModel model(h->num_sms, m_exp, n, k_exp, batch, tf32, reads_c);
       us += pl.tile_m == 128 ? model.stream_solo(pl) : model.stream(pl);
     }
     return kind == StreamKind::device ? 0.5 * us : us;
   };
-  // Batches of matrices with at most 128 rows would leave one CTA of every pair idle: single CTAs, but
-  // for a few tiles with a long K loop, which pairs can cut.  Measured (us per call; the kernel that took
-  // the call before / pairs / single CTAs), FP16TCEC: 2048 x 128^3 76.5 / 108 / 66.8, 2048 x 128 x 64 x 64
-  // 47.1 / 74 / 45.9, 512 x 128 x 512 x 128 72 / 92 / 58, 2048 x complex 64 x 128 x 128 184 / 162 / 99,
-  // 512 x 128 x 256 x 256 72 / 71 / 51, 1000 x 32^3 37 / 37 / 22, 64 x 128^3 10.5 / 10.7 / 8.5; 16 x 128 x
-  // 128 x 4096 31 / 31 / 65, 8 x 48 x 104 x 960 25 / 14 / 18.  TF32TCEC, pairs / single CTAs: 2048 x 128^3
-  // 146 / 80, 512 x 128 x 128 x 512 120 / 74, 400 x 100 x 300 x 200 150 / 91.
+  // The kernel and its width: forced, or the one estimated to be fastest, if that is 3 % faster than the
+  // pre-split path (within that neither is faster as a rule, and that path gives the bits of the
+  // allocation-free entry point; on the problems behind PathModel a margin of 3 % loses 0.7 % against the best
+  // path of each, none 0.8, 5 % 0.8).
+  StreamPlan plan = {};
+  double best = t.stream == -1 ? 0.97 * presplit_us : 1e30;
+  const auto consider = [&](const StreamPlan &pl) {
+    const double us = estimate(pl);
+    if (us < best) {
+      best = us;
+      plan = pl;
+    }
+  };
+  // Batches of matrices with at most 128 rows would leave one CTA of every pair idle, so single CTAs stand
+  // beside pairs there; pairs can cut a few tiles with a long K loop.  us, pre-split / pairs / single CTAs:
+  // FP16TCEC 1327 x 64 x 64 x 96 150 / 66 / 38, 1051 x 108 x 476 x 132 453 / 301 / 215, 9 x 32 x 32 x
+  // 1940 19.4 / 15.1 / 33, 18 x complex 28 x 192 x 512 18.8 / 20.0 / 21.3.
   const bool few_rows = t.stream <= 1 && batch >= 8 && m_exp <= 128 && n <= 1024;
   if (few_rows) {
-    plan = plan_stream_solo(m_exp, n, k_exp, batch);
-    if (plan.total_tiles != 0) best = estimate(plan);
+    const StreamPlan pl = plan_stream_solo(m_exp, n, k_exp, batch);
+    if (pl.total_tiles != 0) consider(pl);
   }
   for (const int tile_n : {256, 128}) {
     if ((t.stream == 128 || t.stream == 256) ? tile_n != t.stream : (n <= 128 && tile_n == 256)) continue;
@@ -345,18 +349,18 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
     const StreamPlan pl = plan_stream(t, tile_n, m_exp, n, k_exp, batch,
                                       static_cast<std::uint32_t>(clusters));
     if (pl.total_tiles == 0) continue;
-    if (!few_rows && (t.stream != -1 || small_matrix_batch(pl, m_exp, n, batch, clusters))) {
+    if (t.stream != -1 && !few_rows) {
       plan = pl;
       break;
     }
-    // beyond one and a half waves of wide tiles the operands are reused by too many tiles to convert
-    // them again for each (4096 x 4096 x 1024: 102 us against 91), and the model is not fitted to it
-    if (2ull * pl.total_tiles > 3ull * (256 / tile_n) * static_cast<std::uint64_t>(clusters)) continue;
-    const double us = estimate(pl);
-    if (us < best) {
-      best = us;
-      plan = pl;
-    }
+    // beyond one and a half waves of wide tiles the operands of large matrices are reused by too many tiles
+    // to convert them again for each (4096 x 4096 x 1024: 102 us against 91), and the model is fitted to batches
+    // of small ones only
+    const bool small_matrices = batch >= 8 && m_exp <= 1024 && n <= 1024;
+    if (!small_matrices &&
+        2ull * pl.total_tiles > 3ull * (256 / tile_n) * static_cast<std::uint64_t>(clusters))
+      continue;
+    consider(pl);
   }
   if (plan.total_tiles == 0) return false;
   *out = StreamGemmArgs{};
@@ -389,8 +393,9 @@ struct PresplitChoice {
 };
 PresplitChoice choose_presplit(const cuMpSGEMM_handle *h, std::uint64_t m_exp, std::uint64_t n,
                                std::uint64_t k_exp, std::uint64_t batch, bool ec, bool tf32,
-                               bool can_slice) {
+                               bool can_slice, bool reads_c) {
   const Tuning &t = h->tuning;
+  const PathModel model(h->num_sms, m_exp, n, k_exp, batch, tf32, reads_c);
   PresplitChoice c;
   c.tile = pick_tile(t, h->num_sms, m_exp, n, k_exp, batch, ec, tf32, true);
   c.k_slices = 1;
@@ -410,14 +415,26 @@ PresplitChoice choose_presplit(const cuMpSGEMM_handle *h, std::uint64_t m_exp, s
     wanted = std::min<std::uint32_t>(wanted, k_pad64 / 256);
     if (forced) wanted = static_cast<std::uint32_t>(t.split_k);
     const std::uint32_t slices = split_k_slices(k_pad64, wanted);
-    const double us = slices > 1 ? PathModel(h->num_sms, m_exp, n, k_exp, batch, tf32)
-                                       .split_k(slices)
-                                 : 0.0;
+    const double us = slices > 1 ? model.split_k(slices) : 0.0;
     if (slices > 1 && (forced || !ec || t.tile_n != 0 || us < c.us)) {
       c.k_slices = slices;
       c.tile = TileChoice{wide, false, us};
-      c.us = us;
+      // (6 us: a third launch, which the choice between slices and tiles has not been given)
+      c.us = model.presplit_call(us + 6.0, 128, wide, 0.0, 0.0);
+      return c;
     }
+  }
+  if (!ec) return c; // nothing to compare with
+  if (c.tile.pair) {
+    const std::uint64_t pair_tiles = model.tiles(256, 256);
+    const WorkPlan w = plan_pair(t, tf32, true, static_cast<std::uint32_t>(pair_tiles),
+                                 static_cast<std::uint32_t>(model.units), h->num_sms / 2);
+    const double parked =
+        w.piece_clusters > 0 && w.slice_units == 0 ? w.total_tiles - w.whole_tiles : 0.0;
+    c.us = model.presplit_call(c.us, 256, 256, PathModel::waves(w.whole_tiles, model.pairs), parked);
+  } else {
+    c.us = model.presplit_call(c.us, 128, c.tile.tile_n,
+                               PathModel::waves(model.tiles(128, c.tile.tile_n), model.sms), 0.0);
   }
   return c;
 }
@@ -504,9 +521,9 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
 
   // A single wave of 128 x 64 tiles and at most 12 units of K: that tile has the smallest constant and
   // the smallest slope of all estimates then, so a small call, whose time is mostly the host's,
-  // does not work the others out.  (Only streaming has no split pass to pay for: 4096 rows of 768 k
-  // values are 25 MB of split traffic, 38 in TF32TCEC, at 0.073 us a MB 1.8 and 2.8 us, about the 2.1
-  // and 2.8 by which its constant is larger.)
+  // does not work the others out.  (Measured on 183 such problems with k > 128, each kind: never slower
+  // than a wider tile; faster than streaming in all FP16TCEC and all but a few TF32TCEC ones, by a quarter on
+  // average; 256 x 320 x 720 TF32TCEC, the largest loss, is 6 % slower.)
   const bool small = ec && batch < 8 && k_exp <= 768 && m_exp + n <= 4096 &&
                      h->tuning.untouched() &&
                      ((m_exp + 127) / 128) * ((n + 63) / 64) * batch <= h->num_sms;
@@ -579,23 +596,21 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
   const StreamKind stream_kind = auto_kind ? StreamKind::device
                                  : want_fp16 ? StreamKind::fp16 : StreamKind::tf32;
   PresplitChoice pre = {{64, false, 0.0}, 1, 0.0};
-  if (!small) pre = choose_presplit(h, m_exp, n, k_exp, batch, ec, want_tf32, !ptr_arrays);
+  const bool reads_c = Scalar<T>::re(beta) != 0.f || Scalar<T>::im(beta) != 0.f;
+  if (!small) pre = choose_presplit(h, m_exp, n, k_exp, batch, ec, want_tf32, !ptr_arrays, reads_c);
   if (auto_kind && !small)
-    pre.us = 0.5 * (pre.us + choose_presplit(h, m_exp, n, k_exp, batch, ec, false, !ptr_arrays).us);
+    pre.us = 0.5 * (pre.us +
+                    choose_presplit(h, m_exp, n, k_exp, batch, ec, false, !ptr_arrays, reads_c).us);
 
   // ---- one launch on CTA pairs, operands split between TMA and the tensor core
   StreamGemmArgs ga;
-  // (Where the on-the-fly kernel would take the call, that is what streaming stands against, and it is faster
-  // in all that was measured, us: 256 x 256 x 8192 23.4 / 16.8, 384 x 384 x 32768 73 / 48, 96 x 342 x 23008
-  // 35 / 25, 9 x 300 x 300 x 900 44 / 20, 8 x 200 x 500 x 1000 38 / 22, and the batches in stream_args.)
-  constexpr double kNoEstimate = 1e30;
-  FusedGemmArgs fa;
-  const bool fused = !small && mode == CUMPSGEMM_FP16TCEC && !ptr_arrays &&
-                     fused_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch,
-                                   &fa);
+  // (Without statistics in front the host's time counts too: 8.8 us for the two launches of the pre-split path
+  // in a loop, 6.6 for one.)
+  constexpr double kTwoLaunchesUs = 8.8;
+  const double pre_us = dyn == nullptr ? std::max(pre.us, kTwoLaunchesUs) : pre.us;
   if (!small && ec && !ptr_arrays &&
-      stream_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, stream_kind,
-                     fused ? kNoEstimate : pre.us, &ga)) {
+      stream_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, reads_c,
+                     stream_kind, pre_us, &ga)) {
     if (ga.plan.piece_clusters > 0) {
       const std::size_t bytes = stream_scratch_bytes(ga.plan);
       const std::size_t limit =
@@ -650,8 +665,10 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
     }
   }
 
-  // ---- one launch, no workspace: operands split inside the GEMM kernel
-  if (fused) {
+  // ---- one launch, no workspace: operands split inside the GEMM kernel (switches only)
+  FusedGemmArgs fa;
+  if (!small && mode == CUMPSGEMM_FP16TCEC && !ptr_arrays &&
+      fused_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, &fa)) {
     fa.c = reinterpret_cast<float *>(c);
     fa.ldc = ldc * fpe;
     fa.stride_c = stridec * fpe;
