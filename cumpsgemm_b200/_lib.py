@@ -90,6 +90,7 @@ PROTOTYPES = {
     "cuMpSGEMM_set_workspace_limit": (None, [vp, C.c_size_t]),
     "cuMpSGEMM_set_count_tail_padding": (None, [vp, i32]),
     "cuMpSGEMM_get_last_route": (i32, [vp, C.POINTER(i32)]),
+    "cuMpSGEMM_get_last_tile": (i32, [vp, C.POINTER(i32), C.POINTER(i32)]),
     "cuMpSGEMM_reload_tuning_env": (None, [vp]),
     "cuMpSGEMM_plan_stream": (i32, [u64, u64, u64, u64, i32, u32, C.POINTER(u32), C.POINTER(u32),
                                     C.POINTER(u32), C.POINTER(u32), C.POINTER(u32)]),

@@ -238,6 +238,12 @@ class Handle:
         route = self._lib.cuMpSGEMM_get_last_route(self._h, C.byref(cut))
         return route, bool(cut.value)
 
+    def last_tile(self) -> tuple[int, int]:
+        """Rows and columns of C in a tile of the last GEMM call (of the real, expanded product)."""
+        rows, cols = C.c_int(0), C.c_int(0)
+        self._lib.cuMpSGEMM_get_last_tile(self._h, C.byref(rows), C.byref(cols))
+        return rows.value, cols.value
+
     def reload_tuning_env(self) -> None:
         """Read the CUMPSGEMM_TILE_N / PAIR / DRAIN_CHUNK / FIRST_CHUNK / PACE / FUSED / STREAM variables
         again (a handle reads them once, at creation)."""

@@ -224,6 +224,13 @@ int cuMpSGEMM_get_last_route(cuMpSGEMM_handle_t h, int *cut_along_k) {
   if (cut_along_k != nullptr) *cut_along_k = h->last_cut_along_k ? 1 : 0;
   return h->last_route;
 }
+int cuMpSGEMM_get_last_tile(cuMpSGEMM_handle_t h, int *rows, int *cols) {
+  if (h == nullptr || rows == nullptr || cols == nullptr) return 1;
+  const bool any = h->last_route != CUMPSGEMM_ROUTE_NONE;
+  *rows = any ? h->last_tile_rows : 0;
+  *cols = any ? h->last_tile_cols : 0;
+  return 0;
+}
 void cuMpSGEMM_reload_tuning_env(cuMpSGEMM_handle_t h) { h->tuning = read_tuning_env(); }
 
 void cuMpSGEMM_set_count_tail_padding(cuMpSGEMM_handle_t h, int enable) {

@@ -588,6 +588,8 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
       return CUBLAS_STATUS_EXECUTION_FAILED;
     }
     h->last_route = CUMPSGEMM_ROUTE_ON_THE_FLY;
+    h->last_tile_rows = 128;
+    h->last_tile_cols = 32;
     return CUBLAS_STATUS_SUCCESS;
   }
 
@@ -661,6 +663,8 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
       }
       h->last_route = CUMPSGEMM_ROUTE_STREAMING;
       h->last_cut_along_k = ga.plan.piece_clusters > 0;
+      h->last_tile_rows = ga.plan.tile_m;
+      h->last_tile_cols = ga.plan.tile_n;
       return CUBLAS_STATUS_SUCCESS;
     }
   }
@@ -727,6 +731,8 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
     }
     h->last_route = CUMPSGEMM_ROUTE_ON_THE_FLY;
     h->last_cut_along_k = fa.k_slices > 1;
+    h->last_tile_rows = 128;
+    h->last_tile_cols = fa.tile_n;
     return CUBLAS_STATUS_SUCCESS;
   }
 
@@ -879,6 +885,8 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
   }
   h->last_route = use_pair ? CUMPSGEMM_ROUTE_PRESPLIT_PAIR : CUMPSGEMM_ROUTE_PRESPLIT_SINGLE;
   h->last_cut_along_k = k_slices > 1 || bytes_tail > 0; // (the scratch is only there to be used)
+  h->last_tile_rows = use_pair ? 256 : 128;
+  h->last_tile_cols = tile_n;
   return CUBLAS_STATUS_SUCCESS;
 }
 

@@ -156,6 +156,7 @@ struct cuMpSGEMM_handle {
 
   // What the last GEMM call launched (see cuMpSGEMM_get_last_route).
   int last_route = 0;
+  int last_tile_rows = 0, last_tile_cols = 0;
   bool last_cut_along_k = false;
 
   // Device status word the GEMM kernel writes when a bounded wait gives up.

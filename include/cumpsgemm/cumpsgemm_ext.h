@@ -134,10 +134,16 @@ enum {
   CUMPSGEMM_ROUTE_NONE = 0,
   CUMPSGEMM_ROUTE_PRESPLIT_SINGLE = 1, /* split pass, then one CTA per tile */
   CUMPSGEMM_ROUTE_PRESPLIT_PAIR = 2,   /* split pass, then one CTA pair per tile */
-  CUMPSGEMM_ROUTE_STREAMING = 3,       /* CTA pairs, operands split between TMA and the tensor core */
-  CUMPSGEMM_ROUTE_ON_THE_FLY = 4       /* single CTAs that load and split the operands themselves */
+  CUMPSGEMM_ROUTE_STREAMING = 3,       /* operands split between TMA and the tensor core; CTA pairs, or
+                                        * single CTAs for batches of matrices with few rows */
+  CUMPSGEMM_ROUTE_ON_THE_FLY = 4       /* single CTAs that load and split the operands themselves: the
+                                        * kernel for small products, or the one that CUMPSGEMM_FUSED=1 or
+                                        * CUMPSGEMM_STREAM=0 select */
 };
 int cuMpSGEMM_get_last_route(cuMpSGEMM_handle_t handle, int *cut_along_k);
+/* Rows and columns of C (of the real, expanded product) in a tile of that call: 256 rows on CTA pairs, 128
+ * on single CTAs; 0 x 0 without a route.  Returns 0, or 1 for a null argument. */
+int cuMpSGEMM_get_last_tile(cuMpSGEMM_handle_t handle, int *rows, int *cols);
 /* Self-test of the bounded wait: a one-CTA kernel waits, with the same routine the GEMM kernels
  * use, on a barrier that nothing signals; after limit_ms it must give up, record its code and
  * return normally.  Returns the status word (expected: 2, the "waited for operands" code) and

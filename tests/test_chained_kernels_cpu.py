@@ -42,6 +42,16 @@ def test_device_decision_is_read_behind_the_wait(source, functions):
         assert body.index("griddep_wait()") < body.index("dyn->"), name
 
 
+@pytest.mark.parametrize("source,function,wait", [
+    ("tcec_gemm_stream.cu", "tcec_gemm_stream_solo_kernel", "griddep_wait()"),
+    ("tcec_gemm_small.cu", "tcec_gemm_small_kernel", "CUMPSGEMM_CHAINED_KERNEL_ENTRY()")])
+def test_device_decision_is_read_behind_the_wait_on_single_ctas(source, function, wait):
+    body = _body((CSRC / source).read_text(), function)
+    assert body.index(wait) < body.index("dyn->")
+    if function == "tcec_gemm_small_kernel":      # all that touches global memory is behind it
+        assert body.index(wait) < body.index("small_body<")
+
+
 @pytest.mark.parametrize("source", ["tcec_gemm.cu", "tcec_gemm_pair.cu", "tcec_gemm_fused.cu",
                                     "tcec_gemm_small.cu", "tcec_gemm_stream.cu"])
 def test_a_warp_that_waits_for_an_accumulator_goes_on_as_a_whole(source):
