@@ -10,9 +10,9 @@
 // fetches them 16 columns at a time.  With beta != 0 the loop loads the next group's C values
 // before it stores the current one.  GEMM kernels before / after, us: 2048^3 beta = 0.5 (128 x 256
 // tiles) 53.3 / 45.6; 1999 x 3001 x 2777 beta = 0.5 (pairs) 118 / 94; complex 1280 x 960 x 1500
-// 71.7 / 64.9; TF32TCEC 4096 x 1024 x 2048 beta = 0 89.7 / 76.5.  (The kernel for batches of small
-// matrices, tcec_gemm_fused.cu, keeps its unrolled stores: it runs them for many tiles per
-// launch, from a warm instruction cache, and the round trip through TMEM cost it 82 -> 93 us on
+// 71.7 / 64.9; TF32TCEC 4096 x 1024 x 2048 beta = 0 89.7 / 76.5.  (Where many short tiles per launch keep
+// the unrolled stores in the instruction cache, they stay: see the direct stores of tcec_gemm_stream.cu;
+// and the on-the-fly kernel, tcec_gemm_fused.cu, which the round trip through TMEM cost 82 -> 93 us on
 // 2048 products of 128^3.)
 #pragma once
 #include "ptx.cuh"

@@ -203,7 +203,7 @@ namespace {
 // scaling) on 16-byte aligned strided operands in the layouts its converters know.  Streaming is faster on
 // all that was measured of what it can take (us, this kernel / streaming: 256 x 256 x 8192 23.4 / 16.8, 384 x
 // 384 x 32768 73 / 48, 9 x 300 x 300 x 900 44 / 20, 2048 x 128^3 76.5 / 66.8), so it runs only where
-// CUMPSGEMM_FUSED=1 asks for it or, by the rule below, where CUMPSGEMM_STREAM=0 switches streaming off.
+// CUMPSGEMM_FUSED=1 asks for it or, by the rule below, where a switch keeps streaming off.
 // Returns false when the call has to take another path.
 template <class T>
 bool fused_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperation_t op_B,
@@ -212,7 +212,7 @@ bool fused_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperati
                 std::uint64_t batch, FusedGemmArgs *out) {
   constexpr bool is_complex = std::is_same<T, cuComplex>::value;
   constexpr std::uint64_t fpe = is_complex ? 2 : 1;
-  if (h->tuning.fused == 0 || (h->tuning.fused != 1 && h->tuning.stream != 0)) return false;
+  if (h->tuning.fused == 0 || (h->tuning.fused != 1 && !h->tuning.streaming_off())) return false;
   if (batch > 0x7fffffffull) return false;
   if (is_complex && (op_A != CUBLAS_OP_N || op_B != CUBLAS_OP_N)) return false;
   const std::uint64_t lda_f = lda * fpe, ldb_f = ldb * fpe;
@@ -296,7 +296,7 @@ bool stream_args(const cuMpSGEMM_handle *h, cublasOperation_t op_A, cublasOperat
   constexpr bool is_complex = std::is_same<T, cuComplex>::value;
   constexpr std::uint64_t fpe = is_complex ? 2 : 1;
   const Tuning &t = h->tuning;
-  if (t.stream == 0 || (t.stream == -1 && t.others_forced())) return false;
+  if (t.streaming_off()) return false;
   const std::uint64_t sa = batch > 1 ? stridea * fpe : 0, sb = batch > 1 ? strideb * fpe : 0;
   const bool aligned = (reinterpret_cast<std::uintptr_t>(a) % 16 == 0) &&
                        (reinterpret_cast<std::uintptr_t>(b) % 16 == 0) && (lda * fpe) % 4 == 0 &&

@@ -72,7 +72,7 @@ struct Profiler {
 // CTA-pair kernel off / on, CUMPSGEMM_DRAIN_CHUNK and CUMPSGEMM_FIRST_CHUNK the number of
 // K stages per accumulator drain and in the first one of a tile (pair and on-the-fly kernels),
 // CUMPSGEMM_PACE = 0 the wave pacing off, CUMPSGEMM_FUSED = 0 / 1 the kernel that splits operands
-// on the fly off / on wherever it is applicable, CUMPSGEMM_SPLIT_K = 0 / n the K-slicing of
+// on the fly off / on wherever it is applicable (-1: by a rule where streaming is off), CUMPSGEMM_SPLIT_K = 0 / n the K-slicing of
 // problems with few tiles off / to n slices.  A switch of one kernel keeps the streaming kernel off,
 // unless CUMPSGEMM_STREAM says otherwise, so that it reaches the kernel it is meant for.
 struct Tuning {
@@ -94,6 +94,7 @@ struct Tuning {
     return tile_n != 0 || pair != -1 || drain_chunk != 0 || first_chunk != 0 || pace != 1 ||
            fused != -1 || split_k > 0 || tail_split > 0;
   }
+  bool streaming_off() const { return stream == 0 || (stream == -1 && others_forced()); }
 };
 Tuning read_tuning_env();
 

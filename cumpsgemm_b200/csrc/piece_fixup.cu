@@ -3,7 +3,7 @@
 // (src/cumpsgemm.cu:272-304, src/dmem_accessor.hpp:352-395).
 //
 // All pieces of a launch end at about the same time, so adding them is a job for the whole GPU:
-// the scratch tiles are still in L2 and every thread has all of its loads in flight.  (Done
+// the scratch tiles are still in L2 and every thread has the loads of four pieces in flight.  (Done
 // instead inside the GEMM kernel by whichever CTA finished a tile last, with a ticket counter per
 // tile, it took 20 us for 40 tiles: a few CTAs, one L2 latency per group of columns and piece.)
 //

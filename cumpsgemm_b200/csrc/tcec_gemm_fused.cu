@@ -12,10 +12,11 @@
 // (hi*hi as it is, the two corrections times 2^-11), and the alpha / beta epilogue stores from the
 // registers (many short tiles per launch: see epilogue.cuh on the rolled one of the other kernels).
 //
-// It pays where the split pass of the two-kernel path costs as much as the GEMM: short K and
-// many small problems (strided batches of at most 128 rows, where a CTA pair of
-// tcec_gemm_stream.cu would leave one CTA idle), where writing the panels to HBM and reading them
-// back is most of the traffic.  It loses for long K on large matrices, where
+// No call reaches it by default: tcec_gemm_stream.cu is faster on all that was measured of what it takes.
+// It runs with CUMPSGEMM_FUSED=1, and, where a switch keeps streaming off, if it is the faster one of the rest (the
+// rule and its figures: fused_args in gemm_api.cu).  That is where the split pass of the two-kernel path
+// costs as much as the GEMM: short K and many small problems, where writing the panels to HBM and reading
+// them back is most of the traffic.  It loses for long K on large matrices, where
 // every operand element is converted once per tile that uses it (n / BN times for A, m / 128
 // times for B) and the converter warps, not the tensor core, set the pace; the dispatch keeps
 // the pre-split path there.  A second regime is a handful of tiles with a very long K loop:

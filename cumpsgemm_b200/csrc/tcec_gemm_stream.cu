@@ -3,7 +3,8 @@
 //
 // The reference splits every FP32 value at fragment load, inside the GEMM kernel
 // (src/device_tcec_wrapper.hpp:72-80 called from src/cumpsgemm_kernel.cuh:58-100).  Here a
-// cluster of two CTAs owns a 256 x BN tile of C (BN = 256 or 128); each CTA
+// cluster of two CTAs owns a 256 x BN tile of C (BN = 256 or 128; for batches of matrices with at most 128
+// rows a single CTA a 128 x 128 one, with the same body); each CTA
 //   * fetches its own 128 rows of op(A) and its own BN / 2 rows of op(B) as plain FP32 through TMA
 //     into a ring of raw slots (32 k values each; edges are zero filled by TMA, so no thread
 //     tests bounds),
@@ -27,7 +28,8 @@
 //
 // What bounds it: with 256 columns shared memory.  Per stage of 64 k values it takes 64 KiB from TMA,
 // gives 64 KiB to the converters, takes 64 KiB of hi / lo tiles back and feeds 112 KiB to the tensor
-// core (A_hi once more for either half): 2432 cycles at 128 bytes a cycle, for 1536 of tensor-core work.
+// core (A_hi once more for either half): 2432 cycles at 128 bytes a cycle, for 1536 of tensor-core work;
+// 2335 were measured at 2048^3, so not all of the tensor core's reads cost what this counts.
 // With 128 columns the instructions of the converters and the epilogue (with A in tensor memory the port
 // has 1088 cycles to do, and the tensor core 768).  Two rules of the code below matter as much:
 // sums are added two at a time (packed), and whatever is live in the loop over the stages besides the 128

@@ -137,8 +137,8 @@ enum {
   CUMPSGEMM_ROUTE_STREAMING = 3,       /* operands split between TMA and the tensor core; CTA pairs, or
                                         * single CTAs for batches of matrices with few rows */
   CUMPSGEMM_ROUTE_ON_THE_FLY = 4       /* single CTAs that load and split the operands themselves: the
-                                        * kernel for small products, or the one that CUMPSGEMM_FUSED=1 or
-                                        * CUMPSGEMM_STREAM=0 select */
+                                        * kernel for small products, or the one that CUMPSGEMM_FUSED=1, or
+                                        * a switch that keeps streaming off, selects */
 };
 int cuMpSGEMM_get_last_route(cuMpSGEMM_handle_t handle, int *cut_along_k);
 /* Rows and columns of C (of the real, expanded product) in a tile of that call: 256 rows on CTA pairs, 128
