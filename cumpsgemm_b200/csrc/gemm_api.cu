@@ -604,15 +604,15 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
     pre.us = 0.5 * (pre.us +
                     choose_presplit(h, m_exp, n, k_exp, batch, ec, false, !ptr_arrays, reads_c).us);
 
-  // ---- one launch on CTA pairs, operands split between TMA and the tensor core
-  StreamGemmArgs ga;
-  // (Without statistics in front the host's time counts too: 8.8 us for the two launches of the pre-split path
-  // in a loop, 6.6 for one.)
-  constexpr double kTwoLaunchesUs = 8.8;
-  const double pre_us = dyn == nullptr ? std::max(pre.us, kTwoLaunchesUs) : pre.us;
-  if (!small && ec && !ptr_arrays &&
-      stream_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, reads_c,
-                     stream_kind, pre_us, &ga)) {
+  // ---- one launch, operands split between TMA and the tensor core.  Returns whether the call was taken, that is
+  // whether the kernel can take it and is estimated to end before `bound_us`.
+  cublasStatus_t stream_status = CUBLAS_STATUS_SUCCESS;
+  const auto stream_call = [&](double bound_us) {
+    StreamGemmArgs ga;
+    if (!ec || ptr_arrays ||
+        !stream_args<T>(h, op_A, op_B, m, n, k, a, lda, stridea, b, ldb, strideb, batch, reads_c,
+                        stream_kind, bound_us, &ga))
+      return false;
     if (ga.plan.piece_clusters > 0) {
       const std::size_t bytes = stream_scratch_bytes(ga.plan);
       const std::size_t limit =
@@ -655,19 +655,23 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
       for (auto &e : tt.e) cudaEventDestroy(e);
     }
     if (prof) h->exp_stats.profiler.stop("gemm_kernel", h->cuda_stream);
-    if (addressable) {
-      mark_stream_work(h);
-      if (gerr != cudaSuccess) {
-        log_error(std::string("kernel launch failed: ") + cudaGetErrorString(gerr));
-        return CUBLAS_STATUS_EXECUTION_FAILED;
-      }
-      h->last_route = CUMPSGEMM_ROUTE_STREAMING;
-      h->last_cut_along_k = ga.plan.piece_clusters > 0;
-      h->last_tile_rows = ga.plan.tile_m;
-      h->last_tile_cols = ga.plan.tile_n;
-      return CUBLAS_STATUS_SUCCESS;
+    if (!addressable) return false;
+    mark_stream_work(h);
+    if (gerr != cudaSuccess) {
+      log_error(std::string("kernel launch failed: ") + cudaGetErrorString(gerr));
+      stream_status = CUBLAS_STATUS_EXECUTION_FAILED;
+      return true;
     }
-  }
+    h->last_route = CUMPSGEMM_ROUTE_STREAMING;
+    h->last_cut_along_k = ga.plan.piece_clusters > 0;
+    h->last_tile_rows = ga.plan.tile_m;
+    h->last_tile_cols = ga.plan.tile_n;
+    return true;
+  };
+  // (Without statistics in front the host's time counts too: 8.8 us for the two launches of the pre-split path
+  // in a loop, 6.6 for one.)
+  constexpr double kTwoLaunchesUs = 8.8;
+  if (!small && stream_call(dyn == nullptr ? std::max(pre.us, kTwoLaunchesUs) : pre.us)) return stream_status;
 
   // ---- one launch, no workspace: operands split inside the GEMM kernel (switches only)
   FusedGemmArgs fa;
@@ -778,6 +782,9 @@ cublasStatus_t gemm_dispatch(cuMpSGEMM_handle *h, cublasOperation_t op_A, cublas
       bytes_tail = bytes;
   }
   if (!ensure_workspace(h, bytes_panels)) {
+    // no memory for the panels (a captured call on a handle that has made none of its size before):
+    // streaming needs none
+    if (stream_call(1e30)) return stream_status;
     log_error(may_allocate(h) ? "failed to allocate the operand workspace"
                               : "the operand workspace cannot grow while the stream is captured; "
                                 "make one call of this size before the capture");

@@ -40,3 +40,37 @@ def test_many_small_matrices(handle, cplx, ops, m, n, k, batch, mode):
     if cplx:
         m, k = m // 2, k // 2
     assert _route(handle, cplx, *ops, m, n, k, batch, mode) == api.ROUTE_STREAMING
+
+
+@pytest.mark.parametrize("mode", [FP16TCEC, TF32TCEC])
+@pytest.mark.parametrize("m,n,k,batch", [(128, 128, 512, 8), (700, 520, 700, 1)])
+def test_a_call_without_memory_for_panels_streams(oracle, mode, m, n, k, batch):
+    """A captured call on a handle without a workspace: pre-split by estimate, but streaming needs no memory."""
+    import torch
+
+    a, b = oracle.gen_uniform(1, batch * m * k), oracle.gen_uniform(2, batch * k * n)
+    da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    c = torch.zeros(batch * m * n, device="cuda")
+
+    def call(h):
+        h.gemm_strided_batch(N, N, m, n, k, 1.0, da, m, m * k, db, k, k * n, 0.0, c, m, m * n, batch, mode)
+        return h.last_route()[0]
+
+    with api.Handle() as h:                       # loads the kernels
+        h.use_current_torch_stream()
+        assert call(h) in PRESPLIT
+        torch.cuda.synchronize()
+    with api.Handle() as h:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            h.use_current_torch_stream()
+            assert call(h) == api.ROUTE_STREAMING
+        c.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        ch = c.cpu().numpy()
+        for i in {0, batch - 1}:
+            truth = oracle.gemm_f64(N, N, m, n, k, 1.0, a[i * m * k:], m, b[i * k * n:], k, 0.0, None, m)
+            assert oracle.residual(truth, ch[i * m * n:(i + 1) * m * n], m) < oracle.error_threshold(True, k)
+        del graph
+        assert h.kernel_status() == 0
